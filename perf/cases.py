@@ -616,28 +616,28 @@ def listed():
     qwen, shard, moe = "Qwen/Qwen3-8B", "Qwen3-32B-tp8-shard", "Qwen/Qwen3-30B-A3B"
     return [
         # one user's chat on one rank of a tensor-parallel group: every kernel is small, latency decides
-        {"name": "decode, one sequence", "of": "decoder", "model": shard, "batch": 1, "tokens": 1, "cached": 333},
+        {"name": "decode 1", "of": "decoder", "model": shard, "batch": 1, "tokens": 1, "cached": 333},
         # a server's running batch: the headline benchmark's step, on a smaller model
-        {"name": "decode, batch of 8", "of": "decoder", "model": qwen, "batch": 8, "tokens": 1, "cached": 2048},
+        {"name": "decode 8", "of": "decoder", "model": qwen, "batch": 8, "tokens": 1, "cached": 2048},
         # three prompts of a chat, no size a multiple of a tile
-        {"name": "prefill, short prompts", "of": "decoder", "model": qwen, "batch": 3, "tokens": 389, "cached": 0},
+        {"name": "prefill short", "of": "decoder", "model": qwen, "batch": 3, "tokens": 389, "cached": 0},
         # one long document
-        {"name": "prefill, long prompt", "of": "decoder", "model": qwen, "batch": 1, "tokens": 16384, "cached": 0},
+        {"name": "prefill long", "of": "decoder", "model": qwen, "batch": 1, "tokens": 16384, "cached": 0},
         # attention alone, over a pack of prompts of 1 K to 3 K tokens
-        {"name": "attention, ragged pack", "of": "prefill attention", "sequences": 5, "mean": 2047, "heads": 64, "kv_heads": 8, "dtype": "bf16",
+        {"name": "attention pack", "of": "prefill attention", "sequences": 5, "mean": 2047, "heads": 64, "kv_heads": 8, "dtype": "bf16",
          "gated": False},
         # the decode attention of long contexts, where the cache's bytes decide
-        {"name": "decode attention, 32 K", "of": "decode attention", "batch": 8, "kv": 32768, "heads": 32, "kv_heads": 8, "page": 64, "dtype": "bf16"},
+        {"name": "decode attention 32K", "of": "decode attention", "batch": 8, "kv": 32768, "heads": 32, "kv_heads": 8, "page": 64, "dtype": "bf16"},
         # latent attention of a short context: many heads share few bytes
-        {"name": "latent attention, 3 K", "of": "latent attention", "batch": 8, "kv": 3000, "heads": 32, "dtype": "bf16"},
+        {"name": "latent attention 3K", "of": "latent attention", "batch": 8, "kv": 3000, "heads": 32, "dtype": "bf16"},
         # experts in a decode step (the weights' bytes decide) and in a prompt (the products do)
-        {"name": "experts, 24 tokens", "of": "moe", "layer": moe, "tokens": 24},
-        {"name": "experts, 4 K tokens", "of": "moe", "layer": moe, "tokens": 4099},
-        {"name": "fp8 experts, 2 K tokens", "of": "fp8 experts", "layer": moe, "tokens": 2048},
+        {"name": "experts 24", "of": "moe", "layer": moe, "tokens": 24},
+        {"name": "experts 4K", "of": "moe", "layer": moe, "tokens": 4099},
+        {"name": "fp8 experts 2K", "of": "fp8 experts", "layer": moe, "tokens": 2048},
         # a recurrent mixer over prompts
-        {"name": "recurrence, 4 prompts", "of": "recurrence", "kind": "wkv", "batch": 4, "tokens": 1500, "heads": 64, "dim": 64, "dtype": "bf16"},
+        {"name": "recurrence prompts", "of": "recurrence", "kind": "wkv", "batch": 4, "tokens": 1500, "heads": 64, "dim": 64, "dtype": "bf16"},
         # a portion of a trace in 32 bits
-        {"name": "feed-forward, 32 bits", "of": "mlp 32", "model": "sizilorn-1b", "tokens": 100},
+        {"name": "feed-forward 32 bits", "of": "mlp 32", "model": "sizilorn-1b", "tokens": 100},
     ]
 
 
