@@ -55,10 +55,11 @@ def test_decode_attention_pipelines_and_fused_merge(ring, fused, B, Hq, Hkv, pag
 
 
 def _attn_ref(q, k, v, scale, causal):
-    """q [lq, Hq, D], k / v [lk, Hkv, D] -> [lq, Hq, D] in fp32 with the bottom-right aligned causal mask."""
+    """q [lq, Hq, D], k / v [lk, Hkv, D] -> [lq, Hq, D] in fp32 (64 bits for 64-bit inputs) with the bottom-right aligned causal mask."""
     lq, lk, G = q.shape[0], k.shape[0], q.shape[1] // k.shape[1]
-    kk, vv = k.float().repeat_interleave(G, dim=1), v.float().repeat_interleave(G, dim=1)
-    s = torch.einsum("qhd,khd->hqk", q.float(), kk) * scale
+    wide = torch.promote_types(q.dtype, torch.float32)
+    kk, vv = k.to(wide).repeat_interleave(G, dim=1), v.to(wide).repeat_interleave(G, dim=1)
+    s = torch.einsum("qhd,khd->hqk", q.to(wide), kk) * scale
     if causal:
         qi = torch.arange(lq, device=q.device)[:, None] + (lk - lq)
         ki = torch.arange(lk, device=q.device)[None, :]
@@ -113,3 +114,40 @@ def test_prefill_attention_reads_keys_in_place():
         qs, ks = int(cu_q[b]), b * stride
         want = _attn_ref(q[qs:qs + lq], k[ks:ks + lk], v[ks:ks + lk], scale, True)
         torch.testing.assert_close(out[qs:qs + lq].float(), want, rtol=3e-2, atol=3e-2)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("lens_q,lens_k,Hq,Hkv,causal,rising", [
+    ([1, 129, 300], [1, 129, 300], 6, 2, True, 0),      # odd group: two row blocks of a head, the last one without a partner
+    ([257, 3], [640, 131], 5, 5, True, 0),              # behind a cached prefix
+    ([128, 2, 255], [127, 0, 384], 4, 1, True, 0),      # a query without keys; the last tile ends with the last key
+    ([70, 260], [1000, 5], 8, 2, False, 0),
+    ([513], [513], 4, 2, True, 40)])                    # scores that grow with the key: every step moves the reference
+def test_prefill_attention_tiles_and_foreign_rows(dtype, lens_q, lens_k, Hq, Hkv, causal, rising):
+    """Edges of the row blocks and key tiles, both ways to pair tiles, values that start between two 16-byte boundaries, and NaN
+    in every key and value row that belongs to no sequence."""
+    from triton_distributed_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(11)
+    D, stride, B = 128, 1024, len(lens_q)
+    q = torch.randn(sum(lens_q), Hq, D, device="cuda", generator=g).to(dtype)
+    k = torch.full((B * stride, Hkv, D), float("nan"), device="cuda", dtype=dtype)
+    v = torch.full((B * stride * Hkv * D + 1,), float("nan"), device="cuda", dtype=dtype)[1:].view(B * stride, Hkv, D)
+    for b, n in enumerate(lens_k):
+        k[b * stride:b * stride + n] = torch.randn(n, Hkv, D, device="cuda", generator=g).to(dtype)
+        v[b * stride:b * stride + n] = torch.randn(n, Hkv, D, device="cuda", generator=g).to(dtype)
+        if rising:  # one channel adds up to `rising` to the scaled scores
+            q[..., 0] = D ** 0.5
+            k[b * stride:b * stride + n, :, 0] = torch.linspace(0, rising, n, device="cuda")[:, None].to(dtype)
+    cu_q = torch.tensor([0] + lens_q, device="cuda").cumsum(0).int()
+    cu_k = torch.arange(0, (B + 1) * stride, stride, dtype=torch.int32, device="cuda")
+    out = ops.prefill_attention(q, k, v, cu_q, cu_k, max(lens_q), stride, D ** -0.5, causal,
+                                seqlens_k=torch.tensor(lens_k, dtype=torch.int32, device="cuda"))
+    ops.check_pipeline_status()
+    for b, (lq, lk) in enumerate(zip(lens_q, lens_k)):
+        qs, ks = int(cu_q[b]), b * stride
+        want = _attn_ref(q[qs:qs + lq].double(), k[ks:ks + lk].double(), v[ks:ks + lk].double(), D ** -0.5, causal)
+        # weights and output are each rounded to the storage type: two half units in the last place of the largest value, and as
+        # much again for the fp32 scores (2^-24 times the sum of 128 products' magnitudes, in the exponent)
+        unit = 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
+        top = float(v[ks:ks + lk].abs().max()) if lk else 0.0
+        torch.testing.assert_close(out[qs:qs + lq].double(), want, rtol=0, atol=4 * unit * top)

@@ -140,6 +140,15 @@ __device__ __forceinline__ uint64_t umma_desc_sw128_kmajor(uint32_t smem_addr) {
   return d;
 }
 
+// MN-major operand in 128-byte-swizzled atoms of 64 (MN) x 8 (K): 8-row K groups 1024 bytes apart, the next 64 MN elements
+// `mn_stride` bytes away
+__device__ __forceinline__ uint64_t umma_desc_sw128_mnmajor(uint32_t smem_addr, uint32_t mn_stride) {
+  uint64_t d = umma_desc_sw128_kmajor(smem_addr);
+  d &= ~(static_cast<uint64_t>(0x3FFF) << 16);
+  d |= static_cast<uint64_t>(mn_stride >> 4) << 16;
+  return d;
+}
+
 // Instruction descriptor of tcgen05.mma.kind::f16 with fp32 accumulation, K-major A and B:
 //   bits [4,6) D format 1 = f32     bits [7,10) A format     bits [10,13) B format (0 = f16, 1 = bf16)
 //   bit 15 / 16 A / B major (0 = K) bits [17,23) N >> 3      bits [24,29) M >> 4
@@ -181,6 +190,17 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint6
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
       "}\n" ::"r"(tmem_d),
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// the same with A in tensor memory: 128 lanes = rows, one 32-bit column = two neighbours along K
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
@@ -286,6 +306,67 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t cluster_addr) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_addr) : "memory");
 }
 
+// the inverse of tmem_ld_32x*: thread t of the warp writes lane (base_lane + t)
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8};"
+      ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, "
+      "%23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+        "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// ------------------------------------------------------------------------------------------
+// Cluster launch control: a running CTA takes over a block of the grid that has not started, so that a kernel with one CTA
+// per SM needs neither a counter in memory nor a guess at the blocks' costs.
+// ------------------------------------------------------------------------------------------
+// Asks for a block; the 16-byte answer lands in `result` (16-byte aligned) and completes 16 bytes on `bar`. Not to be called
+// again after an answer that said there is none.
+__device__ __forceinline__ void clc_try_cancel(uint4* result, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(result)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// Whether the answer holds a block; its coordinates.
+__device__ __forceinline__ bool clc_read(const uint4* result, uint3& block) {
+  uint32_t more, x = 0, y = 0, z = 0;
+  asm volatile(
+      "{\n"
+      ".reg .pred P;\n"
+      ".reg .b128 R;\n"
+      "ld.shared.b128 R, [%4];\n"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 P, R;\n"
+      "selp.u32 %0, 1, 0, P;\n"
+      "@P clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, _}, R;\n"
+      "}\n"
+      : "=r"(more), "+r"(x), "+r"(y), "+r"(z)
+      : "r"(smem_u32(result))
+      : "memory");
+  if (more) block = make_uint3(x, y, z);
+  return more != 0;
+}
 
 }  // namespace b200

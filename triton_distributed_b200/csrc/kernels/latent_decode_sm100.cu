@@ -50,25 +50,11 @@ struct LatentDecodeParams {
   uint32_t* status;
 };
 
-// MN-major operand in 128-byte-swizzled atoms of 64 (MN) x 8 (K): 8-row K groups 1024 bytes apart, the next 64 MN elements
-// `mn_stride` bytes away
-__device__ __forceinline__ uint64_t umma_desc_sw128_mnmajor(uint32_t smem_addr, uint32_t mn_stride) {
-  uint64_t d = umma_desc_sw128_kmajor(smem_addr);
-  d &= ~(static_cast<uint64_t>(0x3FFF) << 16);
-  d |= static_cast<uint64_t>(mn_stride >> 4) << 16;
-  return d;
-}
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
-               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // barrier of the 256 softmax threads, and the same with a vote
 __device__ __forceinline__ void ld_softmax_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ bool ld_softmax_any(bool v) {

@@ -488,17 +488,15 @@ def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seql
     cu_q = cu_seqlens_q.to(device=q.device, dtype=torch.int32).contiguous()
     cu_k = cu_seqlens_k.to(device=q.device, dtype=torch.int32).contiguous()
     k_lens = seqlens_k.to(device=q.device, dtype=torch.int32).contiguous() if seqlens_k is not None else None
-    lib = _lib.load()
-    lib.b200_prefill_attention_scratch_bytes.restype = ctypes.c_longlong
-    nbytes = int(lib.b200_prefill_attention_scratch_bytes(B, Hkv, dv, int(max_seqlen_k)))
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+    if v.data_ptr() % 16:  # the kernel's tile copies start on 16-byte boundaries
+        v = v.clone()
     if out is None:
         out = torch.empty((total_q, Hq, dv), dtype=q.dtype, device=q.device)
     _lib.call("b200_prefill_attention", ptr(q), ptr(k), ptr(v), ptr(cu_q), ptr(cu_k), ptr(k_lens), B, total_q, total_k,
               int(max_seqlen_q), int(max_seqlen_k), Hq, Hkv, D, dv, c_float(scale), 1 if causal else 0, ptr(gate),
-              gate.stride(0) if gate is not None else 0, ptr(scratch), ptr(out),
+              gate.stride(0) if gate is not None else 0, ptr(out),
               dtype_code(q.dtype), ptr(_pipeline_status(q.device)), stream_ptr())
-    _count(2)
+    _count()
     return out
 
 
