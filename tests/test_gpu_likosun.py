@@ -40,6 +40,22 @@ def test_gemm_f32_is_true_fp32(M, N, K):
     assert torch.all(out[:, N:] == 7.0)
 
 
+@pytest.mark.parametrize("N,K,pad", [(64, 32, 0), (65, 31, 0), (129, 130, 0), (200, 257, 4), (2048, 1000, 0), (40000, 300, 0)])
+def test_gemm_f32_tiles_and_parts(N, K, pad):
+    """Both sides of every row-tile height, one to eight parts of K, rows on and off 16-byte boundaries; a row's result is the
+    same whatever rows share the call."""
+    from triton_distributed_b200 import ops
+    a = torch.randn(257, K + pad, device="cuda")[:, :K]
+    b = torch.randn(N, K + pad, device="cuda")[:, :K]
+    want = a.double() @ b.double().t()
+    whole = ops.gemm_f32(a, b)
+    # a sum of K products is off by at most K units in the last place (2^-24) of the sum of their magnitudes
+    bound = K * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t())
+    assert torch.all((whole.double() - want).abs() <= bound)
+    for M in (1, 8, 9, 16, 17, 32, 33, 41, 65, 97, 113, 128, 129):
+        assert torch.equal(ops.gemm_f32(a[:M], b), whole[:M]), M
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("width,center,with_bias", [(75, True, True), (1030, True, True), (2052, False, True), (1000, False, False), (2048, True, False), (5120, True, True), (9001, True, True)])
 def test_embed_norm(dtype, width, center, with_bias):
