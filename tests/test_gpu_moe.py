@@ -236,3 +236,25 @@ def test_silu_mul_fp8_matches_gate_then_block_quant(T, I):
     torch.testing.assert_close(deq, act, rtol=0.07, atol=1e-3)
     deq_ref = (q_ref.float().view(T, I // 128, 128) * s_ref[:, :, None]).view(T, I)
     assert (deq - deq_ref).abs().max() <= 0.07 * act.abs().max()
+
+
+@pytest.mark.parametrize("T,topk,N", [(1, 1, 8), (3, 8, 2048), (257, 3, 1032), (5, 9, 20), (40000, 2, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_reduce_topk_against_64_bits(T, topk, N, dtype, weighted):
+    """Widths with and without whole 16-byte vectors, odd k, more rows than one wave. Error: one rounding to 16 bits of the result and
+    topk + 1 fp32 roundings of the absolute sum. Recording autograd and views keep the torch operators' behaviour."""
+    from triton_distributed_b200.kernels.nvidia import reduce_topk
+    torch.manual_seed(15)
+    x = torch.randn(T * topk, N, device="cuda", dtype=dtype)
+    w = torch.rand(T, topk, device="cuda") if weighted else None
+    wide = x.double().view(T, topk, N) * (w.double().view(T, topk, 1) if weighted else 1.0)
+    want, bound = wide.sum(1), wide.abs().sum(1) * (topk + 1) * 2.0 ** -24
+    half_ulp = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
+    bound = bound + (want.abs() + bound) * 2 * half_ulp + 1e-7
+    assert ((reduce_topk(x, topk, w).double() - want).abs() <= bound).all()
+    leaf = x.clone().requires_grad_()
+    out = reduce_topk(leaf, topk, w)
+    assert out.requires_grad and ((out.detach().double() - want).abs() <= bound).all()
+    shifted = torch.empty(x.numel() + 1, device="cuda", dtype=dtype)[1:].view_as(x).copy_(x)  # no 16-byte alignment
+    assert ((reduce_topk(shifted, topk, w).double() - want).abs() <= bound).all()

@@ -4,6 +4,7 @@
 //                    write of k / v into the paged KV cache, all in one kernel over the fused qkv projection
 //   silu_mul         SwiGLU gate: silu(gate) * up over a fused [gate | up] projection
 //   topk_softmax     router: softmax over experts + top-k (ids, weights)
+//   reduce_topk      sum of the k expert results of every token
 //   embedding        out[t] = table[ids[t]] (token embedding lookup, 16-byte vectors)
 //
 // Role in the reference: flashinfer.norm.rmsnorm, flashinfer.apply_rope_with_cos_sin_cache_inplace and
@@ -256,6 +257,33 @@ __global__ void __launch_bounds__(256) silu_mul_fp8_kernel(const uint4* __restri
   }
 }
 
+// out[t] = sum over j < topk of x[t * topk + j] (* weights[t * topk + j]), added in fp32. Bound by reading x once: a thread owns
+// eight columns of a token, so that the k 16-byte loads are independent of one another and neighbouring threads share lines; no
+// fp32 copy of x exists. 4099 tokens x 8 x 2048 columns: 243 us as a conversion, a reduction and a conversion back,
+// 25 us here (6.0 TB/s).
+template <bool BF16>
+__global__ void __launch_bounds__(256) reduce_topk_kernel(const uint4* __restrict__ x, const float* __restrict__ weights,
+                                                          uint4* __restrict__ out, long long total, int topk, int nv) {
+  griddep_launch_dependents();
+  griddep_wait();
+  for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total; idx += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long t = idx / nv;
+    const uint4* row = x + t * topk * nv + (idx - t * nv);
+    float acc[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+#pragma unroll 8
+    for (int j = 0; j < topk; ++j) {
+      float f[8];
+      unpack8<BF16>(row[static_cast<size_t>(j) * nv], f);
+      const float w = weights != nullptr ? weights[t * topk + j] : 1.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] = weights != nullptr ? acc[e] + f[e] * w : acc[e] + f[e];
+    }
+    out[idx] = pack8<BF16>(acc);
+  }
+}
+
 // Router: one warp per token. logits [T, E] (fp32 or 16-bit), E <= 512. Writes top-k ids (int32) and
 // softmax probabilities (fp32, optionally renormalised over the k winners).
 template <typename LoadF>
@@ -469,6 +497,18 @@ B200_API int b200_silu_mul_fp8(const void* x, void* out8, float* out_scale, int 
     B200_CHECK_CUDA(launch_pdl(silu_mul_fp8_kernel<true>, grid, 256, 0, s, static_cast<const uint4*>(x), static_cast<uint2*>(out8), out_scale, T, inter, ldx));
   else
     B200_CHECK_CUDA(launch_pdl(silu_mul_fp8_kernel<false>, grid, 256, 0, s, static_cast<const uint4*>(x), static_cast<uint2*>(out8), out_scale, T, inter, ldx));
+  return kOk;
+}
+
+// x [T * topk, N] and out [T, N] contiguous, 16-byte aligned; weights fp32 [T * topk] or null.
+B200_API int b200_reduce_topk(const void* x, const float* weights, void* out, int T, int topk, int N, int dtype, void* stream) {
+  B200_REQUIRE(dtype == kBF16 || dtype == kF16, "reduce_topk reads bf16 / f16");
+  B200_REQUIRE(N % 8 == 0 && topk >= 1, "the width (%d) must be a multiple of 8, top-k (%d) positive", N, topk);
+  const long long total = static_cast<long long>(T) * (N / 8), blocks = (total + 255) / 256;
+  if (total == 0) return kOk;
+  const int grid = static_cast<int>(blocks < 64LL * sm_count() ? blocks : 64LL * sm_count());
+  B200_CHECK_CUDA(launch_pdl(dtype == kBF16 ? reduce_topk_kernel<true> : reduce_topk_kernel<false>, grid, 256, 0, static_cast<cudaStream_t>(stream),
+                             static_cast<const uint4*>(x), weights, static_cast<uint4*>(out), total, topk, N / 8));
   return kOk;
 }
 

@@ -129,7 +129,14 @@ histogram_by_expert_triton = histogram_by_expert_torch = histogram_by_expert
 def reduce_topk(x: torch.Tensor, topk: int, weights: torch.Tensor | None = None) -> torch.Tensor:
     """[T * topk, N] -> [T, N]: sum (optionally weighted) of the k copies of every token (fp32 accumulation)."""
     T = x.shape[0] // topk
-    xf = x.view(T, topk, -1).float()
+    rows = x.view(T, topk, -1)
+    # contiguous rows of whole 16-byte vectors: one pass by the native kernel; every other form by torch operators
+    if (rows.dtype in (torch.bfloat16, torch.float16) and rows.is_contiguous() and rows.shape[2] % 8 == 0 and rows.data_ptr() % 16 == 0
+            and ops.plain_tensors(rows, weights)
+            and (weights is None or (weights.dtype == torch.float32 and weights.device == rows.device and weights.is_contiguous()
+                                     and weights.numel() == T * topk))):
+        return ops.reduce_topk(rows, topk, weights)
+    xf = rows.float()
     if weights is not None:
         xf = xf * weights.view(T, topk, 1).float()
     return xf.sum(1).to(x.dtype)

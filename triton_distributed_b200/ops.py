@@ -342,6 +342,26 @@ def topk_softmax(logits: torch.Tensor, k: int, renormalize: bool = False):
     return ids, w
 
 
+def plain_tensors(*tensors: torch.Tensor | None) -> bool:
+    """Whether a native kernel may stand in for torch operators on these: tensors of the ordinary kind on the current CUDA device,
+    with nothing that records or transforms operators (autograd, forward-mode duals, vmap, dispatch modes, tracing) in effect."""
+    ts = [t for t in tensors if t is not None]
+    return (all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.device.index == torch.cuda.current_device() for t in ts)
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
+            and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
+            and torch._C._len_torch_dispatch_stack() == 0 and not torch.compiler.is_compiling() and not torch.jit.is_tracing())
+
+
+def reduce_topk(x: torch.Tensor, topk: int, weights: torch.Tensor | None = None) -> torch.Tensor:
+    """x [T, topk, N] contiguous, 16-bit -> [T, N]: sum over the k rows of a token in fp32, each times its weight (fp32 [T * topk])."""
+    _lib.require_cuda()
+    T, _, N = x.shape
+    out = torch.empty((T, N), dtype=x.dtype, device=x.device)
+    _lib.call("b200_reduce_topk", ptr(x), ptr(weights), ptr(out), T, topk, N, dtype_code(x.dtype), stream_ptr())
+    _count()
+    return out
+
+
 def top_p_sample(logits: torch.Tensor, temperature: float, top_p: float, uniform: torch.Tensor | None = None) -> torch.Tensor:
     """Nucleus sampling without a sort. logits fp32 [B, V]; returns int64 token ids [B, 1]."""
     _lib.require_cuda()
