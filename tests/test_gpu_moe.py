@@ -258,3 +258,43 @@ def test_reduce_topk_against_64_bits(T, topk, N, dtype, weighted):
     assert out.requires_grad and ((out.detach().double() - want).abs() <= bound).all()
     shifted = torch.empty(x.numel() + 1, device="cuda", dtype=dtype)[1:].view_as(x).copy_(x)  # no 16-byte alignment
     assert ((reduce_topk(shifted, topk, w).double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("T,topk,E,bm,segments,ranks", [(1, 1, 1, 128, 1, 1), (128, 8, 128, 128, 1, 1), (1025, 1, 7, 16, 1, 3), (2050, 2, 300, 1, 2, 1),
+                                                        (8192, 8, 1024, 128, 1, 8), (8192, 8, 8, 128, 128, 1), (65537, 1, 128, 128, 1, 1)])
+def test_moe_sort_all_outputs(T, topk, E, bm, segments, ranks):
+    """One to eight CTAs, the edges between them and to the four-launch form, the largest number of groups, ids that are skipped,
+    tiles with rows of several ranks: every output against a stable sort on the CPU."""
+    import numpy as np
+    from triton_distributed_b200.kernels.nvidia import create_sort_plan, moe_sort
+    rng = np.random.default_rng(16)
+    n = T * topk
+    ids = rng.integers(-1, E + 1, (T, topk)).astype(np.int32)   # -1 and E count for nothing
+    plan = create_sort_plan(n, topk, E, bm, segments, with_positions=True)
+    per_rank = (T + ranks - 1) // ranks
+    for _ in range(2):
+        moe_sort(torch.from_numpy(ids).cuda(), plan, tokens_per_rank=per_rank)
+    flat, seg = ids.reshape(-1), np.arange(n) // (n // segments)
+    keep = (flat >= 0) & (flat < E)
+    group = np.where(keep, seg * E + flat, -1)
+    count = np.bincount(group[keep], minlength=segments * E)
+    padded = -(-count // bm) * bm
+    first = np.concatenate([[0], np.cumsum(padded)])
+    order = np.argsort(group, kind="stable")[n - keep.sum():]
+    pos = first[group[order]] + np.arange(len(order)) - (np.cumsum(count) - count)[group[order]]
+    rows = np.full(first[-1], n)
+    rows[pos] = order
+    got = {k: getattr(plan, k).cpu().numpy() for k in ("sorted_ids", "tile_expert", "tile_seg_start", "tile_seg_end", "group_count", "totals", "pair_pos")}
+    tiles = first[-1] // bm
+    assert np.array_equal(got["group_count"], count) and list(got["totals"][:2]) == [first[-1], tiles]
+    assert np.array_equal(got["totals"][2:], first[E::E] // bm)
+    assert np.array_equal(got["sorted_ids"][:first[-1]], rows) and np.array_equal(got["pair_pos"][order], pos)
+    tile_group = np.repeat(np.arange(segments * E), padded // bm)
+    assert np.array_equal(got["tile_expert"][:tiles], tile_group % E)
+    source = rows.reshape(tiles, bm) // topk // per_rank
+    real = rows.reshape(tiles, bm) < n
+    low, high = np.where(real, source, 1 << 30).min(1), np.where(real, source, -1).max(1)
+    if segments > 1:
+        low = high = tile_group // E
+    assert np.array_equal(got["tile_seg_start"][:tiles], low) and np.array_equal(got["tile_seg_end"][:tiles], high)
+    assert int(plan.status[0]) == 0

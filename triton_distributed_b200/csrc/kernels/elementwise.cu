@@ -332,6 +332,8 @@ __device__ __forceinline__ void topk_softmax_warp(LoadF load, int E, int k, int*
 __global__ void topk_softmax_kernel(const void* logits, int dtype, int T, int E, int k, int* ids, float* weights,
                                     int renorm) {
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  griddep_launch_dependents();
+  griddep_wait();
   if (t >= T) return;
   if (dtype == kF32) {
     const float* p = static_cast<const float*>(logits) + static_cast<size_t>(t) * E;
@@ -518,8 +520,7 @@ B200_API int b200_topk_softmax(const void* logits, int dtype, int T, int E, int 
   B200_REQUIRE(k >= 1 && k <= E && k <= 32, "top-k (%d) must be in [1, min(E, 32)]", k);
   B200_REQUIRE(dtype == kF32 || dtype == kBF16 || dtype == kF16, "router logits must be f32/bf16/f16");
   if (T == 0) return kOk;
-  topk_softmax_kernel<<<(T + 7) / 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(logits, dtype, T, E, k, ids, weights,
-                                                                                  renorm);
-  B200_CHECK_CUDA(cudaGetLastError());
+  B200_CHECK_CUDA(launch_pdl(topk_softmax_kernel, (T + 7) / 8, 256, 0, static_cast<cudaStream_t>(stream), logits, dtype, T, E, k, ids,
+                             weights, renorm));
   return kOk;
 }

@@ -1,5 +1,6 @@
 // MoE routing metadata without a host sync, an allocation or a device-wide synchronise, so it can sit inside a
-// CUDA graph. Four short launches (no kernel waits on another CTA, so nothing has to be co-resident):
+// CUDA graph. One launch of one cluster up to 65536 pairs (moe_sort_cluster_kernel); beyond that four short launches (no kernel
+// waits on another CTA, so nothing has to be co-resident):
 //
 //   moe_sort     stable sort of the (token, k) pairs by (segment, expert), every run padded to BLOCK_M rows:
 //                  segments == 1      pairs sorted by expert over all tokens (AG + grouped GEMM, EP dispatch);
@@ -19,6 +20,7 @@
 // moe_reduce_rs.py:79-169.
 #include "b200/host.h"
 #include "b200/primitives.cuh"
+#include "b200/tcgen05.cuh"
 
 #include <cstdlib>
 #include <cstring>
@@ -171,106 +173,141 @@ __global__ void __launch_bounds__(kChunk) moe_scatter_kernel(const MoeSortParams
   }
 }
 
-// ---- small problems in ONE launch (B200DIST_MOE_SORT_SMALL=0 turns it off): at most 8192 pairs and 1024 (segment, expert)
-// groups. One CTA of 32 warps; warp w owns a contiguous block of pairs and counts them per group in its own row of a
-// shared [32][G] table (one leader lane per distinct group and 32-pair chunk, so no atomics), which also gives every
-// pair its rank among the warp's pairs of the same group. A scan over the warps per group, a scan over the groups,
-// and every pair knows its position. Same outputs as the four-kernel path.
-constexpr int kSmallMaxPerLane = 8;
+// ---- up to 65536 pairs and 1024 (segment, expert) groups in ONE launch (B200DIST_MOE_SORT_SMALL=0 turns it off): a cluster of
+// one to eight CTAs of 32 warps. Every warp owns a contiguous block of pairs and counts them per group in its own row of a shared
+// [32][G] table (one leader lane per distinct group and 32-pair chunk, so no atomics), which also gives every pair its rank among
+// the warp's pairs of the same group. A scan over the warps per group, the totals of the other CTAs through distributed shared
+// memory, a scan over the groups (every CTA for itself), and every pair knows its position. Same outputs as the four-kernel path.
+// Bound by latency: the chain of barriers and the launch. One warp per group writes the pad rows (one thread per group stored up to
+// 127 rows one after the other, most of the time of a small sort). 192 pairs, 128 experts: 11.6 us -> 8.6; 32792 pairs: 20.4 us
+// in four launches, with the gaps between them 26 us -> 14.
+constexpr int kSortPerLane = 8;     // pairs per lane
+constexpr int kSortMaxCtas = 8;
+constexpr int kSortCtaPairs = 1024 * kSortPerLane;
 
-__global__ void __launch_bounds__(1024) moe_sort_small_kernel(const MoeSortParams p) {
-  extern __shared__ int32_t wcnt[];          // [32][G] per-warp counts, then exclusive offsets over the warps
+__global__ void __launch_bounds__(1024) moe_sort_cluster_kernel(const MoeSortParams p) {
+  extern __shared__ int32_t sort_smem[];
   __shared__ int32_t warp_tot[32];
-  __shared__ int32_t carry;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int cta = blockIdx.x, ctas = gridDim.x;       // the grid is one cluster
   const int G = p.segments * p.num_experts;
+  int32_t* cta_tot = sort_smem;                       // [G] pairs of this CTA per group; read by the others
+  int32_t* s_total = cta_tot + G;                     // [G] pairs of all CTAs
+  int32_t* s_off = s_total + G;                       // [G] first sorted row
+  int32_t* s_mine = s_off + G;                        // [G] first sorted row of this CTA's pairs
+  uint16_t* wcnt = reinterpret_cast<uint16_t*>(s_mine + G);  // [32][G] per-warp counts, then exclusive offsets over the warps
+  griddep_launch_dependents();
   for (int i = tid; i < 32 * G; i += 1024) wcnt[i] = 0;
-  if (tid == 0) carry = 0;
   __syncthreads();
-  // warp w owns pairs [w * per_warp, (w + 1) * per_warp), per_warp a multiple of 32
-  const int per_warp = ((p.n_pairs + 31) / 32 + 31) / 32 * 32;
-  const int w0 = warp * per_warp;
-  int my_group[kSmallMaxPerLane], my_rank[kSmallMaxPerLane];
-  int32_t* mine = wcnt + warp * G;
+  griddep_wait();
+  // warp w of the cluster owns pairs [w * per_warp, (w + 1) * per_warp), per_warp a multiple of 32
+  const int warps = 32 * ctas;
+  const int per_warp = ((p.n_pairs + warps - 1) / warps + 31) / 32 * 32;
+  const int w0 = (cta * 32 + warp) * per_warp;
+  int my_group[kSortPerLane], my_rank[kSortPerLane];
 #pragma unroll
-  for (int k = 0; k < kSmallMaxPerLane; ++k) {
+  for (int k = 0; k < kSortPerLane; ++k) {
     my_group[k] = -1;
+    const int pair = w0 + k * 32 + lane;
+    if (k * 32 < per_warp && pair < p.n_pairs) {
+      const int e = p.ids[pair];
+      if (e >= 0 && e < p.num_experts) my_group[k] = (pair / p.pairs_per_segment) * p.num_experts + e;
+    }
+  }
+  uint16_t* mine = wcnt + warp * G;
+#pragma unroll
+  for (int k = 0; k < kSortPerLane; ++k) {
     my_rank[k] = 0;
     if (k * 32 < per_warp) {   // uniform over the warp
-      const int pair = w0 + k * 32 + lane;
-      int g = -1;
-      if (pair < p.n_pairs) {
-        const int e = p.ids[pair];
-        if (e >= 0 && e < p.num_experts) g = (pair / p.pairs_per_segment) * p.num_experts + e;
-      }
+      const int g = my_group[k];
       const uint32_t same = __match_any_sync(0xffffffffu, g);
       const int leader = __ffs(same) - 1;
       int old = 0;
       if (g >= 0 && lane == leader) {
         old = mine[g];
-        mine[g] = old + __popc(same);
+        mine[g] = static_cast<uint16_t>(old + __popc(same));
       }
       old = __shfl_sync(0xffffffffu, old, leader);
-      my_group[k] = g;
       my_rank[k] = old + __popc(same & ((1u << lane) - 1u));
       __syncwarp();
     }
   }
   __syncthreads();
-  // per group: exclusive scan of the counts over the warps, total, padded size
-  for (int g0 = 0; g0 < G; g0 += 1024) {
-    const int g = g0 + tid;
-    int total = 0;
-    if (g < G) {
-      for (int w = 0; w < 32; ++w) {
-        const int v = wcnt[w * G + g];
-        wcnt[w * G + g] = total;
+  // per group (G <= 1024: one thread each): exclusive scan of the counts over the warps, the cluster's total, its padded size
+  int before = 0, total = 0;
+  if (tid < G) {
+    int sum = 0;
+    for (int w = 0; w < 32; ++w) {
+      const int v = wcnt[w * G + tid];
+      wcnt[w * G + tid] = static_cast<uint16_t>(sum);
+      sum += v;
+    }
+    cta_tot[tid] = total = sum;
+  }
+  if (ctas > 1) {
+    __syncwarp();
+    cluster_sync_all();
+    if (tid < G) {
+      total = 0;
+      for (int r = 0; r < ctas; ++r) {
+        int v;
+        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(mapa_u32(cta_tot + tid, r)) : "memory");
+        before += r < cta ? v : 0;
         total += v;
       }
-      p.group_count[g] = total;
     }
-    const int padded = (total + p.block_m - 1) / p.block_m * p.block_m;
-    int incl = padded;
+  }
+  const int padded = (total + p.block_m - 1) / p.block_m * p.block_m;
+  int incl = padded;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    int before = carry;
-    for (int w = 0; w < warp; ++w) before += warp_tot[w];
-    const int off = before + incl - padded;
-    if (g < G) {
-      p.group_off[g] = off;
-      const int seg = g / p.num_experts, e = g - seg * p.num_experts;
-      for (int i = total; i < padded; ++i) p.sorted_ids[off + i] = p.n_pairs;
-      for (int t = 0; t < padded / p.block_m; ++t) {
-        p.tile_expert[off / p.block_m + t] = e;
-        p.tile_seg_start[off / p.block_m + t] = p.segments > 1 ? seg : 0x7fffffff;
-        p.tile_seg_end[off / p.block_m + t] = p.segments > 1 ? seg : -1;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_tot[warp] = incl;
+  __syncthreads();
+  int off = incl - padded;
+  for (int w = 0; w < warp; ++w) off += warp_tot[w];
+  if (tid < G) {
+    s_total[tid] = total;
+    s_off[tid] = off;
+    s_mine[tid] = off + before;
+    if (cta == 0) {
+      p.group_count[tid] = total;
+      if ((tid + 1) % p.num_experts == 0) p.totals[2 + tid / p.num_experts] = (off + padded) / p.block_m;   // cumulative
+      if (tid == G - 1) {
+        p.totals[0] = off + padded;
+        p.totals[1] = (off + padded) / p.block_m;
       }
-      if (e == p.num_experts - 1) p.totals[2 + seg] = (off + padded) / p.block_m;
     }
-    __syncthreads();
-    if (tid == 1023) carry = off + padded;
-    __syncthreads();
   }
-  if (tid == 0) {
-    p.totals[0] = carry;
-    p.totals[1] = carry / p.block_m;
+  __syncthreads();
+  // pad rows and tile table, one warp of the cluster per group. The source ranks of a tile's rows are known here unless the
+  // pairs come from several ranks in one segment; then their minimum and maximum follow below
+  const bool many_sources = p.segments == 1 && (p.n_pairs - 1) / p.topk >= p.tokens_per_rank;
+  for (int g = cta * 32 + warp; g < G; g += warps) {
+    const int count = s_total[g], first = s_off[g], seg = g / p.num_experts, e = g - seg * p.num_experts;
+    const int rows = (count + p.block_m - 1) / p.block_m * p.block_m;
+    for (int i = count + lane; i < rows; i += 32) p.sorted_ids[first + i] = p.n_pairs;
+    for (int t = lane; t < rows / p.block_m; t += 32) {
+      const int tile = first / p.block_m + t;
+      p.tile_expert[tile] = e;
+      p.tile_seg_start[tile] = many_sources ? 0x7fffffff : seg;
+      p.tile_seg_end[tile] = many_sources ? -1 : seg;
+    }
   }
-  __threadfence_block();
-  __syncthreads();   // group_off and the tile table (global memory, this CTA) are visible to every thread
+  __syncwarp();
+  if (ctas > 1) cluster_sync_all();   // the tile table stands before the atomics; no CTA leaves while its totals are read
+  else __syncthreads();
 #pragma unroll
-  for (int k = 0; k < kSmallMaxPerLane; ++k) {
+  for (int k = 0; k < kSortPerLane; ++k) {
     const int g = my_group[k];
     if (g >= 0) {
       const int pair = w0 + k * 32 + lane;
-      const int pos = p.group_off[g] + wcnt[warp * G + g] + my_rank[k];
+      const int pos = s_mine[g] + mine[g] + my_rank[k];
       p.sorted_ids[pos] = pair;
       if (p.pair_pos) p.pair_pos[pair] = pos;
-      if (p.segments == 1) {
+      if (many_sources) {
         const int src = (pair / p.topk) / p.tokens_per_rank;
         const int tile = pos / p.block_m;
         atomicMin(p.tile_seg_start + tile, src);
@@ -372,17 +409,34 @@ B200_API int b200_moe_sort(const int32_t* ids, int n_pairs, int topk, int num_ex
   p.chunk_cnt = scratch;
   p.group_off = scratch + static_cast<size_t>(p.chunks_per_segment) * segments * num_experts;
   const int chunks = p.chunks_per_segment * segments;
-  if (small_sort_enabled() && n_pairs <= 32 * 32 * kSmallMaxPerLane && segments * num_experts <= 1024) {
-    const size_t smem = static_cast<size_t>(32) * segments * num_experts * sizeof(int32_t);
+  const int groups = segments * num_experts;
+  if (small_sort_enabled() && n_pairs <= kSortCtaPairs * kSortMaxCtas && groups <= 1024) {
+    // one pair per lane in as few CTAs as that takes: a cluster's barriers cost about a microsecond, eight pairs in a row as much
+    int ctas = 1;
+    while (ctas < kSortMaxCtas && n_pairs > 1024 * ctas) ctas *= 2;
+    const size_t smem = static_cast<size_t>(groups) * (4 * sizeof(int32_t) + 32 * sizeof(uint16_t));
     static bool configured[64] = {false};
     int dev = 0;
     B200_CHECK_CUDA(cudaGetDevice(&dev));
     if (!configured[dev & 63]) {
-      B200_CHECK_CUDA(cudaFuncSetAttribute(moe_sort_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
+      B200_CHECK_CUDA(cudaFuncSetAttribute(moe_sort_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
       configured[dev & 63] = true;
     }
-    moe_sort_small_kernel<<<1, 1024, smem, s>>>(p);
-    B200_CHECK_CUDA(cudaGetLastError());
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(1024);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    B200_CHECK_CUDA(cudaLaunchKernelEx(&cfg, moe_sort_cluster_kernel, p));
     return kOk;
   }
   moe_count_kernel<<<chunks, kChunk, num_experts * sizeof(int32_t), s>>>(p);

@@ -209,13 +209,20 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, topk_ids: torch.Tensor, a_per
                  row_scale: torch.Tensor | None = None, plan: MoeSortPlan | None = None) -> torch.Tensor:
     """Local grouped GEMM: out[t * topk + k] = a[t (or pair)] @ w[topk_ids[t, k]].T (* row_scale). w [E, N, K]."""
     T, topk = topk_ids.shape
-    E, N, K = w.shape
     if plan is None:
-        plan = create_sort_plan(T * topk, topk, E, 128, 1, a.device)
+        plan = create_sort_plan(T * topk, topk, w.shape[0], 128, 1, a.device)
     moe_sort(topk_ids.to(torch.int32).contiguous(), plan)
-    out = torch.empty((T * topk, N), dtype=a.dtype, device=a.device)
+    return grouped_gemm_planned(a, w, plan, 1 if a_per_pair else topk, row_scale)
+
+
+def grouped_gemm_planned(a: torch.Tensor, w: torch.Tensor, plan: MoeSortPlan, a_div: int = 1,
+                         row_scale: torch.Tensor | None = None) -> torch.Tensor:
+    """``grouped_gemm`` of pairs that ``moe_sort`` has put in order: pair p reads row ``p // a_div`` of a."""
+    E, N, K = w.shape
+    n = plan.n_pairs
+    out = torch.empty((n, N), dtype=a.dtype, device=a.device)
     rs = row_scale.reshape(-1).float().contiguous() if row_scale is not None else None
-    _lib.call("b200_grouped_gemm", ptr(a), a.stride(0), 1 if a_per_pair else topk, ptr(w), E, N, K, T * topk,
+    _lib.call("b200_grouped_gemm", ptr(a), a.stride(0), a_div, ptr(w), E, N, K, n,
               ptr(plan.sorted_ids), ptr(plan.tile_expert), None, ptr(plan.totals), plan.max_tiles, ptr(out), out.stride(0),
               ptr(rs), dtype_code(a.dtype), stream_ptr())
     ops._count()

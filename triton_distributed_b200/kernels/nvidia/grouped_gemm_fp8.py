@@ -69,7 +69,7 @@ def grouped_gemm_fp8_planned(a8: torch.Tensor, a_scale: torch.Tensor, w8: torch.
     if out is None:
         out = torch.empty((n_pairs, N), dtype=out_dtype, device=a8.device)
     rs = row_scale.reshape(-1).float().contiguous() if row_scale is not None else None
-    status = torch.zeros(1, dtype=torch.int32, device=a8.device)
+    status = torch.empty(1, dtype=torch.int32, device=a8.device)
     _lib.call("b200_grouped_gemm_fp8", ptr(a8), a8.stride(0), ptr(a_scale), a_scale.stride(0), a_div, ptr(w8), ptr(w_scale),
               E, N, K, n_pairs, ptr(sorted_ids), ptr(tile_expert), ptr(totals), max_tiles, ptr(out), out.stride(0), ptr(rs),
               dtype_code(out.dtype), ptr(status), stream_ptr())

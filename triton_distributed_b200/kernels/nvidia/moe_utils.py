@@ -2,15 +2,16 @@
 
 API parity with ``python/triton_dist/kernels/nvidia/moe_utils.py`` (``calc_gather_scatter_index_triton`` :218,
 ``histogram_by_expert_*`` :32-38, ``reduce_topk_*`` :251-394) and with the CUDA op
-``moe_ag_scatter_align_block_size`` (``csrc/lib/moe_utils.cu``). Four short launches of ``csrc/kernels/moe_align.cu``
-(count, prefix, offsets, scatter) sort the (token, k) pairs by expert (optionally inside every source-rank block), pad
-every run to the tile height and emit the per-tile metadata the grouped GEMMs read; nothing synchronises with the
-host, nothing allocates, and no kernel waits on another CTA.
+``moe_ag_scatter_align_block_size`` (``csrc/lib/moe_utils.cu``). One launch of ``csrc/kernels/moe_align.cu`` (four short
+ones beyond 65536 pairs: count, prefix, offsets, scatter) sorts the (token, k) pairs by expert (optionally inside every
+source-rank block), pads every run to the tile height and emits the per-tile metadata the grouped GEMMs read; nothing
+synchronises with the host and nothing allocates.
 """
 from __future__ import annotations
 
 import ctypes
 import dataclasses
+import functools
 
 import torch
 
@@ -35,8 +36,12 @@ class MoeSortPlan:
     group_count: torch.Tensor     # int32 [segments * E]
     totals: torch.Tensor          # int32 [2 + segments]: m_pad, tiles, cumulative tiles per segment
     scratch: torch.Tensor         # int32: per-chunk expert counts / prefixes and group offsets
-    status: torch.Tensor          # int32 [16], stays zero: the sort has no device-side waits that could expire
     pair_pos: torch.Tensor | None = None  # int32 [n_pairs]: sorted position of every pair (when requested)
+
+    @functools.cached_property
+    def status(self) -> torch.Tensor:
+        """int32 [16], stays zero: the sort has no device-side waits that could expire."""
+        return torch.zeros(16, dtype=torch.int32, device=self.sorted_ids.device)
 
     @property
     def max_tiles(self) -> int:
@@ -51,12 +56,11 @@ def create_sort_plan(n_pairs: int, topk: int, num_experts: int, block_m: int = 1
     tiles = cap // block_m
     lib.b200_moe_sort_scratch_ints.restype = ctypes.c_longlong
     scratch = int(lib.b200_moe_sort_scratch_ints(n_pairs, num_experts, segments))
-    i32 = dict(dtype=torch.int32, device=device)
-    return MoeSortPlan(n_pairs, topk, num_experts, block_m, segments, cap,
-                       torch.empty(cap, **i32), torch.empty(tiles, **i32), torch.empty(tiles, **i32),
-                       torch.empty(tiles, **i32), torch.empty(tiles, **i32), torch.zeros(segments * num_experts, **i32),
-                       torch.zeros(2 + segments, **i32), torch.empty(scratch, **i32), torch.zeros(16, **i32),
-                       torch.empty(n_pairs, **i32) if with_positions else None)
+    # one allocation, cut at 16-byte boundaries; the sort writes all that is read of it
+    sizes = (cap, tiles, tiles, tiles, tiles, segments * num_experts, 2 + segments, scratch, n_pairs if with_positions else 0)
+    parts = torch.empty(sum((n + 3) // 4 * 4 for n in sizes), dtype=torch.int32, device=device).split([(n + 3) // 4 * 4 for n in sizes])
+    parts = [p if p.numel() == n else p[:n] for p, n in zip(parts, sizes)]
+    return MoeSortPlan(n_pairs, topk, num_experts, block_m, segments, cap, *parts[:8], parts[8] if with_positions else None)
 
 
 def moe_sort(topk_ids: torch.Tensor, plan: MoeSortPlan, tokens_per_rank: int | None = None) -> MoeSortPlan:
@@ -70,7 +74,7 @@ def moe_sort(topk_ids: torch.Tensor, plan: MoeSortPlan, tokens_per_rank: int | N
     _lib.call("b200_moe_sort", ptr(ids), plan.n_pairs, plan.topk, plan.num_experts, plan.block_m, plan.segments,
               tokens_per_rank, ptr(plan.sorted_ids), ptr(plan.tile_expert), ptr(plan.tile_seg_start), ptr(plan.tile_seg_end),
               ptr(plan.group_count), ptr(plan.totals), ptr(plan.scratch), ptr(plan.pair_pos), stream_ptr())
-    ops._count(4)
+    ops._count(1 if plan.n_pairs <= 65536 and plan.group_count.numel() <= 1024 else 4)
     return plan
 
 

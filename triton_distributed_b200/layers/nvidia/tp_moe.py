@@ -15,8 +15,9 @@ import torch.nn.functional as F
 
 from ... import _lib, ops
 from ..._lib import dtype_code, ptr, stream_ptr
-from ...kernels.nvidia import (ag_group_gemm, all_reduce, create_ag_group_gemm_context, create_moe_rs_context, grouped_gemm,
-                               moe_reduce_rs, reduce_topk)
+from ...kernels.nvidia import (ag_group_gemm, all_reduce, create_ag_group_gemm_context, create_moe_rs_context, create_sort_plan,
+                               moe_reduce_rs, moe_sort, reduce_topk)
+from ...kernels.nvidia.allgather_group_gemm import grouped_gemm_planned
 from .ep_a2a_layer import EPAll2AllLayer
 
 
@@ -105,9 +106,9 @@ class TP_MoE:
     def partial_fwd(self, x: torch.Tensor) -> torch.Tensor:
         """Replicated activations: this rank's partial sum [T, H] (grouped tcgen05 GEMMs, no communication)."""
         ids, w = self.route(x)
-        up = grouped_gemm(x, self.w_gate_up, ids)
-        act = ops.silu_mul(up)
-        down = grouped_gemm(act, self.w_down, ids, a_per_pair=True, row_scale=w)
+        plan = moe_sort(ids, create_sort_plan(ids.numel(), self.topk, self.num_experts, 128, 1, x.device))  # for both projections
+        act = ops.silu_mul(grouped_gemm_planned(x, self.w_gate_up, plan, self.topk))
+        down = grouped_gemm_planned(act, self.w_down, plan, 1, w)
         return reduce_topk(down, self.topk)
 
     @torch.no_grad()
