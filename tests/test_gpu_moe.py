@@ -298,3 +298,18 @@ def test_moe_sort_all_outputs(T, topk, E, bm, segments, ranks):
         low = high = tile_group // E
     assert np.array_equal(got["tile_seg_start"][:tiles], low) and np.array_equal(got["tile_seg_end"][:tiles], high)
     assert int(plan.status[0]) == 0
+
+
+@pytest.mark.parametrize("T,topk,E,N,K", [(1030, 8, 6, 1320, 128), (500, 4, 9, 1536, 640), (2, 3, 5, 520, 384), (700, 1, 1, 136, 1152)])
+def test_grouped_gemm_fp8_tile_widths(T, topk, E, N, K):
+    """Wide tiles whose second half lies behind N or holds eight columns, one and several k-blocks, more tiles than SMs, and the few
+    pairs that stay on narrow tiles. Error of the oracle's fp32 sum in another order plus one rounding to bf16."""
+    from triton_distributed_b200 import ref
+    from triton_distributed_b200.kernels.nvidia import grouped_gemm_fp8, quantize_fp8_rows, quantize_fp8_weight_blocks
+    torch.manual_seed(17)
+    a8, sa = quantize_fp8_rows(torch.randn(T, K, device="cuda") * torch.rand(T, 1, device="cuda") * 4)
+    w8, sw = quantize_fp8_weight_blocks(torch.randn(E, N, K, device="cuda") * K ** -0.5)
+    ids = torch.stack([torch.randperm(E)[:topk] if topk <= E else torch.randint(0, E, (topk,)) for _ in range(T)]).to(torch.int32).cuda()
+    out = grouped_gemm_fp8(a8, sa, w8, sw, ids)
+    want = ref.grouped_gemm_fp8_ref(a8.repeat_interleave(topk, 0), sa.repeat_interleave(topk, 0), w8, sw, ids.reshape(-1).long())
+    torch.testing.assert_close(out.float(), want, rtol=2.0 ** -8, atol=K * 2.0 ** -22)
