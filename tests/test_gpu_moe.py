@@ -313,3 +313,23 @@ def test_grouped_gemm_fp8_tile_widths(T, topk, E, N, K):
     out = grouped_gemm_fp8(a8, sa, w8, sw, ids)
     want = ref.grouped_gemm_fp8_ref(a8.repeat_interleave(topk, 0), sa.repeat_interleave(topk, 0), w8, sw, ids.reshape(-1).long())
     torch.testing.assert_close(out.float(), want, rtol=2.0 ** -8, atol=K * 2.0 ** -22)
+
+
+@pytest.mark.parametrize("T,topk,E,inter,K", [(1, 2, 4, 64, 128), (300, 4, 16, 768, 512), (1024, 8, 32, 200, 1032), (96, 2, 3, 1000, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gated_grouped_gemm(T, topk, E, inter, K, dtype):
+    """Gate, up and product in one kernel against the per-expert products in fp32: widths that are no multiple of a tile's half, few
+    pairs and many. Error: fp32 sums in another order, then one rounding to 16 bits."""
+    from triton_distributed_b200 import ref
+    from triton_distributed_b200.kernels.nvidia import create_sort_plan, moe_sort
+    from triton_distributed_b200.kernels.nvidia.allgather_group_gemm import grouped_gemm_planned
+    torch.manual_seed(18)
+    a = torch.randn(T, K, device="cuda", dtype=dtype)
+    w = torch.randn(E, 2 * inter, K, device="cuda", dtype=dtype) * K ** -0.5
+    ids = torch.stack([torch.randperm(E)[:topk] for _ in range(T)]).to(torch.int32).cuda()
+    plan = moe_sort(ids, create_sort_plan(T * topk, topk, E, 128, 1))
+    out = grouped_gemm_planned(a, w, plan, topk, gated=True)
+    gate, up = ref.grouped_gemm_ref(a.repeat_interleave(topk, 0), w, ids.reshape(-1).long()).double().chunk(2, dim=1)
+    want = gate * torch.sigmoid(gate) * up
+    # an fp32 sum of K products is off by about sqrt(K) * 2^-24 of their norm (one here); gate and up each carry that error
+    torch.testing.assert_close(out.double(), want, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10, atol=K * 2.0 ** -20)

@@ -1,7 +1,9 @@
 // Grouped (MoE) tcgen05 GEMM for sm_100a: every 128-row tile of expert-sorted (token, k) pairs is multiplied by
 // its expert's weight matrix W[e] [N, K]. Three modes share one mainloop:
 //
-//   PLAIN  out[pair, :] = A[pair / a_div, :] * W[e(pair)]^T (* row_scale[pair])
+//   PLAIN  out[pair, :] = A[pair / a_div, :] * W[e(pair)]^T (* row_scale[pair]). Gated: W[e] holds gate rows, then up rows; a
+//          tile multiplies kBN / 2 of either and its epilogue writes silu(gate) * up, so the projection itself (twice the
+//          bytes, written and read) never exists: 4099 tokens x 8, 1536 x 2048: 205 + 34 us in two kernels, 207 here
 //   AG     the token rows come from all ranks: communication warps pull the peers' token shards over NVLink
 //          into the local gather buffer while tiles whose source ranks have landed are already computed
 //          (ag_group_gemm, python/triton_dist/kernels/nvidia/allgather_group_gemm.py:398-605)
@@ -17,6 +19,7 @@
 //   warp 0 W producer | warp 1 MMA issuer | warps 2-3 communication (AG) | warps 4-7 epilogue | warps 8-11 A gather
 // Tile metadata (sorted pair ids, expert per tile, source-rank range per tile, issue order, tile count) is read
 // from device memory, so the grid is sized for the worst case and no host synchronisation is needed.
+#include "b200/elem.cuh"
 #include "b200/host.h"
 #include "b200/primitives.cuh"
 #include "b200/tcgen05.cuh"
@@ -46,6 +49,7 @@ enum GroupedMode : int { kGPlain = 0, kGAG = 1, kGRS = 2 };
 
 struct GroupedParams {
   int N, K, n_pairs, a_div, lda, ldo, tiles_n, bf16, max_tiles, bn;
+  int n_out;                  // columns of out: N, or N / 2 when gated
   const void* A;
   const int32_t* sorted_ids;
   const int32_t* tile_expert;
@@ -87,7 +91,7 @@ __device__ __forceinline__ int work_tile(const GroupedParams& p, int w, int& n_b
   return p.tile_order ? p.tile_order[slot] : slot;
 }
 
-template <int kMode, int kGN>
+template <int kMode, int kGN, bool kGated = false>
 __global__ void __launch_bounds__(kGThreads, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const GroupedParams p, const SymmCtx ctx) {
   constexpr int kGStages = GTile<kGN>::kStages, kGWBytes = GTile<kGN>::kWBytes, kGStageBytes = GTile<kGN>::kStageBytes;
@@ -105,8 +109,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const GroupedParams
   uint32_t* ready_cache = tmem_slot + 4;  // AG: [kMaxRanks] epoch of the last shard seen complete, per source rank
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int num_tiles = min(p.totals[1], p.max_tiles);
-  const int total_work = num_tiles * p.tiles_n;
   const int num_kb = (p.K + kGK - 1) / kGK;
   const uint64_t pipe_timeout = ctx.timeout_ns;
   uint32_t epoch = 1;
@@ -133,6 +135,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const GroupedParams
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  griddep_launch_dependents();
+  griddep_wait();   // PLAIN is launched before the sort and the producer of A are known to be over
+  const int num_tiles = min(p.totals[1], p.max_tiles);
+  const int total_work = num_tiles * p.tiles_n;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ W producer (TMA)
@@ -162,7 +168,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const GroupedParams
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(empty_bar + stage, phase ^ 1, abort_flag, pipe_timeout)) { ok = false; break; }
           mbar_expect_tx(full_bar + stage, kGWBytes);
-          tma_load_3d(smem + stage * kGStageBytes + kGABytes, &tmW, full_bar + stage, kb * kGK, n_blk * kGN, e);
+          uint8_t* dst = smem + stage * kGStageBytes + kGABytes;
+          if (kGated) {
+            tma_load_3d(dst, &tmW, full_bar + stage, kb * kGK, n_blk * (kGN / 2), e);
+            tma_load_3d(dst + kGWBytes / 2, &tmW, full_bar + stage, kb * kGK, p.n_out + n_blk * (kGN / 2), e);
+          } else {
+            tma_load_3d(dst, &tmW, full_bar + stage, kb * kGK, n_blk * kGN, e);
+          }
           if (++stage == kGStages) { stage = 0; phase ^= 1; }
         }
       }
@@ -266,11 +278,27 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const GroupedParams
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(w4 * 32) << 16) + acc * kGN;
 #pragma unroll 1
-      for (int c = 0; c < kGN / 64; ++c) {
+      for (int c = 0; c < (kGated ? kGN / 128 : kGN / 64); ++c) {
         uint32_t r0[32], r1[32];
-        tmem_ld_32x32(taddr + c * 64, r0);
-        tmem_ld_32x32(taddr + c * 64 + 32, r1);
-        tmem_ld_wait();
+        if (kGated) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t u[32];
+            tmem_ld_32x32(taddr + c * 64 + h * 32, h == 0 ? r0 : r1);
+            tmem_ld_32x32(taddr + kGN / 2 + c * 64 + h * 32, u);
+            tmem_ld_wait();
+            uint32_t* g = h == 0 ? r0 : r1;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) {
+              // (an IEEE division branches, and 128 of them one after the other took longer than the next tile's products)
+              g[q] = __float_as_uint(silu<__nv_bfloat16>(__uint_as_float(g[q])) * __uint_as_float(u[q]));
+            }
+          }
+        } else {
+          tmem_ld_32x32(taddr + c * 64, r0);
+          tmem_ld_32x32(taddr + c * 64 + 32, r1);
+          tmem_ld_wait();
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const uint32_t* r = j < 4 ? r0 + j * 8 : r1 + (j - 4) * 8;
@@ -291,8 +319,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const GroupedParams
           const int rr = i * 4 + (lane >> 3), ch = lane & 7;
           const uint4 v = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((ch ^ (rr & 7)) * 16));
           const int pair = __shfl_sync(0xffffffffu, my_pair, rr);
-          const int gcol = n_blk * kGN + c * 64 + ch * 8;
-          if (pair < p.n_pairs && gcol < p.N)
+          const int gcol = n_blk * (kGated ? kGN / 2 : kGN) + c * 64 + ch * 8;
+          if (pair < p.n_pairs && gcol < p.n_out)
             st_v4(static_cast<uint8_t*>(p.out) + (static_cast<size_t>(pair) * p.ldo + gcol) * 2, v);
         }
         __syncwarp();
@@ -393,24 +421,28 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const GroupedParams
   }
 }
 
-template <int kMode, int kBN>
+template <int kMode, int kBN, bool kGated = false>
 static int launch_grouped_bn(const CUtensorMap& tw, const GroupedParams& p, const SymmCtx& ctx, int grid, cudaStream_t stream) {
   static bool configured[64] = {false};
   int dev = 0;
   B200_CHECK_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    B200_CHECK_CUDA(cudaFuncSetAttribute(grouped_gemm_kernel<kMode, kBN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    B200_CHECK_CUDA(cudaFuncSetAttribute(grouped_gemm_kernel<kMode, kBN, kGated>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          GTile<kBN>::kSmem));
     configured[dev & 63] = true;
   }
   if (kMode == kGRS) {
     // this mode crosses a grid-wide barrier between the GEMM and the reduce-scatter: launched cooperatively, so the
     // driver guarantees (or refuses) the co-residency the barrier needs
-    B200_CHECK_CUDA(launch_cooperative(grouped_gemm_kernel<kMode, kBN>, dim3(grid), dim3(kGThreads), GTile<kBN>::kSmem, stream,
+    B200_CHECK_CUDA(launch_cooperative(grouped_gemm_kernel<kMode, kBN, kGated>, dim3(grid), dim3(kGThreads), GTile<kBN>::kSmem, stream,
                                        tw, p, ctx));
     return kOk;
   }
-  grouped_gemm_kernel<kMode, kBN><<<grid, kGThreads, GTile<kBN>::kSmem, stream>>>(tw, p, ctx);
+  if (kMode == kGPlain) {
+    B200_CHECK_CUDA(launch_pdl(grouped_gemm_kernel<kMode, kBN, kGated>, dim3(grid), dim3(kGThreads), GTile<kBN>::kSmem, stream, tw, p, ctx));
+    return kOk;
+  }
+  grouped_gemm_kernel<kMode, kBN, kGated><<<grid, kGThreads, GTile<kBN>::kSmem, stream>>>(tw, p, ctx);
   B200_CHECK_CUDA(cudaGetLastError());
   return kOk;
 }
@@ -420,8 +452,9 @@ static int launch_grouped(const CUtensorMap& tw, const GroupedParams& p, const S
                      : launch_grouped_bn<kMode, 128>(tw, p, ctx, grid, stream);
 }
 
-// Wide tiles when they waste no more columns than narrow ones would (N = 384 stays on 128-column tiles).
-static int pick_bn(int N) {
+// Wide tiles when they waste no more columns than narrow ones would (N = 384 stays on 128-column tiles), unless so few tiles can
+// exist (each holds at least one pair) that narrow ones spread the weights over more SMs.
+static int pick_bn(int N, int tiles) {
   static int forced = -1;
   if (forced < 0) {
     const char* e = getenv("B200DIST_GROUPED_BN");
@@ -429,23 +462,25 @@ static int pick_bn(int N) {
   }
   if (forced == 128 || forced == 256) return forced;
   const int waste256 = (N + 255) / 256 * 256 - N, waste128 = (N + 127) / 128 * 128 - N;
-  return (N >= 256 && waste256 <= waste128) ? 256 : 128;
+  return (N >= 256 && waste256 <= waste128 && static_cast<long long>(tiles) * ((N + 127) / 128) > sm_count()) ? 256 : 128;
 }
 
 static int fill_grouped(GroupedParams& p, CUtensorMap* tw, const void* W, int E, int N, int K, int n_pairs, int a_div,
                         const int32_t* sorted_ids, const int32_t* tile_expert, const int32_t* tile_order,
-                        const int32_t* totals, int max_tiles, void* out, int ldo, const float* row_scale, int dtype) {
+                        const int32_t* totals, int max_tiles, void* out, int ldo, const float* row_scale, int dtype,
+                        bool gated = false) {
   B200_REQUIRE(dtype == kBF16 || dtype == kF16, "grouped gemm supports bf16/f16");
   B200_REQUIRE(K % 8 == 0 && N % 8 == 0, "K (%d) and N (%d) must be multiples of 8", K, N);
   memset(&p, 0, sizeof(p));
   p.N = N; p.K = K; p.n_pairs = n_pairs; p.a_div = a_div; p.ldo = ldo;
-  p.bn = pick_bn(N);
-  p.tiles_n = (N + p.bn - 1) / p.bn;
+  p.bn = pick_bn(N, n_pairs < max_tiles ? n_pairs : max_tiles);
+  p.n_out = gated ? N / 2 : N;
+  p.tiles_n = gated ? (p.n_out + p.bn / 2 - 1) / (p.bn / 2) : (N + p.bn - 1) / p.bn;
   p.bf16 = dtype == kBF16;
   p.max_tiles = max_tiles;
   p.sorted_ids = sorted_ids; p.tile_expert = tile_expert; p.tile_order = tile_order; p.totals = totals;
   p.out = out; p.row_scale = row_scale;
-  return make_tma_3d(tw, W, dtype, K, N, E, K, static_cast<uint64_t>(N) * K, kGK, p.bn, 1, true);
+  return make_tma_3d(tw, W, dtype, K, N, E, K, static_cast<uint64_t>(N) * K, kGK, gated ? p.bn / 2 : p.bn, 1, true);
 }
 
 }  // namespace b200
@@ -453,15 +488,17 @@ static int fill_grouped(GroupedParams& p, CUtensorMap* tw, const void* W, int E,
 using namespace b200;
 
 // out[pair, :] = A[pair / a_div, :] * W[e]^T (* row_scale[pair]) for the pairs listed in sorted_ids (tiles of 128 rows,
-// one expert per tile, pad rows = n_pairs). W is [E, N, K]; A rows have pitch lda; out rows have pitch ldo.
+// one expert per tile, pad rows = n_pairs). W is [E, N, K]; A rows have pitch lda; out rows have pitch ldo. gated: W[e] is
+// N / 2 gate rows and N / 2 up rows, out [n_pairs, N / 2] = silu(A gate^T) * (A up^T).
 B200_API int b200_grouped_gemm(const void* A, int lda, int a_div, const void* W, int E, int N, int K, int n_pairs,
                                const int32_t* sorted_ids, const int32_t* tile_expert, const int32_t* tile_order,
                                const int32_t* totals, int max_tiles, void* out, int ldo, const float* row_scale, int dtype,
-                               void* stream) {
+                               int gated, void* stream) {
+  B200_REQUIRE(!gated || (N % 16 == 0 && row_scale == nullptr), "a gated projection needs N (%d) a multiple of 16 and no row scale", N);
   GroupedParams p;
   CUtensorMap tw;
   int rc = fill_grouped(p, &tw, W, E, N, K, n_pairs, a_div, sorted_ids, tile_expert, tile_order, totals, max_tiles, out, ldo,
-                        row_scale, dtype);
+                        row_scale, dtype, gated != 0);
   if (rc != kOk) return rc;
   p.A = A; p.lda = lda;
   SymmCtx ctx;
@@ -470,7 +507,10 @@ B200_API int b200_grouped_gemm(const void* A, int lda, int a_div, const void* W,
   ctx.timeout_ns = 4000000000ull;
   int grid = sm_count();
   if (grid > max_tiles * p.tiles_n) grid = max_tiles * p.tiles_n;
-  return launch_grouped<kGPlain>(tw, p, ctx, grid < 1 ? 1 : grid, static_cast<cudaStream_t>(stream));
+  if (grid < 1) grid = 1;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (gated) return p.bn == 256 ? launch_grouped_bn<kGPlain, 256, true>(tw, p, ctx, grid, s) : launch_grouped_bn<kGPlain, 128, true>(tw, p, ctx, grid, s);
+  return launch_grouped<kGPlain>(tw, p, ctx, grid, s);
 }
 
 // AG + grouped GEMM: a_local [Tr, K] are this rank's tokens; pairs index the gathered tokens (pair / topk = token).

@@ -216,14 +216,15 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, topk_ids: torch.Tensor, a_per
 
 
 def grouped_gemm_planned(a: torch.Tensor, w: torch.Tensor, plan: MoeSortPlan, a_div: int = 1,
-                         row_scale: torch.Tensor | None = None) -> torch.Tensor:
-    """``grouped_gemm`` of pairs that ``moe_sort`` has put in order: pair p reads row ``p // a_div`` of a."""
+                         row_scale: torch.Tensor | None = None, gated: bool = False) -> torch.Tensor:
+    """``grouped_gemm`` of pairs that ``moe_sort`` has put in order: pair p reads row ``p // a_div`` of a. gated: w holds gate
+    rows, then up rows, and the result is ``silu(a @ gate.T) * (a @ up.T)``."""
     E, N, K = w.shape
     n = plan.n_pairs
-    out = torch.empty((n, N), dtype=a.dtype, device=a.device)
+    out = torch.empty((n, N // 2 if gated else N), dtype=a.dtype, device=a.device)
     rs = row_scale.reshape(-1).float().contiguous() if row_scale is not None else None
     _lib.call("b200_grouped_gemm", ptr(a), a.stride(0), a_div, ptr(w), E, N, K, n,
               ptr(plan.sorted_ids), ptr(plan.tile_expert), None, ptr(plan.totals), plan.max_tiles, ptr(out), out.stride(0),
-              ptr(rs), dtype_code(a.dtype), stream_ptr())
+              ptr(rs), dtype_code(a.dtype), 1 if gated else 0, stream_ptr())
     ops._count()
     return out

@@ -107,7 +107,7 @@ class TP_MoE:
         """Replicated activations: this rank's partial sum [T, H] (grouped tcgen05 GEMMs, no communication)."""
         ids, w = self.route(x)
         plan = moe_sort(ids, create_sort_plan(ids.numel(), self.topk, self.num_experts, 128, 1, x.device))  # for both projections
-        act = ops.silu_mul(grouped_gemm_planned(x, self.w_gate_up, plan, self.topk))
+        act = grouped_gemm_planned(x, self.w_gate_up, plan, self.topk, gated=True)
         down = grouped_gemm_planned(act, self.w_down, plan, 1, w)
         return reduce_topk(down, self.topk)
 
@@ -179,7 +179,7 @@ class EP_MoE:
         E, N, K = w.shape
         out = torch.zeros((n_rows, N), dtype=a.dtype, device=a.device)
         _lib.call("b200_grouped_gemm", ptr(a), a.stride(0), 1, ptr(w), E, N, K, n_rows, ptr(sorted_ids), ptr(tile_expert), None,
-                  ptr(totals), self.a2a.recv_cap // 128, ptr(out), out.stride(0), None, dtype_code(a.dtype), stream_ptr())
+                  ptr(totals), self.a2a.recv_cap // 128, ptr(out), out.stride(0), None, dtype_code(a.dtype), 0, stream_ptr())
         ops._count()
         return out
 
