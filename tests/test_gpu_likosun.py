@@ -503,3 +503,25 @@ def test_trace_replay_of_another_model(tmp_path):
         got = torch.frombuffer(bytearray((tmp_path / "o" / f"{i}.f32").read_bytes()), dtype=torch.float32).view(len(rows), -1)
         assert lc.rms_error(got, want[rows]).max() < 0.03
     assert _trace(str(tmp_path / "m"), "float32", tmp_path / "o2", steps, 64).returncode == 3
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 130, 200), (100, 300, 1030), (200, 128, 64)])
+def test_gemm_f32_range_of_values(M, N, K):
+    """Magnitudes from 2^-30 to 2^30 in a row, the largest and smallest normal numbers, infinities and NaNs: sums that stay in range
+    keep the bound of an fp32 sum, and rows with infinities and NaNs give what a sum of products gives."""
+    from triton_distributed_b200 import ops
+    a = torch.randn(M, K, device="cuda") * 2.0 ** torch.randint(-30, 31, (M, K), device="cuda")
+    b = torch.randn(N, K, device="cuda") * 2.0 ** torch.randint(-30, 31, (N, K), device="cuda")
+    a[0, :5] = torch.tensor([3.4e38, -3.4e38, 1.2e-38, 0.0, -0.0])
+    b[0], b[1] = 1.0, 2.0 ** -20
+    want, total = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    bound, fits = K * 2.0 ** -24 * total + 1e-37, total < 1e38
+    assert fits[1:].all() and fits[0, 1]
+    assert torch.all(((ops.gemm_f32(a, b).double() - want).abs() <= bound)[fits])
+    a[1, K - 1], a[M - 1, 0], b[N - 1, 7] = torch.inf, torch.nan, -torch.inf
+    want, got = a.double() @ b.double().t(), ops.gemm_f32(a, b)
+    fine = want.isfinite() & fits
+    assert torch.all(((got.double() - want).abs() <= bound)[fine])
+    odd = ~want.isfinite()
+    odd[0] = False  # the first row's fp32 sums may overflow by themselves, before they meet an infinity
+    assert torch.equal(got[odd].double().nan_to_num(7.0), want[odd].nan_to_num(7.0))

@@ -1,183 +1,311 @@
-// fp32 GEMM for the models' 32-bit mode: C[M,N] = A[M,K] * B[N,K]^T, true fp32 products and sums (no TF32).
+// fp32 GEMM for the models' 32-bit mode: C[M,N] = A[M,K] * B[N,K]^T with products and sums as exact as fp32 ones (no TF32).
 //
-// A CTA of 128 threads computes a BM x BN tile over one part of K; the parts of a tile are a cluster, whose CTAs add their partial
-// tiles through distributed shared memory in rank order. The number of parts depends on N and K alone and the sum inside a part
-// runs in the order of K, so a row's result does not depend on how many other rows share the call. Any M, N, K, leading
-// dimensions and alignment.
+// On the tensor cores, with every fp32 operand cut into three bf16 values of eight significant bits each (x = x1 + x2 + x3, exactly:
+// the upper halves of x, x - x1 and x - x1 - x2). Of the nine products x1 y1, x1 y2, x2 y1, x2 y2, x1 y3 and x3 y1 are taken; the
+// three left out are below 2^-23 of x y together. The tensor core's running fp32 sum truncates, so x1 y1 is summed there over 64 k
+// only and the sums of 64 are added up in registers; the other five are 2^-8 smaller and stay in tensor memory over the whole part
+// of K. The error of a SwiGLU block of 2048 / 5632 against 64 bits is 4.2e-7 of its norm (fp32 products on the CUDA cores: 7.7e-7).
+// An infinity or a NaN has no such cut: rows that hold one are marked while they are cut, and their results are summed again, one
+// product after the other, in fp32.
 //
-// What bounds it: for many rows the fp32 pipe, fed by two shared-memory reads of 16 bytes for 32 products (a thread has 8 x 8
-// outputs) and held back by register-bank conflicts of the products; for few rows the bytes of B. Operands stay as they are in
-// memory, rows of 32 consecutive k: cp.async brings them in three or four stages, and with a pitch of 36 words eight
-// neighbouring rows are read without a bank conflict. Above 32 rows tiles are up to 64 x 128, of equal height (100 rows: two of
-// 56 instead of one of 64 and a rest); below, fewer rows would multiply padding, and 64 columns keep enough CTAs (bytes in
-// flight) at narrow N.
-// Measured against a 64 x 64 tile per CTA over all of K with 4 x 4 outputs per thread (11264 x 2048 and 2048 x 5632, us):
-//   M = 1    218, 398 -> 34, 27      M = 16   219, 397 -> 43, 32      M = 32  220, 396 -> 61, 47
-//   M = 100  241, 379 -> 171, 79     M = 256  403, 447 -> 333, 189    M = 1024  1489, 894 -> 1283, 725
-// Products of two neighbours in k at a time (fma.rn.f32x2) were no faster: 36 instead of 40 TFLOP/s at 1024 x 22016 x 4096.
+// A CTA computes 128 columns of C (rows of B, the M side of the MMA) x kT rows over one part of K; the parts of a tile are a
+// cluster, whose CTAs add their partial tiles through distributed shared memory in rank order. The number of parts depends on N
+// and K alone and the sum inside a part runs in the order of K, so a row's result does not depend on how many other rows share the
+// call. Any M, N, K, leading dimensions and alignment.
+//   warps 0-3   promotion: x1 y1 from tensor memory into registers, then the partial tile     warp 4  MMA issuer
+//   warps 8-15  operands: global memory -> registers, one step of 64 k ahead -> three planes in 128-byte-swizzled shared memory
+// What bounds it: for few rows the bytes of B; around 128 rows those bytes, the six products and the cutting (about 1000 clocks of a
+// step's 1500) are near one another; for many rows the tensor cores.
+// Measured against fp32 products on the CUDA cores with 8 x 8 outputs per thread (11264 x 2048 and 2048 x 5632, us):
+//   M = 100  183, 101 -> 62, 46
 #include "b200/host.h"
+#include "b200/packed_f32.cuh"
 #include "b200/primitives.cuh"
 #include "b200/tcgen05.cuh"
 
 namespace b200 {
 
-constexpr int kFK = 32, kFPitch = kFK + 4, kFThreads = 128, kFMaxParts = 8;
+constexpr int kXN = 128, kXK = 64, kXThreads = 512, kXMaxParts = 8;
+constexpr int kXPlaneB = kXN * kXK * 2;
 
-// Thread tiles are TM x TN, lanes 4 x 8, warps kWarpsM x (4 / kWarpsM); rows (columns) of a thread lie 4 (8) apart.
-template <int TM, int TN, int kWarpsM>
+template <int kT>
 struct F32Tile {
-  static constexpr int BM = kWarpsM * 4 * TM, BN = 4 / kWarpsM * 8 * TN;
-  static constexpr int kStages = BN == 128 ? 3 : 4;
-  static constexpr int kStage = (BM + BN) * kFPitch;  // floats
-  static constexpr int kOutPitch = BN + 8;
-  static constexpr int kSmem = 4 * (kStages * kStage > BM * kOutPitch ? kStages * kStage : BM * kOutPitch);
+  static constexpr int kPlaneA = kT * kXK * 2, kStage = 3 * (kXPlaneB + kPlaneA), kStages = 2;
+  static constexpr int kSmem = kStages * kStage + 1024 + 1024;
+  static_assert(kT % 16 == 0 && kT <= 128 && kT * kXN * 4 <= kStages * kStage, "the partial tile takes the stages' place");
 };
 
-__device__ __forceinline__ void cp_async_16(float* dst, const float* src, int bytes) {  // zeros behind `bytes`
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_4(float* dst, const float* src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
-}
+struct F32Params {
+  const float *A, *B;
+  float* C;
+  int M, N, K, parts, part, lda, ldb, ldc;
+  bool vec_a, vec_b;
+};
 
-// `rows` rows of kFK columns from (r0, k0) of X [count, kend] into shared memory: zeros behind the last column; behind the last row
-// that row again (its results are not stored). `vec`: rows start on 16 bytes.
-template <int rows>
-__device__ __forceinline__ void f32_load(float* dst, const float* __restrict__ X, int r0, int count, int k0, int kend, int ld, bool vec) {
-  constexpr int kChunks = kFK / 4;
-  const int chunk = threadIdx.x % kChunks, k = k0 + 4 * chunk;
-  const int left = min(4, max(0, kend - k));
-  const float* src = X + (left > 0 ? k : 0);
-#pragma unroll
-  for (int r = threadIdx.x / kChunks; r < rows; r += kFThreads / kChunks) {
-    const float* from = src + static_cast<size_t>(min(r0 + r, count - 1)) * ld;
-    float* to = dst + r * kFPitch + 4 * chunk;
-    if (vec) {
-      cp_async_16(to, from, 4 * left);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) cp_async_4(to + e, e < left ? from + e : from, e < left ? 4 : 0);
-    }
+// four consecutive k of a row; zeros behind k_end
+__device__ __forceinline__ float4 f32_load4(const float* row, int k, int k_end, bool vec) {
+  if (vec && k + 4 <= k_end) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(row + k));
+    return v;
   }
+  return make_float4(k < k_end ? row[k] : 0.f, k + 1 < k_end ? row[k + 1] : 0.f, k + 2 < k_end ? row[k + 2] : 0.f,
+                     k + 3 < k_end ? row[k + 3] : 0.f);
+}
+__device__ __forceinline__ uint32_t upper_halves(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
+__device__ __forceinline__ float upper_half(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+__device__ __forceinline__ void st_shared_v2(uint32_t at, uint32_t a, uint32_t b) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(a), "r"(b) : "memory");
+}
+// the three planes of four values; whether one of them is no finite number
+__device__ __forceinline__ bool f32_cut(const float4& v, uint32_t at, int plane) {
+  float x[4] = {v.x, v.y, v.z, v.w}, r[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) r[e] = x[e] - upper_half(x[e]);
+  st_shared_v2(at, upper_halves(x[0], x[1]), upper_halves(x[2], x[3]));
+  st_shared_v2(at + plane, upper_halves(r[0], r[1]), upper_halves(r[2], r[3]));
+#pragma unroll
+  for (int e = 0; e < 4; ++e) r[e] -= upper_half(r[e]);
+  st_shared_v2(at + 2 * plane, upper_halves(r[0], r[1]), upper_halves(r[2], r[3]));
+  const float any = (r[0] + r[1]) + (r[2] + r[3]);   // inf - inf and NaN - NaN are NaN
+  return any != any;
 }
 
-template <int TM, int TN, int kWarpsM>
-__global__ void __launch_bounds__(kFThreads) gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B,
-                                                             float* __restrict__ C, int M, int N, int K, int parts, int part, int lda,
-                                                             int ldb, int ldc, bool vec_a, bool vec_b) {
-  using T = F32Tile<TM, TN, kWarpsM>;
-  extern __shared__ __align__(16) float sm[];
-  const int rank = blockIdx.x % parts;  // in the cluster
-  const int n0 = blockIdx.x / parts * T::BN, m0 = blockIdx.y * T::BM;
-  const int k_begin = rank * part, k_end = min(K, k_begin + part);
+template <int kT>
+__global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params p) {
+  using T = F32Tile<kT>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T::kStages * T::kStage);
+  uint64_t *full_bar = bars, *empty_bar = bars + 2, *dfull_bar = bars + 4, *dempty_bar = bars + 6, *done_bar = bars + 8;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+  volatile uint32_t* marked = tmem_slot + 2;                               // a row of this tile holds an infinity or a NaN
+  volatile uint8_t* mark_b = reinterpret_cast<uint8_t*>(tmem_slot + 4);    // [128] which, of B and of A
+  volatile uint8_t* mark_a = mark_b + kXN;                                 // [kT]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = warp % kWarpsM * (4 * TM) + (lane >> 3), col = warp / kWarpsM * (8 * TN) + (lane & 7);
+  const int rank = blockIdx.x % p.parts;  // in the cluster
+  const int n0 = blockIdx.x / p.parts * kXN, m0 = blockIdx.y * kT;
+  const int k_begin = rank * p.part, k_end = min(p.K, k_begin + p.part);
+  const int steps = max(0, (k_end - k_begin + kXK - 1) / kXK);
+  constexpr uint64_t kTimeout = 4000000000ull;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(full_bar + i, 256);
+      mbar_init(empty_bar + i, 1);
+      mbar_init(dfull_bar + i, 1);
+      mbar_init(dempty_bar + i, 4);
+    }
+    mbar_init(done_bar, 1);
+    *abort_flag = 0;
+    *marked = 0;
+    mbar_fence_init();
+  }
+  if (threadIdx.x < kXN) mark_b[threadIdx.x] = 0;
+  if (threadIdx.x < kT) mark_a[threadIdx.x] = 0;
+  if (warp == 4) tmem_alloc(tmem_slot, 512);
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;   // columns: x1 y1 of even and odd steps at 0 and 128, the other products at 256
   griddep_launch_dependents();
   griddep_wait();
-  const int steps = (k_end - k_begin + kFK - 1) / kFK;
-  auto load = [&](int s) {
-    if (s < steps) {
-      float* st = sm + s % T::kStages * T::kStage;
-      f32_load<T::BM>(st, A, m0, M, k_begin + s * kFK, k_end, lda, vec_a);
-      f32_load<T::BN>(st + T::BM * kFPitch, B, n0, N, k_begin + s * kFK, k_end, ldb, vec_b);
+
+  if (warp < 4) {
+    // ------------------------------------------------------------------ promotion: thread = a column of C, kT rows
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");   // 128 * (216 + 40 + 128 + 128) = the launch's 512 * 128
+    f32x2 acc[kT / 2];
+#pragma unroll
+    for (int j = 0; j < kT / 2; ++j) acc[j] = 0ull;
+    const uint32_t lanes = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+    auto add = [&](uint32_t taddr) {
+      uint32_t r0[16], r1[16];
+      tmem_ld_32x16(taddr, r0);
+#pragma unroll
+      for (int h = 0; h < kT / 16; ++h) {
+        tmem_ld_wait();
+        if (h + 1 < kT / 16) tmem_ld_32x16(taddr + (h + 1) * 16, (h & 1) ? r0 : r1);
+        uint32_t* r = (h & 1) ? r1 : r0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[h * 8 + q] = add2(acc[h * 8 + q], pack2(__uint_as_float(r[2 * q]), __uint_as_float(r[2 * q + 1])));
+      }
+    };
+    bool ok = true;
+    for (int s = 0; s < steps && ok; ++s) {
+      ok = mbar_wait(dfull_bar + (s & 1), (s >> 1) & 1, abort_flag, kTimeout);
+      if (!ok) break;
+      tc_fence_after_sync();
+      add(lanes + (s & 1) * 128);
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(dempty_bar + (s & 1));
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  for (int s = 0; s < T::kStages - 1; ++s) load(s);
-  float acc[TM][TN] = {};
-  for (int s = 0; s < steps; ++s) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(T::kStages - 2) : "memory");
-    __syncthreads();  // stage s has landed for all, and stage s - 1 has been read by all
-    load(s + T::kStages - 1);
-    const float* sa = sm + s % T::kStages * T::kStage + row * kFPitch;
-    const float* sb = sm + s % T::kStages * T::kStage + (T::BM + col) * kFPitch;
+    if (steps > 0) {
+      ok = ok && mbar_wait(done_bar, 0, abort_flag, kTimeout);
+      if (ok) {
+        tc_fence_after_sync();
+        add(lanes + 256);
+        tc_fence_before_sync();
+      }
+    }
+    // all products are done: the stages give way to the partial tile [kT][128]
+    float* out = reinterpret_cast<float*>(smem);
+    const int n = threadIdx.x;
 #pragma unroll
-    for (int k = 0; k < kFK; k += 4) {
-      float4 a[TM], b[TN];
+    for (int j = 0; j < kT / 2; ++j) {
+      const float2 v = ok ? unpack2(acc[j]) : make_float2(NAN, NAN);
+      out[(2 * j) * kXN + n] = v.x;
+      out[(2 * j + 1) * kXN + n] = v.y;
+    }
+    if (ok && *marked != 0u) {
+      const float* b = p.B + static_cast<size_t>(min(n0 + n, p.N - 1)) * p.ldb;
+      for (int t = 0; t < kT; ++t) {
+        if (mark_b[n] == 0 && mark_a[t] == 0) continue;
+        const float* a = p.A + static_cast<size_t>(min(m0 + t, p.M - 1)) * p.lda;
+        float sum = 0.f;
+        for (int k = k_begin; k < k_end; ++k) sum = fmaf(a[k], b[k], sum);
+        out[t * kXN + n] = sum;
+      }
+    }
+  } else if (warp < 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == 4 && elect_one()) {
+      // ---------------------------------------------------------------- MMA issuer
+      const uint32_t idesc = umma_idesc_f16(kXN, kT, true);
+      bool ok = true;
+      for (int s = 0; s < steps; ++s) {
+        const uint32_t st = s & 1, phase = (s >> 1) & 1;
+        ok = mbar_wait(dempty_bar + st, phase ^ 1, abort_flag, kTimeout) && mbar_wait(full_bar + st, phase, abort_flag, kTimeout);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t at = smem_u32(smem + st * T::kStage);
+        const uint64_t b1 = umma_desc_sw128_kmajor(at), b2 = umma_desc_sw128_kmajor(at + kXPlaneB), b3 = umma_desc_sw128_kmajor(at + 2 * kXPlaneB);
+        const uint32_t aa = at + 3 * kXPlaneB;
+        const uint64_t a1 = umma_desc_sw128_kmajor(aa), a2 = umma_desc_sw128_kmajor(aa + T::kPlaneA), a3 = umma_desc_sw128_kmajor(aa + 2 * T::kPlaneA);
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(sa + 4 * i * kFPitch + k);
+        for (int k = 0; k < kXK / 16; ++k) umma_f16(tmem_base + st * 128, b1 + 2 * k, a1 + 2 * k, idesc, k != 0 ? 1u : 0u);
+        umma_commit(dfull_bar + st);
+#pragma unroll 1
+        for (int k = 0; k < kXK / 16; ++k) {
+          umma_f16(tmem_base + 256, b3 + 2 * k, a1 + 2 * k, idesc, (s | k) != 0 ? 1u : 0u);
+          umma_f16(tmem_base + 256, b1 + 2 * k, a3 + 2 * k, idesc, 1u);
+          umma_f16(tmem_base + 256, b2 + 2 * k, a2 + 2 * k, idesc, 1u);
+          umma_f16(tmem_base + 256, b2 + 2 * k, a1 + 2 * k, idesc, 1u);
+          umma_f16(tmem_base + 256, b1 + 2 * k, a2 + 2 * k, idesc, 1u);
+        }
+        umma_commit(empty_bar + st);
+      }
+      if (ok && steps > 0) umma_commit(done_bar);
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ operands: half a warp per row of 64 k
+    const int t = threadIdx.x - 256, c = t & 15, r0 = t >> 4;
+    const int k0 = k_begin + 4 * c;
+    const float *rb[kXN / 16], *ra[kT / 16];
+    float4 vb[kXN / 16], va[kT / 16];
 #pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(sb + 8 * j * kFPitch + k);
+    for (int i = 0; i < kXN / 16; ++i) {   // behind the last row that row again: its results are not stored
+      rb[i] = p.B + static_cast<size_t>(min(n0 + r0 + 16 * i, p.N - 1)) * p.ldb;
+      vb[i] = f32_load4(rb[i], k0, k_end, p.vec_b);
+    }
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+    for (int i = 0; i < kT / 16; ++i) {
+      ra[i] = p.A + static_cast<size_t>(min(m0 + r0 + 16 * i, p.M - 1)) * p.lda;
+      va[i] = f32_load4(ra[i], k0, k_end, p.vec_a);
+    }
+    // eight rows down the swizzle repeats: the offset inside a row is the same for all rows of this thread
+    const uint32_t off = static_cast<uint32_t>(r0 * 128 + (((c >> 1) ^ (r0 & 7)) * 16) + (c & 1) * 8);
+    for (int s = 0; s < steps; ++s) {
+      const int next = k0 + (s + 1) * kXK;
+      if (!mbar_wait(empty_bar + (s & 1), ((s >> 1) & 1) ^ 1, abort_flag, kTimeout)) break;
+      const uint32_t at = smem_u32(smem + (s & 1) * T::kStage) + off;
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+      for (int i = 0; i < kXN / 16; ++i) {
+        if (f32_cut(vb[i], at + i * 16 * 128, kXPlaneB)) {
+          mark_b[r0 + 16 * i] = 1;
+          *marked = 1;
+        }
+        vb[i] = f32_load4(rb[i], next, k_end, p.vec_b);
+      }
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+      for (int i = 0; i < kT / 16; ++i) {
+        if (f32_cut(va[i], at + 3 * kXPlaneB + i * 16 * 128, T::kPlaneA)) {
+          mark_a[r0 + 16 * i] = 1;
+          *marked = 1;
+        }
+        va[i] = f32_load4(ra[i], next, k_end, p.vec_a);
+      }
+      fence_view_async_shared();
+      mbar_arrive(full_bar + (s & 1));
     }
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();  // the stages give way to the partial tile
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) sm[(row + 4 * i) * T::kOutPitch + col + 8 * j] = acc[i][j];
+  __syncwarp();
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 4) tmem_dealloc(tmem_base, 512);
   cluster_sync_all();
-  // this CTA's share of the tile: the sum over the parts in order
-  const int share = T::BM * T::BN / 4 / parts;  // BM * BN is a multiple of 4 * kFMaxParts
-  for (int c = threadIdx.x; c < share; c += kFThreads) {
-    const int at = rank * share + c, r = at / (T::BN / 4), n = at % (T::BN / 4) * 4;
-    if (m0 + r >= M || n0 + n >= N) continue;
-    float v[4] = {};
-    for (int q = 0; q < parts; ++q) {
-      float4 x;
-      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                   : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
-                   : "r"(mapa_u32(sm + r * T::kOutPitch + n, q)));
-      v[0] += x.x, v[1] += x.y, v[2] += x.z, v[3] += x.w;
-    }
+  if (warp >= 8) {
+    // this CTA's share of the tile: the sum over the parts in order
+    const float* out = reinterpret_cast<const float*>(smem);
+    for (int i = rank * 256 + threadIdx.x - 256; i < kT * kXN / 4; i += 256 * p.parts) {
+      const int r = i / (kXN / 4), n = i % (kXN / 4) * 4;
+      if (m0 + r >= p.M || n0 + n >= p.N) continue;
+      float v[4] = {};
+      for (int q = 0; q < p.parts; ++q) {
+        float4 x;
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+                     : "r"(mapa_u32(out + r * kXN + n, q)));
+        v[0] += x.x, v[1] += x.y, v[2] += x.z, v[3] += x.w;
+      }
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (n0 + n + e < N) C[static_cast<size_t>(m0 + r) * ldc + n0 + n + e] = v[e];
+      for (int e = 0; e < 4; ++e)
+        if (n0 + n + e < p.N) p.C[static_cast<size_t>(m0 + r) * p.ldc + n0 + n + e] = v[e];
+    }
   }
+  __syncwarp();
   cluster_sync_all();  // the others have read this CTA's partial tile
 }
 
-// Parts of K: up to eight while there are fewer than about two CTAs per SM from N alone, each at least two steps of K.
+// Parts of K, from N and K alone: the fewest steps on the busiest of 148 SMs (one CTA each), where a CTA's start, its sum over the
+// parts and its end cost about as much as three steps.
 static int f32_parts(int N, int K) {
-  int parts = 1;
-  while (parts < kFMaxParts && (N + 127) / 128 * parts * 2 <= 600 && K >= parts * 2 * 2 * kFK) parts *= 2;
-  return parts;
+  const int tiles = (N + kXN - 1) / kXN, steps = (K + kXK - 1) / kXK;
+  int best = 1;
+  long long least = 1ll << 62;
+  for (int parts = 1; parts <= kXMaxParts && parts <= steps; ++parts) {
+    const long long cost = ((static_cast<long long>(tiles) * parts + 147) / 148) * ((steps + parts - 1) / parts + 3);
+    if (cost < least) least = cost, best = parts;
+  }
+  return best;
 }
 
-template <int TM, int TN, int kWarpsM>
-static int launch_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb, int ldc, cudaStream_t stream) {
-  using T = F32Tile<TM, TN, kWarpsM>;
-  const int parts = f32_parts(N, K), part = ((K + parts - 1) / parts + kFK - 1) / kFK * kFK;
+template <int kT>
+static int launch_gemm_f32(const F32Params& p, cudaStream_t stream) {
+  using T = F32Tile<kT>;
   static bool configured[64] = {false};
   int dev = 0;
   B200_CHECK_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    B200_CHECK_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<TM, TN, kWarpsM>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem));
+    B200_CHECK_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<kT>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem));
     configured[dev & 63] = true;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((N + T::BN - 1) / T::BN * parts, (M + T::BM - 1) / T::BM);
-  cfg.blockDim = dim3(kFThreads);
+  cfg.gridDim = dim3((p.N + kXN - 1) / kXN * p.parts, (p.M + kT - 1) / kT);
+  cfg.blockDim = dim3(kXThreads);
   cfg.dynamicSmemBytes = T::kSmem;
   cfg.stream = stream;
-  B200_REQUIRE(cfg.gridDim.y <= 65535, "M (%d) is too large", M);
+  B200_REQUIRE(cfg.gridDim.y <= 65535, "M (%d) is too large", p.M);
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = parts;
+  attr[0].val.clusterDim.x = p.parts;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  auto aligned = [](const float* p, int ld) { return ld % 4 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-  B200_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<TM, TN, kWarpsM>, A, B, C, M, N, K, parts, part, lda, ldb, ldc, aligned(A, lda),
-                                     aligned(B, ldb)));
+  B200_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<kT>, p));
   return kOk;
 }
 
@@ -190,12 +318,19 @@ B200_API int b200_gemm_f32(const float* A, const float* B, float* C, int M, int 
   B200_REQUIRE(M > 0 && N > 0 && K > 0, "empty problem %dx%dx%d", M, N, K);
   B200_REQUIRE(lda >= K && ldb >= K && ldc >= N, "leading dimensions are smaller than the rows");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (M <= 8) return launch_gemm_f32<2, 2, 1>(A, B, C, M, N, K, lda, ldb, ldc, s);     // 8 x 64
-  if (M <= 16) return launch_gemm_f32<4, 2, 1>(A, B, C, M, N, K, lda, ldb, ldc, s);    // 16 x 64
-  if (M <= 32) return launch_gemm_f32<4, 4, 2>(A, B, C, M, N, K, lda, ldb, ldc, s);    // 32 x 64
-  const int tiles = (M + 63) / 64, rows = (M + tiles - 1) / tiles;                     // even tiles of up to 64 rows x 128
-  if (rows <= 40) return launch_gemm_f32<5, 8, 2>(A, B, C, M, N, K, lda, ldb, ldc, s);
-  if (rows <= 48) return launch_gemm_f32<6, 8, 2>(A, B, C, M, N, K, lda, ldb, ldc, s);
-  if (rows <= 56) return launch_gemm_f32<7, 8, 2>(A, B, C, M, N, K, lda, ldb, ldc, s);
-  return launch_gemm_f32<8, 8, 2>(A, B, C, M, N, K, lda, ldb, ldc, s);
+  auto aligned = [](const float* x, int ld) { return ld % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0; };
+  F32Params p = {A, B, C, M, N, K, f32_parts(N, K), 0, lda, ldb, ldc, aligned(A, lda), aligned(B, ldb)};
+  p.part = ((K + p.parts - 1) / p.parts + kXK - 1) / kXK * kXK;
+  // row tiles of even height: 100 rows are one of 112, 150 two of 80
+  const int tiles = (M + 127) / 128, rows = (M + tiles - 1) / tiles;
+  switch ((rows + 15) / 16) {
+    case 1: return launch_gemm_f32<16>(p, s);
+    case 2: return launch_gemm_f32<32>(p, s);
+    case 3: return launch_gemm_f32<48>(p, s);
+    case 4: return launch_gemm_f32<64>(p, s);
+    case 5: return launch_gemm_f32<80>(p, s);
+    case 6: return launch_gemm_f32<96>(p, s);
+    case 7: return launch_gemm_f32<112>(p, s);
+    default: return launch_gemm_f32<128>(p, s);
+  }
 }
