@@ -300,3 +300,23 @@ def test_embedding_with_norm_outputs():
     assert torch.equal(out, table[ids.reshape(-1)])
     torch.testing.assert_close(xg.float(), out.float() * gain.float(), rtol=1e-2, atol=1e-2)
     torch.testing.assert_close(ss[:4], out.float().pow(2).sum(-1), rtol=1e-4, atol=1e-3)
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 8, 64), (1167, 4096, 72), (1167, 6144, 64), (129, 25000, 136), (260, 16392, 64), (520, 7560, 328), (2000, 2056, 64)])
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gemm_tile_widths(M, N, K, gated, dtype):
+    """Sizes for which the pairs' tiles are 128 to 256 columns wide, none of them a multiple of the tile, into rows with a pitch, and
+    the gated form. An fp32 sum of K products of norm one is off by less than K * 2^-20, then one rounding to 16 bits."""
+    from triton_distributed_b200 import ops
+    torch.manual_seed(19)
+    a = torch.randn(M, K, device="cuda", dtype=dtype)
+    b = torch.randn(2 * N if gated else N, K, device="cuda", dtype=dtype) * K ** -0.5
+    out = torch.full((M, N + 8), 7.0, device="cuda", dtype=dtype)
+    (ops.gemm_gated if gated else ops.gemm)(a, b, out[:, :N])
+    want = a.double() @ b.double().t()
+    if gated:
+        gate, up = want.chunk(2, dim=1)
+        want = gate * torch.sigmoid(gate) * up
+    assert (out[:, N:] == 7).all()
+    torch.testing.assert_close(out[:, :N].double(), want, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10, atol=K * 2.0 ** -20)

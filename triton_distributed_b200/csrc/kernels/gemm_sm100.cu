@@ -25,8 +25,15 @@
 //   RS mode ends with a reduce phase in which all threads sum the `world` slots of this rank's
 //   rows (fp32) as the blocks complete.
 //
+// PLAIN pairs take tiles of 256 rows x kW columns, kW from 128 to 256: with one pair on every two SMs the last wave of wide
+// tiles can be nearly empty, and the host picks the width whose waves cost least (1167 x 4096 over 12288: 80 tiles of 256
+// columns are two waves on 74 pairs, 128 us; 130 tiles of 160 are two waves of 0.63 of the work, 98 us). Gated: B holds
+// gate rows, then up rows; one CTA of a pair loads kW / 2 gate rows, the other as many up rows, the accumulator holds both
+// side by side, and the epilogue writes silu(gate) * up (1167 x 24576 over 4096: 153 + 20 us in two kernels, 151 here).
+//
 // All cross-rank and cross-CTA waits are bounded; on expiry the kernel records a status, unwinds
 // every role through a CTA-wide abort flag, frees its TMEM and returns.
+#include "b200/elem.cuh"
 #include "b200/host.h"
 #include "b200/primitives.cuh"
 #include "b200/tcgen05.cuh"
@@ -138,13 +145,16 @@ __device__ __forceinline__ void comm_copy(uint8_t* dst, const uint8_t* src, size
   for (; i < nvec; i += kCommThreads) st_v4(d + i, ld_v4_relaxed_sys(s + i));
 }
 
-template <int kMode, int kCtas>
+template <int kMode, int kCtas, int kW = kBN, bool kGated = false>
 __global__ void __launch_bounds__(256, 1)
 gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                   const __grid_constant__ CUtensorMap tmB, const GemmParams p, const SymmCtx ctx) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr bool kPair = kCtas == 2;
+  static_assert(kW == kBN || (kPair && kMode == kPlain), "other tile widths: pairs without communication");
+  static_assert(kW % 32 == 0 && (!kGated || kPair), "the N of a pair's MMA is a multiple of 32");
+  constexpr int kOutW = kGated ? kW / 2 : kW;  // columns of C per tile
   constexpr int kNS = kPair ? kPairStages : kStages;              // pipeline depth
   constexpr int kSB = kPair ? kPairStageBytes : kStageBytes;      // bytes per stage in this CTA
   uint8_t* epi_smem = smem + kStages * kStageBytes;
@@ -196,6 +206,10 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constan
   if (kPair) cluster_sync_all();  // the peer's barriers exist before anything signals them
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  if (kMode == kPlain) {  // launched before the kernels in front of it are known to be over
+    griddep_launch_dependents();
+    griddep_wait();
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -223,9 +237,10 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constan
           uint8_t* sa = smem + stage * kSB;
           if (kPair) {
             // both CTAs' loads credit the leader's barrier; the leader announces the bytes of the whole pair
-            if (leader) mbar_expect_tx(full_bar + stage, 2 * kSB);
+            if (leader) mbar_expect_tx(full_bar + stage, 2 * (kABytes + kW / 2 * kBK * 2));
             tma_load_2d_pair(sa, tmA, full_bar + stage, kb * kBK, m_blk * kBM);
-            tma_load_2d_pair(sa + kABytes, &tmB, full_bar + stage, kb * kBK, n_blk * kBN + static_cast<int>(cta_rank) * 128);
+            const int b_row = kGated ? static_cast<int>(cta_rank) * p.N + n_blk * (kW / 2) : n_blk * kW + static_cast<int>(cta_rank) * (kW / 2);
+            tma_load_2d_pair(sa + kABytes, &tmB, full_bar + stage, kb * kBK, b_row);
           } else {
             mbar_expect_tx(full_bar + stage, kSB);
             tma_load_2d(sa, tmA, full_bar + stage, kb * kBK, m_blk * kBM);
@@ -239,7 +254,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constan
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (leader && elect_one()) {
-      const uint32_t idesc = umma_idesc_f16(kBM * kCtas, kBN, p.bf16 != 0);
+      const uint32_t idesc = umma_idesc_f16(kBM * kCtas, kW, p.bf16 != 0);
       uint32_t stage = 0, phase = 0, it = 0;
       bool ok = true;
       for (int t = unit; t < total_tiles && ok; t += num_units, ++it) {
@@ -412,11 +427,24 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constan
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(w * 32) << 16) + acc * kBN;
       const int row_base = m_blk * kBM + w * 32;
 #pragma unroll 1
-      for (int c = 0; c < kBN / 64; ++c) {
+      for (int c = 0; c < (kOutW + 63) / 64; ++c) {  // columns of the last part behind kOutW are read and not stored
         uint32_t r0[32], r1[32];
-        tmem_ld_32x32(taddr + c * 64, r0);
-        tmem_ld_32x32(taddr + c * 64 + 32, r1);
-        tmem_ld_wait();
+        if (kGated) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t u[32];
+            tmem_ld_32x32(taddr + c * 64 + h * 32, h == 0 ? r0 : r1);
+            tmem_ld_32x32(taddr + kW / 2 + c * 64 + h * 32, u);
+            tmem_ld_wait();
+            uint32_t* g = h == 0 ? r0 : r1;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) g[q] = __float_as_uint(silu<__nv_bfloat16>(__uint_as_float(g[q])) * __uint_as_float(u[q]));
+          }
+        } else {
+          tmem_ld_32x32(taddr + c * 64, r0);
+          tmem_ld_32x32(taddr + c * 64 + 32, r1);
+          tmem_ld_wait();
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const uint32_t* r = j < 4 ? r0 + j * 8 : r1 + (j - 4) * 8;
@@ -441,8 +469,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constan
           const int ch = lane & 7;
           const uint4 v = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((ch ^ (rr & 7)) * 16));
           const int grow = row_base + rr;
-          const int gcol = n_blk * kBN + c * 64 + ch * 8;
-          if (grow < p.M && gcol < p.N) {
+          const int gcol = n_blk * kOutW + c * 64 + ch * 8;
+          if (grow < p.M && gcol < p.N && (kOutW % 64 == 0 || c * 64 + ch * 8 < kOutW)) {
             if (kMode == kRS) {
               const int owner = grow / p.Mr;
               const int lrow = grow - owner * p.Mr;
@@ -612,14 +640,14 @@ static bool two_cta_enabled() {
   return g_two_cta == 1;
 }
 
-template <int kMode, int kCtas>
+template <int kMode, int kCtas, int kW = kBN, bool kGated = false>
 static int launch_gemm_impl(const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& b, const GemmParams& p,
                             const SymmCtx& ctx, int grid, cudaStream_t stream) {
   static bool configured[64] = {false};
   int dev = 0;
   B200_CHECK_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    B200_CHECK_CUDA(cudaFuncSetAttribute(gemm_sm100_kernel<kMode, kCtas>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
+    B200_CHECK_CUDA(cudaFuncSetAttribute(gemm_sm100_kernel<kMode, kCtas, kW, kGated>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
     configured[dev & 63] = true;
   }
   cudaLaunchConfig_t cfg;
@@ -628,14 +656,16 @@ static int launch_gemm_impl(const CUtensorMap& a0, const CUtensorMap& a1, const 
   cfg.blockDim = dim3(256);
   cfg.dynamicSmemBytes = kGemmSmem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = kCtas;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = kCtas > 1 ? 1 : 0;
-  B200_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_sm100_kernel<kMode, kCtas>, a0, a1, b, p, ctx));
+  cfg.numAttrs = kMode == kPlain && pdl_enabled() ? 2 : 1;
+  B200_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_sm100_kernel<kMode, kCtas, kW, kGated>, a0, a1, b, p, ctx));
   return kOk;
 }
 
@@ -674,9 +704,23 @@ static int fill_common(GemmParams& p, int M, int N, int K, int dtype, int group_
 
 using namespace b200;
 
-// C[M,N] = A[M,K] * B[N,K]^T, all row-major with leading dimensions lda/ldb/ldc (elements).
+// Width of a pair's tiles: a wave of tiles takes about as long as their width and a fixed part (the first loads and the last
+// store, worth about 24 columns); the narrower ones read A more often, so a tie goes to the wider.
+static int pick_width(int tiles_m, int cols, int step, int units) {
+  int best = 256;
+  long long least = 1ll << 62;
+  for (int w = 256; w >= 128; w -= step) {
+    const long long tiles = static_cast<long long>(tiles_m) * ((cols + w - 1) / w);
+    const long long cost = (tiles + units - 1) / units * (w + 24);
+    if (cost < least) least = cost, best = w;
+  }
+  return best;
+}
+
+// C[M,N] = A[M,K] * B[N,K]^T, all row-major with leading dimensions lda/ldb/ldc (elements). gated: B [2 * N, K] holds gate rows,
+// then up rows, and C = silu(A gate^T) * (A up^T); more than 128 rows.
 B200_API int b200_gemm(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int dtype,
-                       int max_ctas, void* stream) {
+                       int max_ctas, int gated, void* stream) {
   GemmParams p;
   memset(&p, 0, sizeof(p));
   int rc = fill_common(p, M, N, K, dtype, 16);
@@ -686,9 +730,17 @@ B200_API int b200_gemm(const void* A, const void* B, void* C, int M, int N, int 
   CUtensorMap ta, tb;
   rc = make_tma_2d(&ta, A, dtype, M, K, lda, kBM, kBK, true);
   if (rc != kOk) return rc;
-  const bool pair = use_pair(M);
+  const bool pair = use_pair(M) || gated;
+  B200_REQUIRE(!gated || M > kBM, "a gated product needs more than %d rows, got %d", kBM, M);
   set_tiles(p, pair, 0);
-  rc = make_tma_2d(&tb, B, dtype, N, K, ldb, pair ? 128 : kBN, kBK, true);
+  int width = kBN;
+  if (pair) {
+    int units = sm_count() / 2;
+    if (max_ctas > 1) units = min(units, max_ctas / 2);
+    width = gated ? pick_width(p.tiles_m, 2 * N, 64, units) : pick_width(p.tiles_m, N, 32, units);
+    p.tiles_n = gated ? (2 * N + width - 1) / width : (N + width - 1) / width;
+  }
+  rc = make_tma_2d(&tb, B, dtype, gated ? 2 * N : N, K, ldb, pair ? width / 2 : kBN, kBK, true);
   if (rc != kOk) return rc;
   SymmCtx ctx;
   memset(&ctx, 0, sizeof(ctx));
@@ -697,7 +749,21 @@ B200_API int b200_gemm(const void* A, const void* B, void* C, int M, int N, int 
   int grid = min(p.tiles_m * p.tiles_n * (pair ? 2 : 1), sm_count());
   if (max_ctas > 0) grid = min(grid, max_ctas);
   if (pair && grid < 2) grid = 2;
-  return launch_gemm<kPlain>(pair, ta, ta, tb, p, ctx, grid, static_cast<cudaStream_t>(stream));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (!pair) return launch_gemm_impl<kPlain, 1>(ta, ta, tb, p, ctx, grid, st);
+  grid &= ~1;
+  if (gated) {
+    if (width == 128) return launch_gemm_impl<kPlain, 2, 128, true>(ta, ta, tb, p, ctx, grid, st);
+    if (width == 192) return launch_gemm_impl<kPlain, 2, 192, true>(ta, ta, tb, p, ctx, grid, st);
+    return launch_gemm_impl<kPlain, 2, 256, true>(ta, ta, tb, p, ctx, grid, st);
+  }
+  switch (width) {
+    case 128: return launch_gemm_impl<kPlain, 2, 128>(ta, ta, tb, p, ctx, grid, st);
+    case 160: return launch_gemm_impl<kPlain, 2, 160>(ta, ta, tb, p, ctx, grid, st);
+    case 192: return launch_gemm_impl<kPlain, 2, 192>(ta, ta, tb, p, ctx, grid, st);
+    case 224: return launch_gemm_impl<kPlain, 2, 224>(ta, ta, tb, p, ctx, grid, st);
+    default: return launch_gemm_impl<kPlain, 2>(ta, ta, tb, p, ctx, grid, st);
+  }
 }
 
 // AG-GEMM. a_local [Mr, K] is this rank's shard; ag_buf0/1 are the two symmetric gather buffers

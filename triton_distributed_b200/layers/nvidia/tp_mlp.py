@@ -92,8 +92,7 @@ class TP_MLP:
         if T <= 128:
             act = ops.gemm_skinny(x, self.gate_up_proj, swiglu=True)
             return ops.gemm_skinny(act, self.down_proj)
-        act = ops.silu_mul(ops.gemm(x, self.gate_up_proj))
-        return ops.linear(act, self.down_proj)
+        return ops.linear(ops.gemm_gated(x, self.gate_up_proj), self.down_proj)
 
     @torch.no_grad()
     def dist_triton_AR_fwd(self, x: torch.Tensor) -> torch.Tensor:

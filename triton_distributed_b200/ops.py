@@ -35,17 +35,27 @@ def _check_2d(t: torch.Tensor, name: str) -> None:
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, max_ctas: int = 0) -> torch.Tensor:
-    """``a[M,K] @ b[N,K].T`` on the persistent tcgen05 kernel (128x256x64 tiles, fp32 accumulation)."""
+    """``a[M,K] @ b[N,K].T`` on the persistent tcgen05 kernel (fp32 accumulation)."""
+    return _gemm(a, b, b.shape[0], out, max_ctas, False)
+
+
+def gemm_gated(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    """``silu(a @ gate.T) * (a @ up.T)`` for b = [gate rows | up rows] and more than 128 rows of a, in one kernel."""
+    if b.shape[0] % 2:
+        raise ValueError("gemm_gated: b holds as many up rows as gate rows")
+    return _gemm(a, b, b.shape[0] // 2, out, 0, True)
+
+
+def _gemm(a, b, N, out, max_ctas, gated):
     _lib.require_cuda()
     _check_2d(a, "a"), _check_2d(b, "b")
     M, K = a.shape
-    N = b.shape[0]
     if b.shape[1] != K or a.dtype != b.dtype:
         raise ValueError("gemm: shape/dtype mismatch")
     if out is None:
         out = torch.empty((M, N), dtype=a.dtype, device=a.device)
     _lib.call("b200_gemm", ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-              dtype_code(a.dtype), max_ctas, stream_ptr())
+              dtype_code(a.dtype), max_ctas, 1 if gated else 0, stream_ptr())
     _count()
     return out
 
