@@ -154,3 +154,22 @@ def test_latent_split_choice():
                 assert 1 <= splits <= 64 and splits <= (kv + 63) // 64 and per_cta in (16, 32, 64)
                 assert per_cta == 16 or rows > per_cta // 2
     assert choose_latent_splits(8, 64, 16384) == (18, 64) and choose_latent_splits(1, 16, 2048) == (32, 16)
+
+
+def test_latent_split_choice_is_the_least_of_all_splits():
+    """The choice visits one number of splits per number of tiles: the same as trying every number."""
+    import random
+    from triton_distributed_b200 import ops
+    rng = random.Random(3)
+    for _ in range(400):
+        batch, rows, kv, sms = rng.randint(1, 64), rng.choice((1, 9, 16, 17, 33, 64, 200)), int(2 ** rng.uniform(0, 16)), rng.choice((148, 20))
+        n, best = max(1, (kv + 63) // 64), (float("inf"), 1, 16)
+        for per_cta, us in ((16, 1.2), (32, 1.25), (64, 1.4)):
+            if per_cta > 16 and rows <= per_cta // 2:
+                continue
+            for splits in range(1, min(64, n) + 1):
+                tiles = -(-n // splits)
+                cost = -(-batch * -(-rows // per_cta) * splits // sms) * tiles * us + 7e-4 * batch * rows * splits
+                if cost < best[0]:
+                    best = (cost, -(-n // tiles), per_cta)
+        assert ops.choose_latent_splits(batch, rows, kv, sms) == best[1:]

@@ -114,13 +114,21 @@ def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
 
 
 def stream_ptr(stream: torch.cuda.Stream | None = None) -> ctypes.c_void_p:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))  # no Stream object per launch
+
+
+_have_cuda = False  # asked of the driver until there is one
 
 
 def require_cuda() -> None:
     """Ops call this first: on a GPU machine the native path is the only path."""
-    if not torch.cuda.is_available():
+    global _have_cuda
+    if _have_cuda:
+        return
+    _have_cuda = torch.cuda.is_available()
+    if not _have_cuda:
         raise RuntimeError("this op needs a CUDA device (sm_100a); use triton_distributed_b200.ref on CPU")
 
 

@@ -811,17 +811,23 @@ def choose_latent_splits(batch: int, rows: int, max_kv_len: int, sm_count: int =
     """(splits, query rows per CTA) of the absorbed latent attention, for `rows` query rows of each of `batch` sequences: the
     least estimated time, from what a 64-key tile takes by rows per CTA (measured; a CTA has an SM to itself) and what writing
     and merging the partial results of one more split costs."""
-    n_tiles = max(1, (max_kv_len + 63) // 64)
+    return _latent_splits(batch, rows, max(1, (max_kv_len + 63) // 64), sm_count)
+
+
+@functools.lru_cache(maxsize=1024)  # by sizes alone: a decode step asks for the same every 64 tokens, in every layer
+def _latent_splits(batch: int, rows: int, n_tiles: int, sm_count: int) -> tuple[int, int]:
     best = (float("inf"), 1, 16)
     for per_cta, tile_us in ((16, 1.2), (32, 1.25), (64, 1.4)):
         if per_cta > 16 and rows <= per_cta // 2:
             continue
         ctas = batch * ((rows + per_cta - 1) // per_cta)
-        for splits in range(1, min(64, n_tiles) + 1):
+        splits = 1
+        while splits <= min(64, n_tiles):  # of all splits with the same tiles per CTA, the fewest
             tiles = -(-n_tiles // splits)
             cost = -(-ctas * splits // sm_count) * tiles * tile_us + 7e-4 * batch * rows * splits
             if cost < best[0]:
                 best = (cost, -(-n_tiles // tiles), per_cta)
+            splits = -(-n_tiles // (tiles - 1)) if tiles > 1 else n_tiles + 1
     return best[1], best[2]
 
 
@@ -850,13 +856,10 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, kv_lens: torch.Tensor
         _lib.call("b200_latent_attention_plain", ptr(q), ptr(cache), *shape, ptr(sink), ptr(out), dtype_code(q.dtype), stream_ptr())
         _count()
         return out
-    o_part = torch.empty((T * H, num_splits, P), dtype=torch.float32, device=q.device)
-    lse_part = torch.empty((T * H, num_splits), dtype=torch.float32, device=q.device)
+    part = torch.empty(T * H * num_splits * (P + 1), dtype=torch.float32, device=q.device)  # [T * H, splits, P] and its log-sum-exps
     per_cta = rows_per_cta or (16 if tokens * H <= 16 else 32 if tokens * H <= 32 else 64)
-    _lib.call("b200_latent_decode", ptr(q), ptr(cache), ctypes.c_longlong(cache.shape[0] * page), *shape, num_splits, per_cta,
-              ptr(o_part), ptr(lse_part), dtype_code(q.dtype), ptr(_pipeline_status(q.device)), stream_ptr())
-    _lib.call("b200_latent_combine", ptr(o_part), ptr(lse_part), ptr(sink), T * H, H, num_splits, P, ptr(out), dtype_code(q.dtype),
-              stream_ptr())
+    _lib.call("b200_latent_attention", ptr(q), ptr(cache), ctypes.c_longlong(cache.shape[0] * page), *shape, num_splits, per_cta,
+              ptr(part), ptr(sink), ptr(out), dtype_code(q.dtype), ptr(_pipeline_status(q.device)), stream_ptr())
     _count(2)
     return out
 
