@@ -178,6 +178,21 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kernel(const uint2* __restri
   }
 }
 
+// What the layers of a step read of its token positions: positions in 32 bits, cache slots, lengths. One launch instead of the
+// seven element-wise ones of a captured decode step (about 1.4 us each, in front of everything else).
+__global__ void __launch_bounds__(256) step_tables_kernel(const int64_t* __restrict__ ids, int B, int S, int64_t per_seq,
+                                                          int* __restrict__ pos, int64_t* __restrict__ slots, int* __restrict__ kv_lens) {
+  griddep_launch_dependents();
+  griddep_wait();
+  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  if (i >= static_cast<long long>(B) * S) return;
+  const int b = static_cast<int>(i / S);
+  const int64_t at = ids[i];
+  pos[i] = static_cast<int>(at);
+  slots[i] = b * per_seq + at;
+  if (i - static_cast<long long>(b) * S == S - 1) kv_lens[b] = static_cast<int>(at + 1);
+}
+
 // out[t, i] = silu(x[t, i]) * x[t, inter + i]; x is [T, 2 * inter] with row pitch ldx.
 template <bool BF16>
 __global__ void __launch_bounds__(256) silu_mul_kernel(const uint4* __restrict__ x, uint4* __restrict__ out, int T,
@@ -464,6 +479,15 @@ B200_API int b200_qk_norm_rope(const void* qkv, const int* positions, const int6
                                static_cast<uint2*>(q_out), static_cast<uint2*>(k_cache), static_cast<uint2*>(v_cache), T, Hq,
                                Hkv, eps));
   B200_CHECK_CUDA(cudaGetLastError());
+  return kOk;
+}
+
+// ids int64 [B, S] -> pos int32 [B * S], slots int64 [B * S] (b * per_seq + position), kv_lens int32 [B] (last position + 1)
+B200_API int b200_step_tables(const int64_t* ids, int B, int S, long long per_seq, int* pos, int64_t* slots, int* kv_lens, void* stream) {
+  const long long total = static_cast<long long>(B) * S;
+  if (total <= 0) return kOk;
+  B200_CHECK_CUDA(launch_pdl(step_tables_kernel, static_cast<unsigned>((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), ids, B, S,
+                             per_seq, pos, slots, kv_lens));
   return kOk;
 }
 

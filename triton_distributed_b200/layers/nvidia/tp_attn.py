@@ -105,8 +105,7 @@ class TP_Attn:
         `step` carries per-step tensors precomputed by the model (positions int32, slots, kv_lens)."""
         kp, vp = kv_cache.layer(layer_idx)
         if step is None:
-            pos = position_ids.reshape(-1).to(torch.int32)
-            step = {"pos": pos, "slots": kv_cache.slots(position_ids), "kv_lens": (position_ids[:, -1] + 1).to(torch.int32)}
+            step = ops.step_tables(position_ids, kv_cache.blocks_per_seq * kv_cache.page_size)
         q = ops.qk_norm_rope(qkv, step["pos"], cos_sin_cache, self.q_heads_local, self.kv_heads_local,
                              kp.view(-1, self.kv_heads_local, self.head_dim), vp.view(-1, self.kv_heads_local, self.head_dim),
                              step["slots"], self.q_norm_w, self.k_norm_w, self.eps)
@@ -121,8 +120,9 @@ class TP_Attn:
         if self.head_dim != 128:
             raise NotImplementedError("the native prefill attention is specialised for head_dim 128")
         L = kv_cache.blocks_per_seq * kv_cache.page_size
-        cu_q = torch.arange(0, (bsz + 1) * seqlen, seqlen, dtype=torch.int32, device=qkv.device)
-        cu_k = torch.arange(0, (bsz + 1) * L, L, dtype=torch.int32, device=qkv.device)
+        if "bounds" not in step:  # the same for every layer of a step
+            step["bounds"] = [torch.arange(0, (bsz + 1) * n, n, dtype=torch.int32, device=qkv.device) for n in (seqlen, L)]
+        cu_q, cu_k = step["bounds"]
         o = ops.prefill_attention(q, kp.view(-1, self.kv_heads_local, self.head_dim), vp.view(-1, self.kv_heads_local, self.head_dim),
                                   cu_q, cu_k, seqlen, min(L, step.get("kv_len") or kv_cache.max_length), self.scale, True, seqlens_k=step["kv_lens"])
         return o.reshape(bsz * seqlen, -1)

@@ -55,7 +55,7 @@ class Engine:
         m.set_fwd(backend)
 
     def _decode_step(self) -> None:
-        self._static_pos.copy_(self.kv_cache.kv_offset.to(torch.int64)[:, None])
+        self._static_pos.copy_(self.kv_cache.kv_offset[:, None])
         self._static_logits = self.model.inference(self._static_ids, self._static_pos, self.kv_cache)
 
     def _init_cuda_graph(self) -> None:

@@ -239,8 +239,7 @@ class Qwen3:
     def _inference_AR(self, input_ids, position_ids, kv_cache, kv_len=None):
         """Returns the final-normed hidden states [B, S, H]."""
         bsz, seqlen = input_ids.shape
-        step = {"pos": position_ids.reshape(-1).to(torch.int32), "slots": kv_cache.slots(position_ids), "kv_len": kv_len,
-                "kv_lens": (position_ids[:, -1] + 1).to(torch.int32)}
+        step = ops.step_tables(position_ids, kv_cache.blocks_per_seq * kv_cache.page_size) | {"kv_len": kv_len}
         residual = ops.embedding(input_ids.reshape(-1), self.embed_tokens)  # [T, H], becomes the residual stream
         x = ops.rmsnorm(residual, self.layers[0].input_norm_w, self.eps)
         for i, layer in enumerate(self.layers):
@@ -268,8 +267,7 @@ class Qwen3:
             if native:
                 bl = bsz // self.world_size
                 hidden = hidden[self.rank * bl:(self.rank + 1) * bl].contiguous()
-                step = {"pos": position_ids.reshape(-1).to(torch.int32), "slots": kv_cache.slots(position_ids),
-                        "kv_lens": (position_ids[:, -1] + 1).to(torch.int32)}
+                step = ops.step_tables(position_ids, kv_cache.blocks_per_seq * kv_cache.page_size)
             for layer in self.layers:
                 hidden = layer.fwd(hidden, position_ids, self.cos_sin_cache, kv_cache, step)
             if native and not wo_lm_head and native_gather:

@@ -266,6 +266,20 @@ def rmsnorm(x: torch.Tensor, gamma: torch.Tensor, eps: float, residual: torch.Te
     return o2.reshape(x.shape)
 
 
+def step_tables(position_ids: torch.Tensor, slots_per_seq: int) -> dict[str, torch.Tensor]:
+    """What every layer of a step reads of its token positions [B, S] (int64), in one launch: ``pos`` int32 [B * S], ``slots`` int64
+    [B * S] (the slot in a paged cache where sequence b owns slots ``b * slots_per_seq`` ...) and ``kv_lens`` int32 [B]."""
+    _lib.require_cuda()
+    B, S = position_ids.shape
+    ids = position_ids.to(torch.int64).contiguous()
+    pos = torch.empty(B * S, dtype=torch.int32, device=ids.device)
+    slots = torch.empty(B * S, dtype=torch.int64, device=ids.device)
+    kv_lens = torch.empty(B, dtype=torch.int32, device=ids.device)
+    _lib.call("b200_step_tables", ptr(ids), B, S, ctypes.c_longlong(slots_per_seq), ptr(pos), ptr(slots), ptr(kv_lens), stream_ptr())
+    _count()
+    return {"pos": pos, "slots": slots, "kv_lens": kv_lens}
+
+
 def qk_norm_rope(qkv: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Tensor, num_q_heads: int,
                  num_kv_heads: int, k_cache: torch.Tensor, v_cache: torch.Tensor, slots: torch.Tensor | None,
                  q_gamma: torch.Tensor | None, k_gamma: torch.Tensor | None, eps: float = 1e-6,
