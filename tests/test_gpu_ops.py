@@ -320,3 +320,33 @@ def test_gemm_tile_widths(M, N, K, gated, dtype):
         want = gate * torch.sigmoid(gate) * up
     assert (out[:, N:] == 7).all()
     torch.testing.assert_close(out[:, :N].double(), want, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10, atol=K * 2.0 ** -20)
+
+
+@pytest.mark.parametrize("lens,Hq,Hkv,page,splits", [((1, 15, 16, 17), 8, 1, 64, 1), ((63, 64, 65, 300), 6, 2, 16, 2), ((129, 1000, 2, 777), 32, 4, 48, 5),
+                                                     ((500, 31, 64, 4000), 3, 3, 10, 4)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rising", [False, True])
+def test_decode_attention_small_groups(lens, Hq, Hkv, page, splits, dtype, rising):
+    """Up to eight heads per KV head: lengths around the 16-token slices, pages that slices cross, groups that fill a part of the tile, and
+    scores that rise along the keys, so that the reference maximum moves again and again. Error against 64 bits: probabilities and
+    the result are rounded to 16 bits, half a unit (2^-9, 2^-12) of the largest value each, doubled for the sums."""
+    from triton_distributed_b200 import ops
+    torch.manual_seed(21)
+    B, D, blocks = len(lens), 128, -(-max(lens) // page)
+    table = torch.randperm(B * blocks, device="cuda").to(torch.int32).view(B, blocks)
+    q = torch.randn(B, Hq, D, device="cuda", dtype=dtype)
+    k, v = (torch.randn(B * blocks, page, Hkv, D, device="cuda", dtype=dtype) for _ in range(2))
+    if rising:  # scores climb by up to 60 along the sequence
+        for b, n in enumerate(lens):
+            at = torch.arange(blocks * page, device="cuda").clamp(max=n - 1) / n
+            lift = (q[b].view(Hkv, -1, D)[:, 0].float() / q[b].view(Hkv, -1, D)[:, 0].float().norm(dim=-1, keepdim=True) * 60)
+            k[table[b].long()] += (at.view(blocks, page, 1, 1) * lift).to(dtype)
+    kv = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    out, lse = ops.decode_attention(q, k, v, kv, table, D ** -0.5, 0.0, splits, return_lse=True)
+    for b, n in enumerate(lens):
+        kb, vb = (c[table[b].long()].flatten(0, 1)[:n].double().repeat_interleave(Hq // Hkv, 1) for c in (k, v))
+        s = torch.einsum("hd,nhd->hn", q[b].double(), kb) * D ** -0.5
+        want = torch.einsum("hn,nhd->hd", torch.softmax(s, -1), vb)
+        half = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
+        assert ((out[b].double() - want).abs() <= 2 * half * (want.abs() + vb.abs().amax())).all()
+        torch.testing.assert_close(lse[b].double(), torch.logsumexp(s, -1), rtol=1e-5, atol=1e-4)

@@ -555,6 +555,252 @@ __global__ void __launch_bounds__(kAttnThreads) decode_split_ring_kernel(const D
   if (FUSE && !p.direct) combine_by_last_cta<BF16>(p, b, head0, nrows);
 }
 
+// ------------------------------------------------------------------------------------------------
+// Groups of at most eight query heads per KV head: the same rings, with tokens on the wide side of the products.
+//
+// The kernel above puts the query heads on the 16 rows of mma.m16n8k16, of which a group of four or eight fills a part, and
+// reduces and rescales in every 16-token slice: 785 instructions a slice at 4.4 clocks each, which bound it (4.65 of 8.2 TB/s
+// under the profiler) with two warps per scheduler. Here the scores are S^T [16 tokens, 8 heads] = K Q^T and the output is
+// O^T [128, 8 heads] += V^T P^T: half the products and half the accumulators, P^T gets its layout from two movmatrix, and the
+// reference maximum of a head moves only when a score exceeds it by more than 2^8 (one vote per slice), so that a slice has
+// no reduction and no rescale. Sums and output share the reference, which cancels in the merge.
+// 8 sequences of 24 K to 32 K tokens, 32 / 8 heads: 192.6 us -> 153.4 (6.2 TB/s); 64 of 4 K 180.9 -> 141.1; one of 128 K
+// 92.9 -> 89.8; 8 of 128 K with one KV head 93.1 -> 84.0; 2 of 4 K 19.9 -> 20.8 (the latency of starting and merging).
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+  return d;
+}
+
+template <bool BF16, int kNST, bool FUSE = false>
+__global__ void __launch_bounds__(kAttnThreads) decode_split_narrow_kernel(const DecodeParams p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  griddep_launch_dependents();
+  griddep_wait();
+  constexpr int kSlice = 16;                      // tokens per slice
+  constexpr int kSliceBytes = kSlice * kD * 2;    // 4 KB (K or V)
+  constexpr int kHeads = 8;
+  constexpr float kSlack = 8.f;                   // log2
+  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int nrows = p.Hq / p.Hkv, head0 = kvh * nrows;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kv_len = p.kv_lens[b];
+  int chunk = (kv_len + p.S - 1) / p.S;
+  chunk = (chunk + kTile - 1) / kTile * kTile;
+  const int t0 = split * chunk;
+  const int t1 = min(kv_len, t0 + chunk);
+  const int row = lane >> 2, col = (lane & 3) * 2;   // of an accumulator tile: token (or output column), head and the next
+
+  if (t0 >= t1) {  // empty split: mark it so that the combine skips it
+    if (!p.direct) {
+      for (int r = threadIdx.x; r < nrows; r += blockDim.x)
+        p.lse_part[(static_cast<size_t>(b) * p.Hq + head0 + r) * p.S + split] = -INFINITY;
+      if (FUSE) combine_by_last_cta<BF16>(p, b, head0, nrows);
+    } else {
+      for (int i = threadIdx.x; i < nrows * kD; i += blockDim.x) {
+        const size_t o = (static_cast<size_t>(b) * p.Hq + head0 + i / kD) * kD + (i % kD);
+        if (BF16) static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16(0.f);
+        else static_cast<__half*>(p.out)[o] = __float2half(0.f);
+      }
+      if (p.out_lse)
+        for (int r = threadIdx.x; r < nrows; r += blockDim.x) p.out_lse[static_cast<size_t>(b) * p.Hq + head0 + r] = -INFINITY;
+    }
+    return;
+  }
+
+  uint32_t qb[8][2];   // Q^T fragments: head lane / 4, elements 16 kk + col, + 1 and eight further
+  {
+    const uint32_t* q32 = static_cast<const uint32_t*>(p.q) + (static_cast<size_t>(b) * p.Hq + head0 + min(row, nrows - 1)) * (kD / 2);
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) {
+      qb[kk][0] = row < nrows ? q32[kk * 8 + (lane & 3)] : 0u;
+      qb[kk][1] = row < nrows ? q32[kk * 8 + 4 + (lane & 3)] : 0u;
+    }
+  }
+
+  // this warp's ring: slot s holds K at +0 and V at +kSliceBytes
+  const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + warp * (kNST * 2 * kSliceBytes);
+  const uint8_t* kc = static_cast<const uint8_t*>(p.k_cache);
+  const uint8_t* vc = static_cast<const uint8_t*>(p.v_cache);
+  const int nslices_cta = (t1 - t0 + kSlice - 1) / kSlice;
+  const int my_slices = nslices_cta > warp ? (nslices_cta - warp + 3) / 4 : 0;   // slices warp, warp + 4, ...
+  const bool page_fast = (p.page % kSlice) == 0;   // a 16-token slice never crosses a page (t0 is a multiple of 64)
+  const int* table = p.block_table + static_cast<size_t>(b) * p.bt_stride;
+  const int hi = lane >> 4, c16 = lane & 15;       // copies: half a warp per token of 256 bytes
+  const size_t step = static_cast<size_t>(p.Hkv) * (2 * 2 * kD);                 // bytes between every other token
+  const size_t lane_off = (static_cast<size_t>(hi) * p.Hkv + kvh) * (2 * kD) + c16 * 16;
+  uint32_t so[4];                                  // swizzled places of tokens 2 i + hi, i = 0..3; eight tokens down they repeat
+#pragma unroll
+  for (int i = 0; i < 4; ++i) so[i] = static_cast<uint32_t>((2 * i + hi) * 256 + ((c16 ^ (2 * i + hi)) * 16));
+  int next_blk = page_fast && my_slices > 0 ? table[(t0 + warp * kSlice) / p.page] : 0;   // one slice ahead of its copies
+
+  auto load_slice = [&](int j) {   // j-th slice of this warp; always commits a group so that the counting stays uniform
+    if (j < my_slices) {
+      const int st0 = t0 + (warp + 4 * j) * kSlice;
+      const uint32_t slot = ring + (j % kNST) * (2 * kSliceBytes);
+      if (page_fast) {
+        const size_t base = (static_cast<size_t>(next_blk) * p.page + st0 % p.page) * (static_cast<size_t>(p.Hkv) * 2 * kD) + lane_off;
+        if (j + 1 < my_slices) next_blk = table[(st0 + 4 * kSlice) / p.page];
+        const uint8_t *ks = kc + base, *vs = vc + base;
+        if (st0 + kSlice <= t1) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t at = slot + so[i & 3] + (i >> 2) * (8 * 256);
+            cp_async_16(at, ks + i * step, 16);
+            cp_async_16(at + kSliceBytes, vs + i * step, 16);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t at = slot + so[i & 3] + (i >> 2) * (8 * 256);
+            const bool in = st0 + 2 * i + hi < t1;
+            cp_async_16(at, in ? ks + i * step : kc, in ? 16 : 0);
+            cp_async_16(at + kSliceBytes, in ? vs + i * step : vc, in ? 16 : 0);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t at = slot + so[i & 3] + (i >> 2) * (8 * 256);
+          const int tok = st0 + 2 * i + hi;
+          const bool in = tok < t1;
+          size_t off = 0;
+          if (in) off = ((static_cast<size_t>(table[tok / p.page]) * p.page + tok % p.page) * p.Hkv + kvh) * (2 * kD) + c16 * 16;
+          cp_async_16(at, kc + off, in ? 16 : 0);
+          cp_async_16(at + kSliceBytes, vc + off, in ? 16 : 0);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+
+  float m_ref[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};   // of heads col, col + 1; l_run: this lane's tokens
+  float oacc[8][4];   // tile dn: columns 16 dn + row (and + 8) of heads col, col + 1
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) oacc[i][e] = 0.f;
+
+  const float kLog2e = 1.4426950408889634f;
+  const float scale2 = p.scale * kLog2e;
+  const int mi = lane >> 3, mr = lane & 7;
+  // lane addresses of the fragments: K chunks 2 kk + (mi >> 1) of token (mi & 1) * 8 + mr; V chunks 2 dn + (mi & 1) of token (mi >> 1) * 8 + mr
+  const uint32_t k_row = ((mi & 1) * 8 + mr) * 256, v_row = ((mi >> 1) * 8 + mr) * 256;
+#pragma unroll
+  for (int j = 0; j < kNST - 1; ++j) load_slice(j);
+  for (int j = 0; j < my_slices; ++j) {
+    load_slice(j + kNST - 1);        // into the slot that was computed in the previous iteration
+    cp_async_wait<kNST - 1>();       // slice j has landed (for this lane); the barrier below covers the other lanes
+    __syncwarp();
+    const uint32_t ks = ring + (j % kNST) * (2 * kSliceBytes), vs = ks + kSliceBytes;
+    const int wt0 = t0 + (warp + 4 * j) * kSlice;  // first token of this slice
+    // ---- S^T: two sums, so that no product waits for the one before it
+    float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) {
+      uint32_t a[4];
+      ldmatrix_x4(ks + k_row + (((2 * kk + (mi >> 1)) ^ mr) * 16), a[0], a[1], a[2], a[3]);
+      mma16816<BF16>((kk & 1) ? sb : sa, a, qb[kk][0], qb[kk][1]);
+    }
+    float v[4];   // tokens row, row, row + 8, row + 8 of heads col, col + 1, col, col + 1
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = (sa[e] + sb[e]) * scale2;
+    if (p.soft_cap > 0.f) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = p.soft_cap * tanhf((sa[e] + sb[e]) * p.scale / p.soft_cap) * kLog2e;
+    }
+    if (wt0 + kSlice > t1) {
+      if (wt0 + row >= t1) v[0] = v[1] = -INFINITY;
+      if (wt0 + row + 8 >= t1) v[2] = v[3] = -INFINITY;
+    }
+    const float top0 = fmaxf(v[0], v[2]), top1 = fmaxf(v[1], v[3]);
+    if (__any_sync(0xffffffffu, top0 > m_ref[0] + kSlack || top1 > m_ref[1] + kSlack)) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float mx = h ? top1 : top0;
+#pragma unroll
+        for (int m = 4; m < 32; m <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, m));
+        const float m_new = fmaxf(m_ref[h], mx);
+        const float corr = m_new == -INFINITY ? 0.f : exp2f(m_ref[h] - m_new);   // m_ref = -inf -> 0
+        m_ref[h] = m_new;
+        l_run[h] *= corr;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          oacc[i][h] *= corr;
+          oacc[i][2 + h] *= corr;
+        }
+      }
+    }
+    float pr[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) pr[e] = exp2f(v[e] - (m_ref[e & 1] == -INFINITY ? 0.f : m_ref[e & 1]));
+    l_run[0] += pr[0] + pr[2];
+    l_run[1] += pr[1] + pr[3];
+    const uint32_t b0 = movmatrix_trans(BF16 ? pack_bf16x2(pr[0], pr[1]) : pack_f16x2(pr[0], pr[1]));
+    const uint32_t b1 = movmatrix_trans(BF16 ? pack_bf16x2(pr[2], pr[3]) : pack_f16x2(pr[2], pr[3]));
+#pragma unroll
+    for (int dn = 0; dn < 8; ++dn) {
+      uint32_t a[4];
+      ldmatrix_x4_trans(vs + v_row + (((2 * dn + (mi & 1)) ^ mr) * 16), a[0], a[1], a[2], a[3]);
+      mma16816<BF16>(oacc[dn], a, b0, b1);
+    }
+    __syncwarp();  // every lane is done with this slot before the next iteration's copies overwrite the previous one
+  }
+  cp_async_wait<0>();
+  __syncthreads();   // all rings are idle: their memory becomes the merge area
+
+  // ---- merge the four warps ----
+  float* red_m = reinterpret_cast<float*>(smem);            // [4][8]
+  float* red_l = red_m + 4 * kHeads;                        // [4][8]
+  float* red_o = red_l + 4 * kHeads;                        // [4][8][128]
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int m = 4; m < 32; m <<= 1) l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], m);
+    if (row == 0) {
+      red_m[warp * kHeads + col + h] = m_ref[h];
+      red_l[warp * kHeads + col + h] = l_run[h];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = col + h;
+    const float mg = fmaxf(fmaxf(red_m[r], red_m[kHeads + r]), fmaxf(red_m[2 * kHeads + r], red_m[3 * kHeads + r]));
+    const float scale_w = m_ref[h] == -INFINITY ? 0.f : exp2f(m_ref[h] - mg);
+    float* o = red_o + (warp * kHeads + r) * kD + row;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      o[16 * i] = oacc[i][h] * scale_w;
+      o[16 * i + 8] = oacc[i][2 + h] * scale_w;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nrows * kD; i += blockDim.x) {
+    const int r = i / kD, c = i - r * kD;
+    const float mg = fmaxf(fmaxf(red_m[r], red_m[kHeads + r]), fmaxf(red_m[2 * kHeads + r], red_m[3 * kHeads + r]));
+    float lg = 0.f, og = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float mw = red_m[w * kHeads + r];
+      lg += mw == -INFINITY ? 0.f : red_l[w * kHeads + r] * exp2f(mw - mg);
+      og += red_o[(w * kHeads + r) * kD + c];
+    }
+    const float o = lg > 0.f ? og / lg : 0.f;
+    const size_t bh = static_cast<size_t>(b) * p.Hq + head0 + r;
+    const float lse = lg > 0.f ? mg * 0.6931471805599453f + logf(lg) : -INFINITY;
+    if (p.direct) {
+      if (BF16) static_cast<__nv_bfloat16*>(p.out)[bh * kD + c] = __float2bfloat16(o);
+      else static_cast<__half*>(p.out)[bh * kD + c] = __float2half(o);
+      if (c == 0 && p.out_lse) p.out_lse[bh] = lse;
+    } else {
+      p.o_part[(bh * p.S + split) * kD + c] = o;
+      if (c == 0) p.lse_part[bh * p.S + split] = lse;
+    }
+  }
+  if (FUSE && !p.direct) combine_by_last_cta<BF16>(p, b, head0, nrows);
+}
+
 // With `gate` ([B, Hq], row pitch ldg) every head's merged output is multiplied by sigmoid(gate).
 // out[bh, :] = sum_s w_s o[bh, s, :] / sum_s w_s with w_s = exp(lse_s - max lse); partials with
 // lse = -inf are skipped. Strides are in elements so the same kernel merges split partials
@@ -584,7 +830,7 @@ __global__ void __launch_bounds__(kD) decode_combine_kernel(const float* o_part,
 
 // Pipeline variant when the caller passes ring < 0: B200DIST_ATTN_V2 = 0 (two-stage CTA-wide pipeline), 3 or 6
 // (per-warp rings of that depth) forces one; unset picks the three-deep rings (two CTAs of 96 KB per SM), which
-// measured fastest from 2 K to 128 K tokens per sequence: 4.7-4.9 TB/s at batch 8 x 16 K and batch 32 x 4 K against
+// measured fastest from 2 K to 128 K tokens per sequence (with 16-row tiles): 4.7-4.9 TB/s at batch 8 x 16 K and 32 x 4 K against
 // 3.7-3.8 TB/s for the CTA-wide pipeline and 3.1-3.2 TB/s for six-deep rings (one CTA per SM).
 static int attn_ring_default() {
   static int stages = -1;
@@ -638,6 +884,7 @@ B200_API int b200_decode_attn(const void* q, const void* k_cache, const void* v_
 #define B200_ATTN_SMEM(BF, FU)                                                                \
     if (rc == kOk) rc = set_smem(decode_split_kernel<BF, FU>, kAttnSmem);                       \
     if (rc == kOk) rc = set_smem(decode_split_ring_kernel<BF, 3, FU>, 96 * 1024);               \
+    if (rc == kOk) rc = set_smem(decode_split_narrow_kernel<BF, 3, FU>, 96 * 1024);             \
     if (rc == kOk) rc = set_smem(decode_split_ring_kernel<BF, 6, FU>, 192 * 1024);
     B200_ATTN_SMEM(true, false) B200_ATTN_SMEM(false, false) B200_ATTN_SMEM(true, true) B200_ATTN_SMEM(false, true)
 #undef B200_ATTN_SMEM
@@ -662,6 +909,11 @@ B200_API int b200_decode_attn(const void* q, const void* k_cache, const void* v_
     else if (bf) B200_ATTN_LAUNCH((decode_split_kernel<true, false>));
     else if (fuse) B200_ATTN_LAUNCH((decode_split_kernel<false, true>));
     else B200_ATTN_LAUNCH((decode_split_kernel<false, false>));
+  } else if (ring == 3 && G <= 8) {
+    if (bf && fuse) B200_ATTN_LAUNCH((decode_split_narrow_kernel<true, 3, true>));
+    else if (bf) B200_ATTN_LAUNCH((decode_split_narrow_kernel<true, 3, false>));
+    else if (fuse) B200_ATTN_LAUNCH((decode_split_narrow_kernel<false, 3, true>));
+    else B200_ATTN_LAUNCH((decode_split_narrow_kernel<false, 3, false>));
   } else if (ring == 3) {
     if (bf && fuse) B200_ATTN_LAUNCH((decode_split_ring_kernel<true, 3, true>));
     else if (bf) B200_ATTN_LAUNCH((decode_split_ring_kernel<true, 3, false>));
