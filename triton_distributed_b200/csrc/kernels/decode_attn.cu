@@ -562,8 +562,9 @@ __global__ void __launch_bounds__(kAttnThreads) decode_split_ring_kernel(const D
 // reduces and rescales in every 16-token slice: 785 instructions a slice at 4.4 clocks each, which bound it (4.65 of 8.2 TB/s
 // under the profiler) with two warps per scheduler. Here the scores are S^T [16 tokens, 8 heads] = K Q^T and the output is
 // O^T [128, 8 heads] += V^T P^T: half the products and half the accumulators, P^T gets its layout from two movmatrix, and the
-// reference maximum of a head moves only when a score exceeds it by more than 2^8 (one vote per slice), so that a slice has
-// no reduction and no rescale. Sums and output share the reference, which cancels in the merge.
+// running maximum of a head, its reduction over the tokens and the rescale are left out of a slice that holds no new maximum of
+// any head (one vote). Letting the maximum lag by up to 2^8 was no faster and cost a tenth of the precision: probabilities just
+// below one, where most of the weight is, are rounded by half as much as those just above a power of two.
 // 8 sequences of 24 K to 32 K tokens, 32 / 8 heads: 192.6 us -> 153.4 (6.2 TB/s); 64 of 4 K 180.9 -> 141.1; one of 128 K
 // 92.9 -> 89.8; 8 of 128 K with one KV head 93.1 -> 84.0; 2 of 4 K 19.9 -> 20.8 (the latency of starting and merging).
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
@@ -580,7 +581,6 @@ __global__ void __launch_bounds__(kAttnThreads) decode_split_narrow_kernel(const
   constexpr int kSlice = 16;                      // tokens per slice
   constexpr int kSliceBytes = kSlice * kD * 2;    // 4 KB (K or V)
   constexpr int kHeads = 8;
-  constexpr float kSlack = 8.f;                   // log2
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int nrows = p.Hq / p.Hkv, head0 = kvh * nrows;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(kAttnThreads) decode_split_narrow_kernel(const
       if (wt0 + row + 8 >= t1) v[2] = v[3] = -INFINITY;
     }
     const float top0 = fmaxf(v[0], v[2]), top1 = fmaxf(v[1], v[3]);
-    if (__any_sync(0xffffffffu, top0 > m_ref[0] + kSlack || top1 > m_ref[1] + kSlack)) {
+    if (__any_sync(0xffffffffu, top0 > m_ref[0] || top1 > m_ref[1])) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         float mx = h ? top1 : top0;
