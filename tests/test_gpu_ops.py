@@ -350,3 +350,23 @@ def test_decode_attention_small_groups(lens, Hq, Hkv, page, splits, dtype, risin
         half = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
         assert ((out[b].double() - want).abs() <= 2 * half * (want.abs() + vb.abs().amax())).all()
         torch.testing.assert_close(lse[b].double(), torch.logsumexp(s, -1), rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("E,k", [(1, 1), (8, 8), (33, 4), (128, 8), (129, 8), (256, 32), (257, 3), (512, 8)])
+def test_topk_softmax_widths_and_ties(E, k):
+    """Every number of values per lane and its edges, equal logits (the lower expert goes first) and -inf logits, against a stable sort
+    in fp64; a probability is off by a few units of fp32."""
+    from triton_distributed_b200 import ops
+    torch.manual_seed(22)
+    T = 300
+    logits = (torch.randn(T, E, device="cuda") * 4).round() / 2   # many ties
+    logits[0] = 0.0
+    if E > k:
+        logits[1, : E - k] = -torch.inf
+    for renorm in (False, True):
+        ids, w = ops.topk_softmax(logits, k, renorm)
+        p = torch.softmax(logits.double(), -1)
+        want_p, want = torch.sort(p, dim=-1, descending=True, stable=True)
+        want_p = want_p[:, :k] / (want_p[:, :k].sum(-1, keepdim=True) if renorm else 1.0)
+        assert torch.equal(ids.long(), want[:, :k])
+        torch.testing.assert_close(w.double(), want_p, rtol=1e-5, atol=1e-9)
