@@ -102,9 +102,13 @@ _DTYPE_CODE = {
 }
 
 
-def dtype_code(dt: torch.dtype) -> int:
+_SETTLED = 0x100  # ``kSettled`` of csrc/include/b200/host.h
+
+
+def dtype_code(dt: torch.dtype, settled: bool = False) -> int:
+    """The native code of a type; ``settled``: no kernel in flight on the stream writes the call's parameters."""
     try:
-        return _DTYPE_CODE[dt]
+        return _DTYPE_CODE[dt] | (_SETTLED if settled else 0)
     except KeyError:
         raise TypeError(f"dtype {dt} is not supported by the native kernels") from None
 

@@ -36,9 +36,9 @@ def main() -> None:
     if args.kind == "tiled":
         fn = lambda: ops.gemm(a, b, c)
     elif args.kind == "skinny":
-        fn = lambda: ops.gemm_skinny(a, b, c)
+        fn = lambda: ops.gemm_skinny(a, b, c, settled=True)
     else:
-        fn = lambda: ops.gemm_skinny(a, b, c, swiglu=True)
+        fn = lambda: ops.gemm_skinny(a, b, c, swiglu=True, settled=True)
     _, ms, ts = perf_func_cold(fn, args.iters, args.warmup)
     flops = 2.0 * args.m * rows * args.k
     wbytes = 2.0 * rows * args.k

@@ -134,7 +134,7 @@ def main() -> None:
         g = torch.ones(D, device=dev, dtype=dt)
         ss = torch.full((16,), float(H), device=dev)
         ep = ops.skinny_row_scale(ss, H, 1e-6, base=ops.skinny_qkv_heads(pos, None, cs, Hq, Hkv, qo, kcache, vcache, g, g, 1e-6))
-        fn = lambda: ops.gemm_skinny(x, w, epilogue=ep)
+        fn = lambda: ops.gemm_skinny(x, w, epilogue=ep, settled=True)
         info = {"bytes": 2.0 * w.numel()}
     elif args.op in ("decode_attn", "sp_decode"):
         B, Hq, Hkv, D, page, L = 8, 64, 8, 128, 64, args.kv_len
@@ -163,7 +163,7 @@ def main() -> None:
     elif args.op == "rmsnorm":
         x = torch.randn(16384, 8192, device=dev, dtype=dt)
         g = torch.ones(8192, device=dev, dtype=dt)
-        fn = lambda: ops.rmsnorm(x, g, 1e-6)
+        fn = lambda: ops.rmsnorm(x, g, 1e-6, settled=True)
         info = {"bytes": 2.0 * x.numel() * 2}
     elif args.op == "latent_decode":  # batch 8, 32 heads, latent rank 512
         B, H, r = 8, 32, 512
@@ -172,7 +172,7 @@ def main() -> None:
         lens, q = torch.full((B,), args.kv_len, dtype=torch.int32, device=dev), torch.randn(B, H, r, device=dev, dtype=dt)
         splits, rows = ops.choose_latent_splits(B, H, args.kv_len)
         sink = torch.zeros(H, device=dev)
-        fn = lambda: ops.latent_attention(q, cache, lens, table, 1, 0.05, sink, args.splits or splits, rows)
+        fn = lambda: ops.latent_attention(q, cache, lens, table, 1, 0.05, sink, args.splits or splits, rows, settled=True)
         info = {"bytes": 2.0 * cache.numel(), "splits": args.splits or splits}
     elif args.op == "residual_norm":  # 4096 tokens, 16 earlier states
         T, W, n = 4096, 4096, 16
@@ -180,7 +180,7 @@ def main() -> None:
         a, b = torch.randn(2, T, W, device=dev, dtype=dt)
         gates, w = torch.randn(T, 2 * W, device=dev, dtype=dt), torch.ones(n + 1, device=dev)
         g = torch.ones(W, device=dev, dtype=dt)
-        fn = lambda: ops.residual_norm(x, W, 0.5, a, gates[:, :W], g, b, gates[:, W:], g, states=states, weights=w, keep=True, gain=g, bias=g)
+        fn = lambda: ops.residual_norm(x, W, 0.5, a, gates[:, :W], g, b, gates[:, W:], g, states=states, weights=w, keep=True, gain=g, bias=g, settled=True)
         info = {"bytes": T * W * (8 + 8 + 4 + 4.0 * n + 4 + 2)}
     elif args.op in ("wkv", "gated_delta"):  # batch 8 x 512 tokens; 64 heads of 64, or 32 heads of 128
         B, S = 8, 512
@@ -188,11 +188,11 @@ def main() -> None:
         rows = [torch.randn(B * S, H * D, device=dev, dtype=dt) for _ in range(5)]
         st, c = torch.zeros(B, H, D, D, device=dev), torch.ones(H * D, device=dev)
         if args.op == "wkv":
-            fn = lambda: ops.wkv(*rows, c, c, c, st, D, D, 1e-6)
+            fn = lambda: ops.wkv(*rows, c, c, c, st, D, D, 1e-6, settled=True)
         else:
             ab = torch.randn(B * S, 2 * H, device=dev, dtype=dt)
             fn = lambda: ops.gated_delta(rows[0][:, : H // 2 * D], rows[1][:, : H // 2 * D], rows[2], ab[:, :H], ab[:, H:], rows[3], c[:H], c[:H], c[:D],
-                                         st, D, D, 1e-6)
+                                         st, D, D, 1e-6, settled=True)
         info = {"flops": (5.0 if args.op == "wkv" else 7.0) * B * S * H * D * D}
     else:  # qk_norm_rope
         T, Hq, Hkv, D = 16384, 64, 8, 128
@@ -204,7 +204,7 @@ def main() -> None:
         kcache = torch.zeros(T, Hkv, D, device=dev, dtype=dt)
         vcache = torch.zeros_like(kcache)
         g = torch.ones(D, device=dev, dtype=dt)
-        fn = lambda: ops.qk_norm_rope(qkv, pos, cs, Hq, Hkv, kcache, vcache, None, g, g)
+        fn = lambda: ops.qk_norm_rope(qkv, pos, cs, Hq, Hkv, kcache, vcache, None, g, g, settled=True)
         info = {"bytes": 2.0 * qkv.numel() * 2}
     _, ms, ts = perf_func_cold(fn, args.iters, args.warmup)
     utils.get_heap().check_status(args.op)

@@ -121,7 +121,7 @@ def kernels(name: str, batch: int = 8, prompt: int = 2048) -> list[dict]:
         table = torch.arange(pages, dtype=torch.int32, device=dev).view(batch, -1)
         cache, qc, sink = rnd(pages, 64, r), rnd(batch, H, r), torch.zeros(H, device=dev)
         splits, rows = ops.choose_latent_splits(batch, H, kv)
-        new = _row(f"latent attention + combine, kv {kv}", lambda: ops.latent_attention(qc, cache, lens, table, 1, 0.1, sink, splits, rows),
+        new = _row(f"latent attention + combine, kv {kv}", lambda: ops.latent_attention(qc, cache, lens, table, 1, 0.1, sink, splits, rows, settled=True),
                    2.0 * batch * kv * r, 4.0 * batch * H * kv * r)
         kc, vc, qq = rnd(pages, 64, Hkv, 128), rnd(pages, 64, Hkv, 128), rnd(batch, H, 128)
         ws: dict = {}
@@ -135,8 +135,8 @@ def kernels(name: str, batch: int = 8, prompt: int = 2048) -> list[dict]:
     for label, N, K in (("absorb queries", r, d), ("values from latents", v, r)):
         xh, wh = rnd(batch, H, K), rnd(H, N, K)
         wl = rnd(H * N * K // W // 128 * 128, W)   # a decode GEMM of as many weight bytes
-        pair(_row(f"head_linear, {label}, {batch} tokens", lambda: ops.head_linear(xh, wh), 2.0 * H * N * K),
-             _row("gemm_skinny of equal bytes", lambda: ops.gemm_skinny(x, wl), 2.0 * wl.numel()))
+        pair(_row(f"head_linear, {label}, {batch} tokens", lambda: ops.head_linear(xh, wh, settled=True), 2.0 * H * N * K),
+             _row("gemm_skinny of equal bytes", lambda: ops.gemm_skinny(x, wl, settled=True), 2.0 * wl.numel()))
     for T in (batch, batch * prompt):                                                 # ---- row-wise kernels
         cols = H * d + r + ff + 2 * W
         proj, gain = rnd(T, cols), rnd(r)
@@ -151,14 +151,14 @@ def kernels(name: str, batch: int = 8, prompt: int = 2048) -> list[dict]:
         n = L // 2
         states, wts = torch.zeros(n + 1, T, W, device=dev), torch.ones(n + 1, device=dev)
         new = _row(f"residual_norm with {n} earlier states, {T} tokens",
-                   lambda: ops.residual_norm(xs, W, 0.5, s1, ga, b, s2, gb, b, states=states, weights=wts, keep=True, gain=g, bias=b, eps=1e-6),
+                   lambda: ops.residual_norm(xs, W, 0.5, s1, ga, b, s2, gb, b, states=states, weights=wts, keep=True, gain=g, bias=b, eps=1e-6, settled=True),
                    T * W * (8 + 8 + 4 + 4 * n + 4 + 2.0))
         res = rnd(T, W)
-        pair(new, _row(f"rmsnorm with residual, {T} tokens", lambda: ops.rmsnorm(s1, g, 1e-6, residual=res), 8.0 * T * W))
+        pair(new, _row(f"rmsnorm with residual, {T} tokens", lambda: ops.rmsnorm(s1, g, 1e-6, residual=res, settled=True), 8.0 * T * W))
         del states, proj
         ids, tab = torch.randint(0, a.vocab_size, (T,), device=dev), rnd(a.vocab_size, W)
         st0 = torch.empty(T, W, device=dev)
-        new = _row(f"embed_norm, {T} tokens", lambda: ops.embed_norm(ids, tab, 2.0, W, g, b, 1e-6, True, state0=st0), T * W * 12.0)
+        new = _row(f"embed_norm, {T} tokens", lambda: ops.embed_norm(ids, tab, 2.0, W, g, b, 1e-6, True, state0=st0, settled=True), T * W * 12.0)
         pair(new, _row(f"embedding, {T} tokens", lambda: ops.embedding(ids, tab), 4.0 * T * W))
     S, B = prompt, batch                                                              # ---- prompts
     R = B * S
@@ -167,7 +167,7 @@ def kernels(name: str, batch: int = 8, prompt: int = 2048) -> list[dict]:
     w_like = rnd(H * 128, W)
     like = _row(f"gemm {R} x {H * 128} x {W}", lambda: ops.linear(xp, w_like),
                 2.0 * (R * W + R * H * 128 + H * 128 * W), 2.0 * R * H * 128 * W)
-    pair(_row(f"expand keys: gemm {R} x {H * d} x {r}", lambda: ops.linear(c, uk), 2.0 * (R * r + H * d * r + R * H * d), 2.0 * R * H * d * r), like)
+    pair(_row(f"expand keys: gemm {R} x {H * d} x {r}", lambda: ops.linear(c, uk, settled=True), 2.0 * (R * r + H * d * r + R * H * d), 2.0 * R * H * d * r), like)
     pair(_row(f"expand values: gemm {H * v} x {R} x {r}", lambda: ops.linear(uv, c), 2.0 * (R * r + H * v * r + R * H * v), 2.0 * R * H * v * r), like)
     qp, kp, vt = rnd(B * S, H, d), rnd(B * S, H, d), rnd(H, v, B * S)
     cu = torch.arange(0, (B + 1) * S, S, dtype=torch.int32, device=dev)

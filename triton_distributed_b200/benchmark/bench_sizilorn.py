@@ -94,14 +94,14 @@ def kernels(name: str, batch: int = 8, prompt: int = 2048) -> list[dict]:
         N = m.heads * m.dim
         rows = [rnd(T, N) for _ in range(5)]
         st, c = torch.zeros(batch, m.heads, m.dim, m.dim, device=dev), torch.ones(N, device=dev)
-        pair(_row(f"wkv, {m.heads} heads of {m.dim}, {tag}", lambda: ops.wkv(*rows, c, c, c, st, m.dim, m.dim, 1e-6),
+        pair(_row(f"wkv, {m.heads} heads of {m.dim}, {tag}", lambda: ops.wkv(*rows, c, c, c, st, m.dim, m.dim, 1e-6, settled=True),
                   12.0 * T * N + 8.0 * st.numel(), fp32(5.0 * T * N * m.dim), iters=6), decode_like if tokens == 1 else prefill_like)
         qk, E = de.kv_heads * de.dim, de.heads * de.vdim
         rows, ab = [rnd(T, qk), rnd(T, qk), rnd(T, E), rnd(T, E)], rnd(T, 2 * de.heads)
         st, c = torch.zeros(batch, de.heads, de.dim, de.vdim, device=dev), torch.ones(max(de.heads, de.vdim), device=dev)
         pair(_row(f"gated_delta, {de.heads} heads of {de.dim}, {tag}",
                   lambda: ops.gated_delta(rows[0], rows[1], rows[2], ab[:, : de.heads], ab[:, de.heads:], rows[3], c[: de.heads], c[: de.heads], c[: de.vdim],
-                                          st, de.dim, de.vdim, 1e-6),
+                                          st, de.dim, de.vdim, 1e-6, settled=True),
                   2.0 * T * (2 * qk + 3 * E) + 8.0 * st.numel(), fp32(7.0 * T * E * de.dim), iters=6), decode_like if tokens == 1 else prefill_like)
         del rows, ab, st
         # ---- row-wise kernels
@@ -109,16 +109,16 @@ def kernels(name: str, batch: int = 8, prompt: int = 2048) -> list[dict]:
         glu = _row(f"silu_mul, {tag}", lambda: ops.silu_mul(gu), 6.0 * T * q3.intermediate_size)
         del gu
         g, b, s1, s2, res = rnd(W), rnd(W), rnd(T, W), rnd(T, W), rnd(T, W)
-        norm = _row(f"rmsnorm with residual, {tag}", lambda: ops.rmsnorm(s1, g, 1e-6, residual=res), 8.0 * T * W)
+        norm = _row(f"rmsnorm with residual, {tag}", lambda: ops.rmsnorm(s1, g, 1e-6, residual=res, settled=True), 8.0 * T * W)
         xs, tanh = rnd(T, W, dt=torch.float32), ops.TanhNorm(0.5)
-        pair(_row(f"residual_norm, tanh, {tag}", lambda: ops.residual_norm(xs, W, 1.0, s1, gain=g, bias=b, center=tanh), 12.0 * T * W), norm)
-        pair(_row(f"residual_post of one, tanh, {tag}", lambda: ops.residual_post(xs, W, 1.0, s1, g, post_eps=1e-6, gain=g, bias=b, center=tanh), 12.0 * T * W), norm)
-        pair(_row(f"residual_post of two, tanh, {tag}", lambda: ops.residual_post(xs, W, 0.5, s1, g, s2, g, 1e-6, gain=g, bias=b, center=tanh), 14.0 * T * W), norm)
+        pair(_row(f"residual_norm, tanh, {tag}", lambda: ops.residual_norm(xs, W, 1.0, s1, gain=g, bias=b, center=tanh, settled=True), 12.0 * T * W), norm)
+        pair(_row(f"residual_post of one, tanh, {tag}", lambda: ops.residual_post(xs, W, 1.0, s1, g, post_eps=1e-6, gain=g, bias=b, center=tanh, settled=True), 12.0 * T * W), norm)
+        pair(_row(f"residual_post of two, tanh, {tag}", lambda: ops.residual_post(xs, W, 0.5, s1, g, s2, g, 1e-6, gain=g, bias=b, center=tanh, settled=True), 14.0 * T * W), norm)
         mu, last = rnd(5, W), rnd(batch, W)
-        pair(_row(f"token_mix, {tag}", lambda: ops.token_mix(s1, mu, last), 12.0 * T * W), glu)
+        pair(_row(f"token_mix, {tag}", lambda: ops.token_mix(s1, mu, last, settled=True), 12.0 * T * W), glu)
         C = 2 * qk + E
         wide, taps, hist = rnd(T, C + 8), rnd(de.conv, C, dt=torch.float32), rnd(batch, de.conv - 1, C)
-        pair(_row(f"short_conv, {tag}", lambda: ops.short_conv(wide[:, :C], taps, hist), 4.0 * T * C), glu)
+        pair(_row(f"short_conv, {tag}", lambda: ops.short_conv(wide[:, :C], taps, hist, settled=True), 4.0 * T * C), glu)
         del wide
         ids, tab, gs = torch.randint(0, a.vocab_size, (T,), device=dev), rnd(a.vocab_size, side * 4), rnd(T, side)
         emb_table = rnd(a.vocab_size, side)
@@ -130,20 +130,20 @@ def kernels(name: str, batch: int = 8, prompt: int = 2048) -> list[dict]:
         cs, gq = torch.randn(prompt, 128, device=dev), rnd(128)
         pq, pk, pv = proj.split([at.heads * 128, Hkv * 128, Hkv * 128], dim=1)
         pair(_row(f"head_norm_rope, {tag}", lambda: ops.head_norm_rope(pq, pk, pv, at.heads, Hkv, 128, gq, gq, 1e-6, cs, pos, slots, kc, vc), 4.0 * T * cols),
-             _row(f"qk_norm_rope, {tag}", lambda: ops.qk_norm_rope(proj, pos, cs, at.heads, Hkv, kc.view(T, Hkv, 128), vc.view(T, Hkv, 128), slots, gq, gq),
+             _row(f"qk_norm_rope, {tag}", lambda: ops.qk_norm_rope(proj, pos, cs, at.heads, Hkv, kc.view(T, Hkv, 128), vc.view(T, Hkv, 128), slots, gq, gq, settled=True),
                   4.0 * T * cols))
         del proj, kc, vc
         # ---- products of another form than the partner's
         x, w = rnd(T, 5, W), rnd(4 * N + 128, W)
         xl = rnd(T, W)
-        new = _row(f"linear_groups, five inputs, {tag}", lambda: ops.linear_groups(x, w, [N] * 4 + [128]), 2.0 * (w.numel() + x.numel() + T * w.shape[0]),
+        new = _row(f"linear_groups, five inputs, {tag}", lambda: ops.linear_groups(x, w, [N] * 4 + [128], settled=True), 2.0 * (w.numel() + x.numel() + T * w.shape[0]),
                    2.0 * T * w.numel())
-        big = _row(f"linear of equal size, {tag}", lambda: ops.linear(xl, w), 2.0 * (w.numel() + xl.numel() + T * w.shape[0]), 2.0 * T * w.numel())
+        big = _row(f"linear of equal size, {tag}", lambda: ops.linear(xl, w, settled=True), 2.0 * (w.numel() + xl.numel() + T * w.shape[0]), 2.0 * T * w.numel())
         pair(new, big)
         low, w2 = rnd(T, m.decay_rank), rnd(N, m.decay_rank)
-        pair(_row(f"tanh_linear, rank {m.decay_rank}, {tag}", lambda: ops.tanh_linear(low, w2),
+        pair(_row(f"tanh_linear, rank {m.decay_rank}, {tag}", lambda: ops.tanh_linear(low, w2, settled=True),
                   2.0 * (low.numel() + w2.numel() + T * N), 2.0 * T * w2.numel()),
-             _row(f"linear of equal size, {tag}", lambda: ops.linear(low, w2), 2.0 * (low.numel() + w2.numel() + T * N), 2.0 * T * w2.numel()))
+             _row(f"linear of equal size, {tag}", lambda: ops.linear(low, w2, settled=True), 2.0 * (low.numel() + w2.numel() + T * N), 2.0 * T * w2.numel()))
         del x
     ops.check_pipeline_status()
     torch.cuda.empty_cache()

@@ -81,6 +81,16 @@ struct DriverApi {
 const DriverApi* driver();
 
 // Element kinds understood by the launchers (values are part of the C ABI).
+// Added to the dtype of an entry point that reads parameters (weights, gains, ...): no kernel in flight on the stream writes them,
+// so they may be fetched before the kernels in front of this one are over. Kernels of a dependent-launch chain start under one
+// another several deep, so "in flight" is more than the launch just before. Without it everything is read behind the wait.
+constexpr int kSettled = 0x100;
+inline bool take_settled(int& dtype) {
+  const bool settled = (dtype & kSettled) != 0;
+  dtype &= ~kSettled;
+  return settled;
+}
+
 enum DType : int { kBF16 = 0, kF16 = 1, kF32 = 2, kE4M3 = 3, kU8 = 4, kI32 = 5 };
 inline int dtype_size(int dt) {
   switch (dt) {

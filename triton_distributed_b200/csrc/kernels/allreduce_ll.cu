@@ -38,6 +38,7 @@ struct ArLLParams {
   const uint32_t* gamma;       // [hidden / 2]
   uint32_t* normed_out;        // [rows, hidden / 2]
   float eps;
+  bool settled;                // gamma may be read before the kernels in front are over
 };
 
 __device__ __forceinline__ float2 ll_unpack(uint32_t w, bool bf16) { return bf16 ? unpack_bf16x2(w) : unpack_f16x2(w); }
@@ -50,8 +51,8 @@ __global__ void __launch_bounds__(kLLThreads) allreduce_ll_kernel(const ArLLPara
   const int row_words = p.hidden / 2;
   const bool bf16 = p.bf16 != 0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // the gain is a weight (never an output of the kernel launched just before this one): fetched before the dependency
-  // wait, past L1, so that it costs no round trip after the sum
+  // a settled gain is fetched before the dependency wait, so that it costs no round trip after the sum; past L1
+  if (!p.settled) griddep_wait();
   uint32_t gw[kLLWordsPerThread];
 #pragma unroll
   for (int u = 0; u < kLLWordsPerThread; ++u) {
@@ -201,6 +202,7 @@ B200_API int b200_allreduce_ll(const void* symm_ctx, const void* in, int rows, i
                                void* normed_out, float eps, int use_multimem, void* stream) {
   SymmCtx ctx;
   memcpy(&ctx, symm_ctx, sizeof(ctx));
+  const bool settled = take_settled(dtype);
   B200_REQUIRE(dtype == kBF16 || dtype == kF16, "the LL all-reduce handles bf16 and f16");
   B200_REQUIRE(rows >= 1 && hidden >= 2 && hidden % 2 == 0, "bad shape %d x %d", rows, hidden);
   B200_REQUIRE(hidden / 2 <= kLLThreads * kLLWordsPerThread, "hidden (%d) exceeds %d", hidden, 2 * kLLThreads * kLLWordsPerThread);
@@ -219,6 +221,7 @@ B200_API int b200_allreduce_ll(const void* symm_ctx, const void* in, int rows, i
   p.gamma = static_cast<const uint32_t*>(gamma);
   p.normed_out = static_cast<uint32_t*>(normed_out);
   p.eps = eps;
+  p.settled = settled;
   int grid = rows < sm_count() ? rows : sm_count();
   if (grid > kLLMaxCtas) grid = kLLMaxCtas;
   B200_CHECK_CUDA(launch_pdl(allreduce_ll_kernel, dim3(grid), dim3(kLLThreads), 0, static_cast<cudaStream_t>(stream), p, ctx));

@@ -38,12 +38,12 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 template <bool BF16>
 __global__ void __launch_bounds__(512) rmsnorm_kernel(const uint4* __restrict__ x, const uint4* residual_in,
                                                       uint4* residual_out, const uint4* __restrict__ gamma,
-                                                      uint4* __restrict__ y, int rows, int hidden, float eps) {
+                                                      uint4* __restrict__ y, int rows, int hidden, float eps, bool settled) {
   __shared__ float red[32];
   const int nv = hidden / 8;
   griddep_launch_dependents();
-  // the gain is a weight (not an output of the kernel launched just before this one): it is fetched before the
-  // dependency wait, past L1, and stays in registers for every row
+  // a settled gain is fetched before the dependency wait; past L1, and it stays in registers for every row
+  if (!settled) griddep_wait();
   uint4 gv[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kernel(const uint2* __restri
                                                            const int64_t* __restrict__ slots, const uint2* q_gamma,
                                                            const uint2* k_gamma, const float* __restrict__ cos_sin,
                                                            uint2* __restrict__ q_out, uint2* k_cache, uint2* v_cache,
-                                                           int T, int Hq, int Hkv, float eps) {
+                                                           int T, int Hq, int Hkv, float eps, bool settled) {
   const int heads = Hq + 2 * Hkv;
   griddep_launch_dependents();
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -128,7 +128,8 @@ __global__ void __launch_bounds__(256) qk_norm_rope_kernel(const uint2* __restri
   const int t = warp_global / heads;
   const int h = warp_global - t * heads;
   const uint2* gamma = h < Hq ? q_gamma : k_gamma;
-  // the gains are weights (not outputs of the kernel launched just before this one): fetched before the wait, past L1
+  // settled gains are fetched before the wait; past L1
+  if (!settled) griddep_wait();
   const uint2 g = (gamma != nullptr && warp_global < T * heads && h < Hq + Hkv) ? __ldcg(gamma + lane) : make_uint2(0, 0);
   griddep_wait();
   if (warp_global >= T * heads) return;
@@ -439,6 +440,7 @@ B200_API int b200_embedding(const long long* ids, const void* table, void* out, 
 
 B200_API int b200_rmsnorm(const void* x, const void* residual_in, void* residual_out, const void* gamma, void* y,
                           int rows, int hidden, float eps, int dtype, void* stream) {
+  const bool settled = take_settled(dtype);
   B200_REQUIRE(dtype == kBF16 || dtype == kF16, "rmsnorm supports bf16/f16");
   B200_REQUIRE(hidden % 8 == 0 && hidden <= 8 * 4 * 512, "hidden (%d) must be a multiple of 8 and <= 16384", hidden);
   if (rows == 0) return kOk;
@@ -450,11 +452,11 @@ B200_API int b200_rmsnorm(const void* x, const void* residual_in, void* residual
   if (dtype == kBF16)
     B200_CHECK_CUDA(launch_pdl(rmsnorm_kernel<true>, grid, threads, 0, s, static_cast<const uint4*>(x),
                                static_cast<const uint4*>(residual_in), static_cast<uint4*>(residual_out),
-                               static_cast<const uint4*>(gamma), static_cast<uint4*>(y), rows, hidden, eps));
+                               static_cast<const uint4*>(gamma), static_cast<uint4*>(y), rows, hidden, eps, settled));
   else
     B200_CHECK_CUDA(launch_pdl(rmsnorm_kernel<false>, grid, threads, 0, s, static_cast<const uint4*>(x),
                                static_cast<const uint4*>(residual_in), static_cast<uint4*>(residual_out),
-                               static_cast<const uint4*>(gamma), static_cast<uint4*>(y), rows, hidden, eps));
+                               static_cast<const uint4*>(gamma), static_cast<uint4*>(y), rows, hidden, eps, settled));
   B200_CHECK_CUDA(cudaGetLastError());
   return kOk;
 }
@@ -462,6 +464,7 @@ B200_API int b200_rmsnorm(const void* x, const void* residual_in, void* residual
 B200_API int b200_qk_norm_rope(const void* qkv, const int* positions, const int64_t* slots, const void* q_gamma,
                                const void* k_gamma, const float* cos_sin, void* q_out, void* k_cache, void* v_cache,
                                int T, int Hq, int Hkv, int head_dim, float eps, int dtype, void* stream) {
+  const bool settled = take_settled(dtype);
   B200_REQUIRE(dtype == kBF16 || dtype == kF16, "qk_norm_rope supports bf16/f16");
   B200_REQUIRE(head_dim == 128, "qk_norm_rope is specialised for head_dim 128, got %d", head_dim);
   if (T == 0) return kOk;
@@ -472,12 +475,12 @@ B200_API int b200_qk_norm_rope(const void* qkv, const int* positions, const int6
     B200_CHECK_CUDA(launch_pdl(qk_norm_rope_kernel<true>, grid, 256, 0, s, static_cast<const uint2*>(qkv), positions, slots,
                                static_cast<const uint2*>(q_gamma), static_cast<const uint2*>(k_gamma), cos_sin,
                                static_cast<uint2*>(q_out), static_cast<uint2*>(k_cache), static_cast<uint2*>(v_cache), T, Hq,
-                               Hkv, eps));
+                               Hkv, eps, settled));
   else
     B200_CHECK_CUDA(launch_pdl(qk_norm_rope_kernel<false>, grid, 256, 0, s, static_cast<const uint2*>(qkv), positions, slots,
                                static_cast<const uint2*>(q_gamma), static_cast<const uint2*>(k_gamma), cos_sin,
                                static_cast<uint2*>(q_out), static_cast<uint2*>(k_cache), static_cast<uint2*>(v_cache), T, Hq,
-                               Hkv, eps));
+                               Hkv, eps, settled));
   B200_CHECK_CUDA(cudaGetLastError());
   return kOk;
 }

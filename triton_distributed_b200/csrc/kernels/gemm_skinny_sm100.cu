@@ -78,6 +78,7 @@ struct SkinnyParams {
   int units_total;    // tiles * num_kb
   int units_per_cta;  // contiguous (tile, k-block) units owned by one CTA
   int up_row0;        // dual: first row of the `up` projection inside W
+  int settled;        // W may be read before the kernels in front are over
   int bf16;
   void* C;
   int ldc;
@@ -284,9 +285,13 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 0) {
     if (elect_one()) {
-      // Weight producer. The weights do not depend on the previous kernel, so this thread never waits for it: it
+      // Weight producer. Settled weights do not depend on any kernel in flight, so this thread never waits for one: it
       // arms each stage's barrier for the whole stage (weights + activations), requests the weight tiles and
       // publishes how many k-blocks are armed. The activation tiles are requested by the thread below.
+      if (!p.settled) {
+        griddep_wait();
+        fence_proxy_async();
+      }
       uint32_t stage = 0, phase = 0, armed = 0;
       int u = u_begin;
       Segment sg;
@@ -542,12 +547,14 @@ B200_API long long b200_gemm_skinny_scratch_floats(int M, int N, int dual) {
 // X [M, K] (row pitch ldx), W [Nw, K] (row pitch ldw), C [M, N] (row pitch ldc).
 // dual == 0: N = Nw. dual == 1: W = [gate (N rows); up (N rows)], C = silu(X gate^T) * (X up^T).
 // scratch / tickets: zero-initialised once by the caller; every call leaves them zeroed.
+// dtype + kSettled (here and below): no kernel in flight writes W, which is then streamed from the start.
 // splits <= 0: one CTA per SM (stream-K); splits > 0 forces tiles * splits CTAs.
 static unsigned long long* g_skinny_trace = nullptr;
 
 static int skinny_impl(const void* X, const void* W, void* C, int M, int N, int K, int ldx, int ldw, int ldc, int dual,
                        int dtype, float* scratch, uint32_t* tickets, int splits, const SkinnyEpilogue* ep, void* stream,
                        int groups = 1, const int* group_tiles = nullptr) {
+  const bool settled = take_settled(dtype);
   B200_REQUIRE(dtype == kBF16 || dtype == kF16, "gemm_skinny supports bf16/f16");
   B200_REQUIRE(M >= 1 && M <= 256, "gemm_skinny handles 1..256 tokens, got %d", M);
   B200_REQUIRE(K % 8 == 0, "K (%d) must be a multiple of 8", K);
@@ -563,6 +570,7 @@ static int skinny_impl(const void* X, const void* W, void* C, int M, int N, int 
   if (p.stages < 2) p.stages = kSkSmemBudget / p.stage_bytes < 2 ? 0 : 2;
   B200_REQUIRE(p.stages >= 2, "tile does not fit in shared memory");
   p.up_row0 = N;
+  p.settled = settled;
   p.bf16 = dtype == kBF16;
   p.C = C; p.ldc = ldc; p.scratch = scratch; p.tickets = tickets;
   p.trace = g_skinny_trace;

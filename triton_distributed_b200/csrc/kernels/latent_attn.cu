@@ -78,6 +78,7 @@ struct HeadLinearParams {
   void* y;          // y[t * ldy + h * yh + n]
   int T, H, N, K;
   long long ldx, xh, ldy, yh;
+  bool settled;     // w may be read before the kernels in front are over
 };
 
 enum HeadLinearAct : int { kActNone = 0, kActTanh = 1 };   // applied to x on its way into the product
@@ -112,11 +113,12 @@ __global__ void __launch_bounds__(256) head_linear_kernel(const HeadLinearParams
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int k = kc + 32 * i + 8 * tq;
-      w0[i] = (k < k_end && n0 + g < p.N) ? ld_v4_nc(w + static_cast<size_t>(n0 + g) * p.K + k) : zero;
-      w1[i] = (k < k_end && n0 + g + 8 < p.N) ? ld_v4_nc(w + static_cast<size_t>(n0 + g + 8) * p.K + k) : zero;
+      w0[i] = (k < k_end && n0 + g < p.N) ? __ldcg(reinterpret_cast<const uint4*>(w + static_cast<size_t>(n0 + g) * p.K + k)) : zero;
+      w1[i] = (k < k_end && n0 + g + 8 < p.N) ? __ldcg(reinterpret_cast<const uint4*>(w + static_cast<size_t>(n0 + g + 8) * p.K + k)) : zero;
     }
   };
-  load_w(k_begin);  // weights: read before the dependency wait
+  if (!p.settled) griddep_wait();
+  load_w(k_begin);
   griddep_wait();
   float acc[kHlTok][4] = {};
   for (int kc = k_begin; kc < k_end; kc += 128) {
@@ -202,11 +204,12 @@ struct LatentParams {
 // value: the merged row is scaled by exp(lse) / (exp(lse) + exp(sink)).
 template <typename T>
 __global__ void __launch_bounds__(128) latent_combine_kernel(const float* o_part, const float* lse_part, const float* sink, int H,
-                                                             int splits, int pitch, T* out) {
+                                                             int splits, int pitch, T* out, bool settled) {
   const size_t row = blockIdx.y;
   const int c = blockIdx.x * 128 + threadIdx.x;
   griddep_launch_dependents();
-  const float sk = sink != nullptr ? __ldg(sink + row % H) : -CUDART_INF_F;
+  if (!settled) griddep_wait();
+  const float sk = sink != nullptr ? __ldcg(sink + row % H) : -CUDART_INF_F;
   griddep_wait();
   if (c >= pitch) return;
   float o, lse;
@@ -310,13 +313,14 @@ static int launch_head_linear(const HeadLinearParams& p, int dtype, cudaStream_t
 }
 
 // y[t * ldy + h * yh + n] = sum_k W[h, n, k] act(x[t * ldx + h * xh + k]), act 0 = none, 1 = tanh. 16-bit: K, strides in
-// multiples of 8 elements.
+// multiples of 8 elements. dtype + kSettled: no kernel in flight writes W.
 B200_API int b200_head_linear(const void* x, const void* w, void* y, int T, int H, int N, int K, long long ldx, long long xh,
                               long long ldy, long long yh, int act, int dtype, void* stream) {
   if (T <= 0) return kOk;
   B200_REQUIRE(H >= 1 && N >= 1 && K >= 1 && H <= 65535, "bad head_linear shape");
   B200_REQUIRE(act == kActNone || act == kActTanh, "head_linear: unknown activation %d", act);
-  const HeadLinearParams p{x, w, y, T, H, N, K, ldx, xh, ldy, yh};
+  const bool settled = take_settled(dtype);
+  const HeadLinearParams p{x, w, y, T, H, N, K, ldx, xh, ldy, yh, settled};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   return act == kActTanh ? launch_head_linear<kActTanh>(p, dtype, s) : launch_head_linear<kActNone>(p, dtype, s);
 }
@@ -332,13 +336,15 @@ static int fill_latent(LatentParams& p, const void* q, const void* cache, const 
 }
 
 // Merges partial results o_part fp32 [rows, splits, pitch] with log-sum-exps lse_part fp32 [rows, splits]; row % H is the head.
+// dtype + kSettled: no kernel in flight writes the sink.
 B200_API int b200_latent_combine(const float* o_part, const float* lse_part, const float* sink, int rows, int H, int splits, int pitch,
                                  void* out, int dtype, void* stream) {
   if (rows <= 0) return kOk;
+  const bool settled = take_settled(dtype);
   B200_REQUIRE(rows <= 65535, "latent_combine: too many rows (%d)", rows);
   const dim3 grid((pitch + 127) / 128, rows);
   B200_DISPATCH_FLOAT(dtype, B200_CHECK_CUDA(launch_pdl(latent_combine_kernel<T>, grid, dim3(128), 0, static_cast<cudaStream_t>(stream),
-                                                        o_part, lse_part, sink, H, splits, pitch, static_cast<T*>(out)));
+                                                        o_part, lse_part, sink, H, splits, pitch, static_cast<T*>(out), settled));
                       return kOk;);
 }
 

@@ -482,11 +482,12 @@ B200_API int b200_latent_combine(const float* o_part, const float* lse_part, con
                                  void* out, int dtype, void* stream);
 
 // Both launches of a call: part fp32 [B * S * H * splits * (pitch + 1)] holds the partial results, then their log-sum-exps.
+// dtype + kSettled: no kernel in flight writes the sink.
 B200_API int b200_latent_attention(const void* q, const void* cache, long long num_slots, const int* block_table, int bt_stride,
                                    const int* kv_lens, int B, int S, int H, int pitch, int page, float scale, int splits,
                                    int rows_per_cta, float* part, const float* sink, void* out, int dtype, uint32_t* status, void* stream) {
   float* lse = part + static_cast<size_t>(B) * S * H * splits * pitch;
   const int rc = b200_latent_decode(q, cache, num_slots, block_table, bt_stride, kv_lens, B, S, H, pitch, page, scale, splits, rows_per_cta,
-                                    part, lse, dtype, status, stream);
+                                    part, lse, dtype & ~kSettled, status, stream);
   return rc != kOk ? rc : b200_latent_combine(part, lse, sink, B * S * H, H, splits, pitch, out, dtype, stream);
 }

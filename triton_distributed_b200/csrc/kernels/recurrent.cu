@@ -37,6 +37,7 @@ struct TokenMixParams {
   void* last;        // [B, pitch] the previous token of every sequence, updated
   void* out;         // [B * S, G, pitch]
   int S, G, pitch;
+  bool settled;      // mu may be read before the kernels in front are over
 };
 
 // grid (column blocks, token blocks, B). The thread of the first token block alone reads and replaces the carried row.
@@ -47,6 +48,7 @@ __global__ void __launch_bounds__(128) token_mix_kernel(const TokenMixParams p) 
   griddep_launch_dependents();
   if (c >= p.pitch) return;
   float4 mu[G];
+  if (!p.settled) griddep_wait();
 #pragma unroll
   for (int g = 0; g < G; ++g) mu[g] = load4(static_cast<const T*>(p.mu) + static_cast<size_t>(g) * p.pitch + c);
   griddep_wait();
@@ -91,6 +93,7 @@ struct ShortConvParams {
   void* last;         // [B, n - 1, C] the previous inputs of every sequence, oldest first, updated
   void* out;          // [B * S, C]
   int S, C, n, ldx;
+  bool settled;       // the taps may be read before the kernels in front are over
 };
 
 // grid (channel blocks, token blocks, B), four channels per thread. kN > 0: that many taps, kept in registers.
@@ -102,6 +105,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const ShortConvParams p
   if (c >= p.C) return;
   const int n = kN > 0 ? kN : p.n;
   float4 w[kN > 0 ? kN : 1];
+  if (!p.settled) griddep_wait();
   if (kN > 0) {
 #pragma unroll
     for (int j = 0; j < (kN > 0 ? kN : 0); ++j) w[j] = load4(p.taps + static_cast<size_t>(j) * p.C + c);
@@ -156,6 +160,7 @@ struct RecurrentParams {
   int S, H, per;                  // tokens per sequence, heads, heads per q / k head
   int D, E, Dp, Ep;               // key and value sizes of a head, and padded to multiples of 8
   float eps;
+  bool settled;                   // the per-channel constants may be read before the kernels in front are over
 };
 
 __device__ __forceinline__ float softplus(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
@@ -260,6 +265,7 @@ __global__ void __launch_bounds__(2 * kP, kP == 128 ? 2 : 4) recurrent_kernel(co
   // the state comes from an earlier call: it may be fetched into L2, but not read, before that call is known to be over
   for (int i = threadIdx.x * 32; i < p.Dp * p.Ep; i += kThreads * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(state + i));
   const int ic = threadIdx.x % (kP / 8) * 8, it = threadIdx.x / (kP / 8);   // this thread's eight elements of a chunk
+  if (!p.settled) griddep_wait();
   if (threadIdx.x < kP) s_gain[threadIdx.x] = threadIdx.x < p.Ep ? p.gain[h * p.gain_stride + threadIdx.x] : 0.f;
   if (kKind == kWkv && threadIdx.x < kP) {
     const bool in = threadIdx.x < p.Dp;
@@ -611,6 +617,7 @@ __global__ void __launch_bounds__(2 * kP) recurrent_step_kernel(const RecurrentP
   griddep_launch_dependents();
   // the state comes from an earlier call: it may be fetched into L2, but not read, before that call is known to be over
   for (int i = threadIdx.x * 32; i < p.Dp * p.Ep; i += kThreads * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(state + i));
+  if (!p.settled) griddep_wait();
   const float base = kKind == kWkv && ch < p.Dp ? p.decay_base[h * p.Dp + ch] : 0.f, bonus = kKind == kWkv && ch < p.Dp ? p.bonus[h * p.Dp + ch] : 0.f;
   const float gain = ch < p.Ep ? p.gain[h * p.gain_stride + ch] : 0.f;
   griddep_wait();
@@ -831,7 +838,7 @@ using namespace b200;
 B200_API int b200_token_mix(const void* h, const void* mu, void* last, void* out, int B, int S, int G, int pitch, int dtype, void* stream) {
   if (B <= 0 || S <= 0) return kOk;
   B200_REQUIRE(G >= 1 && G <= kMixMax && pitch % 4 == 0 && B <= 65535, "token_mix: 1..%d mixes and a pitch in multiples of 4", kMixMax);
-  const TokenMixParams p{h, mu, last, out, S, G, pitch};
+  const TokenMixParams p{h, mu, last, out, S, G, pitch, take_settled(dtype)};
   const dim3 grid((pitch / 4 + 127) / 128, (S + kMixTokens - 1) / kMixTokens, B);
   B200_REQUIRE(grid.y <= 65535, "token_mix: too many tokens");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -857,7 +864,7 @@ B200_API int b200_short_conv(const void* x, const float* taps, void* last, void*
                              void* stream) {
   if (B <= 0 || S <= 0) return kOk;
   B200_REQUIRE(n >= 1 && C % 4 == 0 && ldx % 4 == 0 && B <= 65535, "short_conv: channels (%d) and pitch (%d) must be multiples of 4", C, ldx);
-  const ShortConvParams p{x, taps, last, out, S, C, n, ldx};
+  const ShortConvParams p{x, taps, last, out, S, C, n, ldx, take_settled(dtype)};
   const dim3 grid((C / 4 + 127) / 128, (S + kConvTokens - 1) / kConvTokens, B);
   B200_REQUIRE(grid.y <= 65535, "short_conv: too many tokens");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -878,6 +885,7 @@ B200_API int b200_wkv(const void* r, int ldr, const void* k, int ldk, const void
   memset(&p, 0, sizeof(p));
   p.q = r; p.ldq = ldr; p.k = k; p.ldk = ldk; p.v = v; p.ldv = ldv; p.decay = z; p.ld_decay = ldz; p.gate = gate; p.ldg = ldg;
   p.decay_base = w0; p.bonus = u; p.gain = gain; p.gain_stride = Ep; p.eps = eps; p.state = state; p.out = out;
+  p.settled = take_settled(dtype);
   p.S = S; p.H = H; p.per = 1; p.D = D; p.Dp = Dp; p.E = E; p.Ep = Ep;
   return run_recurrent<kWkv>(p, B, H, plain, dtype, stream);
 }
@@ -892,6 +900,7 @@ B200_API int b200_gated_delta(const void* q, int ldq, const void* k, int ldk, co
   B200_REQUIRE(G >= 1, "gated_delta needs at least one key head");
   p.q = q; p.ldq = ldq; p.k = k; p.ldk = ldk; p.v = v; p.ldv = ldv; p.decay = a; p.beta = b; p.ld_decay = lda; p.gate = gate; p.ldg = ldg;
   p.decay_base = A; p.decay_bias = dt; p.gain = gain; p.gain_stride = 0; p.eps = eps; p.state = state; p.out = out;
+  p.settled = take_settled(dtype);
   p.S = S; p.H = H; p.per = H / G; p.D = D; p.Dp = Dp; p.E = E; p.Ep = Ep;
   return run_recurrent<kDelta>(p, B, G, plain, dtype, stream);
 }

@@ -34,6 +34,7 @@ struct NormParams {
   const void* gain;   // [pitch] (not read by kNormCopy)
   const void* bias;   // [pitch] or null
   void* h;            // [T, pitch]; null: no norm
+  bool settled;       // gain and bias may be read before the kernels in front are over
 };
 
 struct ResidualParams {
@@ -175,7 +176,7 @@ __device__ __forceinline__ void norm_row(const NormParams& n, const Slice<kCl>& 
   }
 }
 
-// the gain and bias are weights: read before the dependency wait
+// with settled gains and biases the call stands before the dependency wait
 template <typename T, int U, int kCl>
 __device__ __forceinline__ void load_norm_weights(const NormParams& n, const Slice<kCl>& sl, float4 (&gain)[U], float4 (&bias)[U]) {
 #pragma unroll
@@ -198,6 +199,7 @@ __global__ void __launch_bounds__(kRnThreads) embed_norm_kernel(const EmbedParam
   const Slice<kCl> sl(pitch);
   griddep_launch_dependents();
   float4 gain[U], bias[U], v[U];
+  if (!p.norm.settled) griddep_wait();
   load_norm_weights<T, U, kCl>(p.norm, sl, gain, bias);
   if (kCl > 1) cluster_sync_all();  // every CTA of the cluster runs before any writes to another's shared memory
   griddep_wait();
@@ -242,6 +244,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_norm_kernel(const Residua
   const Slice<kCl> sl(pitch);
   griddep_launch_dependents();
   float4 gain[U], bias[U], x[U];
+  if (!p.norm.settled) griddep_wait();
   load_norm_weights<T, U, kCl>(p.norm, sl, gain, bias);
   if (kCl > 1) cluster_sync_all();  // every CTA of the cluster runs before any writes to another's shared memory
   griddep_wait();
@@ -323,6 +326,7 @@ __global__ void __launch_bounds__(kRnThreads) residual_post_kernel(const PostPar
   const Slice<kCl> sl(pitch);
   griddep_launch_dependents();
   float4 gain[U], bias[U], a[U], b[U], x[U];
+  if (!p.norm.settled) griddep_wait();
   load_norm_weights<T, U, kCl>(p.norm, sl, gain, bias);
   if (kCl > 1) cluster_sync_all();  // every CTA of the cluster runs before any writes to another's shared memory
   griddep_wait();
@@ -430,7 +434,7 @@ B200_API int b200_embed_norm(const long long* ids, const void* table, int rows, 
   EmbedParams p;
   memset(&p, 0, sizeof(p));
   p.ids = ids; p.table = table; p.V = V; p.scale = scale; p.x = x; p.state0 = state0;
-  p.norm = NormParams{width, pitch, kind, eps, gain, bias, h};
+  p.norm = NormParams{width, pitch, kind, eps, gain, bias, h, take_settled(dtype)};
   int rc = check_norm(p.norm);
   if (rc != kOk) return rc;
   B200_DISPATCH_FLOAT(dtype, B200_ROW_KERNELS(embed_norm_kernel, EmbedParams););
@@ -450,7 +454,7 @@ B200_API int b200_residual_norm(const void* a, const void* gate_a, const void* b
   memset(&p, 0, sizeof(p));
   p.a = a; p.b = b; p.gate_a = gate_a; p.gate_b = gate_b; p.bias_a = bias_a; p.bias_b = bias_b; p.ldg = ldg; p.mult = mult;
   p.x = x; p.states = states; p.state_stride = state_stride; p.weights = weights; p.n_prev = n_prev; p.keep = keep;
-  p.norm = NormParams{width, pitch, kind, eps, gain, bias, h};
+  p.norm = NormParams{width, pitch, kind, eps, gain, bias, h, take_settled(dtype)};
   int rc = check_norm(p.norm);
   if (rc != kOk) return rc;
   B200_DISPATCH_FLOAT(dtype, B200_ROW_KERNELS(residual_norm_kernel, ResidualParams););
@@ -466,7 +470,7 @@ B200_API int b200_residual_post(const void* a, const void* gain_a, const void* b
   PostParams p;
   memset(&p, 0, sizeof(p));
   p.a = a; p.b = b; p.gain_a = gain_a; p.gain_b = gain_b; p.eps = post_eps; p.mult = mult; p.x = x;
-  p.norm = NormParams{width, pitch, kind, eps, gain, bias, h};
+  p.norm = NormParams{width, pitch, kind, eps, gain, bias, h, take_settled(dtype)};
   int rc = check_norm(p.norm);
   if (rc != kOk) return rc;
   B200_DISPATCH_FLOAT(dtype, B200_ROW_KERNELS(residual_post_kernel, PostParams););

@@ -166,10 +166,11 @@ def all_reduce(x: torch.Tensor, output: torch.Tensor | None = None, method: AllR
 def all_reduce_rmsnorm(x: torch.Tensor, residual: torch.Tensor | None, gamma: torch.Tensor, eps: float,
                        ctx: AllReduceContext, method: AllReduceMethod | None = None,
                        normed_out: torch.Tensor | None = None, residual_out: torch.Tensor | None = None,
-                       max_sm: int = -1):
+                       max_sm: int = -1, settled: bool = False):
     """Fused ``h = all_reduce(x) + residual; y = rmsnorm(h) * gamma``. x: [rows, hidden].
 
     Returns (y, h). `residual_out` defaults to `residual` (in place) when a residual is given.
+    ``settled``: no kernel in flight on the stream writes gamma, which may then be fetched early (see ``ops.linear``).
     """
     rows, hidden = x.shape
     es = x.element_size()
@@ -180,7 +181,7 @@ def all_reduce_rmsnorm(x: torch.Tensor, residual: torch.Tensor | None, gamma: to
             normed_out = torch.empty_like(x)
         if residual_out is None:
             residual_out = residual if residual is not None else torch.empty_like(x)
-        _lib.call("b200_allreduce_ll", ctx.heap.ctx, ptr(x), rows, hidden, dtype_code(x.dtype), ptr(ctx.ll_ws[0]),
+        _lib.call("b200_allreduce_ll", ctx.heap.ctx, ptr(x), rows, hidden, dtype_code(x.dtype, settled), ptr(ctx.ll_ws[0]),
                   ptr(ctx.ll_ws[1]), ptr(ctx.ll_sync), ptr(residual), ptr(residual_out), ptr(gamma), ptr(normed_out),
                   c_float(eps), 1 if (_AR_LL_MC and ctx.heap.has_multicast) else 0, stream_ptr())
         ops._count()

@@ -92,4 +92,4 @@ class GatedAttention:
                                       step["cu_k"], S, step["kv_len"], 1.0, True, seqlens_k=step["kv_lens"], gate=gate)
         else:
             o = ops.gqa_attention_plain(q, kp, vp, step["kv_lens"], cache.block_table, S, 1.0, gate=gate)
-        return ops.linear(o.view(B * S, -1), self.wo, out=out)
+        return ops.linear(o.view(B * S, -1), self.wo, out=out, settled=True)

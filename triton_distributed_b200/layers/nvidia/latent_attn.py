@@ -90,17 +90,17 @@ class LatentAttention:
 
     def _attend_absorbed(self, q3, kv_cache, layer_idx, step):
         cache = kv_cache.layer(layer_idx)
-        qc = ops.head_linear(q3, self.uk_t)
+        qc = ops.head_linear(q3, self.uk_t, settled=True)
         splits, rows = ops.choose_latent_splits(step["bsz"], step["seqlen"] * self.heads, step["kv_len"] or kv_cache.max_length)
-        ctx = ops.latent_attention(qc, cache, step["kv_lens"], kv_cache.block_table, step["seqlen"], self.scale, self.sink, splits, rows)
-        return ops.head_linear(ctx, self.uv.view(self.heads, self.vdim, self.pitch))
+        ctx = ops.latent_attention(qc, cache, step["kv_lens"], kv_cache.block_table, step["seqlen"], self.scale, self.sink, splits, rows, settled=True)
+        return ops.head_linear(ctx, self.uv.view(self.heads, self.vdim, self.pitch), settled=True)
 
     def _attend_expanded(self, q3, kv_cache, layer_idx, step):
         B, S, kv = step["bsz"], step["seqlen"], step["kv_len"]
         kv8 = pad_up(kv)
         kv_cache.blank(layer_idx, kv, kv8)  # the rows in between are unused slots: masked, and must be finite
         c = kv_cache.rows(layer_idx, kv8)   # [B * kv8, pitch]
-        k = ops.linear(c, self.uk)
+        k = ops.linear(c, self.uk, settled=True)
         vt = ops.linear(self.uv, c)         # values already transposed: [heads * vdim, B * kv8]
         if "cu_q" not in step:  # the same for every layer of the step
             step["cu_q"] = torch.arange(0, (B + 1) * S, S, dtype=torch.int32, device=q3.device)
@@ -111,7 +111,7 @@ class LatentAttention:
     @torch.no_grad()
     def partial_fwd(self, q, kv_cache, layer_idx: int, step, out: torch.Tensor | None = None) -> torch.Tensor:
         """Attention and output projection without the reduction over ranks."""
-        return ops.linear(self.attend(q, kv_cache, layer_idx, step), self.wo, out=out)
+        return ops.linear(self.attend(q, kv_cache, layer_idx, step), self.wo, out=out, settled=True)
 
 
 __all__ = ["LatentAttention", "pad_heads", "pad_matrix", "pad_up", "pad_vector", "shard_local"]

@@ -52,13 +52,13 @@ class WkvMixer:
     @torch.no_grad()
     def partial_fwd(self, h: torch.Tensor, cache: HybridCache, layer_idx: int, out: torch.Tensor) -> torch.Tensor:
         """h [B * S, width] -> this rank's partial sum in `out`."""
-        mixes = ops.token_mix(h, self.mu, cache.state(layer_idx, "last"))
-        r, k, v, gate, low = ops.linear_groups(mixes, self.w_in, self.rows).split(self.rows, dim=1)
+        mixes = ops.token_mix(h, self.mu, cache.state(layer_idx, "last"), settled=True)
+        r, k, v, gate, low = ops.linear_groups(mixes, self.w_in, self.rows, settled=True).split(self.rows, dim=1)
         N = self.heads * self.dim
-        z = ops.tanh_linear(low[:, : self.rank], self.w2)
+        z = ops.tanh_linear(low[:, : self.rank], self.w2, settled=True)
         o = ops.wkv(r[:, :N], k[:, :N], v[:, :N], z, gate[:, :N], self.w0, self.u, self.gain, cache.state(layer_idx, "memory"), self.spec.dim,
-                    self.spec.dim, self.eps)
-        return ops.linear(o, self.wo, out=out)
+                    self.spec.dim, self.eps, settled=True)
+        return ops.linear(o, self.wo, out=out, settled=True)
 
 
 class GatedDelta:
@@ -94,7 +94,7 @@ class GatedDelta:
     def partial_fwd(self, parts, cache: HybridCache, layer_idx: int, out: torch.Tensor) -> torch.Tensor:
         """`parts`: this block's slices of the fused projection; `out` receives this rank's partial sum."""
         qkv, b, a, gate = parts
-        q, k, v = ops.short_conv(qkv, self.taps, cache.state(layer_idx, "inputs")).split(self.sizes, dim=1)
+        q, k, v = ops.short_conv(qkv, self.taps, cache.state(layer_idx, "inputs"), settled=True).split(self.sizes, dim=1)
         o = ops.gated_delta(q, k, v, a[:, : self.heads], b[:, : self.heads], gate, self.a_log, self.dt_bias, self.gain,
-                            cache.state(layer_idx, "memory"), self.spec.dim, self.spec.vdim, self.eps)
-        return ops.linear(o, self.wo, out=out)
+                            cache.state(layer_idx, "memory"), self.spec.dim, self.spec.vdim, self.eps, settled=True)
+        return ops.linear(o, self.wo, out=out, settled=True)

@@ -28,7 +28,7 @@ from .tp_mlp import shard_local
 def layer_norm(hidden: torch.Tensor, eps: float, w: torch.Tensor) -> torch.Tensor:
     """RMSNorm (the reference names it layer_norm, tp_attn.py:60-66). Native on CUDA, torch on CPU."""
     if hidden.is_cuda:
-        return ops.rmsnorm(hidden, w, eps)
+        return ops.rmsnorm(hidden, w, eps, settled=True)
     hf = hidden.float()
     return (hf * torch.rsqrt(hf.pow(2).mean(-1, keepdim=True) + eps) * w.float()).to(hidden.dtype)
 
@@ -108,7 +108,7 @@ class TP_Attn:
             step = ops.step_tables(position_ids, kv_cache.blocks_per_seq * kv_cache.page_size)
         q = ops.qk_norm_rope(qkv, step["pos"], cos_sin_cache, self.q_heads_local, self.kv_heads_local,
                              kp.view(-1, self.kv_heads_local, self.head_dim), vp.view(-1, self.kv_heads_local, self.head_dim),
-                             step["slots"], self.q_norm_w, self.k_norm_w, self.eps)
+                             step["slots"], self.q_norm_w, self.k_norm_w, self.eps, settled=True)
         if seqlen == 1:
             splits = step.get("splits") or ops.choose_kv_splits(bsz, self.kv_heads_local, self.q_heads_local // self.kv_heads_local,
                                                                 kv_cache.max_length)
@@ -159,9 +159,9 @@ class TP_Attn:
     @torch.no_grad()
     def partial_fwd(self, x2, position_ids, cos_sin_cache, kv_cache, layer_idx, bsz, seqlen, step=None):
         """Native path without the final reduction: x2 [B*S, H] -> partial o_proj output [B*S, H]."""
-        qkv = ops.linear(x2, self.wqkv)
+        qkv = ops.linear(x2, self.wqkv, settled=True)
         o = self._attn_native(qkv, position_ids, cos_sin_cache, kv_cache, layer_idx, bsz, seqlen, step)
-        return ops.linear(o, self.wo)
+        return ops.linear(o, self.wo, settled=True)
 
     @torch.no_grad()
     def dist_triton_AR_fwd(self, x, position_ids, cos_sin_cache, kv_cache, layer_idx: int):

@@ -90,9 +90,9 @@ class TP_MLP:
         if x.dtype == torch.float32:
             return ops.linear(ops.silu_mul(ops.linear(x, self.gate_up_proj)), self.down_proj)
         if T <= 128:
-            act = ops.gemm_skinny(x, self.gate_up_proj, swiglu=True)
-            return ops.gemm_skinny(act, self.down_proj)
-        return ops.linear(ops.gemm_gated(x, self.gate_up_proj), self.down_proj)
+            act = ops.gemm_skinny(x, self.gate_up_proj, swiglu=True, settled=True)
+            return ops.gemm_skinny(act, self.down_proj, settled=True)
+        return ops.linear(ops.gemm_gated(x, self.gate_up_proj), self.down_proj, settled=True)
 
     @torch.no_grad()
     def dist_triton_AR_fwd(self, x: torch.Tensor) -> torch.Tensor:

@@ -90,7 +90,7 @@ class TP_MoE:
 
     def route(self, x: torch.Tensor):
         """Router on the native kernels: (ids int32 [T, topk], weights fp32 [T, topk])."""
-        logits = ops.linear(x, self.gate)
+        logits = ops.linear(x, self.gate, settled=True)
         return ops.topk_softmax(logits, self.topk, self.norm_topk_prob)
 
     @torch.no_grad()
@@ -186,7 +186,7 @@ class EP_MoE:
     @torch.no_grad()
     def dist_triton_fwd(self, x_local: torch.Tensor) -> torch.Tensor:
         """x_local [T_local, H] (this rank's tokens) -> [T_local, H]."""
-        ids, w = ops.topk_softmax(ops.linear(x_local, self.gate), self.topk, self.norm_topk_prob)
+        ids, w = ops.topk_softmax(ops.linear(x_local, self.gate, settled=True), self.topk, self.norm_topk_prob)
         res = self.a2a.dispatch(x_local, ids)
         if self.fp8_experts:
             from ...kernels.nvidia.grouped_gemm_fp8 import grouped_gemm_fp8_planned

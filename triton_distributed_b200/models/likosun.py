@@ -62,7 +62,7 @@ class LikosunLayer:
 
     def sublayers(self, h: torch.Tensor, kv_cache: LatentCache, step: dict):
         """h [T, P] -> (partial sums [2 or 1, T, P] of the sublayers, gate logits of the mixer, of the feed-forward or None)."""
-        proj = ops.linear(h, self.w_in)
+        proj = ops.linear(h, self.w_in, settled=True)
         parts = proj.split(self.splits, dim=1)
         q, latent, gate1 = parts[0], parts[1], parts[-1] if self.down is None else parts[-2]
         up, gate2 = (None, None) if self.down is None else (parts[2], parts[-1])
@@ -71,7 +71,7 @@ class LikosunLayer:
         out = torch.empty((1 if self.down is None else 2, *h.shape), dtype=h.dtype, device=h.device)
         self.attn.partial_fwd(q, kv_cache, self.layer_idx, step, out=out[0])
         if self.down is not None:
-            ops.linear(act, self.down, out=out[1])
+            ops.linear(act, self.down, out=out[1], settled=True)
         return out, gate1, gate2
 
 
@@ -161,7 +161,7 @@ class Likosun:
         states = torch.empty((max(self.num_layers, 1), T, self.pitch), dtype=torch.float32, device=self.device)
         first = self.layers[0]
         x, h = ops.embed_norm(input_ids, self.embed, a.embedding_scale, a.hidden_size, first.norm_w, first.norm_b, a.norm_eps, True,
-                              state0=states[0])
+                              state0=states[0], settled=True)
         for i, layer in enumerate(self.layers):
             out, gate1, gate2 = layer.sublayers(h, kv_cache, step)
             if self.world_size > 1:
@@ -171,7 +171,8 @@ class Likosun:
             gain, bias = (self.norm_w, self.norm_b) if last else (self.layers[i + 1].norm_w, self.layers[i + 1].norm_b)
             h = ops.residual_norm(x, a.hidden_size, a.residual_mult, out[0], gate1, layer.gate1_b,
                                   out[1] if gate2 is not None else None, gate2, layer.gate2_b, states=states,
-                                  weights=layer.depth_weights, keep=not last, gain=gain, bias=bias, eps=a.norm_eps, center=True)
+                                  weights=layer.depth_weights, keep=not last, gain=gain, bias=bias, eps=a.norm_eps, center=True,
+                                  settled=True)
             if self.layer_taps is not None:
                 self.layer_taps.append(x[:, : a.hidden_size].clone())
         hidden = h.view(bsz, S, self.pitch)
@@ -180,5 +181,5 @@ class Likosun:
     def lm_logits(self, hidden: torch.Tensor) -> torch.Tensor:
         """fp32 logits [B, n, V] of normed hidden states [B, n, P]. (The head is replicated over ranks.)"""
         rows = hidden.reshape(-1, self.pitch).contiguous()
-        logits = ops.linear(rows, self.head)[:, : self.arch.vocab_size]
+        logits = ops.linear(rows, self.head, settled=True)[:, : self.arch.vocab_size]
         return logits.float().view(*hidden.shape[:-1], -1)

@@ -231,9 +231,9 @@ class Qwen3:
     def _reduce_norm(self, partial, residual, gamma):
         """h = all_reduce(partial) + residual (in place); returns rmsnorm(h) * gamma."""
         if self.world_size > 1:
-            y, _ = all_reduce_rmsnorm(partial, residual, gamma, self.eps, self.ar_ctx, self.ar_method)
+            y, _ = all_reduce_rmsnorm(partial, residual, gamma, self.eps, self.ar_ctx, self.ar_method, settled=True)
             return y
-        return ops.rmsnorm(partial, gamma, self.eps, residual=residual)
+        return ops.rmsnorm(partial, gamma, self.eps, residual=residual, settled=True)
 
     @torch.no_grad()
     def _inference_AR(self, input_ids, position_ids, kv_cache, kv_len=None):
@@ -241,7 +241,7 @@ class Qwen3:
         bsz, seqlen = input_ids.shape
         step = ops.step_tables(position_ids, kv_cache.blocks_per_seq * kv_cache.page_size) | {"kv_len": kv_len}
         residual = ops.embedding(input_ids.reshape(-1), self.embed_tokens)  # [T, H], becomes the residual stream
-        x = ops.rmsnorm(residual, self.layers[0].input_norm_w, self.eps)
+        x = ops.rmsnorm(residual, self.layers[0].input_norm_w, self.eps, settled=True)
         for i, layer in enumerate(self.layers):
             part = layer.attn.partial_fwd(x, position_ids, self.cos_sin_cache, kv_cache, i, bsz, seqlen, step)
             x = self._reduce_norm(part, residual, layer.post_norm_w)
@@ -300,12 +300,12 @@ class Qwen3:
             # the head writes its vocabulary shard straight into this rank's slot of the symmetric gather buffer
             vloc = self.lm_head.shape[0]
             slot = self.logit_buf.view(-1)[: self.world_size * bsz * vloc].view(self.world_size, bsz, vloc)[self.rank]
-            ops.linear(last, self.lm_head, out=slot)
+            ops.linear(last, self.lm_head, out=slot, settled=True)
             gathered = self._gather_rows(self.logit_buf, bsz)
             local = gathered.permute(1, 0, 2).reshape(bsz, -1)
             return local[:, : self.arch.vocab_size].float().unsqueeze(1)
         else:
-            local = ops.linear(last, self.lm_head)
+            local = ops.linear(last, self.lm_head, settled=True)
         if self.world_size > 1:
             gathered = torch.empty((self.world_size, bsz, local.shape[-1]), dtype=local.dtype, device=local.device)
             dist.all_gather_into_tensor(gathered, local.contiguous(), group=self.group)

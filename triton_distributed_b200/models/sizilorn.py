@@ -96,7 +96,7 @@ class SizilornLayer:
         if not self.parallel:
             self.mixer.partial_fwd(h, cache, self.layer_idx, out[0])
             return out
-        parts = ops.linear(h, self.w_in).split(self.splits, dim=1)
+        parts = ops.linear(h, self.w_in, settled=True).split(self.splits, dim=1)
         self.left.partial_fwd(parts[: self.n_left], cache, self.layer_idx, step, out[0])
         self.right.partial_fwd(parts[self.n_left:], cache, self.layer_idx, out[1])
         return out
@@ -197,20 +197,20 @@ class Sizilorn:
         step = {"bsz": bsz, "seqlen": S, "kv_len": kv_len if S > 1 else None, "slots": kv_cache.slots(position_ids),
                 "positions": position_ids.reshape(-1).to(torch.int32), "kv_lens": (position_ids[:, -1] + 1).to(torch.int32)}
         first = self.layers[0].norm1
-        x, h = ops.embed_norm(ids, self.embed, 1.0, W, first.gain, first.bias, 0.0, first.kind)
+        x, h = ops.embed_norm(ids, self.embed, 1.0, W, first.gain, first.bias, 0.0, first.kind, settled=True)
         for i, layer in enumerate(self.layers):
             out = self._reduced(layer.mix(h, kv_cache, step))
             then = layer.norm2.kw if layer.mlp is not None else {"center": ops.COPY}
             if layer.parallel:
-                h = ops.residual_post(x, W, 0.5, out[0], layer.left_gain, out[1], layer.right_gain, a.norm_eps, **then)
+                h = ops.residual_post(x, W, 0.5, out[0], layer.left_gain, out[1], layer.right_gain, a.norm_eps, **then, settled=True)
             else:
-                h = ops.residual_norm(x, W, 1.0, out[0], **then)
+                h = ops.residual_norm(x, W, 1.0, out[0], **then, settled=True)
             if layer.mlp is not None:
                 h = ops.residual_norm(x, W, 1.0, self._reduced(layer.mlp.partial_fwd(h)), center=ops.COPY)
-            act = ops.token_side(ops.linear(h, layer.side_gate), ids, self.side_embed, i * a.side_dim, a.side_dim)
-            y = ops.linear(act, layer.side_proj)
+            act = ops.token_side(ops.linear(h, layer.side_gate, settled=True), ids, self.side_embed, i * a.side_dim, a.side_dim)
+            y = ops.linear(act, layer.side_proj, settled=True)
             norm = self.final_norm if i + 1 == self.num_layers else self.layers[i + 1].norm1
-            h = ops.residual_post(x, W, 1.0, y, layer.side_gain, post_eps=a.norm_eps, **norm.kw)
+            h = ops.residual_post(x, W, 1.0, y, layer.side_gain, post_eps=a.norm_eps, **norm.kw, settled=True)
             if self.layer_taps is not None:
                 self.layer_taps.append(x[:, :W].clone())
         hidden = h.view(bsz, S, self.pitch)
@@ -219,5 +219,5 @@ class Sizilorn:
     def lm_logits(self, hidden: torch.Tensor) -> torch.Tensor:
         """fp32 logits [B, n, V] of normed hidden states [B, n, P]. (The head is replicated over ranks.)"""
         rows = hidden.reshape(-1, self.pitch).contiguous()
-        logits = ops.linear(rows, self.head)[:, : self.arch.vocab_size]
+        logits = ops.linear(rows, self.head, settled=True)[:, : self.arch.vocab_size]
         return logits.float().view(*hidden.shape[:-1], -1)

@@ -153,8 +153,8 @@ def skinny_residual(residual: torch.Tensor, sumsq_out: torch.Tensor | None, next
 
 
 def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, swiglu: bool = False,
-                splits: int = 0, epilogue: SkinnyEpilogue | None = None) -> torch.Tensor | None:
-    """Decode GEMM for ``M <= 256`` tokens: ``x[M,K] @ w[N,K].T`` with the weights streamed once.
+                splits: int = 0, epilogue: SkinnyEpilogue | None = None, settled: bool = False) -> torch.Tensor | None:
+    """Decode GEMM for ``M <= 256`` tokens: ``x[M,K] @ w[N,K].T`` with the weights streamed once. ``settled``: see ``linear``.
 
     With ``swiglu=True``, ``w`` is ``[gate; up]`` (2*I rows) and the result is ``silu(x gate^T) * (x up^T)`` [M, I].
     With ``epilogue`` (M <= 16) the finished tiles go through a fused epilogue instead of (or before) the plain store;
@@ -180,34 +180,39 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = Non
     ldc = out.stride(0) if out is not None else (epilogue._keep[0].stride(0) if epilogue.kind == 2 else N)
     if epilogue is None:
         _lib.call("b200_gemm_skinny", ptr(x), ptr(w), ptr(out), M, N, K, x.stride(0), w.stride(0), ldc,
-                  1 if swiglu else 0, dtype_code(x.dtype), ptr(scratch), ptr(tickets), splits, stream_ptr())
+                  1 if swiglu else 0, dtype_code(x.dtype, settled), ptr(scratch), ptr(tickets), splits, stream_ptr())
     else:
         if ctypes.sizeof(SkinnyEpilogue) != lib.b200_gemm_skinny_epilogue_bytes():
             raise RuntimeError("SkinnyEpilogue layout differs between the Python binding and the native library")
         _lib.call("b200_gemm_skinny_fused", ptr(x), ptr(w), ptr(out), M, N, K, x.stride(0), w.stride(0), ldc,
-                  1 if swiglu else 0, dtype_code(x.dtype), ptr(scratch), ptr(tickets), ctypes.byref(epilogue), stream_ptr())
+                  1 if swiglu else 0, dtype_code(x.dtype, settled), ptr(scratch), ptr(tickets), ctypes.byref(epilogue), stream_ptr())
     _count()
     return out
 
 
-def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """``x @ w.T`` for any leading shape: the skinny kernel for <= 256 rows, else the tiled one; fp32 has its own kernel."""
+def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, settled: bool = False) -> torch.Tensor:
+    """``x @ w.T`` for any leading shape: the skinny kernel for <= 256 rows, else the tiled one; fp32 has its own kernel.
+
+    ``settled`` (here and in the other ops that take it) is the caller's word that nothing in flight on the stream writes the call's
+    parameters (weights, gains, mixing rows, sinks), as for the weights of a model: the kernel may then fetch them while the kernels
+    in front of it still run. Kernels of a chain start under one another several deep (programmatic dependent launch), so an operand
+    that any recent launch computed is not settled. By default everything is read behind the kernels in front."""
     lead = x.shape[:-1]
     x2 = x.reshape(-1, x.shape[-1])
     o2 = out.reshape(-1, w.shape[0]) if out is not None else None
     if x2.dtype == torch.float32:
         y = gemm_f32(x2, w, o2)
     else:
-        y = gemm_skinny(x2, w, o2) if x2.shape[0] <= 256 else gemm(x2, w, o2)
+        y = gemm_skinny(x2, w, o2, settled=settled) if x2.shape[0] <= 256 else gemm(x2, w, o2)
     return y.reshape(*lead, w.shape[0])
 
 
 _GROUP_TILE = 128  # rows of a decode-GEMM tile
 
 
-def linear_groups(x: torch.Tensor, w: torch.Tensor, rows: list[int]) -> torch.Tensor:
+def linear_groups(x: torch.Tensor, w: torch.Tensor, rows: list[int], settled: bool = False) -> torch.Tensor:
     """Several inputs, each with its own rows of one weight matrix: x [T, G, K], w [sum(rows), K] with ``rows[g]`` rows (multiples
-    of 128) for input g; returns ``[x_0 @ w_0.T | x_1 @ w_1.T | ...]`` [T, sum(rows)]. Up to 256 tokens are one launch."""
+    of 128) for input g; returns ``[x_0 @ w_0.T | x_1 @ w_1.T | ...]`` [T, sum(rows)]. Up to 256 tokens are one launch. ``settled``: see ``linear``."""
     _lib.require_cuda()
     T, G, K = x.shape
     if not x.is_contiguous() or w.shape != (sum(rows), K) or w.stride(1) != 1 or len(rows) != G or any(r % _GROUP_TILE for r in rows):
@@ -219,7 +224,7 @@ def linear_groups(x: torch.Tensor, w: torch.Tensor, rows: list[int]) -> torch.Te
         scratch, tickets = _skinny_scratch.get(x.device, lib.b200_gemm_skinny_scratch_floats(T, w.shape[0], 0), w.shape[0] // _GROUP_TILE)
         tiles = (ctypes.c_int * G)(*[r // _GROUP_TILE for r in rows])
         _lib.call("b200_gemm_skinny_groups", ptr(x), ptr(w), ptr(out), T, K, G, tiles, G * K, w.stride(0), out.stride(0),
-                  dtype_code(x.dtype), ptr(scratch), ptr(tickets), stream_ptr())
+                  dtype_code(x.dtype, settled), ptr(scratch), ptr(tickets), stream_ptr())
         _count()
         return out
     at = 0
@@ -245,12 +250,9 @@ def gemm_f32(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None) 
 
 
 def rmsnorm(x: torch.Tensor, gamma: torch.Tensor, eps: float, residual: torch.Tensor | None = None,
-            out: torch.Tensor | None = None) -> torch.Tensor:
-    """RMSNorm over the last dim. With `residual`, computes ``residual += x`` in place first and normalises the sum.
-
-    ``gamma`` is treated as a weight: the kernel fetches it before it waits for the kernel launched just before it
-    (programmatic dependent launch), so it must not be an output of that kernel. The same holds for the gains of
-    ``qk_norm_rope`` and of the fused all-reduce + RMSNorm."""
+            out: torch.Tensor | None = None, settled: bool = False) -> torch.Tensor:
+    """RMSNorm over the last dim. With `residual`, computes ``residual += x`` in place first and normalises the sum. ``settled``: see
+    ``linear``."""
     _lib.require_cuda()
     hidden = x.shape[-1]
     x2 = x.reshape(-1, hidden)
@@ -261,7 +263,7 @@ def rmsnorm(x: torch.Tensor, gamma: torch.Tensor, eps: float, residual: torch.Te
     o2 = out.reshape(-1, hidden)
     r2 = residual.reshape(-1, hidden) if residual is not None else None
     _lib.call("b200_rmsnorm", ptr(x2), ptr(r2), ptr(r2), ptr(gamma), ptr(o2), x2.shape[0], hidden, c_float(eps),
-              dtype_code(x.dtype), stream_ptr())
+              dtype_code(x.dtype, settled), stream_ptr())
     _count()
     return o2.reshape(x.shape)
 
@@ -283,12 +285,12 @@ def step_tables(position_ids: torch.Tensor, slots_per_seq: int) -> dict[str, tor
 def qk_norm_rope(qkv: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Tensor, num_q_heads: int,
                  num_kv_heads: int, k_cache: torch.Tensor, v_cache: torch.Tensor, slots: torch.Tensor | None,
                  q_gamma: torch.Tensor | None, k_gamma: torch.Tensor | None, eps: float = 1e-6,
-                 q_out: torch.Tensor | None = None) -> torch.Tensor:
+                 q_out: torch.Tensor | None = None, settled: bool = False) -> torch.Tensor:
     """Per-head RMSNorm of q/k, neox RoPE, and the write of k/v into the KV cache at `slots`, in one kernel.
 
     qkv: [T, (Hq + 2 Hkv) * 128]; positions: int32 [T]; cos_sin: fp32 [max_pos, 128] (cos | sin);
     caches: [num_slots, Hkv, 128] (any view whose first dim is the slot); slots: int64 [T] (None = identity).
-    Returns q [T, Hq, 128].
+    ``settled`` (of the gains): see ``linear``. Returns q [T, Hq, 128].
     """
     _lib.require_cuda()
     T = qkv.shape[0]
@@ -301,7 +303,7 @@ def qk_norm_rope(qkv: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Tens
         q_out = torch.empty((T, num_q_heads, D), dtype=qkv.dtype, device=qkv.device)
     _lib.call("b200_qk_norm_rope", ptr(qkv), ptr(positions), ptr(slots), ptr(q_gamma), ptr(k_gamma), ptr(cos_sin),
               ptr(q_out), ptr(k_cache), ptr(v_cache), T, num_q_heads, num_kv_heads, D, c_float(eps),
-              dtype_code(qkv.dtype), stream_ptr())
+              dtype_code(qkv.dtype, settled), stream_ptr())
     _count()
     return q_out
 
@@ -576,17 +578,17 @@ def _norm_args(width, gain, bias, eps, center, h):
 
 
 def embed_norm(ids: torch.Tensor, table: torch.Tensor, scale: float, width: int, gain: torch.Tensor, bias: torch.Tensor | None,
-               eps: float, center: bool | TanhNorm, state0: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:
+               eps: float, center: bool | TanhNorm, state0: torch.Tensor | None = None, settled: bool = False) -> tuple[torch.Tensor, torch.Tensor]:
     """``x = table[ids] * scale`` in fp32 and ``h = norm(x)`` in the table's type, one kernel. ids int64 [T]; table [V, P]
     with P >= width columns (padding columns zero). ``center``: layer norm, else RMS norm, or a ``TanhNorm``. ``state0`` fp32 [T, P]
-    receives a copy of x. Returns (x fp32 [T, P], h [T, P])."""
+    receives a copy of x. ``settled`` (of gain and bias): see ``linear``. Returns (x fp32 [T, P], h [T, P])."""
     _lib.require_cuda()
     flat = ids.reshape(-1).to(torch.int64).contiguous()
     T, P = flat.numel(), table.shape[1]
     x = torch.empty((T, P), dtype=torch.float32, device=table.device)
     h = torch.empty((T, P), dtype=table.dtype, device=table.device)
     _lib.call("b200_embed_norm", ptr(flat), ptr(table), T, ctypes.c_longlong(table.shape[0]), width, P, c_float(scale), ptr(x),
-              ptr(state0), *_norm_args(width, gain, bias, eps, center, h), dtype_code(table.dtype), stream_ptr())
+              ptr(state0), *_norm_args(width, gain, bias, eps, center, h), dtype_code(table.dtype, settled), stream_ptr())
     _count()
     return x, h
 
@@ -595,13 +597,13 @@ def residual_norm(x: torch.Tensor, width: int, mult: float, a: torch.Tensor, gat
                   bias_a: torch.Tensor | None = None, b: torch.Tensor | None = None, gate_b: torch.Tensor | None = None,
                   bias_b: torch.Tensor | None = None, states: torch.Tensor | None = None, weights: torch.Tensor | None = None,
                   keep: bool = False, gain: torch.Tensor | None = None, bias: torch.Tensor | None = None, eps: float = 0.0,
-                  center: bool | TanhNorm | str = True) -> torch.Tensor | None:
+                  center: bool | TanhNorm | str = True, settled: bool = False) -> torch.Tensor | None:
     """One pass over the fp32 residual stream ``x`` [T, P] (updated in place):
     ``s = x + mult * (sigmoid(gate_a + bias_a) * a + sigmoid(gate_b + bias_b) * b)``; with ``weights`` (fp32 [n + 1])
     ``x = sum_j weights[j] * states[j] + weights[n] * s`` over the n earlier states (``states`` fp32 [>= n, T, P]; s is stored
     as state n with ``keep``), else ``x = s``; returns ``norm(x)`` when ``gain`` is given (see ``_norm_args`` for ``center``; ``COPY``
     returns x in the type of a and takes no gain). a, b [T, P]; the gate logits may be
-    column slices of a wider GEMM output (same row pitch)."""
+    column slices of a wider GEMM output (same row pitch). ``settled`` (of gain and bias): see ``linear``."""
     _lib.require_cuda()
     T, P = x.shape
     if x.dtype != torch.float32 or a.shape != x.shape or not a.is_contiguous() or (b is not None and (b.shape != x.shape or not b.is_contiguous())):
@@ -618,23 +620,25 @@ def residual_norm(x: torch.Tensor, width: int, mult: float, a: torch.Tensor, gat
     h = torch.empty((T, P), dtype=a.dtype, device=a.device) if gain is not None or center == COPY else None
     _lib.call("b200_residual_norm", ptr(a), ptr(gate_a), ptr(bias_a), ptr(b), ptr(gate_b), ptr(bias_b), ldg, c_float(mult), ptr(x),
               ptr(states), ctypes.c_longlong(T * P), ptr(weights), n, 1 if keep else 0, T, width, P,
-              *_norm_args(width, gain, bias, eps, center, h), dtype_code(a.dtype), stream_ptr())
+              *_norm_args(width, gain, bias, eps, center, h), dtype_code(a.dtype, settled), stream_ptr())
     _count()
     return h
 
 
 def residual_post(x: torch.Tensor, width: int, mult: float, a: torch.Tensor, gain_a: torch.Tensor, b: torch.Tensor | None = None,
                   gain_b: torch.Tensor | None = None, post_eps: float = 0.0, gain: torch.Tensor | None = None,
-                  bias: torch.Tensor | None = None, eps: float = 0.0, center: bool | TanhNorm | str = True) -> torch.Tensor | None:
+                  bias: torch.Tensor | None = None, eps: float = 0.0, center: bool | TanhNorm | str = True,
+                  settled: bool = False) -> torch.Tensor | None:
     """``x += mult * (rms(a) * gain_a + rms(b) * gain_b)`` on the fp32 stream x [T, P] (in place; b optional): sublayer results [T, P]
-    that are RMS-normed over the width on their way in. Returns ``norm(x)`` as ``residual_norm`` does."""
+    that are RMS-normed over the width on their way in. Returns ``norm(x)`` as ``residual_norm`` does.
+    ``settled`` (of gain and bias): see ``linear``."""
     _lib.require_cuda()
     T, P = x.shape
     if x.dtype != torch.float32 or a.shape != x.shape or not a.is_contiguous() or (b is not None and (b.shape != x.shape or not b.is_contiguous())):
         raise ValueError("residual_post: x must be fp32 [T, P] and the sublayer results contiguous [T, P]")
     h = torch.empty((T, P), dtype=a.dtype, device=a.device) if gain is not None or center == COPY else None
     _lib.call("b200_residual_post", ptr(a), ptr(gain_a), ptr(b), ptr(gain_b), c_float(post_eps), c_float(mult), ptr(x), T, width, P,
-              *_norm_args(width, gain, bias, eps, center, h), dtype_code(a.dtype), stream_ptr())
+              *_norm_args(width, gain, bias, eps, center, h), dtype_code(a.dtype, settled), stream_ptr())
     _count()
     return h
 
@@ -653,35 +657,36 @@ def token_side(g: torch.Tensor, ids: torch.Tensor, table: torch.Tensor, offset: 
 
 
 # ---- recurrent mixers (csrc/kernels/recurrent.cu) ---------------------------------------------
-def token_mix(h: torch.Tensor, mu: torch.Tensor, last: torch.Tensor) -> torch.Tensor:
+def token_mix(h: torch.Tensor, mu: torch.Tensor, last: torch.Tensor, settled: bool = False) -> torch.Tensor:
     """``h_t + (h_{t-1} - h_t) * mu_g`` for every row of mu [G, P]: h [B * S, P] -> [B * S, G, P]. ``last`` [B, P] is the token before
-    the call and is replaced by the call's last one."""
+    the call and is replaced by the call's last one. ``settled`` (of mu): see ``linear``."""
     _lib.require_cuda()
     T, P = h.shape
     B, G = last.shape[0], mu.shape[0]
     if not (h.is_contiguous() and mu.is_contiguous() and last.is_contiguous()) or T % B or mu.shape[1] != P or last.shape[1] != P:
         raise ValueError("token_mix: shape/layout mismatch")
     out = torch.empty((T, G, P), dtype=h.dtype, device=h.device)
-    _lib.call("b200_token_mix", ptr(h), ptr(mu), ptr(last), ptr(out), B, T // B, G, P, dtype_code(h.dtype), stream_ptr())
+    _lib.call("b200_token_mix", ptr(h), ptr(mu), ptr(last), ptr(out), B, T // B, G, P, dtype_code(h.dtype, settled), stream_ptr())
     _count()
     return out
 
 
-def tanh_linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def tanh_linear(x: torch.Tensor, w: torch.Tensor, settled: bool = False) -> torch.Tensor:
     """``tanh(x) @ w.T``, the second half of a low-rank map: x [T, K] (rows may be strided), w [N, K]. One launch for few tokens, tanh
-    and the tiled GEMM for many."""
+    and the tiled GEMM for many. ``settled``: see ``linear``."""
     if x.shape[0] <= 256:
-        return head_linear(x[:, None], w[None], tanh=True)[:, 0]
+        return head_linear(x[:, None], w[None], tanh=True, settled=settled)[:, 0]
     _check_2d(x, "x")
     act = torch.empty(x.shape, dtype=x.dtype, device=x.device)
     _lib.call("b200_tanh_rows", ptr(x), ptr(act), x.shape[0], x.shape[1], x.stride(0), dtype_code(x.dtype), stream_ptr())
     _count()
-    return linear(act, w)
+    return linear(act, w, settled=settled)
 
 
-def short_conv(x: torch.Tensor, taps: torch.Tensor, last: torch.Tensor) -> torch.Tensor:
+def short_conv(x: torch.Tensor, taps: torch.Tensor, last: torch.Tensor, settled: bool = False) -> torch.Tensor:
     """Causal convolution per channel, then silu: x [B * S, C] (rows may be strided), taps fp32 [n, C] (the last weighs the current
-    token), ``last`` [B, n - 1, C] the inputs before the call, replaced by the last ones of the call. Returns [B * S, C]."""
+    token), ``last`` [B, n - 1, C] the inputs before the call, replaced by the last ones of the call. ``settled`` (of the taps): see
+    ``linear``. Returns [B * S, C]."""
     _lib.require_cuda()
     T, C = x.shape
     n, B = taps.shape[0], last.shape[0]
@@ -689,7 +694,7 @@ def short_conv(x: torch.Tensor, taps: torch.Tensor, last: torch.Tensor) -> torch
             or last.shape[1:] != (n - 1, C) or last.dtype != x.dtype or T % B:
         raise ValueError("short_conv: shape/layout mismatch")
     out = torch.empty((T, C), dtype=x.dtype, device=x.device)
-    _lib.call("b200_short_conv", ptr(x), ptr(taps), ptr(last), ptr(out), B, T // B, C, n, x.stride(0), dtype_code(x.dtype), stream_ptr())
+    _lib.call("b200_short_conv", ptr(x), ptr(taps), ptr(last), ptr(out), B, T // B, C, n, x.stride(0), dtype_code(x.dtype, settled), stream_ptr())
     _count()
     return out
 
@@ -702,11 +707,11 @@ def _check_recurrent(state, rows, fp32, name):
 
 
 def wkv(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, gate: torch.Tensor, w0: torch.Tensor, u: torch.Tensor,
-        gain: torch.Tensor, state: torch.Tensor, dim: int, vdim: int, eps: float, plain: bool = False) -> torch.Tensor:
+        gain: torch.Tensor, state: torch.Tensor, dim: int, vdim: int, eps: float, plain: bool = False, settled: bool = False) -> torch.Tensor:
     """Decayed outer-product memory with a bonus ``u`` for the current token and decays ``exp(-exp(z + w0))`` per key channel, then
     the RMS norm of every head, ``gain`` and ``silu(gate)``. r, k, z [B * S, H * D], v, gate [B * S, H * E] (rows may be strided);
     w0, u [H * D], gain [H * E]; ``state`` [B, H, D, E] is updated. D and E are multiples of 8, ``dim`` / ``vdim`` the true sizes.
-    Returns [B * S, H * E]."""
+    ``settled`` (of w0, u and gain): see ``linear``. Returns [B * S, H * E]."""
     _lib.require_cuda()
     B, H, D, E = state.shape
     _check_recurrent(state, (r, k, v, z, gate), (w0, u, gain), "wkv")
@@ -717,17 +722,18 @@ def wkv(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, gate
     out = torch.empty((T, H * E), dtype=r.dtype, device=r.device)
     _lib.call("b200_wkv", ptr(r), r.stride(0), ptr(k), k.stride(0), ptr(v), v.stride(0), ptr(z), z.stride(0), ptr(gate), gate.stride(0),
               ptr(w0), ptr(u), ptr(gain), c_float(eps), ptr(state), ptr(out), B, T // B, H, dim, D, vdim, E, int(plain),
-              dtype_code(r.dtype), stream_ptr())
+              dtype_code(r.dtype, settled), stream_ptr())
     _count()
     return out
 
 
 def gated_delta(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tensor, b: torch.Tensor, gate: torch.Tensor,
                 a_log: torch.Tensor, dt_bias: torch.Tensor, gain: torch.Tensor, state: torch.Tensor, dim: int, vdim: int, eps: float,
-                plain: bool = False) -> torch.Tensor:
+                plain: bool = False, settled: bool = False) -> torch.Tensor:
     """Gated delta rule on unit-length q (times dim ** -0.5) and k, then the RMS norm of every head, ``gain`` and ``silu(gate)``. q, k
     [B * S, G * D], v, gate [B * S, H * E], a (decay) and b (step size) logits [B * S, H] (rows may be strided; a and b with one
-    pitch); a_log, dt_bias [H], gain [E]; ``state`` [B, H, D, E] is updated. Returns [B * S, H * E]."""
+    pitch); a_log, dt_bias [H], gain [E]; ``state`` [B, H, D, E] is updated. ``settled`` (of a_log, dt_bias and gain): see ``linear``.
+    Returns [B * S, H * E]."""
     _lib.require_cuda()
     B, H, D, E = state.shape
     _check_recurrent(state, (q, k, v, a, b, gate), (a_log, dt_bias, gain), "gated_delta")
@@ -738,7 +744,7 @@ def gated_delta(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tens
     out = torch.empty((T, H * E), dtype=q.dtype, device=q.device)
     _lib.call("b200_gated_delta", ptr(q), q.stride(0), ptr(k), k.stride(0), ptr(v), v.stride(0), ptr(a), ptr(b), a.stride(0), ptr(gate),
               gate.stride(0), ptr(a_log), ptr(dt_bias), ptr(gain), c_float(eps), ptr(state), ptr(out), B, T // B, H, G, dim, D, vdim, E,
-              int(plain), dtype_code(q.dtype), stream_ptr())
+              int(plain), dtype_code(q.dtype, settled), stream_ptr())
     _count()
     return out
 
@@ -804,9 +810,9 @@ def latent_prep(latent_in: torch.Tensor | None, gain: torch.Tensor | None, cache
     return act
 
 
-def head_linear(x: torch.Tensor, w: torch.Tensor, tanh: bool = False) -> torch.Tensor:
+def head_linear(x: torch.Tensor, w: torch.Tensor, tanh: bool = False, settled: bool = False) -> torch.Tensor:
     """Per-head GEMM ``y[t, h, :] = w[h] @ x[t, h, :]``: x [T, H, K] (unit inner stride), w [H, N, K] -> y [T, H, N]. With ``tanh`` of
-    tanh(x)."""
+    tanh(x). ``settled``: see ``linear``."""
     _lib.require_cuda()
     T, H, K = x.shape
     N = w.shape[1]
@@ -815,7 +821,7 @@ def head_linear(x: torch.Tensor, w: torch.Tensor, tanh: bool = False) -> torch.T
     y = torch.empty((T, H, N), dtype=x.dtype, device=x.device)
     ll = ctypes.c_longlong
     _lib.call("b200_head_linear", ptr(x), ptr(w), ptr(y), T, H, N, K, ll(x.stride(0)), ll(x.stride(1)), ll(y.stride(0)),
-              ll(y.stride(1)), int(tanh), dtype_code(x.dtype), stream_ptr())
+              ll(y.stride(1)), int(tanh), dtype_code(x.dtype, settled), stream_ptr())
     _count()
     return y
 
@@ -847,13 +853,13 @@ def _latent_splits(batch: int, rows: int, n_tiles: int, sm_count: int) -> tuple[
 
 def latent_attention(q: torch.Tensor, cache: torch.Tensor, kv_lens: torch.Tensor, block_table: torch.Tensor, tokens: int,
                      scale: float, sink: torch.Tensor | None = None, num_splits: int = 1, rows_per_cta: int = 0,
-                     variant: str | None = None) -> torch.Tensor:
+                     variant: str | None = None, settled: bool = False) -> torch.Tensor:
     """Attention of absorbed queries over paged latents that are both keys and values. q [B * tokens, H, P]; cache
     [blocks, page, P]; kv_lens int32 [B] (the new tokens included); block_table int32 [B, *]; query token i of a sequence attends
     keys j <= kv_len - tokens + i. ``sink`` fp32 [H]. Returns [B * tokens, H, P].
 
     ``variant``: "tc" (tcgen05 tiles; 16-bit, ranks up to 512) or "plain" (one warp per row, any type and rank); None picks the
-    first that handles the operands."""
+    first that handles the operands. ``settled`` (of the sink): see ``linear``."""
     _lib.require_cuda()
     T, H, P = q.shape
     B = kv_lens.numel()
@@ -873,7 +879,7 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, kv_lens: torch.Tensor
     part = torch.empty(T * H * num_splits * (P + 1), dtype=torch.float32, device=q.device)  # [T * H, splits, P] and its log-sum-exps
     per_cta = rows_per_cta or (16 if tokens * H <= 16 else 32 if tokens * H <= 32 else 64)
     _lib.call("b200_latent_attention", ptr(q), ptr(cache), ctypes.c_longlong(cache.shape[0] * page), *shape, num_splits, per_cta,
-              ptr(part), ptr(sink), ptr(out), dtype_code(q.dtype), ptr(_pipeline_status(q.device)), stream_ptr())
+              ptr(part), ptr(sink), ptr(out), dtype_code(q.dtype, settled), ptr(_pipeline_status(q.device)), stream_ptr())
     _count(2)
     return out
 
