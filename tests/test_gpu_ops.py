@@ -370,3 +370,24 @@ def test_topk_softmax_widths_and_ties(E, k):
         want_p = want_p[:, :k] / (want_p[:, :k].sum(-1, keepdim=True) if renorm else 1.0)
         assert torch.equal(ids.long(), want[:, :k])
         torch.testing.assert_close(w.double(), want_p, rtol=1e-5, atol=1e-9)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_prefill_attention_largest_weight_is_exact(dtype):
+    """A key of a later step outweighs the ones before it by a power of two that is no whole number: its weight is held as one, so the
+    columns of a row share no rounding error of their own."""
+    from triton_distributed_b200 import ops
+    torch.manual_seed(8)
+    S, n, D = 128, 300, 128
+    q, k, v = torch.zeros(S, 1, D), torch.zeros(n, 1, D), torch.zeros(n, 1, D)
+    q[:, 0, 0], k[200, 0, 0] = torch.linspace(0.1, 5.5, S), 1.0
+    v[200] = torch.rand(1, D) + 1.0
+    q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+    ends = [torch.tensor([0, m], dtype=torch.int32, device="cuda") for m in (S, n)]
+    out = ops.prefill_attention(q.cuda(), k.cuda(), v.cuda(), *ends, S, n, 1.0, False).double().cpu()
+    w = torch.exp(q[:, 0].double() @ k[:, 0].double().t())
+    want = w @ v[:, 0].double() / w.sum(1, keepdim=True)
+    # fp32 sums (2^-21 of the result with the exponentials) move the rounding of hardly any of the outputs: up to four of a row's 128,
+    # by a unit in the last place each, which is 2^-7 of a value just above a power of two in bf16
+    unit = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
+    assert ((out[:, 0] - want.to(dtype).double()) / want).mean(1).abs().max() <= 4 * unit / D

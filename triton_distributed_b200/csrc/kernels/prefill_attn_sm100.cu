@@ -13,8 +13,12 @@
 //   warp 10     asks the hardware for the next item (cluster launch control) while the current one is worked on
 // Tensor memory: S of tile t at columns 128 t, O of tile t at 256 + 128 t. The softmax thread reads its row of S, keeps it in
 // registers, and writes P as 16-bit pairs over the same columns: P is the A operand of the second product straight from tensor
-// memory. O stays in tensor memory: rows are rescaled only when a new maximum exceeds the reference by more than 2^8 (exact for
-// any reference: numerator and denominator use the same one), which after the first steps of a row hardly ever happens.
+// memory. O stays in tensor memory; the rows of a warp are rescaled when one of them has a new maximum. A reference that lags behind
+// the maximum would do (by up to 2^8: 397 us for 449 on the pack below), but it costs precision: a row's largest weight is one, which
+// 16 bits hold exactly, only while the reference is the maximum itself (error against 64 bits 2.07e-3 of the norm for 2.03e-3).
+// The sum over all keys is the tensor core's running fp32 sum, which truncates where the former kernel added the sums of 128 keys to
+// registers: no difference in the error of random values (2.03e-3 on the pack, 2.11e-3 over 16384 keys in bf16, 2.63e-4 in f16);
+// with values of mean one, results over 16384 keys lie 3.8e-5 low, which shows in f16 alone (2.26e-4 for 2.22e-4).
 // V is read in place, row-major, as an MN-major operand (b200_prefill_attention_vt reads V^T as a K-major one). Rows behind a
 // sequence's last key belong to others: their scores are masked and their values are zeroed in shared memory, so nothing that
 // stands there (not even NaN) reaches the output.
@@ -22,9 +26,10 @@
 // two blocks the K and V rings have two stages, with three K has two, with four both have one, which is what shared memory holds.
 // Every barrier wait is bounded; on expiry the CTA unwinds through an abort flag and reports a status.
 //
-// What bounds it: the special-function unit and the tensor core, evenly (128 x 128 scores are 1024 cycles of either), and in long
-// calls the power cap. One query tile per CTA, P through shared memory, O in registers and a launch that transposed V before it
-// gave 502 TFLOP/s (causal, 8 x 2048 tokens, 64 / 8 heads, bf16) and 598 (1 x 16384, 32 / 8 heads); this form 991 and 1289.
+// What bounds it: the special-function unit and the tensor core, evenly (128 x 128 scores are 1024 cycles of either), the rescaling,
+// and in long calls the power cap. One query tile per CTA, P through shared memory, O in registers and a launch that transposed V
+// before it took 769 us for five causal sequences of 1 K to 3 K tokens (64 / 8 heads, bf16) and 851 for one of 16384 (8 / 1 heads);
+// this form 449 and 516.
 //
 // Role in the reference: flash_attn_with_kvcache in layers/nvidia/tp_attn.py:194-195 (prefill) and the Triton
 // flash-attention consumer of the sequence-parallel all-gather path, kernels/nvidia/sp_ag_attention_intra_node.py:255-425.
@@ -369,7 +374,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2e;
         if (j == 0) {
           ref = top;
-        } else if (__any_sync(0xffffffffu, top > ref + 8.f)) {
+        } else if (__any_sync(0xffffffffu, top > ref)) {
           // the scores of this step were issued after the tile's last product, so O is complete and nothing writes it now
           const float next = fmaxf(ref, top);
           const float corr = fast_exp2(ref - (next == -INFINITY ? 0.f : next));
