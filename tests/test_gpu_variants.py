@@ -151,3 +151,37 @@ def test_prefill_attention_tiles_and_foreign_rows(dtype, lens_q, lens_k, Hq, Hkv
         unit = 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
         top = float(v[ks:ks + lk].abs().max()) if lk else 0.0
         torch.testing.assert_close(out[qs:qs + lq].double(), want, rtol=0, atol=4 * unit * top)
+
+
+def test_entry_points_of_native_callers():
+    """The forms that programs without the Python layer call keep their arguments: GEMM, grouped GEMM, prefill attention with a scratch
+    for transposed values (here also with values between two 16-byte boundaries)."""
+    import ctypes
+    from triton_distributed_b200 import _lib, ops
+    from triton_distributed_b200._lib import ptr, stream_ptr
+    from triton_distributed_b200.kernels.nvidia import create_sort_plan, grouped_gemm, moe_sort
+    torch.manual_seed(5)
+    bf, null, one = torch.bfloat16, None, ctypes.c_float(0.1)
+    a, b = torch.randn(200, 64, device="cuda").to(bf), torch.randn(72, 64, device="cuda").to(bf)
+    out = torch.empty(200, 72, dtype=bf, device="cuda")
+    _lib.call("b200_gemm", ptr(a), ptr(b), ptr(out), 200, 72, 64, 64, 64, 72, 0, 0, stream_ptr())
+    assert torch.equal(out, ops.gemm(a, b))
+    w, ids = torch.randn(4, 72, 64, device="cuda").to(bf), torch.randint(0, 4, (200, 1), dtype=torch.int32, device="cuda")
+    plan, scale = moe_sort(ids, create_sort_plan(200, 1, 4, 128, 1)), torch.rand(200, device="cuda")
+    _lib.call("b200_grouped_gemm", ptr(a), 64, 1, ptr(w), 4, 72, 64, 200, ptr(plan.sorted_ids), ptr(plan.tile_expert), null, ptr(plan.totals),
+              plan.max_tiles, ptr(out), 72, ptr(scale), 0, stream_ptr())
+    assert torch.equal(out, grouped_gemm(a, w, ids, row_scale=scale))
+    lib = _lib.load()
+    lib.b200_prefill_attention_scratch_bytes.restype = ctypes.c_longlong
+    n = lib.b200_prefill_attention_scratch_bytes(2, 2, 64, 130)
+    assert n == 2 * 2 * 64 * 256 * 2
+    q, k = torch.randn(200, 4, 64, device="cuda").to(bf), torch.randn(200, 2, 64, device="cuda").to(bf)
+    ends, scratch = torch.tensor([0, 70, 200], dtype=torch.int32, device="cuda"), torch.empty(n, dtype=torch.uint8, device="cuda")
+    for shift in (0, 1):
+        v = torch.randn(200 * 2 * 64 + shift, device="cuda").to(bf)[shift:].view(200, 2, 64)
+        got = torch.empty(200, 4, 64, dtype=bf, device="cuda")
+        args = (ptr(q), ptr(k), ptr(v), ptr(ends), ptr(ends), null, 2, 200, 200, 130, 130, 4, 2, 64, 64, one, 1, null, 0)
+        _lib.call("b200_prefill_attention", *args, ptr(scratch), ptr(got), 0, null, stream_ptr())
+        assert torch.equal(got, ops.prefill_attention(q, k, v, ends, ends, 130, 130, 0.1, True))
+        with pytest.raises(_lib.NativeError):
+            _lib.call("b200_prefill_attention", *args, null, ptr(got), 0, null, stream_ptr())

@@ -718,10 +718,8 @@ static int pick_width(int tiles_m, int cols, int step, int units) {
   return best;
 }
 
-// C[M,N] = A[M,K] * B[N,K]^T, all row-major with leading dimensions lda/ldb/ldc (elements). gated: B [2 * N, K] holds gate rows,
-// then up rows, and C = silu(A gate^T) * (A up^T); more than 128 rows.
-B200_API int b200_gemm(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int dtype,
-                       int max_ctas, int gated, void* stream) {
+static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int dtype,
+                     int max_ctas, bool gated, void* stream) {
   GemmParams p;
   memset(&p, 0, sizeof(p));
   int rc = fill_common(p, M, N, K, dtype, 16);
@@ -765,6 +763,18 @@ B200_API int b200_gemm(const void* A, const void* B, void* C, int M, int N, int 
     case 224: return launch_gemm_impl<kPlain, 2, 224>(ta, ta, tb, p, ctx, grid, st);
     default: return launch_gemm_impl<kPlain, 2>(ta, ta, tb, p, ctx, grid, st);
   }
+}
+
+// C[M,N] = A[M,K] * B[N,K]^T, all row-major with leading dimensions lda/ldb/ldc (elements).
+B200_API int b200_gemm(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int dtype,
+                       int max_ctas, void* stream) {
+  return gemm_impl(A, B, C, M, N, K, lda, ldb, ldc, dtype, max_ctas, false, stream);
+}
+
+// B [2 * N, K] holds gate rows, then up rows, and C [M, N] = silu(A gate^T) * (A up^T); more than 128 rows of A.
+B200_API int b200_gemm_gated(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int dtype,
+                             void* stream) {
+  return gemm_impl(A, B, C, M, N, K, lda, ldb, ldc, dtype, 0, true, stream);
 }
 
 // AG-GEMM. a_local [Mr, K] is this rank's shard; ag_buf0/1 are the two symmetric gather buffers

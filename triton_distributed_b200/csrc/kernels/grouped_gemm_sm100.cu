@@ -487,18 +487,14 @@ static int fill_grouped(GroupedParams& p, CUtensorMap* tw, const void* W, int E,
 
 using namespace b200;
 
-// out[pair, :] = A[pair / a_div, :] * W[e]^T (* row_scale[pair]) for the pairs listed in sorted_ids (tiles of 128 rows,
-// one expert per tile, pad rows = n_pairs). W is [E, N, K]; A rows have pitch lda; out rows have pitch ldo. gated: W[e] is
-// N / 2 gate rows and N / 2 up rows, out [n_pairs, N / 2] = silu(A gate^T) * (A up^T).
-B200_API int b200_grouped_gemm(const void* A, int lda, int a_div, const void* W, int E, int N, int K, int n_pairs,
+static int grouped_gemm_impl(const void* A, int lda, int a_div, const void* W, int E, int N, int K, int n_pairs,
                                const int32_t* sorted_ids, const int32_t* tile_expert, const int32_t* tile_order,
                                const int32_t* totals, int max_tiles, void* out, int ldo, const float* row_scale, int dtype,
-                               int gated, void* stream) {
-  B200_REQUIRE(!gated || (N % 16 == 0 && row_scale == nullptr), "a gated projection needs N (%d) a multiple of 16 and no row scale", N);
+                             bool gated, void* stream) {
   GroupedParams p;
   CUtensorMap tw;
   int rc = fill_grouped(p, &tw, W, E, N, K, n_pairs, a_div, sorted_ids, tile_expert, tile_order, totals, max_tiles, out, ldo,
-                        row_scale, dtype, gated != 0);
+                        row_scale, dtype, gated);
   if (rc != kOk) return rc;
   p.A = A; p.lda = lda;
   SymmCtx ctx;
@@ -511,6 +507,25 @@ B200_API int b200_grouped_gemm(const void* A, int lda, int a_div, const void* W,
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (gated) return p.bn == 256 ? launch_grouped_bn<kGPlain, 256, true>(tw, p, ctx, grid, s) : launch_grouped_bn<kGPlain, 128, true>(tw, p, ctx, grid, s);
   return launch_grouped<kGPlain>(tw, p, ctx, grid, s);
+}
+
+// out[pair, :] = A[pair / a_div, :] * W[e]^T (* row_scale[pair]) for the pairs listed in sorted_ids (tiles of 128 rows,
+// one expert per tile, pad rows = n_pairs). W is [E, N, K]; A rows have pitch lda; out rows have pitch ldo.
+B200_API int b200_grouped_gemm(const void* A, int lda, int a_div, const void* W, int E, int N, int K, int n_pairs,
+                               const int32_t* sorted_ids, const int32_t* tile_expert, const int32_t* tile_order,
+                               const int32_t* totals, int max_tiles, void* out, int ldo, const float* row_scale, int dtype,
+                               void* stream) {
+  return grouped_gemm_impl(A, lda, a_div, W, E, N, K, n_pairs, sorted_ids, tile_expert, tile_order, totals, max_tiles, out, ldo, row_scale,
+                           dtype, false, stream);
+}
+
+// As b200_grouped_gemm where W[e] is N / 2 gate rows, then N / 2 up rows: out [n_pairs, N / 2] = silu(A gate^T) * (A up^T).
+B200_API int b200_grouped_gemm_gated(const void* A, int lda, int a_div, const void* W, int E, int N, int K, int n_pairs,
+                                     const int32_t* sorted_ids, const int32_t* tile_expert, const int32_t* tile_order,
+                                     const int32_t* totals, int max_tiles, void* out, int ldo, int dtype, void* stream) {
+  B200_REQUIRE(N % 16 == 0, "a gated projection needs N (%d) a multiple of 16", N);
+  return grouped_gemm_impl(A, lda, a_div, W, E, N, K, n_pairs, sorted_ids, tile_expert, tile_order, totals, max_tiles, out, ldo, nullptr,
+                           dtype, true, stream);
 }
 
 // AG + grouped GEMM: a_local [Tr, K] are this rank's tokens; pairs index the gathered tokens (pair / topk = token).

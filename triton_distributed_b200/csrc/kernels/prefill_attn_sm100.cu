@@ -534,11 +534,11 @@ using namespace b200;
 // KV cache whose sequences own contiguous runs of slots. With causal != 0 query i of a sequence attends keys
 // <= i + (k_len - q_len). gate: nullable [total_q, Hq] with row pitch ldg, every head's output times sigmoid(gate).
 // q, k and v 16-byte aligned; dk, dv: multiples of 8, dk <= 256. dtype 0 = bf16, 1 = f16.
-B200_API int b200_prefill_attention(const void* q, const void* k, const void* v, const int* cu_q, const int* cu_k,
-                                    const int* k_lens, int B,
-                                    int total_q, int total_k, int max_q, int max_k, int Hq, int Hkv, int dk, int dv,
-                                    float scale, int causal, const void* gate, int ldg, void* out, int dtype,
-                                    uint32_t* status, void* stream) {
+B200_API int b200_prefill_attention_direct(const void* q, const void* k, const void* v, const int* cu_q, const int* cu_k,
+                                           const int* k_lens, int B,
+                                           int total_q, int total_k, int max_q, int max_k, int Hq, int Hkv, int dk, int dv,
+                                           float scale, int causal, const void* gate, int ldg, void* out, int dtype,
+                                           uint32_t* status, void* stream) {
   B200_REQUIRE(dtype == kBF16 || dtype == kF16, "prefill attention supports bf16/f16");
   B200_REQUIRE(dk >= 8 && dk % 8 == 0 && dk <= 256 && dv >= 8 && dv % 8 == 0,
                "prefill attention needs head sizes in multiples of 8, keys up to 256; got %d and %d", dk, dv);
@@ -549,7 +549,34 @@ B200_API int b200_prefill_attention(const void* q, const void* k, const void* v,
                         causal, nullptr, gate, ldg, out, dtype, status, static_cast<cudaStream_t>(stream));
 }
 
-// As b200_prefill_attention for values that are already transposed:
+// The form of callers that bring a scratch for transposed values: b200_prefill_attention_scratch_bytes(...) bytes, which nothing is
+// written to any more. Values that do not start on a 16-byte boundary are copied to one that does, in stream order.
+B200_API long long b200_prefill_attention_scratch_bytes(int B, int Hkv, int dv, int max_k) {
+  const long long s_pad = (static_cast<long long>(max_k) + 127) / 128 * 128;
+  return static_cast<long long>(B) * Hkv * dv * s_pad * 2;
+}
+B200_API int b200_prefill_attention(const void* q, const void* k, const void* v, const int* cu_q, const int* cu_k,
+                                    const int* k_lens, int B,
+                                    int total_q, int total_k, int max_q, int max_k, int Hq, int Hkv, int dk, int dv,
+                                    float scale, int causal, const void* gate, int ldg, void* vt_scratch, void* out, int dtype,
+                                    uint32_t* status, void* stream) {
+  B200_REQUIRE(vt_scratch != nullptr, "the transposed-V scratch is required");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  void* copy = nullptr;
+  if (reinterpret_cast<uintptr_t>(v) % 16 != 0 && total_k > 0 && Hkv > 0 && dv > 0) {
+    const size_t bytes = static_cast<size_t>(total_k) * Hkv * dv * 2;
+    B200_CHECK_CUDA(cudaMallocAsync(&copy, bytes, s));
+    const cudaError_t e = cudaMemcpyAsync(copy, v, bytes, cudaMemcpyDeviceToDevice, s);
+    if (e != cudaSuccess) cudaFreeAsync(copy, s);
+    B200_CHECK_CUDA(e);
+  }
+  const int rc = b200_prefill_attention_direct(q, k, copy != nullptr ? copy : v, cu_q, cu_k, k_lens, B, total_q, total_k, max_q, max_k, Hq, Hkv, dk,
+                                               dv, scale, causal, gate, ldg, out, dtype, status, stream);
+  if (copy != nullptr) B200_CHECK_CUDA(cudaFreeAsync(copy, s));
+  return rc;
+}
+
+// As b200_prefill_attention_direct for values that are already transposed:
 //   q [total_q, Hq, dk] with ldq elements between two tokens; k [total_k, Hkv, dk] contiguous; vt [Hkv, dv, total_k], the keys of
 //   a sequence at columns cu_k[b] ... (multiples of 8). Whole tiles of 128 keys are read: what follows a sequence must be finite;
 //   sink: nullable fp32 [Hq] on the device, a logit that joins every row's softmax denominator unscaled and has no value;

@@ -223,8 +223,13 @@ def grouped_gemm_planned(a: torch.Tensor, w: torch.Tensor, plan: MoeSortPlan, a_
     n = plan.n_pairs
     out = torch.empty((n, N // 2 if gated else N), dtype=a.dtype, device=a.device)
     rs = row_scale.reshape(-1).float().contiguous() if row_scale is not None else None
-    _lib.call("b200_grouped_gemm", ptr(a), a.stride(0), a_div, ptr(w), E, N, K, n,
-              ptr(plan.sorted_ids), ptr(plan.tile_expert), None, ptr(plan.totals), plan.max_tiles, ptr(out), out.stride(0),
-              ptr(rs), dtype_code(a.dtype), 1 if gated else 0, stream_ptr())
+    args = (ptr(a), a.stride(0), a_div, ptr(w), E, N, K, n, ptr(plan.sorted_ids), ptr(plan.tile_expert), None, ptr(plan.totals),
+            plan.max_tiles, ptr(out), out.stride(0))
+    if gated:
+        if rs is not None:
+            raise ValueError("grouped_gemm_planned: the gated form takes no row_scale")
+        _lib.call("b200_grouped_gemm_gated", *args, dtype_code(a.dtype), stream_ptr())
+    else:
+        _lib.call("b200_grouped_gemm", *args, ptr(rs), dtype_code(a.dtype), stream_ptr())
     ops._count()
     return out

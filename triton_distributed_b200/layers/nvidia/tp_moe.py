@@ -179,7 +179,7 @@ class EP_MoE:
         E, N, K = w.shape
         out = torch.zeros((n_rows, N), dtype=a.dtype, device=a.device)
         _lib.call("b200_grouped_gemm", ptr(a), a.stride(0), 1, ptr(w), E, N, K, n_rows, ptr(sorted_ids), ptr(tile_expert), None,
-                  ptr(totals), self.a2a.recv_cap // 128, ptr(out), out.stride(0), None, dtype_code(a.dtype), 0, stream_ptr())
+                  ptr(totals), self.a2a.recv_cap // 128, ptr(out), out.stride(0), None, dtype_code(a.dtype), stream_ptr())
         ops._count()
         return out
 

@@ -54,8 +54,11 @@ def _gemm(a, b, N, out, max_ctas, gated):
         raise ValueError("gemm: shape/dtype mismatch")
     if out is None:
         out = torch.empty((M, N), dtype=a.dtype, device=a.device)
-    _lib.call("b200_gemm", ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-              dtype_code(a.dtype), max_ctas, 1 if gated else 0, stream_ptr())
+    args = ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0), dtype_code(a.dtype)
+    if gated:
+        _lib.call("b200_gemm_gated", *args, stream_ptr())
+    else:
+        _lib.call("b200_gemm", *args, max_ctas, stream_ptr())
     _count()
     return out
 
@@ -538,7 +541,7 @@ def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seql
         v = v.clone()
     if out is None:
         out = torch.empty((total_q, Hq, dv), dtype=q.dtype, device=q.device)
-    _lib.call("b200_prefill_attention", ptr(q), ptr(k), ptr(v), ptr(cu_q), ptr(cu_k), ptr(k_lens), B, total_q, total_k,
+    _lib.call("b200_prefill_attention_direct", ptr(q), ptr(k), ptr(v), ptr(cu_q), ptr(cu_k), ptr(k_lens), B, total_q, total_k,
               int(max_seqlen_q), int(max_seqlen_k), Hq, Hkv, D, dv, c_float(scale), 1 if causal else 0, ptr(gate),
               gate.stride(0) if gate is not None else 0, ptr(out),
               dtype_code(q.dtype), ptr(_pipeline_status(q.device)), stream_ptr())
