@@ -391,3 +391,29 @@ def test_prefill_attention_largest_weight_is_exact(dtype):
     # by a unit in the last place each, which is 2^-7 of a value just above a power of two in bf16
     unit = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
     assert ((out[:, 0] - want.to(dtype).double()) / want).mean(1).abs().max() <= 4 * unit / D
+
+
+@pytest.mark.parametrize("form", ["tiled", "grouped", "wide grouped"])
+def test_gated_epilogues_of_very_negative_gates(form):
+    """Gates down to the end of the exponential's range: small numbers, not zero, and of full precision times a large up value."""
+    from triton_distributed_b200 import ops
+    from triton_distributed_b200.kernels.nvidia import create_sort_plan, moe_sort
+    from triton_distributed_b200.kernels.nvidia.allgather_group_gemm import grouped_gemm_planned
+    M, N, K = {"tiled": 200, "grouped": 8, "wide grouped": 600}[form], 256, 64
+    a = torch.zeros(M, K, device="cuda", dtype=torch.bfloat16)
+    a[:, 0] = 1.0
+    b = torch.zeros(2 * N, K, device="cuda", dtype=torch.bfloat16)
+    b[:N, 0] = -torch.linspace(80.0, 90.0, N).to(torch.bfloat16)
+    b[N:, 0] = 2.0 ** 20
+    if form == "tiled":
+        out = ops.gemm_gated(a, b)
+    else:
+        plan = moe_sort(torch.zeros(M, 1, dtype=torch.int32, device="cuda"), create_sort_plan(M, 1, 4, 128, 1))
+        out = grouped_gemm_planned(a, torch.stack([b] * 4), plan, 1, gated=True)
+    z = b[:N, 0].double()
+    want = (z * torch.exp(z) * 2.0 ** 20).expand(M, N)
+    # exp(-z) itself overflows behind 88.7: zero there, as an IEEE division of z by infinity gives. 2^-9 of the rounding to 16 bits and
+    # 2 + |z| units of 2^-23 of the exponential, twice
+    near = z > -88.7
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs())[:, near].all()
+    assert (out[:, z < -88.8] == 0).all()

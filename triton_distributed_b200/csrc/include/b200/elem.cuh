@@ -41,8 +41,11 @@ __device__ __forceinline__ void store4(__half* p, float4 v) {
 // forms whose error (about 1e-6) is far below a rounding of the result.
 template <typename T>
 __device__ __forceinline__ float exp_t(float z) { return sizeof(T) == 4 ? expf(z) : __expf(z); }
+// (__fdividef gives zero for divisors above 2^126, which 1 + exp(-z) reaches at z = -87.4: both sides are divided by four)
 template <typename T>
-__device__ __forceinline__ float silu(float z) { return sizeof(T) == 4 ? z / (1.f + expf(-z)) : __fdividef(z, 1.f + __expf(-z)); }
+__device__ __forceinline__ float silu(float z) {
+  return sizeof(T) == 4 ? z / (1.f + expf(-z)) : __fdividef(0.25f * z, fmaf(0.25f, __expf(-z), 0.25f));
+}
 template <typename T>
 __device__ __forceinline__ float inv_sqrt(float z) { return sizeof(T) == 4 ? 1.f / sqrtf(z) : rsqrtf(z); }
 template <typename T>
