@@ -94,3 +94,22 @@ def test_moe_model_native_modes_match_torch(dist1):
     for mode in ("triton_dist_AR", "triton_dist"):
         torch.testing.assert_close(outs[mode], outs["torch"], rtol=3e-2, atol=3e-2)
     model.finalize()
+
+
+def test_attention_only_reads_the_step_tables(dist1):
+    """One dictionary of step tables, refilled by its owner for prompts of another length: nothing of the first call is left in it."""
+    from triton_distributed_b200 import ops
+    from triton_distributed_b200.layers.nvidia import TP_Attn, _set_cos_sin_cache
+    from triton_distributed_b200.models import KV_Cache
+    torch.manual_seed(6)
+    att = TP_Attn(0, 1)
+    rnd = lambda *shape: torch.randn(shape, device="cuda", dtype=torch.bfloat16)
+    att._init_parameters(q=rnd(512, 256), k=rnd(256, 256), v=rnd(256, 256), o=rnd(256, 512), q_norm=rnd(128), k_norm=rnd(128), num_heads=4, num_kv_heads=2)
+    cos = _set_cos_sin_cache(10000.0 ** (-torch.arange(64, device="cuda") / 64), 256)
+    step = {}
+    for seqlen in (40, 70, 9):
+        kv, own = (KV_Cache(1, 2, 128, 2, 128, torch.bfloat16, 1) for _ in range(2))
+        pos, qkv = torch.arange(seqlen, device="cuda")[None].repeat(2, 1), rnd(2 * seqlen, 1024)
+        step.update(ops.step_tables(pos, kv.blocks_per_seq * kv.page_size))
+        got = att._attn_native(qkv, pos, cos, kv, 0, 2, seqlen, step)
+        assert torch.equal(got, att._attn_native(qkv, pos, cos, own, 0, 2, seqlen))

@@ -42,6 +42,11 @@ def _set_cos_sin_cache(inv_freq: torch.Tensor, max_length: int) -> torch.Tensor:
 
 _rope_torch = golden.rope_torch
 
+def prompt_bounds(bsz: int, seqlen: int, slots_per_seq: int, device) -> tuple[torch.Tensor, torch.Tensor]:
+    """First query row and first cache slot of every sequence of a batch of prompts, int32 [bsz + 1] each: the same for every layer."""
+    return tuple(torch.arange(0, (bsz + 1) * n, n, dtype=torch.int32, device=device) for n in (seqlen, slots_per_seq))
+
+
 class TP_Attn:
 
     def __init__(self, rank: int = 0, world_size: int = 8, group=None):
@@ -102,7 +107,8 @@ class TP_Attn:
 
     def _attn_native(self, qkv, position_ids, cos_sin_cache, kv_cache, layer_idx, bsz, seqlen, step=None):
         """qkv [B*S, (Hq + 2 Hkv) D] -> attention output [B*S, Hq*D] with k/v appended to the paged cache.
-        `step` carries per-step tensors precomputed by the model (positions int32, slots, kv_lens)."""
+        `step` carries per-step tensors precomputed by the model (positions int32, slots, kv_lens and, for a prompt, ``bounds``: see
+        ``prompt_bounds``); it is only read."""
         kp, vp = kv_cache.layer(layer_idx)
         if step is None:
             step = ops.step_tables(position_ids, kv_cache.blocks_per_seq * kv_cache.page_size)
@@ -120,9 +126,7 @@ class TP_Attn:
         if self.head_dim != 128:
             raise NotImplementedError("the native prefill attention is specialised for head_dim 128")
         L = kv_cache.blocks_per_seq * kv_cache.page_size
-        if "bounds" not in step:  # the same for every layer of a step
-            step["bounds"] = [torch.arange(0, (bsz + 1) * n, n, dtype=torch.int32, device=qkv.device) for n in (seqlen, L)]
-        cu_q, cu_k = step["bounds"]
+        cu_q, cu_k = step["bounds"] if "bounds" in step else prompt_bounds(bsz, seqlen, L, qkv.device)
         o = ops.prefill_attention(q, kp.view(-1, self.kv_heads_local, self.head_dim), vp.view(-1, self.kv_heads_local, self.head_dim),
                                   cu_q, cu_k, seqlen, min(L, step.get("kv_len") or kv_cache.max_length), self.scale, True, seqlens_k=step["kv_lens"])
         return o.reshape(bsz * seqlen, -1)

@@ -25,6 +25,7 @@ from ..kernels.allreduce import AllReduceMethod
 from ..kernels.nvidia import (all_reduce_rmsnorm, create_ag_gemm_context, create_allreduce_ctx,
                               create_fast_allgather_context, create_gemm_rs_context, fast_allgather)
 from ..layers.nvidia import TP_MLP, TP_Attn, _set_cos_sin_cache, golden, layer_norm
+from ..layers.nvidia.tp_attn import prompt_bounds
 from .config import ArchConfig, ModelConfig
 from .kv_cache import KV_Cache
 from .weights import RandomSource, SafetensorsSource, WeightSource
@@ -235,11 +236,21 @@ class Qwen3:
             return y
         return ops.rmsnorm(partial, gamma, self.eps, residual=residual, settled=True)
 
+    @staticmethod
+    def _step(position_ids, kv_cache):
+        """What the layers of a step share (``TP_Attn._attn_native``)."""
+        bsz, seqlen = position_ids.shape
+        slots = kv_cache.blocks_per_seq * kv_cache.page_size
+        step = ops.step_tables(position_ids, slots)
+        if seqlen > 1:
+            step["bounds"] = prompt_bounds(bsz, seqlen, slots, position_ids.device)
+        return step
+
     @torch.no_grad()
     def _inference_AR(self, input_ids, position_ids, kv_cache, kv_len=None):
         """Returns the final-normed hidden states [B, S, H]."""
         bsz, seqlen = input_ids.shape
-        step = ops.step_tables(position_ids, kv_cache.blocks_per_seq * kv_cache.page_size) | {"kv_len": kv_len}
+        step = self._step(position_ids, kv_cache) | {"kv_len": kv_len}
         residual = ops.embedding(input_ids.reshape(-1), self.embed_tokens)  # [T, H], becomes the residual stream
         x = ops.rmsnorm(residual, self.layers[0].input_norm_w, self.eps, settled=True)
         for i, layer in enumerate(self.layers):
@@ -267,7 +278,7 @@ class Qwen3:
             if native:
                 bl = bsz // self.world_size
                 hidden = hidden[self.rank * bl:(self.rank + 1) * bl].contiguous()
-                step = ops.step_tables(position_ids, kv_cache.blocks_per_seq * kv_cache.page_size)
+                step = self._step(position_ids, kv_cache)
             for layer in self.layers:
                 hidden = layer.fwd(hidden, position_ids, self.cos_sin_cache, kv_cache, step)
             if native and not wo_lm_head and native_gather:
