@@ -333,3 +333,16 @@ def test_gated_grouped_gemm(T, topk, E, inter, K, dtype):
     want = gate * torch.sigmoid(gate) * up
     # an fp32 sum of K products is off by about sqrt(K) * 2^-24 of their norm (one here); gate and up each carry that error
     torch.testing.assert_close(out.double(), want, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10, atol=K * 2.0 ** -20)
+
+
+def test_plan_before_its_first_sort():
+    """A new plan holds no pairs and no tiles, whatever the memory held before."""
+    from triton_distributed_b200.kernels.nvidia import create_sort_plan
+    shapes = [(24, 3, 8, 128, 1), (4096, 8, 64, 128, 4)]
+    for args in shapes:
+        plan = create_sort_plan(*args)
+        whole = plan.sorted_ids._base if plan.sorted_ids._base is not None else plan.sorted_ids
+        junk = [torch.full_like(whole, 77) for _ in range(4)]
+        del plan, whole, junk
+        plan = create_sort_plan(*args)
+        assert int(plan.totals.abs().sum()) == 0 and int(plan.group_count.abs().sum()) == 0 and int(plan.status.abs().sum()) == 0

@@ -210,7 +210,7 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, topk_ids: torch.Tensor, a_per
     """Local grouped GEMM: out[t * topk + k] = a[t (or pair)] @ w[topk_ids[t, k]].T (* row_scale). w [E, N, K]."""
     T, topk = topk_ids.shape
     if plan is None:
-        plan = create_sort_plan(T * topk, topk, w.shape[0], 128, 1, a.device)
+        plan = create_sort_plan(T * topk, topk, w.shape[0], 128, 1, a.device, cleared=False)
     moe_sort(topk_ids.to(torch.int32).contiguous(), plan)
     return grouped_gemm_planned(a, w, plan, 1 if a_per_pair else topk, row_scale)
 

@@ -84,7 +84,7 @@ def grouped_gemm_fp8(a8: torch.Tensor, a_scale: torch.Tensor, w8: torch.Tensor, 
     T, topk = topk_ids.shape
     E = w8.shape[0]
     if plan is None:
-        plan = create_sort_plan(T * topk, topk, E, 128, 1, a8.device)
+        plan = create_sort_plan(T * topk, topk, E, 128, 1, a8.device, cleared=False)
     moe_sort(topk_ids.to(torch.int32).contiguous(), plan)
     return grouped_gemm_fp8_planned(a8, a_scale, w8, w_scale, plan.sorted_ids, plan.tile_expert, plan.totals, plan.max_tiles,
                                     T * topk, 1 if a_per_pair else topk, row_scale, None, out_dtype)

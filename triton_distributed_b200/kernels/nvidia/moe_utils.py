@@ -49,17 +49,19 @@ class MoeSortPlan:
 
 
 def create_sort_plan(n_pairs: int, topk: int, num_experts: int, block_m: int = 128, segments: int = 1,
-                     device="cuda", with_positions: bool = False) -> MoeSortPlan:
+                     device="cuda", with_positions: bool = False, cleared: bool = True) -> MoeSortPlan:
     lib = _lib.load()
     lib.b200_moe_sorted_capacity.restype = ctypes.c_longlong
     cap = int(lib.b200_moe_sorted_capacity(n_pairs, num_experts, block_m, segments))
     tiles = cap // block_m
     lib.b200_moe_sort_scratch_ints.restype = ctypes.c_longlong
     scratch = int(lib.b200_moe_sort_scratch_ints(n_pairs, num_experts, segments))
-    # one allocation, cut at 16-byte boundaries; the sort writes all that is read of it
+    # one allocation, cut at 16-byte boundaries
     sizes = (cap, tiles, tiles, tiles, tiles, segments * num_experts, 2 + segments, scratch, n_pairs if with_positions else 0)
     parts = torch.empty(sum((n + 3) // 4 * 4 for n in sizes), dtype=torch.int32, device=device).split([(n + 3) // 4 * 4 for n in sizes])
     parts = [p if p.numel() == n else p[:n] for p, n in zip(parts, sizes)]
+    if cleared:  # a plan that has not been sorted holds no tile: a GEMM over it does nothing
+        parts[5].zero_(), parts[6].zero_()
     return MoeSortPlan(n_pairs, topk, num_experts, block_m, segments, cap, *parts[:8], parts[8] if with_positions else None)
 
 

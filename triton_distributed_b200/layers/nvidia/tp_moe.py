@@ -106,7 +106,7 @@ class TP_MoE:
     def partial_fwd(self, x: torch.Tensor) -> torch.Tensor:
         """Replicated activations: this rank's partial sum [T, H] (grouped tcgen05 GEMMs, no communication)."""
         ids, w = self.route(x)
-        plan = moe_sort(ids, create_sort_plan(ids.numel(), self.topk, self.num_experts, 128, 1, x.device))  # for both projections
+        plan = moe_sort(ids, create_sort_plan(ids.numel(), self.topk, self.num_experts, 128, 1, x.device, cleared=False))  # for both projections
         act = grouped_gemm_planned(x, self.w_gate_up, plan, self.topk, gated=True)
         down = grouped_gemm_planned(act, self.w_down, plan, 1, w)
         return reduce_topk(down, self.topk)
