@@ -346,3 +346,24 @@ def test_plan_before_its_first_sort():
         del plan, whole, junk
         plan = create_sort_plan(*args)
         assert int(plan.totals.abs().sum()) == 0 and int(plan.group_count.abs().sum()) == 0 and int(plan.status.abs().sum()) == 0
+
+
+def test_expired_waits_are_reported(monkeypatch):
+    """The fp8 grouped GEMM and the 32-bit GEMM get the status word that ``check_pipeline_status`` reads and clears."""
+    from triton_distributed_b200 import _lib, ops
+    from triton_distributed_b200.kernels.nvidia import quantize_fp8_rows, quantize_fp8_weight_blocks
+    from triton_distributed_b200.kernels.nvidia.grouped_gemm_fp8 import grouped_gemm_fp8
+    seen, call = {}, _lib.call
+    monkeypatch.setattr(_lib, "call", lambda name, *args: (seen.update({name: args}), call(name, *args)))
+    x = torch.randn(9, 256, device="cuda")
+    ops.gemm_f32(x, x)
+    ids = torch.zeros(9, 1, dtype=torch.int32, device="cuda")
+    grouped_gemm_fp8(*quantize_fp8_rows(x), *quantize_fp8_weight_blocks(torch.randn(2, 128, 256, device="cuda")), ids)
+    word = ops._pipeline_status(x.device)
+    for name in ("b200_gemm_f32_checked", "b200_grouped_gemm_fp8"):
+        assert seen[name][-2].value == word.data_ptr()
+    ops.check_pipeline_status()
+    word.fill_(3)
+    with pytest.raises(RuntimeError):
+        ops.check_pipeline_status()
+    ops.check_pipeline_status()

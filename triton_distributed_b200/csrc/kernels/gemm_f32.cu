@@ -53,6 +53,7 @@ struct F32Params {
   float* C;
   int M, N, K, parts, part, lda, ldb, ldc;
   bool vec_a, vec_b;
+  uint32_t* status;   // nullable: set non-zero when a pipeline wait expired (the tile's results are NaN then)
 };
 
 // four consecutive k of a row; zeros behind k_end
@@ -299,6 +300,7 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 4) tmem_dealloc(tmem_base, 512);
+  if (threadIdx.x == 0 && *abort_flag != 0u && p.status != nullptr) atomicMax(p.status, static_cast<uint32_t>(kStatusPipeTimeout));
   cluster_sync_all();
   if (warp >= 8) {
     // this CTA's share of the tile: the sum over the parts in order
@@ -368,13 +370,14 @@ static int launch_gemm_f32(const F32Params& p, cudaStream_t stream) {
 
 using namespace b200;
 
-B200_API int b200_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb, int ldc,
-                           void* stream) {
+// status (device, nullable): raised when a wait inside the kernel runs out.
+B200_API int b200_gemm_f32_checked(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb, int ldc,
+                                   uint32_t* status, void* stream) {
   B200_REQUIRE(M > 0 && N > 0 && K > 0, "empty problem %dx%dx%d", M, N, K);
   B200_REQUIRE(lda >= K && ldb >= K && ldc >= N, "leading dimensions are smaller than the rows");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto aligned = [](const float* x, int ld) { return ld % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0; };
-  F32Params p = {A, B, C, M, N, K, f32_parts(N, K), 0, lda, ldb, ldc, aligned(A, lda), aligned(B, ldb)};
+  F32Params p = {A, B, C, M, N, K, f32_parts(N, K), 0, lda, ldb, ldc, aligned(A, lda), aligned(B, ldb), status};
   p.part = ((K + p.parts - 1) / p.parts + kXK - 1) / kXK * kXK;
   // row tiles of even height: 100 rows are one of 112, 150 two of 80
   const int tiles = (M + 127) / 128, rows = (M + tiles - 1) / tiles;
@@ -388,4 +391,8 @@ B200_API int b200_gemm_f32(const float* A, const float* B, float* C, int M, int 
     case 7: return launch_gemm_f32<112>(p, s);
     default: return launch_gemm_f32<128>(p, s);
   }
+}
+B200_API int b200_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb, int ldc,
+                           void* stream) {
+  return b200_gemm_f32_checked(A, B, C, M, N, K, lda, ldb, ldc, nullptr, stream);
 }

@@ -55,7 +55,8 @@ def grouped_gemm_fp8_planned(a8: torch.Tensor, a_scale: torch.Tensor, w8: torch.
 
     a8 e4m3 (or uint8 bytes) [rows, K]; a_scale fp32 [rows, K / 128]; w8 [E, N, K]; w_scale fp32 [E, ceil(N / 128), K / 128].
     Row ``sorted_ids[i] // a_div`` of a8 feeds sorted row i; the result of pair p lands in ``out[p]`` ([n_pairs, N]).
-    Rows of ``out`` that no tile covers are left untouched (pass a zeroed ``out`` if that matters)."""
+    Rows of ``out`` that no tile covers are left untouched (pass a zeroed ``out`` if that matters). A wait inside the kernel that
+    runs out is reported by ``ops.check_pipeline_status``."""
     _lib.require_cuda()
     E, N, K = w8.shape
     if a8.shape[1] != K or a8.element_size() != 1 or w8.element_size() != 1:
@@ -69,10 +70,9 @@ def grouped_gemm_fp8_planned(a8: torch.Tensor, a_scale: torch.Tensor, w8: torch.
     if out is None:
         out = torch.empty((n_pairs, N), dtype=out_dtype, device=a8.device)
     rs = row_scale.reshape(-1).float().contiguous() if row_scale is not None else None
-    status = torch.empty(1, dtype=torch.int32, device=a8.device)
     _lib.call("b200_grouped_gemm_fp8", ptr(a8), a8.stride(0), ptr(a_scale), a_scale.stride(0), a_div, ptr(w8), ptr(w_scale),
               E, N, K, n_pairs, ptr(sorted_ids), ptr(tile_expert), ptr(totals), max_tiles, ptr(out), out.stride(0), ptr(rs),
-              dtype_code(out.dtype), ptr(status), stream_ptr())
+              dtype_code(out.dtype), ptr(ops._pipeline_status(a8.device)), stream_ptr())
     ops._count()
     return out
 

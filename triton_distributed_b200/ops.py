@@ -247,7 +247,8 @@ def gemm_f32(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None) 
         raise ValueError("gemm_f32: shape/dtype mismatch")
     if out is None:
         out = torch.empty((M, N), dtype=a.dtype, device=a.device)
-    _lib.call("b200_gemm_f32", ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0), stream_ptr())
+    _lib.call("b200_gemm_f32_checked", ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+              ptr(_pipeline_status(a.device)), stream_ptr())
     _count()
     return out
 
