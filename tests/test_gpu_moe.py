@@ -367,3 +367,26 @@ def test_expired_waits_are_reported(monkeypatch):
     with pytest.raises(RuntimeError):
         ops.check_pipeline_status()
     ops.check_pipeline_status()
+
+
+@pytest.mark.parametrize("T,I", [(3, 128), (30, 256), (700, 2176), (500, 4224), (9, 1920)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_silu_mul_fp8_bytes(T, I, dtype):
+    """Gates of 32, whose silu is 32, make the products exact: scales and bytes are those of IEEE divisions, ties included. Rows in
+    more than one block of CTAs, more rows than CTAs, and scales from 2^-30 on."""
+    from triton_distributed_b200 import ops
+    g = torch.Generator().manual_seed(21)
+    u = torch.randn(T, I // 128, 128, generator=g)
+    # a block's largest value is 448 s and others are s times values halfway between two bytes
+    s = torch.tensor([1.0, 3.0, 5.0, 7.0])[torch.randint(0, 4, (T, I // 128, 1), generator=g)] / 32
+    odd = torch.randint(0, 8, (T, I // 128, 64), generator=g) * 2 + 17
+    u[:, :, :64] = s * odd / 16 * 2.0 ** torch.randint(-4, 8, odd.shape, generator=g)
+    u[:, :, 64:127] = u[:, :, 64:127].to(dtype).float().clamp(-10, 10) * s
+    u[:, :, 127:] = 448 * s
+    u[T // 2] *= 2.0 ** (-30 if dtype == torch.bfloat16 else -5)
+    u = u.view(T, I).to(dtype)
+    q, scale = ops.silu_mul_fp8(torch.cat([torch.full_like(u, 32.0), u], dim=1).cuda())
+    blocks = (32 * u.float()).view(T, I // 128, 128)
+    want = blocks.abs().amax(2) / 448
+    assert torch.equal(scale.cpu(), want)
+    assert torch.equal(q.cpu().view(torch.uint8), (blocks / want[:, :, None]).view(T, I).to(torch.float8_e4m3fn).view(torch.uint8))

@@ -236,9 +236,9 @@ __global__ void __launch_bounds__(256) silu_mul_fp8_kernel(const uint4* __restri
   griddep_wait();
   const int nblk = inter / 128;
   const int lane = threadIdx.x & 31, hl = lane & 15;
-  // half-warps take blocks of 128 channels, then rows: the grid covers the blocks of a row in x, so no index is divided. (64-bit
-  // index divisions and 16 IEEE divisions per eight values bound this kernel, not its bytes: 16384 x 768, 33 us -> 18.) Every
-  // lane runs the same number of iterations (the shuffles below need the whole warp); the memory accesses are predicated instead.
+  // half-warps take blocks of 128 channels, then rows: the grid covers the blocks of a row in x, so no index is divided (by
+  // 64-bit divisions of its own). Every lane runs the same number of iterations (the shuffles below need the whole warp); the memory
+  // accesses are predicated instead.
   const int blk = blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4);
   for (int t = blockIdx.y; t < T; t += gridDim.y) {
     const bool in = blk < nblk;
@@ -249,21 +249,15 @@ __global__ void __launch_bounds__(256) silu_mul_fp8_kernel(const uint4* __restri
     float amax = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      o[e] = __fdividef(g[e], 1.f + __expf(-g[e])) * u[e];
+      o[e] = g[e] / (1.f + __expf(-g[e])) * u[e];
       amax = fmaxf(amax, fabsf(o[e]));
     }
 #pragma unroll
     for (int s = 8; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
     const float scale = amax / 448.f;
-    // one division per block and a product per value (within an ulp of a division each); a scale whose reciprocal overflows divides
-    if (scale >= 1e-30f || scale == 0.f) {
-      const float inv = scale > 0.f ? __fdiv_rn(1.f, scale) : 1.f;
+    const float den = scale > 0.f ? scale : 1.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] *= inv;
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = __fdiv_rn(o[e], scale);
-    }
+    for (int e = 0; e < 8; ++e) o[e] = __fdiv_rn(o[e], den);   // a product with the reciprocal would move ties to the other byte
     uint32_t lo = 0, hi = 0;
 #pragma unroll
     for (int q = 0; q < 4; q += 2) {
