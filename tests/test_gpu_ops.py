@@ -417,3 +417,22 @@ def test_gated_epilogues_of_very_negative_gates(form):
     near = z > -88.7
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs())[:, near].all()
     assert (out[:, z < -88.8] == 0).all()
+
+
+@pytest.mark.parametrize("B,S", [(1, 1), (3, 1), (1, 257), (3, 300), (70, 5)])
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+def test_step_tables(B, S, dtype):
+    """Positions from an offset of each sequence, also as rows of a wider matrix and as columns of a transposed one."""
+    from triton_distributed_b200 import ops
+    from triton_distributed_b200.models import KV_Cache
+    torch.manual_seed(9)
+    kv = KV_Cache(1, B, 1024, 1, 128, torch.bfloat16, 1)
+    pos = (torch.randint(0, 500, (B, 1)) + torch.arange(S)[None]).to(dtype).cuda()
+    wide = torch.full((B, S + 3), -1, dtype=dtype, device="cuda")
+    wide[:, 2:2 + S] = pos
+    for ids in (pos, wide[:, 2:2 + S], pos.t().contiguous().t()):
+        step = ops.step_tables(ids, kv.blocks_per_seq * kv.page_size)
+        assert step["pos"].dtype == step["kv_lens"].dtype == torch.int32 and step["slots"].dtype == torch.int64
+        assert torch.equal(step["pos"], pos.reshape(-1).to(torch.int32))
+        assert torch.equal(step["slots"], kv.slots(pos))
+        assert torch.equal(step["kv_lens"], (pos[:, -1] + 1).to(torch.int32))

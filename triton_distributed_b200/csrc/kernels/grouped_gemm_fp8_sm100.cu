@@ -54,7 +54,7 @@ struct FTile {
 };
 
 struct Fp8GroupedParams {
-  int N, K, n_pairs, a_div, lda, ldo, tiles_n, max_tiles, num_kb, sa_ld, bf16, bn, sw_blocks;
+  int N, K, n_pairs, a_div, lda, ldo, tiles_n, max_tiles, num_kb, sa_ld, bf16, sw_blocks;
   const uint8_t* A;           // e4m3 rows, pitch lda bytes
   const float* sa;            // [rows, sa_ld] activation scales, one per 128 channels
   const float* sw;            // [E, sw_blocks, num_kb] weight scales, one per 128 x 128 block
@@ -505,7 +505,6 @@ static int fp8_fill(Fp8GroupedParams& p, CUtensorMap* tw, const void* A8, int ld
   B200_REQUIRE(a_div >= 1 && max_tiles >= 1, "bad a_div / max_tiles");
   memset(&p, 0, sizeof(p));
   p.N = N; p.K = K; p.n_pairs = n_pairs; p.a_div = a_div; p.lda = lda; p.ldo = ldo;
-  p.bn = bn;
   p.tiles_n = (N + bn - 1) / bn;
   p.sw_blocks = (N + kFN - 1) / kFN;
   p.max_tiles = max_tiles;

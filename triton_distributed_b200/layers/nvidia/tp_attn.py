@@ -28,7 +28,7 @@ from .tp_mlp import shard_local
 def layer_norm(hidden: torch.Tensor, eps: float, w: torch.Tensor) -> torch.Tensor:
     """RMSNorm (the reference names it layer_norm, tp_attn.py:60-66). Native on CUDA, torch on CPU."""
     if hidden.is_cuda:
-        return ops.rmsnorm(hidden, w, eps, settled=True)
+        return ops.rmsnorm(hidden, w, eps)
     hf = hidden.float()
     return (hf * torch.rsqrt(hf.pow(2).mean(-1, keepdim=True) + eps) * w.float()).to(hidden.dtype)
 
