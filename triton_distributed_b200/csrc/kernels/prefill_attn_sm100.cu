@@ -5,7 +5,8 @@
 //
 // A CTA works on two tiles of 128 query rows at a time and walks the keys in steps of 128. The tiles are the same rows of two
 // heads that share a KV head, or, where the group size is odd, two row blocks of one head: either way both tiles use the K and V
-// tiles in shared memory. While the softmax of one tile runs, the tensor core computes the other tile's products:
+// tiles in shared memory. While the softmax of one tile runs, the tensor core computes the other tile's products (two tiles in
+// turn: published as ping-pong scheduling, FlashAttention-3, Shah et al. 2024):
 //   warps 0-3   softmax of tile 0, one thread per query row
 //   warps 4-7   softmax of tile 1
 //   warp 8      TMA producer: both Q tiles of an item, then K and V tiles through their rings (128-byte swizzle)
