@@ -1,0 +1,64 @@
+"""Decode GEMM whose tiles hold all of K, against the fp32 statement of the same chain."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,swiglu", [
+    (1, 8, 64, False),          # one granule, one k-block (a stage has two)
+    (8, 1280, 5120, False),     # a tile per SM or less
+    (9, 1001, 192, False),      # the second half of the tokens, a ragged last tile, a ragged last stage
+    (16, 6144, 1088, False),
+    (3, 60000, 128, False),     # several tiles per CTA
+    (1, 3200, 5120, True), (8, 12288, 256, True), (16, 100, 320, True),
+])
+def test_gemm_rows(M, N, K, swiglu, dtype):
+    from triton_distributed_b200 import ops
+    torch.manual_seed(5)
+    x = torch.randn(M, K, device="cuda").to(dtype)
+    w = (torch.randn(N * (2 if swiglu else 1), K, device="cuda") * K ** -0.5).to(dtype)
+    y = ops.gemm_rows(x, w, swiglu=swiglu)
+    ref = x.double() @ w.double().T
+    if swiglu:
+        ref = torch.nn.functional.silu(ref[:, :N]) * ref[:, N:]
+    # sums of K products of values around one in fp32, one rounding of the result
+    eps = torch.finfo(dtype).eps
+    torch.testing.assert_close(y.double(), ref, rtol=eps, atol=2e-5)
+    for _ in range(20):  # the order of the sums is fixed, whatever order the boxes land in
+        assert torch.equal(ops.gemm_rows(x, w, swiglu=swiglu, out_f32=True), y.float())
+    if not swiglu:
+        h = torch.randn(M, N, device="cuda").to(dtype)
+        want = ref + h.double()
+        ops.gemm_rows(x, w, out=h, residual=h)
+        torch.testing.assert_close(h.double(), want, rtol=eps, atol=2e-5)
+
+
+@pytest.mark.parametrize("M,N,K,swiglu", [(1, 1280, 5120, False), (8, 128, 64, False), (16, 3000, 4160, False), (5, 700, 704, True)])
+def test_gemm_rows_norm(M, N, K, swiglu):
+    from triton_distributed_b200 import ops
+    torch.manual_seed(6)
+    h = (torch.randn(M, K, device="cuda") * torch.logspace(-6, 6, M, device="cuda")[:, None]).bfloat16()
+    gamma = (1 + torch.randn(K, device="cuda")).bfloat16()
+    w = (torch.randn(N * (2 if swiglu else 1), K, device="cuda") * K ** -0.5).bfloat16()
+    y = ops.gemm_rows(h, w, swiglu=swiglu, gamma=gamma, eps=1e-6)
+    hd = h.double()
+    scale = torch.rsqrt(hd.square().mean(-1, keepdim=True) + 1e-6)
+    # the product of h and the gain is rounded to bf16, then everything is fp32 up to the result
+    ref = ((hd * gamma.double()).to(torch.bfloat16).double() @ w.double().T) * scale
+    if swiglu:
+        ref = torch.nn.functional.silu(ref[:, :N]) * ref[:, N:]
+    torch.testing.assert_close(y.double(), ref, rtol=2 ** -7, atol=2e-5)
+
+
+def test_gemm_rows_refuses():
+    from triton_distributed_b200 import _lib, ops
+    x = torch.zeros(4, 128, device="cuda", dtype=torch.float16)
+    w = torch.zeros(64, 128, device="cuda", dtype=torch.float16)
+    with pytest.raises(_lib.NativeError):
+        ops.gemm_rows(x, w, gamma=torch.ones(128, device="cuda", dtype=torch.float16), eps=1e-6)
+    with pytest.raises(_lib.NativeError):
+        ops.gemm_rows(x[:, :120], w[:, :120])
+    with pytest.raises(_lib.NativeError):
+        ops.gemm_rows(x.new_zeros(17, 128), w)

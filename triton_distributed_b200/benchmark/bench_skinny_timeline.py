@@ -7,7 +7,7 @@ when each checkpoint was reached by the slowest CTA, in microseconds after the p
 What it shows is the fixed cost of a decode GEMM beyond its weight stream: dependency hand-over, first activation
 load, MMA drain, and the stream-K fix-up through L2.
 
-    python -m triton_distributed_b200.benchmark.bench_skinny_timeline [--tokens 8]
+    python -m triton_distributed_b200.benchmark.bench_skinny_timeline [--tokens 24]   (up to 16 tokens take ops.gemm_rows)
 """
 from __future__ import annotations
 
@@ -63,7 +63,7 @@ def timeline(M: int, N: int, K: int, swiglu: bool, calls: int = 6) -> list[dict]
 
 def main() -> None:
     ap = argparse.ArgumentParser()
-    ap.add_argument("--tokens", type=int, default=8)
+    ap.add_argument("--tokens", type=int, default=24)
     args = ap.parse_args()
     for name, N, K, swiglu in SHAPES:
         for row in timeline(args.tokens, N, K, swiglu):

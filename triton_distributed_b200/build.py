@@ -35,7 +35,7 @@ LIB_PATH = LIB_DIR / "libb200dist.so"
 DEBUG_LIB_PATH = LIB_DIR / "libb200dist_debug.so"
 
 # what a model family launches on one GPU: no heap, no collectives
-_GEMMS = ("runtime/host.cc", "kernels/gemm_sm100.cu", "kernels/gemm_skinny_sm100.cu", "kernels/prefill_attn_sm100.cu")
+_GEMMS = ("runtime/host.cc", "kernels/gemm_sm100.cu", "kernels/gemm_skinny_sm100.cu", "kernels/gemm_rows.cu", "kernels/prefill_attn_sm100.cu")
 SUBSETS = {
     "likosun": _GEMMS + ("kernels/gemm_f32.cu", "kernels/latent_attn.cu", "kernels/latent_decode_sm100.cu", "kernels/residual.cu"),
     "sizilorn": _GEMMS + ("kernels/gemm_f32.cu", "kernels/latent_attn.cu", "kernels/residual.cu", "kernels/elementwise.cu",

@@ -246,6 +246,27 @@ class Qwen3:
             step["bounds"] = prompt_bounds(bsz, seqlen, slots, position_ids.device)
         return step
 
+    def _few_tokens(self, tokens: int) -> bool:
+        """Whether a step runs on ``_step_rows``: one GPU, bf16 (the gain is multiplied into h, which f16 may not hold) and sizes of
+        ``ops.gemm_rows``."""
+        a = self.arch
+        return (self.world_size == 1 and tokens <= 16 and self.dtype == torch.bfloat16 and not a.num_experts and a.hidden_size <= 16384
+                and a.hidden_size % 64 == 0 and a.intermediate_size % 64 == 0)
+
+    def _step_rows(self, input_ids, position_ids, kv_cache, kv_len=None):
+        """The residual stream [B * S, H] behind the last layer. Norms and residual adds are part of the projections."""
+        bsz, seqlen = input_ids.shape
+        step = self._step(position_ids, kv_cache) | {"kv_len": kv_len}
+        h = ops.embedding(input_ids.reshape(-1), self.embed_tokens)
+        for i, layer in enumerate(self.layers):
+            attn, mlp = layer.attn, layer.mlp
+            qkv = ops.gemm_rows(h, attn.wqkv, gamma=layer.input_norm_w, eps=self.eps, settled=True)
+            o = attn._attn_native(qkv, position_ids, self.cos_sin_cache, kv_cache, i, bsz, seqlen, step)
+            ops.gemm_rows(o, attn.wo, out=h, residual=h, settled=True)
+            act = ops.gemm_rows(h, mlp.gate_up_proj, swiglu=True, gamma=layer.post_norm_w, eps=self.eps, settled=True)
+            ops.gemm_rows(act, mlp.down_proj, out=h, residual=h, settled=True)
+        return h
+
     @torch.no_grad()
     def _inference_AR(self, input_ids, position_ids, kv_cache, kv_len=None):
         """Returns the final-normed hidden states [B, S, H]."""
@@ -269,6 +290,13 @@ class Qwen3:
         longest sequence after this step when the host knows it (bounds the work of a prefill)."""
         bsz, seqlen = input_ids.shape
         native_gather = self.world_size > 1 and self.gather_ctx is not None and bsz <= self.gather_rows
+        if self.mode == "triton_dist_AR" and self._few_tokens(bsz * seqlen):
+            h = self._step_rows(input_ids, position_ids, kv_cache, kv_len)
+            if wo_lm_head:
+                return ops.rmsnorm(h, self.norm_w, self.eps, settled=True).view(bsz, seqlen, -1)
+            last = h if seqlen == 1 else h.view(bsz, seqlen, -1)[:, -1].contiguous()
+            logits = ops.gemm_rows(last, self.lm_head, gamma=self.norm_w, eps=self.eps, out_f32=True, settled=True)
+            return logits[:, : self.arch.vocab_size].unsqueeze(1)
         if self.mode == "triton_dist_AR":
             hidden = self._inference_AR(input_ids, position_ids, kv_cache, kv_len)
         else:

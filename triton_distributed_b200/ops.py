@@ -172,6 +172,12 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = Non
     M, K = x.shape
     n_rows = w.shape[0]
     N = n_rows // 2 if swiglu else n_rows
+    # Few tokens and all of K on one SM: 1.1 to 2.3 times as fast at the projections of 1280 x 5120 to 151936 x 4096. A long K with
+    # few rows to it stays with the kernel that spreads K over the SMs.
+    if (1 <= M <= 16 and K % 64 == 0 and 64 <= K <= 1024 + 8 * N and splits == 0 and epilogue is None and w.shape[1] == K and w.dtype == x.dtype
+            and n_rows % (2 if swiglu else 1) == 0
+            and (out is None or (out.shape == (M, N) and out.stride(1) == 1 and out.dtype == x.dtype))):
+        return gemm_rows(x, w, out, swiglu, settled=settled)
     own_output = epilogue is not None and epilogue.kind in (1, 2)
     if out is None and not own_output:
         out = torch.empty((M, N), dtype=x.dtype, device=x.device)
@@ -189,6 +195,32 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = Non
             raise RuntimeError("SkinnyEpilogue layout differs between the Python binding and the native library")
         _lib.call("b200_gemm_skinny_fused", ptr(x), ptr(w), ptr(out), M, N, K, x.stride(0), w.stride(0), ldc,
                   1 if swiglu else 0, dtype_code(x.dtype, settled), ptr(scratch), ptr(tickets), ctypes.byref(epilogue), stream_ptr())
+    _count()
+    return out
+
+
+def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, swiglu: bool = False, gamma: torch.Tensor | None = None,
+              eps: float = 0.0, residual: torch.Tensor | None = None, out_f32: bool = False, settled: bool = False) -> torch.Tensor:
+    """Decode GEMM for ``M <= 16`` tokens and K in multiples of 64 whose tiles hold all of K: ``x @ w.T``, or with ``swiglu``
+    ``silu(x gate^T) * (x up^T)`` for w = [gate; up]. ``gamma`` (bf16): of ``rmsnorm(x) * gamma`` in the place of x. ``residual`` [M, N] is
+    added to the product; `out` may be the residual itself. ``out_f32``: fp32 results, rounded to the storage type all the same.
+    ``settled`` (of w and gamma): see ``linear``."""
+    _lib.require_cuda()
+    _check_2d(x, "x"), _check_2d(w, "w")
+    M, K = x.shape
+    N = w.shape[0] // 2 if swiglu else w.shape[0]
+    if w.shape[1] != K or w.dtype != x.dtype or (swiglu and w.shape[0] % 2):
+        raise ValueError("gemm_rows: shape/dtype mismatch")
+    if out is None:
+        out = torch.empty((M, N), dtype=torch.float32 if out_f32 else x.dtype, device=x.device)
+    if out.shape != (M, N) or out.stride(1) != 1 or out.dtype != (torch.float32 if out_f32 else x.dtype):
+        raise ValueError("gemm_rows: the output is [M, N] with unit inner stride")
+    if gamma is not None and (gamma.shape != (K,) or gamma.dtype != x.dtype or not gamma.is_contiguous()):
+        raise ValueError("gemm_rows: gamma is [K] in the type of x")
+    if residual is not None and (residual.shape != (M, N) or residual.dtype != x.dtype or residual.stride() != out.stride()):
+        raise ValueError("gemm_rows: the residual is laid out like the output")
+    _lib.call("b200_gemm_rows", ptr(x), ptr(w), ptr(out), M, N, K, x.stride(0), w.stride(0), out.stride(0), 1 if swiglu else 0, ptr(gamma),
+              c_float(eps), ptr(residual), 1 if out_f32 else 0, dtype_code(x.dtype, settled), ptr(_pipeline_status(x.device)), stream_ptr())
     _count()
     return out
 
