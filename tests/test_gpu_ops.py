@@ -109,6 +109,44 @@ def test_qk_norm_rope_and_cache_write():
     torch.testing.assert_close(vc[slots], qkv.view(T, -1, D)[:, Hq + Hkv:])
 
 
+@pytest.mark.parametrize("T,Hq,Hkv", [(1, 1, 1), (3, 8, 1), (2367, 4, 2), (2368, 4, 2), (1200, 8, 1), (800, 16, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_qk_norm_rope_groups_of_heads(T, Hq, Hkv, dtype):
+    """Two and eight heads a warp (eight from 16 warps an SM on), with groups that q, k and v share and that no head fills."""
+    from triton_distributed_b200 import ops
+    torch.manual_seed(14)
+    D, n = 128, Hq + 2 * Hkv
+    qkv = torch.randn(T, n * D, device="cuda").to(dtype)
+    pos = torch.randint(0, 4000, (T,), device="cuda", dtype=torch.int32)
+    inv = 1.0 / (1e6 ** (torch.arange(0, D, 2, device="cuda", dtype=torch.float32) / D))
+    ang = torch.arange(4096, device="cuda", dtype=torch.float32)[:, None] * inv[None, :]
+    cos_sin = torch.cat([ang.cos(), ang.sin()], -1).contiguous()
+    kg = torch.randn(D, device="cuda").to(dtype)
+    slots = torch.randperm(T + 5, device="cuda")[:T].to(torch.int64)
+    slots[T // 2] = -1   # not cached
+    kc = torch.zeros(T + 5, Hkv, D, device="cuda", dtype=dtype)
+    vc = torch.zeros_like(kc)
+    q = ops.qk_norm_rope(qkv, pos, cos_sin, Hq, Hkv, kc, vc, slots, None, kg, 1e-6)
+    x = qkv.float().view(T, n, D)
+
+    def turned(v):
+        c, s = cos_sin[pos.long()][:, None].chunk(2, -1)
+        v1, v2 = v.chunk(2, -1)
+        return torch.cat([v1 * c - v2 * s, v2 * c + v1 * s], -1)
+
+    eps = torch.finfo(dtype).eps
+    kx = x[:, Hq:Hq + Hkv]
+    k = (kx * torch.rsqrt(kx.pow(2).mean(-1, keepdim=True) + 1e-6) * kg.float()).to(dtype).float()
+    torch.testing.assert_close(q.float(), turned(x[:, :Hq]), rtol=eps, atol=1e-5)   # one rounding of an fp32 value
+    keep = slots >= 0
+    # the norm's rounding may fall to the other side: a place of it on either partner, and one of the result
+    torch.testing.assert_close(kc[slots[keep]].float(), turned(k)[keep], rtol=2 * eps, atol=2 * eps * float(k.abs().max()))
+    assert torch.equal(vc[slots[keep]], qkv.view(T, n, D)[keep, Hq + Hkv:])
+    free = torch.ones(T + 5, dtype=torch.bool, device="cuda")
+    free[slots[keep]] = False
+    assert not kc[free].any() and not vc[free].any()
+
+
 def test_silu_mul_and_topk():
     from triton_distributed_b200 import ops
     torch.manual_seed(5)
