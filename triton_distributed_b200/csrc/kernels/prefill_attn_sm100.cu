@@ -9,13 +9,14 @@
 // turn: published as ping-pong scheduling, FlashAttention-3, Shah et al. 2024):
 //   warps 0-3   softmax of tile 0, one thread per query row
 //   warps 4-7   softmax of tile 1
-//   warp 8      TMA producer: both Q tiles of an item, then K and V tiles through their rings (128-byte swizzle)
-//   warp 9      one elected thread issues tcgen05.mma, for each step and tile O += P V of this step, then S = Q K^T of the next
-//   warp 10     asks the hardware for the next item (cluster launch control) while the current one is worked on
+//   warps 8-11  rescale O of either tile while the softmax warps compute the exponentials, and store the finished rows
+//   warp 12     TMA producer: both Q tiles of an item, then K and V tiles through their rings (128-byte swizzle)
+//   warp 13     one elected thread issues tcgen05.mma, for each step and tile O += P V of this step, then S = Q K^T of the next
+//   warp 14     asks the hardware for the next item (cluster launch control) while the current one is worked on
 // Tensor memory: S of tile t at columns 128 t, O of tile t at 256 + 128 t. The softmax thread reads its row of S, keeps it in
 // registers, and writes P as 16-bit pairs over the same columns: P is the A operand of the second product straight from tensor
 // memory. O stays in tensor memory; the rows of a warp are rescaled when one of them has a new maximum. A reference that lags behind
-// the maximum would do (by up to 2^8: 397 us for 449 on the pack below), but it costs precision: a row's largest weight is one, which
+// the maximum would do (by up to 2^8), but it costs precision: a row's largest weight is one, which
 // 16 bits hold exactly, only while the reference is the maximum itself (error against 64 bits 2.07e-3 of the norm for 2.03e-3).
 // The sum over all keys is the tensor core's running fp32 sum, which truncates where the former kernel added the sums of 128 keys to
 // registers: no difference in the error of random values (2.03e-3 on the pack, 2.11e-3 over 16384 keys in bf16, 2.63e-4 in f16);
@@ -27,10 +28,14 @@
 // two blocks the K and V rings have two stages, with three K has two, with four both have one, which is what shared memory holds.
 // Every barrier wait is bounded; on expiry the CTA unwinds through an abort flag and reports a status.
 //
-// What bounds it: the special-function unit and the tensor core, evenly (128 x 128 scores are 1024 cycles of either), the rescaling,
-// and in long calls the power cap. One query tile per CTA, P through shared memory, O in registers and a launch that transposed V
+// What bounds it: a tile's chain of softmax and both products (with nothing but the products the pack below takes 315 us, without the
+// exponentials 370, without the rescaling 390), and in long calls the power cap. The special-function unit and the tensor core are busy 42 % of
+// the time each. Rescaling and storing by the softmax warps themselves took 450 us where it is 424 now; stored row by row from the registers
+// it was 525, since a warp that stores 32 rows at a time keeps the next item's rescaling waiting. Two threads per row (16 softmax warps)
+// took 470, steps of 64 keys with the next step's scores in front of this step's product 524: products of 64 columns are slow.
+// One query tile per CTA, P through shared memory, O in registers and a launch that transposed V
 // before it took 769 us for five causal sequences of 1 K to 3 K tokens (64 / 8 heads, bf16) and 851 for one of 16384 (8 / 1 heads);
-// this form 449 and 516.
+// this form 424 and 516 or less.
 //
 // Role in the reference: flash_attn_with_kvcache in layers/nvidia/tp_attn.py:194-195 (prefill) and the Triton
 // flash-attention consumer of the sequence-parallel all-gather path, kernels/nvidia/sp_ag_attention_intra_node.py:255-425.
@@ -49,13 +54,17 @@ constexpr int kPAtom = 128 * 64 * 2;        // one 128-row x 64-column 16-bit sw
 constexpr int kPTile = 2 * kPAtom;          // a 128 x 128 tile: 32 KB
 constexpr int prefill_k_stages(int dk_atoms) { return dk_atoms <= 3 ? 2 : 1; }
 constexpr int prefill_v_stages(int dk_atoms) { return dk_atoms <= 2 ? 2 : 1; }
+// Output rows go to memory through shared memory, a warp's 32 rows at once, where rows of Q and K leave 32 KB for it.
+constexpr bool prefill_staged(int dk_atoms) { return dk_atoms <= 2; }
 constexpr int prefill_smem(int dk_atoms) {
   return 2 * dk_atoms * kPAtom /*Q*/ + prefill_k_stages(dk_atoms) * dk_atoms * kPAtom /*K*/ + prefill_v_stages(dk_atoms) * kPTile /*V*/ +
-         1024 + 256;
+         1024 + 256 + 2 * kPM * 4 /*factors*/ + (prefill_staged(dk_atoms) ? kPM * kPD * 2 : 0);
 }
-constexpr int kPThreads = 384;
-// 384 threads start with 168 registers each: 2 x 128 x 216 + 128 x 72 is the same total
-constexpr int kPSoftmaxRegs = 216, kPOtherRegs = 72;
+constexpr int kPThreads = 512;
+// 512 threads start with 128 registers each; 2 x 128 x softmax + 128 x rescaling + 128 x others is the same total. Who stores needs more.
+constexpr int prefill_softmax_regs(int dk_atoms) { return prefill_staged(dk_atoms) ? 176 : 184; }
+constexpr int prefill_scale_regs(int dk_atoms) { return prefill_staged(dk_atoms) ? 88 : 72; }
+constexpr int kPOtherRegs = 72;
 
 struct PrefillParams {
   int Hq, Hkv, causal, bf16;
@@ -116,6 +125,63 @@ __device__ __forceinline__ PrefillItem prefill_item(const PrefillParams& p, uint
   return w;
 }
 
+// Stores a warp's 32 rows of a tile's output times inv. Staged: through 8 KB of shared memory, two whole rows per instruction;
+// o_empty is signalled as soon as the rows have left tensor memory.
+template <bool kStaged, bool BF16>
+__device__ __forceinline__ void prefill_store(const PrefillParams& p, const PrefillItem& w, int t, int steps, uint32_t o_addr, float inv,
+                                              uint8_t* stg, uint64_t* o_empty) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q_pos = w.m_blk_of(t) * kPM + (warp & 3) * 32 + lane;
+  const bool store = q_pos < w.q_len;
+  const size_t pitch = static_cast<size_t>(p.Hq) * p.dv * 2;   // from a token to the next
+  uint8_t* dst = static_cast<uint8_t*>(p.out) + static_cast<size_t>(w.q_start + q_pos) * pitch + (static_cast<size_t>(w.head_of(t)) * p.dv + w.v_col0) * 2;
+  // 16-byte chunk c of this thread's row lies at number c xor lane % 8 (opaque: the sixteen addresses would be kept, and spill)
+  uint32_t mine = smem_u32(stg + lane * 256 + (lane & 7) * 16);
+  asm volatile("" : "+r"(mine));
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t o[32];
+    if (steps > 0) {
+      tmem_ld_32x32(o_addr + c * 32, o);
+      tmem_ld_wait();
+    } else {
+#pragma unroll
+      for (int e = 0; e < 32; ++e) o[e] = 0u;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint32_t v[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float a = __uint_as_float(o[q * 8 + 2 * e]) * inv, b = __uint_as_float(o[q * 8 + 2 * e + 1]) * inv;
+        v[e] = BF16 ? pack_bf16x2(a, b) : pack_f16x2(a, b);
+      }
+      if (kStaged)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(mine ^ ((c * 4 + q) * 16)), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+      else if (store && w.v_col0 + c * 32 + q * 8 < p.dv)
+        *reinterpret_cast<uint4*>(dst + c * 64 + q * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+  }
+  if (steps > 0) {
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(o_empty);
+  }
+  if (kStaged) {   // two whole rows per store
+    __syncwarp();
+    const int chunk = lane & 15;
+    const bool in = w.v_col0 + chunk * 8 < p.dv;
+    const uint8_t* from = stg + (lane >> 4) * 256;
+    uint8_t* to = dst + chunk * 16 - (lane - (lane >> 4)) * pitch;   // of row lane / 16 of the warp
+    int left = w.q_len - (q_pos - lane) - (lane >> 4);               // rows from there to the sequence's end
+#pragma unroll 4
+    for (int r = 0; r < 32; r += 2, left -= 2, to += 2 * pitch) {
+      const uint4 v4 = *reinterpret_cast<const uint4*>(from + r * 256 + (chunk ^ ((r + (lane >> 4)) & 7)) * 16);
+      if (in && left > 0) *reinterpret_cast<uint4*>(to) = v4;
+    }
+    __syncwarp();
+  }
+}
+
 template <int kDkAtoms, bool BF16>
 __global__ void __launch_bounds__(kPThreads, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -135,7 +201,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* v_full = bars + 6;      // [2]
   uint64_t* v_empty = bars + 8;     // [2]
   uint64_t* s_full = bars + 10;     // [2 tiles] scores are in tensor memory (and the tile's earlier products are done)
-  uint64_t* p_full = bars + 12;     // [2 tiles] probabilities are in tensor memory
+  uint64_t* p_full = bars + 12;     // [2 tiles] probabilities are in tensor memory, and the output has been rescaled
   uint64_t* o_full = bars + 14;     // [2 tiles] the item's last product is done
   uint64_t* o_empty = bars + 16;    // [2 tiles] the item's output has been read
   uint64_t* next_full = bars + 18;  // [1]
@@ -143,6 +209,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint4* next_item = reinterpret_cast<uint4*>(bars + 20);  // 16-byte answer of the launch control
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  uint64_t* c_full = bars + 24;     // [2 tiles] a step's factors of the output have been written
+  uint64_t* f_full = bars + 26;     // [2 tiles] an item's last factors have been written
+  float* s_factor = reinterpret_cast<float*>(bars + 32);   // [2 tiles][128 rows]
+  uint8_t* s_out = reinterpret_cast<uint8_t*>(s_factor + 2 * kPM);   // [4 warps][32 rows][256 bytes]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint64_t timeout_ns = 4000000000ull;
@@ -156,19 +226,21 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(v_full + i, 1);
       mbar_init(v_empty + i, 1);
       mbar_init(s_full + i, 1);
-      mbar_init(p_full + i, 4);
+      mbar_init(p_full + i, 8);
       mbar_init(o_full + i, 1);
       mbar_init(o_empty + i, 4);
+      mbar_init(c_full + i, 4);
+      mbar_init(f_full + i, 4);
     }
     mbar_init(next_full, 1);
-    mbar_init(next_empty, 10);  // producer, MMA issuer, eight softmax warps
+    mbar_init(next_empty, 14);  // producer, MMA issuer, eight softmax warps, four that rescale
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
   }
-  if (warp == 11) tmem_alloc(tmem_slot, 512);
+  if (warp == 15) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -187,9 +259,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     return more;
   };
 
-  if (warp >= 8) {
+  if (warp >= 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPOtherRegs));
-    if (warp == 8) {
+    if (warp == 12) {
       // ---------------------------------------------------------------- TMA producer
       if (elect_one()) {
         int kc = 0, vc = 0, qc = 0;
@@ -237,7 +309,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       }
       __syncwarp();
-    } else if (warp == 9) {
+    } else if (warp == 13) {
       // ---------------------------------------------------------------- MMA issuer
       if (elect_one()) {
         const uint32_t idesc_s = umma_idesc_f16(kPM, kPN, BF16);
@@ -315,7 +387,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       }
       __syncwarp();
-    } else if (warp == 10) {
+    } else if (warp == 14) {
       // ---------------------------------------------------------------- next items
       if (elect_one()) {
         bool more = true;
@@ -334,13 +406,67 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       __syncwarp();
     }
+  } else if (warp >= 8) {
+    // ------------------------------------------------------------------ rescaling and output, one thread per query row of either tile
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(prefill_scale_regs(kDkAtoms)));
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t o_lanes = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 2 * kPN;
+    uint32_t c_phase = 0, f_phase = 0;   // bit t: parity of tile t's next phase
+    bool ok = true;
+    for (int i = 0; ok; ++i) {
+      const PrefillItem w = prefill_item(p, at, gridDim.y);
+      for (int j = 1; j < w.n && ok; ++j) {
+        for (int t = 0; t < 2; ++t) {
+          if (j < w.steps_of(t)) {
+            ok = __all_sync(0xffffffffu, mbar_wait(c_full + t, c_phase >> t & 1, abort_flag, timeout_ns));
+            c_phase ^= 1u << t;
+            if (!ok) break;
+            tc_fence_after_sync();
+            const float corr = s_factor[t * kPM + row];
+            if (__any_sync(0xffffffffu, corr != 1.f)) {
+              // the scores of this step were issued after the tile's last product, so O is complete and nothing writes it now
+              const uint32_t o_addr = o_lanes + t * kPD;
+              uint32_t o[2][16];
+              tmem_ld_32x16(o_addr, o[0]);
+#pragma unroll
+              for (int c = 0; c < 8; ++c) {
+                tmem_ld_wait();
+                if (c < 7) tmem_ld_32x16(o_addr + (c + 1) * 16, o[(c + 1) & 1]);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) o[c & 1][e] = __float_as_uint(__uint_as_float(o[c & 1][e]) * corr);
+                tmem_st_32x16(o_addr + c * 16, o[c & 1]);
+              }
+              tmem_st_wait();
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_full + t);
+          }
+        }
+      }
+      // ---- the rows' output
+      for (int t = 0; t < 2 && ok && prefill_staged(kDkAtoms); ++t) {
+        const int steps = w.steps_of(t);
+        float inv = 0.f;
+        if (steps > 0) {
+          ok = __all_sync(0xffffffffu, mbar_wait(f_full + t, f_phase >> t & 1, abort_flag, timeout_ns) &&
+                                           mbar_wait(o_full + t, f_phase >> t & 1, abort_flag, timeout_ns));
+          f_phase ^= 1u << t;
+          if (!ok) break;
+          tc_fence_after_sync();
+          inv = s_factor[t * kPM + row];
+        }
+        prefill_store<prefill_staged(kDkAtoms), BF16>(p, w, t, steps, o_lanes + t * kPD, inv, s_out + (warp & 3) * 32 * 256, o_empty + t);
+      }
+      if (!ok || !advance(i, true)) break;
+    }
   } else {
     // ------------------------------------------------------------------ softmax, one thread per query row
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPSoftmaxRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(prefill_softmax_regs(kDkAtoms)));
     const int t = warp >> 2;  // tile
     const int row = (warp & 3) * 32 + lane;
     const uint32_t lanes = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-    const uint32_t s_addr = lanes + t * kPN, o_addr = lanes + 2 * kPN + t * kPD;
+    const uint32_t s_addr = lanes + t * kPN;
     int sc = 0, oc = 0, vc = 0;
     bool ok = true;
     for (int i = 0; ok; ++i) {
@@ -375,22 +501,17 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2e;
         if (j == 0) {
           ref = top;
-        } else if (__any_sync(0xffffffffu, top > ref)) {
-          // the scores of this step were issued after the tile's last product, so O is complete and nothing writes it now
-          const float next = fmaxf(ref, top);
-          const float corr = fast_exp2(ref - (next == -INFINITY ? 0.f : next));
-          ref = next;
-          sum *= corr;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t o[32];
-            tmem_ld_32x32(o_addr + c * 32, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
-            tmem_st_32x32(o_addr + c * 32, o);
+        } else {
+          // (the factors of the step before have been used: this step's scores were issued behind that step's product)
+          float corr = 1.f;
+          if (top > ref) {
+            corr = fast_exp2(ref - top);
+            ref = top;
           }
-          tmem_st_wait();
+          sum *= corr;
+          s_factor[t * kPM + row] = corr;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(c_full + t);
         }
         const float base = ref == -INFINITY ? 0.f : ref;
         const f32x2 scale2 = pack2(p.scale_log2e, p.scale_log2e), base2 = pack2(-base, -base);
@@ -422,50 +543,34 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_full + t);
+        if (lane == 0) {
+          mbar_arrive(p_full + t);
+          if (j == 0) mbar_arrive(p_full + t);   // for the warp that rescales: nothing to do yet
+        }
       }
       vc += w.n;
-      // ---- the row's output
-      if (ok && steps > 0) {
-        ok = __all_sync(0xffffffffu, mbar_wait(o_full + t, oc++ & 1, abort_flag, timeout_ns));
-        tc_fence_after_sync();
-      }
       if (!ok) break;
-      if (p.sink != nullptr) sum += exp2f(p.sink[head] * 1.4426950408889634f - ref);  // the sink counts once, unscaled
-      float inv = sum > 0.f ? 1.f / sum : 0.f;
-      const bool store = q_pos < w.q_len;
-      if (store && p.gate != nullptr) {
-        const size_t g = static_cast<size_t>(w.q_start + q_pos) * p.ldg + head;
-        const float z = BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.gate)[g]) : __half2float(static_cast<const __half*>(p.gate)[g]);
-        inv /= 1.f + expf(-z);
-      }
-      uint8_t* dst = static_cast<uint8_t*>(p.out) + ((static_cast<size_t>(w.q_start + q_pos) * p.Hq + head) * p.dv + w.v_col0) * 2;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t o[32];
-        if (steps > 0) {
-          tmem_ld_32x32(o_addr + c * 32, o);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] = 0u;
+      float inv = 0.f;
+      if (steps > 0) {   // the row's factor; whoever rescaled the output also stores it, if through shared memory
+        if (p.sink != nullptr) sum += exp2f(p.sink[head] * 1.4426950408889634f - ref);  // the sink counts once, unscaled
+        inv = sum > 0.f ? 1.f / sum : 0.f;
+        if (q_pos < w.q_len && p.gate != nullptr) {
+          const size_t g = static_cast<size_t>(w.q_start + q_pos) * p.ldg + head;
+          const float z = BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.gate)[g]) : __half2float(static_cast<const __half*>(p.gate)[g]);
+          inv /= 1.f + expf(-z);
         }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (!store || w.v_col0 + c * 32 + q * 8 >= p.dv) continue;
-          uint32_t v[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float a = __uint_as_float(o[q * 8 + 2 * e]) * inv, b = __uint_as_float(o[q * 8 + 2 * e + 1]) * inv;
-            v[e] = BF16 ? pack_bf16x2(a, b) : pack_f16x2(a, b);
-          }
-          *reinterpret_cast<uint4*>(dst + c * 64 + q * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+        // The last step's factor may still be needed: it has been used once the item's last product is done.
+        ok = __all_sync(0xffffffffu, mbar_wait(o_full + t, oc++ & 1, abort_flag, timeout_ns));
+        if (!ok) break;
+        if (prefill_staged(kDkAtoms)) {
+          s_factor[t * kPM + row] = inv;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(f_full + t);
         }
       }
-      if (steps > 0) {
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(o_empty + t);
+      if (!prefill_staged(kDkAtoms)) {   // eight warps store faster than four
+        tc_fence_after_sync();
+        prefill_store<false, BF16>(p, w, t, steps, tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 2 * kPN + t * kPD, steps > 0 ? inv : 0.f, nullptr, o_empty + t);
       }
       if (!advance(i, true)) break;
     }
@@ -474,7 +579,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // ---------------------------------------------------------------------- teardown
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 11) tmem_dealloc(tmem_base, 512);
+  if (warp == 15) tmem_dealloc(tmem_base, 512);
   if (threadIdx.x == 0 && *abort_flag != 0u && p.status != nullptr) atomicMax(p.status, static_cast<uint32_t>(kStatusPipeTimeout));
 }
 
