@@ -527,6 +527,29 @@ def test_gemm_f32_range_of_values(M, N, K):
     assert torch.equal(got[odd].double().nan_to_num(7.0), want[odd].nan_to_num(7.0))
 
 
+@pytest.mark.parametrize("M", [1, 16, 17, 112, 113, 128, 129, 300])
+@pytest.mark.parametrize("N,K,pad", [(130, 1, 0), (70, 63, 1), (300, 64, 0), (2048, 257, 3), (129, 1030, 2)])
+def test_gemm_f32_planes(M, N, K, pad):
+    """A cut beforehand gives the bits of a cut inside, with infinities, NaNs and the smallest numbers in it, from a workspace that held
+    something else."""
+    import ctypes
+    from triton_distributed_b200 import _lib, ops
+    from triton_distributed_b200._lib import ptr, stream_ptr
+    a, b = torch.randn(M, K + pad, device="cuda")[:, :K], torch.randn(N, K + pad, device="cuda")[:, :K]
+    a[M // 2, K // 2] = 1e-45
+    a[M - 1, 0] = torch.inf if K > 1 else 1e-40
+    if M > 16:
+        a[3, K - 1] = torch.nan
+    fn = _lib.load().b200_gemm_f32_workspace_bytes
+    fn.restype = ctypes.c_longlong
+    ws = torch.full((fn(M, K),), 0xff, dtype=torch.uint8, device="cuda")
+    out = [torch.empty(M, N, device="cuda") for _ in range(2)]
+    for o, w in zip(out, (None, ws)):
+        _lib.call("b200_gemm_f32_planes", ptr(a), ptr(b), ptr(o), M, N, K, a.stride(0), b.stride(0), N, ptr(w), ptr(ops._pipeline_status(a.device)), stream_ptr())
+    assert torch.equal(out[0].view(torch.int32), out[1].view(torch.int32))
+    ops.check_pipeline_status()
+
+
 @pytest.mark.parametrize("K", [1, 2, 3, 5, 8, 40])
 @pytest.mark.parametrize("kind", ["full mantissas", "any", "one sign"])
 def test_gemm_f32_short_sums(K, kind):

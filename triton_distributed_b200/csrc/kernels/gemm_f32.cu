@@ -22,12 +22,19 @@
 // and K alone and the sum inside a part runs in the order of K, so a row's result does not depend on how many other rows share the
 // call. Any M, N, K, leading dimensions and alignment.
 //   warps 0-3   promotion: x1 y1 from tensor memory into registers, then the partial tile     warp 4  MMA issuer
-//   warps 8-15  operands: global memory -> registers, one step of 64 k ahead -> three planes in 128-byte-swizzled shared memory
-// What bounds it: for few rows the bytes of B; from about 100 rows on the cutting (two products less are no faster; without the
-// look for small numbers 5 % are gained). The rare cases are left to a second look per step: a branch for every four values kept
-// the loads, the arithmetic and the stores of neighbouring values apart (100 x 11264 x 2048: 78 us for 70).
-// Measured against fp32 products on the CUDA cores with 4 x 4 outputs per thread (11264 x 2048 and 2048 x 5632, us, back to back):
-//   M = 1  227, 268 -> 37, 32     M = 100  242, 336 -> 62, 58     M = 1000 (the first)  1488 -> 513
+//   warp 5      A's planes into shared memory by bulk copies, where A was cut beforehand
+//   warps 8-15  operands: global memory -> registers, one or two steps of 64 k ahead -> three planes in 128-byte-swizzled shared memory
+// More than 16 rows of A are cut once, by a kernel in front, when the caller brings room for the planes: every column tile would cut them again,
+// and without them the registers hold two steps of B's loads instead of one. The planes and their sums are the same either way.
+// What bounds it: the products, 1830 of 2330 clocks a step at 100 rows (the planes' copies are asked for when their place is free and take
+// about as long as a step), and at the end of a CTA 13000 clocks for the partial tile and the sum over the parts. The rare cases are left to a
+// second look per step: a branch for every four values kept the loads, the arithmetic and the stores of neighbouring values apart.
+// us, back to back over several B, with A cut by every CTA and one step of loads -> now (planes from 17 rows on; parts by clusters that fit):
+//   11264 x 2048   1 row 40 -> 38    100 rows 61 -> 57    1024 rows 516 -> 451
+//   2048 x 5632    1 row 39 -> 24    100 rows 60 -> 36    1024 rows 297 -> 211
+//   22016 x 4096   1 row 154 -> 123  100 rows 223 -> 165  1024 rows 1954 -> 1384
+//   4096 x 11008   1 row 68 -> 62    100 rows 90 -> 81    1024 rows 925 -> 630
+// fp32 products on the CUDA cores with 4 x 4 outputs per thread took 227 us for 1 x 11264 x 2048 and 336 for 100 x 2048 x 5632.
 #include "b200/host.h"
 #include "b200/packed_f32.cuh"
 #include "b200/primitives.cuh"
@@ -54,6 +61,8 @@ struct F32Params {
   int M, N, K, parts, part, lda, ldb, ldc;
   bool vec_a, vec_b;
   uint32_t* status;   // nullable: set non-zero when a pipeline wait expired (the tile's results are NaN then)
+  uint8_t* planes;          // nullable: A cut beforehand, [row tiles][steps of 64 k][three planes of kT rows as a stage holds them]
+  uint32_t* planes_tiny;    // [row tiles][steps of 64 k] non-zero: the upper half of a value there is zero and the value is not
 };
 
 // four consecutive k of a row; zeros behind k_end
@@ -72,38 +81,84 @@ __device__ __forceinline__ void st_shared_v2(uint32_t at, uint32_t a, uint32_t b
   asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(a), "r"(b) : "memory");
 }
 // the planes of four values from their first ones
-__device__ __forceinline__ void f32_store_planes(const float4& v, const float (&h)[4], uint32_t at, int plane, float& any) {
+__device__ __forceinline__ void f32_planes(const float4& v, const float (&h)[4], uint2 (&out)[3], float& any) {
   const f32x2 minus = pack2(-1.f, -1.f), up = pack2(256.f, 256.f);
   f32x2 r[2] = {fma2(pack2(h[0], h[1]), minus, pack2(v.x, v.y)), fma2(pack2(h[2], h[3]), minus, pack2(v.z, v.w))};
   any = fmaf(sum2(add2(r[0], r[1])), 0.f, any);
-  st_shared_v2(at, upper_halves(h[0], h[1]), upper_halves(h[2], h[3]));
+  out[0] = make_uint2(upper_halves(h[0], h[1]), upper_halves(h[2], h[3]));
 #pragma unroll
   for (int g = 1; g < 3; ++g) {
     const float2 a = unpack2(mul2(r[0], up)), b = unpack2(mul2(r[1], up));
-    st_shared_v2(at + g * plane, upper_halves(a.x, a.y), upper_halves(b.x, b.y));
+    out[g] = make_uint2(upper_halves(a.x, a.y), upper_halves(b.x, b.y));
     r[0] = fma2(pack2(upper_half(a.x), upper_half(a.y)), minus, pack2(a.x, a.y));
     r[1] = fma2(pack2(upper_half(b.x), upper_half(b.y)), minus, pack2(b.x, b.y));
   }
 }
-// The cut of four values. `any` becomes NaN when one of them is an infinity or a NaN (or their differences overflow), `least` falls
-// below 0x1ffff when the upper half of one holds no bit of it (zero is none of these: it wraps around).
-__device__ __forceinline__ void f32_cut(const float4& v, uint32_t at, int plane, float& any, uint32_t& least) {
-  const float h[4] = {upper_half(v.x), upper_half(v.y), upper_half(v.z), upper_half(v.w)};
+__device__ __forceinline__ void f32_store_planes(const float4& v, const float (&h)[4], uint32_t at, int plane, float& any) {
+  uint2 out[3];
+  f32_planes(v, h, out, any);
+#pragma unroll
+  for (int g = 0; g < 3; ++g) st_shared_v2(at + g * plane, out[g].x, out[g].y);
+}
+// falls below 0x1ffff when the upper half of one of the four holds no bit of it (zero is none of these: it wraps around)
+__device__ __forceinline__ uint32_t f32_least(const float4& v) {
   const uint32_t ab = min((__float_as_uint(v.x) << 1) - 1u, (__float_as_uint(v.y) << 1) - 1u);
   const uint32_t cd = min((__float_as_uint(v.z) << 1) - 1u, (__float_as_uint(v.w) << 1) - 1u);
-  least = min(least, min(ab, cd));
+  return min(ab, cd);
+}
+// The cut of four values. `any` becomes NaN when one of them is an infinity or a NaN (or their differences overflow), `least` follows
+// f32_least.
+__device__ __forceinline__ void f32_cut(const float4& v, uint32_t at, int plane, float& any, uint32_t& least) {
+  const float h[4] = {upper_half(v.x), upper_half(v.y), upper_half(v.z), upper_half(v.w)};
+  least = min(least, f32_least(v));
   f32_store_planes(v, h, at, plane, any);
 }
 // the same with a bit in the upper half of every NaN, which an infinity would stand for otherwise
-__device__ __noinline__ void f32_cut_odd(float4 v, uint32_t at, int plane) {
+__device__ __forceinline__ void f32_first_odd(const float4& v, float (&h)[4]) {
   const float x[4] = {v.x, v.y, v.z, v.w};
-  float h[4], any = 0.f;
 #pragma unroll
   for (int e = 0; e < 4; ++e) h[e] = x[e] != x[e] ? __uint_as_float(0x7fff0000u) : upper_half(x[e]);
+}
+__device__ __noinline__ void f32_cut_odd(float4 v, uint32_t at, int plane) {
+  float h[4], any = 0.f;
+  f32_first_odd(v, h);
   f32_store_planes(v, h, at, plane, any);
 }
 
+// A cut once for all column tiles, in the form of the GEMM's stages. grid (steps of 64 k, row tiles).
 template <int kT>
+__global__ void __launch_bounds__(256) f32_planes_kernel(const F32Params p) {
+  constexpr int kPlane = F32Tile<kT>::kPlaneA;
+  const int c = threadIdx.x & 15, r0 = threadIdx.x >> 4, k = blockIdx.x * kXK + 4 * c, m0 = blockIdx.y * kT;
+  const size_t at = static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x;
+  uint8_t* out = p.planes + at * (3 * kPlane) + r0 * 128 + (((c >> 1) ^ (r0 & 7)) * 16) + (c & 1) * 8;
+  griddep_launch_dependents();
+  griddep_wait();
+  float4 v[kT / 16];
+#pragma unroll
+  for (int i = 0; i < kT / 16; ++i) v[i] = f32_load4(p.A + static_cast<size_t>(min(m0 + r0 + 16 * i, p.M - 1)) * p.lda, k, p.K, p.vec_a);
+  uint32_t least = ~0u;
+#pragma unroll
+  for (int i = 0; i < kT / 16; ++i) {
+    float h[4], any = 0.f;
+    uint2 x[3];
+    f32_first_odd(v[i], h);
+    f32_planes(v[i], h, x, any);
+    least = min(least, f32_least(v[i]));
+#pragma unroll
+    for (int g = 0; g < 3; ++g) *reinterpret_cast<uint2*>(out + g * kPlane + i * 16 * 128) = x[g];
+  }
+  const int tiny = __syncthreads_or(least < 0x1ffffu);
+  if (threadIdx.x == 0) p.planes_tiny[at] = tiny;
+}
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
+// kPlanes: A has been cut by f32_planes_kernel and arrives by bulk copies
+template <int kT, bool kPlanes>
 __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params p) {
   using T = F32Tile<kT>;
   extern __shared__ uint8_t smem_raw[];
@@ -113,6 +168,7 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* tiny = tmem_slot + 2;   // an operand's upper half is zero and the operand is not
+  uint64_t* afull_bar = bars + 12;           // kPlanes: A's planes have landed
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x % p.parts;  // in the cluster
   const int n0 = blockIdx.x / p.parts * kXN, m0 = blockIdx.y * kT;
@@ -125,8 +181,9 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
       mbar_init(empty_bar + i, 1);
       mbar_init(dfull_bar + i, 1);
       mbar_init(dempty_bar + i, 4);
+      mbar_init(afull_bar + i, 1);
     }
-    mbar_init(done_bar, 1);
+    mbar_init(done_bar, kPlanes ? 2 : 1);
     *abort_flag = 0;
     *tiny = 0;
     mbar_fence_init();
@@ -221,7 +278,8 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
       bool ok = true;
       for (int s = 0; s < steps; ++s) {
         const uint32_t st = s & 1, phase = (s >> 1) & 1, main = s % T::kMain;
-        ok = mbar_wait(dempty_bar + main, ((s / T::kMain) & 1) ^ 1, abort_flag, kTimeout) && mbar_wait(full_bar + st, phase, abort_flag, kTimeout);
+        ok = mbar_wait(dempty_bar + main, ((s / T::kMain) & 1) ^ 1, abort_flag, kTimeout) && mbar_wait(full_bar + st, phase, abort_flag, kTimeout) &&
+             (!kPlanes || mbar_wait(afull_bar + st, phase, abort_flag, kTimeout));
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t at = smem_u32(smem + st * T::kStage);
@@ -247,53 +305,85 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
       }
       if (ok && steps > 0) umma_commit(done_bar);
     }
+    if (kPlanes && warp == 5) {
+      // ---------------------------------------------------------------- A's planes
+      const size_t first = static_cast<size_t>(blockIdx.y) * ((p.K + kXK - 1) / kXK) + k_begin / kXK;
+      if (lane == 0) {
+        fence_proxy_async();
+        int s = 0;
+        for (; s < steps; ++s) {
+          if (!mbar_wait(empty_bar + (s & 1), ((s >> 1) & 1) ^ 1, abort_flag, kTimeout)) break;
+          mbar_expect_tx(afull_bar + (s & 1), 3 * T::kPlaneA);
+          bulk_load(smem + (s & 1) * T::kStage + 3 * kXPlaneB, p.planes + (first + s) * (3 * T::kPlaneA), 3 * T::kPlaneA, afull_bar + (s & 1));
+        }
+        volatile uint32_t never = 0;   // the last copies have to land before shared memory is given back, also after an abort
+        for (int c = max(0, s - 2); c < s; ++c) mbar_wait(afull_bar + (c & 1), (c >> 1) & 1, &never, kTimeout);
+      }
+      __syncwarp();
+      uint32_t small = 0;
+      for (int s = lane; s < steps; s += 32) small |= __ldcg(p.planes_tiny + first + s);
+      if (__any_sync(0xffffffffu, small != 0u) && lane == 0) *tiny = 1;
+      __syncwarp();
+      if (lane == 0 && steps > 0) mbar_arrive(done_bar);
+    }
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ operands: half a warp per row of 64 k
     const int t = threadIdx.x - 256, c = t & 15, r0 = t >> 4;
     const int k0 = k_begin + 4 * c;
-    const float *rb[kXN / 16], *ra[kT / 16];
-    float4 vb[kXN / 16], va[kT / 16];
-#pragma unroll
-    for (int i = 0; i < kXN / 16; ++i) {   // behind the last row that row again: its results are not stored
-      rb[i] = p.B + static_cast<size_t>(min(n0 + r0 + 16 * i, p.N - 1)) * p.ldb;
-      vb[i] = f32_load4(rb[i], k0, k_end, p.vec_b);
-    }
-#pragma unroll
-    for (int i = 0; i < kT / 16; ++i) {
-      ra[i] = p.A + static_cast<size_t>(min(m0 + r0 + 16 * i, p.M - 1)) * p.lda;
-      va[i] = f32_load4(ra[i], k0, k_end, p.vec_a);
-    }
     // eight rows down the swizzle repeats: the offset inside a row is the same for all rows of this thread
     const uint32_t off = static_cast<uint32_t>(r0 * 128 + (((c >> 1) ^ (r0 & 7)) * 16) + (c & 1) * 8);
-    for (int s = 0; s < steps; ++s) {
-      const int next = k0 + (s + 1) * kXK;
-      if (!mbar_wait(empty_bar + (s & 1), ((s >> 1) & 1) ^ 1, abort_flag, kTimeout)) break;
-      const uint32_t at = smem_u32(smem + (s & 1) * T::kStage) + off;
-      float any = 0.f;
-      uint32_t least = ~0u;
+    constexpr int kRowsB = kXN / 16, kRowsA = kPlanes ? 0 : kT / 16;
+    constexpr int kDepth = kRowsA <= 2 ? 2 : 1;   // steps of loads in flight, as many as the registers hold
+    const float *rb[kRowsB], *ra[kRowsA + 1];
+    float4 vb[kDepth][kRowsB], va[kDepth][kRowsA + 1];
 #pragma unroll
-      for (int i = 0; i < kXN / 16; ++i) {
-        f32_cut(vb[i], at + i * 16 * 128, kXPlaneB, any, least);
-        vb[i] = f32_load4(rb[i], next, k_end, p.vec_b);
-      }
+    for (int i = 0; i < kRowsB; ++i) rb[i] = p.B + static_cast<size_t>(min(n0 + r0 + 16 * i, p.N - 1)) * p.ldb;   // behind the last row
 #pragma unroll
-      for (int i = 0; i < kT / 16; ++i) {
-        f32_cut(va[i], at + 3 * kXPlaneB + i * 16 * 128, T::kPlaneA, any, least);
-        va[i] = f32_load4(ra[i], next, k_end, p.vec_a);
-      }
-      if (least < 0x1ffffu) *tiny = 1;
-      if (any != any) {   // rare: this step's values are read again, and cut with a look at each
-#pragma unroll 1
-        for (int i = 0; i < kXN / 16 + kT / 16; ++i) {
-          const bool of_b = i < kXN / 16;
-          const int r = r0 + 16 * (of_b ? i : i - kXN / 16);
-          const float* row = of_b ? p.B + static_cast<size_t>(min(n0 + r, p.N - 1)) * p.ldb : p.A + static_cast<size_t>(min(m0 + r, p.M - 1)) * p.lda;
-          f32_cut_odd(f32_load4(row, next - kXK, k_end, of_b ? p.vec_b : p.vec_a), at + (of_b ? 0 : 3 * kXPlaneB) + (r - r0) * 128, of_b ? kXPlaneB : T::kPlaneA);
+    for (int i = 0; i < kRowsA; ++i) ra[i] = p.A + static_cast<size_t>(min(m0 + r0 + 16 * i, p.M - 1)) * p.lda;   // that row again: not stored
+#pragma unroll
+    for (int d = 0; d < kDepth; ++d) {
+#pragma unroll
+      for (int i = 0; i < kRowsB; ++i) vb[d][i] = f32_load4(rb[i], k0 + d * kXK, k_end, p.vec_b);
+#pragma unroll
+      for (int i = 0; i < kRowsA; ++i) va[d][i] = f32_load4(ra[i], k0 + d * kXK, k_end, p.vec_a);
+    }
+    bool ok = true;
+    for (int s0 = 0; s0 < steps && ok; s0 += 2) {
+#pragma unroll
+      for (int st = 0; st < 2; ++st) {
+        const int s = s0 + st, next = k0 + (s + kDepth) * kXK;
+        constexpr int kSets = kDepth - 1;
+        const int d = st & kSets;
+        if (s >= steps) break;
+        ok = mbar_wait(empty_bar + st, ((s >> 1) & 1) ^ 1, abort_flag, kTimeout);
+        if (!ok) break;
+        const uint32_t at = smem_u32(smem + st * T::kStage) + off;
+        float any = 0.f;
+        uint32_t least = ~0u;
+#pragma unroll
+        for (int i = 0; i < kRowsB; ++i) {
+          f32_cut(vb[d][i], at + i * 16 * 128, kXPlaneB, any, least);
+          vb[d][i] = f32_load4(rb[i], next, k_end, p.vec_b);
         }
+#pragma unroll
+        for (int i = 0; i < kRowsA; ++i) {
+          f32_cut(va[d][i], at + 3 * kXPlaneB + i * 16 * 128, T::kPlaneA, any, least);
+          va[d][i] = f32_load4(ra[i], next, k_end, p.vec_a);
+        }
+        if (least < 0x1ffffu) *tiny = 1;
+        if (any != any) {   // rare: this step's values are read again, and cut with a look at each
+#pragma unroll 1
+          for (int i = 0; i < kRowsB + kRowsA; ++i) {
+            const bool of_b = i < kRowsB;
+            const int r = r0 + 16 * (of_b ? i : i - kRowsB);
+            const float* row = of_b ? p.B + static_cast<size_t>(min(n0 + r, p.N - 1)) * p.ldb : p.A + static_cast<size_t>(min(m0 + r, p.M - 1)) * p.lda;
+            f32_cut_odd(f32_load4(row, next - kDepth * kXK, k_end, of_b ? p.vec_b : p.vec_a), at + (of_b ? 0 : 3 * kXPlaneB) + (r - r0) * 128, of_b ? kXPlaneB : T::kPlaneA);
+          }
+        }
+        fence_view_async_shared();
+        mbar_arrive(full_bar + st);
       }
-      fence_view_async_shared();
-      mbar_arrive(full_bar + (s & 1));
     }
   }
   __syncwarp();
@@ -325,27 +415,31 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
   cluster_sync_all();  // the others have read this CTA's partial tile
 }
 
-// Parts of K, from N and K alone: the fewest steps on the busiest of 148 SMs (one CTA each), where a CTA's start, its sum over the
-// parts and its end cost about as much as three steps. (148 whatever the device has: the parts are part of the result's rounding.)
+// Parts of K, from N and K alone: the fewest steps on the busiest SM, where a CTA's start, its sum over the parts and its end cost about
+// as much as four steps. A cluster's CTAs, one per SM, lie in one part of the chip, so clusters leave SMs over: 15 of eight run at a time
+// and not 18 (2048 x 5632, 100 rows: 16 clusters of eight, two waves, 53 us; of six, one wave, 35). The counts are a B200's, whatever the
+// device has: the parts are part of the result's rounding.
 static int f32_parts(int N, int K) {
+  constexpr int kClusters[kXMaxParts] = {148, 74, 45, 33, 26, 22, 15, 15};
   const int tiles = (N + kXN - 1) / kXN, steps = (K + kXK - 1) / kXK;
   int best = 1;
   long long least = 1ll << 62;
   for (int parts = 1; parts <= kXMaxParts && parts <= steps; ++parts) {
-    const long long cost = ((static_cast<long long>(tiles) * parts + 147) / 148) * ((steps + parts - 1) / parts + 3);
+    const long long waves = (tiles + kClusters[parts - 1] - 1) / kClusters[parts - 1];
+    const long long cost = waves * ((steps + parts - 1) / parts + 4);
     if (cost < least) least = cost, best = parts;
   }
   return best;
 }
 
-template <int kT>
-static int launch_gemm_f32(const F32Params& p, cudaStream_t stream) {
+template <int kT, bool kPlanes>
+static int launch_gemm_f32_form(const F32Params& p, cudaStream_t stream) {
   using T = F32Tile<kT>;
   static bool configured[64] = {false};
   int dev = 0;
   B200_CHECK_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    B200_CHECK_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<kT>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem));
+    B200_CHECK_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<kT, kPlanes>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem));
     configured[dev & 63] = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -362,37 +456,65 @@ static int launch_gemm_f32(const F32Params& p, cudaStream_t stream) {
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  B200_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<kT>, p));
+  if (kPlanes)
+    B200_CHECK_CUDA(launch_pdl(f32_planes_kernel<kT>, dim3((p.K + kXK - 1) / kXK, cfg.gridDim.y), dim3(256), 0, stream, p));
+  B200_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<kT, kPlanes>, p));
   return kOk;
+}
+template <int kT>
+static int launch_gemm_f32(F32Params& p, void* workspace, cudaStream_t stream) {
+  if (workspace == nullptr) return launch_gemm_f32_form<kT, false>(p, stream);
+  const size_t stages = static_cast<size_t>((p.M + kT - 1) / kT) * ((p.K + kXK - 1) / kXK);
+  p.planes = static_cast<uint8_t*>(workspace);
+  p.planes_tiny = reinterpret_cast<uint32_t*>(p.planes + stages * (3 * F32Tile<kT>::kPlaneA));
+  return launch_gemm_f32_form<kT, true>(p, stream);
 }
 
 }  // namespace b200
 
 using namespace b200;
 
-// status (device, nullable): raised when a wait inside the kernel runs out.
-B200_API int b200_gemm_f32_checked(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb, int ldc,
-                                   uint32_t* status, void* stream) {
+// row tiles of even height: 100 rows are one of 112, 150 two of 80
+static int f32_rows(int M) {
+  const int tiles = (M + 127) / 128;
+  return ((M + tiles - 1) / tiles + 15) / 16 * 16;
+}
+
+// Bytes of b200_gemm_f32_planes' workspace.
+B200_API long long b200_gemm_f32_workspace_bytes(int M, int K) {
+  if (M <= 0 || K <= 0) return 0;
+  const int rows = f32_rows(M);
+  return static_cast<long long>((M + rows - 1) / rows) * ((K + kXK - 1) / kXK) * (3ll * rows * kXK * 2 + 4);
+}
+
+// workspace (nullable, on a 16-byte boundary): A is cut into its planes there, once for all column tiles; results are the same. status
+// (device, nullable): raised when a wait inside the kernel runs out.
+B200_API int b200_gemm_f32_planes(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb, int ldc,
+                                  void* workspace, uint32_t* status, void* stream) {
   B200_REQUIRE(M > 0 && N > 0 && K > 0, "empty problem %dx%dx%d", M, N, K);
   B200_REQUIRE(lda >= K && ldb >= K && ldc >= N, "leading dimensions are smaller than the rows");
+  B200_REQUIRE(reinterpret_cast<uintptr_t>(workspace) % 16 == 0, "the workspace must be 16-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto aligned = [](const float* x, int ld) { return ld % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0; };
-  F32Params p = {A, B, C, M, N, K, f32_parts(N, K), 0, lda, ldb, ldc, aligned(A, lda), aligned(B, ldb), status};
+  F32Params p = {A, B, C, M, N, K, f32_parts(N, K), 0, lda, ldb, ldc, aligned(A, lda), aligned(B, ldb), status, nullptr, nullptr};
   p.part = ((K + p.parts - 1) / p.parts + kXK - 1) / kXK * kXK;
-  // row tiles of even height: 100 rows are one of 112, 150 two of 80
-  const int tiles = (M + 127) / 128, rows = (M + tiles - 1) / tiles;
-  switch ((rows + 15) / 16) {
-    case 1: return launch_gemm_f32<16>(p, s);
-    case 2: return launch_gemm_f32<32>(p, s);
-    case 3: return launch_gemm_f32<48>(p, s);
-    case 4: return launch_gemm_f32<64>(p, s);
-    case 5: return launch_gemm_f32<80>(p, s);
-    case 6: return launch_gemm_f32<96>(p, s);
-    case 7: return launch_gemm_f32<112>(p, s);
-    default: return launch_gemm_f32<128>(p, s);
+  switch (f32_rows(M) / 16) {
+    case 1: return launch_gemm_f32<16>(p, workspace, s);
+    case 2: return launch_gemm_f32<32>(p, workspace, s);
+    case 3: return launch_gemm_f32<48>(p, workspace, s);
+    case 4: return launch_gemm_f32<64>(p, workspace, s);
+    case 5: return launch_gemm_f32<80>(p, workspace, s);
+    case 6: return launch_gemm_f32<96>(p, workspace, s);
+    case 7: return launch_gemm_f32<112>(p, workspace, s);
+    default: return launch_gemm_f32<128>(p, workspace, s);
   }
+}
+// The same without a workspace.
+B200_API int b200_gemm_f32_checked(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb, int ldc,
+                                   uint32_t* status, void* stream) {
+  return b200_gemm_f32_planes(A, B, C, M, N, K, lda, ldb, ldc, nullptr, status, stream);
 }
 B200_API int b200_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, int lda, int ldb, int ldc,
                            void* stream) {
-  return b200_gemm_f32_checked(A, B, C, M, N, K, lda, ldb, ldc, nullptr, stream);
+  return b200_gemm_f32_planes(A, B, C, M, N, K, lda, ldb, ldc, nullptr, nullptr, stream);
 }
