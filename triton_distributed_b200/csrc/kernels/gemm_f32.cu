@@ -27,13 +27,13 @@
 // More than 16 rows of A are cut once, by a kernel in front, when the caller brings room for the planes: every column tile would cut them again,
 // and without them the registers hold two steps of B's loads instead of one. The planes and their sums are the same either way.
 // What bounds it: the products, 1830 of 2330 clocks a step at 100 rows (the planes' copies are asked for when their place is free and take
-// about as long as a step), and at the end of a CTA 13000 clocks for the partial tile and the sum over the parts. The rare cases are left to a
+// about as long as a step), and the start and end of a CTA. The rare cases are left to a
 // second look per step: a branch for every four values kept the loads, the arithmetic and the stores of neighbouring values apart.
 // us, back to back over several B, with A cut by every CTA and one step of loads -> now (planes from 17 rows on; parts by clusters that fit):
-//   11264 x 2048   1 row 40 -> 38    100 rows 61 -> 57    1024 rows 516 -> 451
-//   2048 x 5632    1 row 39 -> 24    100 rows 60 -> 36    1024 rows 297 -> 211
-//   22016 x 4096   1 row 154 -> 123  100 rows 223 -> 165  1024 rows 1954 -> 1384
-//   4096 x 11008   1 row 68 -> 62    100 rows 90 -> 81    1024 rows 925 -> 630
+//   11264 x 2048   1 row 40 -> 38    100 rows 61 -> 54    1024 rows 516 -> 411
+//   2048 x 5632    1 row 39 -> 24    100 rows 60 -> 34    1024 rows 297 -> 195
+//   22016 x 4096   1 row 154 -> 123  100 rows 223 -> 159  1024 rows 1954 -> 1347
+//   4096 x 11008   1 row 68 -> 62..68  100 rows 90 -> 82  1024 rows 925 -> 636
 // fp32 products on the CUDA cores with 4 x 4 outputs per thread took 227 us for 1 x 11264 x 2048 and 336 for 100 x 2048 x 5632.
 #include "b200/host.h"
 #include "b200/packed_f32.cuh"
@@ -152,6 +152,51 @@ __global__ void __launch_bounds__(256) f32_planes_kernel(const F32Params p) {
   if (threadIdx.x == 0) p.planes_tiny[at] = tiny;
 }
 
+// The partial tile from its sums of x1 y1 and the scaled groups in tensor memory: three warpgroups, every third 16 rows each, a thread
+// a column of C. (One warpgroup took 8800 of a CTA's 45000 clocks for it at 112 rows, with the other warps idle.)
+template <int kT>
+__device__ __forceinline__ void f32_finish(const F32Params& p, uint32_t tmem_base, float* out, int warp, int group, int m0, int n0, int k_begin,
+                                           int k_end, int steps, volatile uint32_t* abort_flag, volatile uint32_t* tiny) {
+  asm volatile("bar.sync 1, 384;" ::: "memory");   // x1 y1 is there, whatever became of the waits
+  const int n = (warp & 3) * 32 + (threadIdx.x & 31);
+  const uint32_t lanes = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  const bool ok = __all_sync(0xffffffffu, *abort_flag == 0u), small = *tiny != 0u;
+  tc_fence_after_sync();
+#pragma unroll 1
+  for (int h = group; h < kT / 16; h += 3) {
+    float* at = out + h * 16 * kXN + n;
+    uint32_t c1[16] = {}, c2[16] = {}, c3[16] = {};
+    __syncwarp();
+    if (steps > 0 && ok) {
+      tmem_ld_32x16(lanes + 128 + h * 16, c1);
+      tmem_ld_32x16(lanes + 256 + h * 16, c2);
+      tmem_ld_32x16(lanes + 384 + h * 16, c3);
+      tmem_ld_wait();
+    }
+    // rows whose sum is finite in x1 y1 but not in the scaled groups, or is no number where an infinity may have met such a value
+    uint32_t again = 0;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const float main = at[q * kXN];
+      const float rest = fmaf(fmaf(__uint_as_float(c3[q]), 0x1p-8f, __uint_as_float(c2[q])), 0x1p-8f, __uint_as_float(c1[q]));
+      const bool finite = fabsf(main) <= FLT_MAX;
+      const float v = finite ? fmaf(rest, 0x1p-8f, main) : main;
+      if (finite ? !(fabsf(rest) <= FLT_MAX) : small && main != main) again |= 1u << q;
+      at[q * kXN] = ok ? v : NAN;
+    }
+    if (!ok) again = 0u;
+    const float* b = p.B + static_cast<size_t>(min(n0 + n, p.N - 1)) * p.ldb;
+    for (uint32_t left = again; left != 0u; left &= left - 1) {
+      const int q = __ffs(left) - 1;
+      const float* a = p.A + static_cast<size_t>(min(m0 + h * 16 + q, p.M - 1)) * p.lda;
+      float sum = 0.f;
+      for (int k = k_begin; k < k_end; ++k) sum = fmaf(a[k], b[k], sum);
+      at[q * kXN] = sum;
+    }
+  }
+  tc_fence_before_sync();
+}
+
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
@@ -227,49 +272,15 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
       __syncwarp();
       if (lane == 0) mbar_arrive(dempty_bar + at);
     }
-    if (steps > 0 && ok) {
-      ok = mbar_wait(done_bar, 0, abort_flag, kTimeout);
-      tc_fence_after_sync();
-    }
-    // all products are done: the stages give way to the partial tile [kT][128]
+    if (steps > 0 && ok) mbar_wait(done_bar, 0, abort_flag, kTimeout);
+    // all products are done: the stages give way to the partial tile [kT][128], first of x1 y1
     float* out = reinterpret_cast<float*>(smem);
-    const int n = threadIdx.x;
-    // rows whose sum is finite in x1 y1 but not in the scaled groups, or is no number where an infinity may have met such a value
-    uint32_t again[(kT + 31) / 32] = {};
-    const bool small = ok && *tiny != 0u;
 #pragma unroll
-    for (int h = 0; h < kT / 16; ++h) {
-      uint32_t c1[16] = {}, c2[16] = {}, c3[16] = {};
-      if (steps > 0 && ok) {
-        tmem_ld_32x16(lanes + 128 + h * 16, c1);
-        tmem_ld_32x16(lanes + 256 + h * 16, c2);
-        tmem_ld_32x16(lanes + 384 + h * 16, c3);
-        tmem_ld_wait();
-      }
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const float2 pair = unpack2(acc[h * 8 + q / 2]);
-        const float main = (q & 1) ? pair.y : pair.x;
-        const float rest = fmaf(fmaf(__uint_as_float(c3[q]), 0x1p-8f, __uint_as_float(c2[q])), 0x1p-8f, __uint_as_float(c1[q]));
-        const bool finite = fabsf(main) <= FLT_MAX;
-        const float v = finite ? fmaf(rest, 0x1p-8f, main) : main;
-        if (finite ? !(fabsf(rest) <= FLT_MAX) : small && main != main) again[(h * 16 + q) / 32] |= 1u << ((h * 16 + q) & 31);
-        out[(h * 16 + q) * kXN + n] = ok ? v : NAN;
-      }
+    for (int r = 0; r < kT; ++r) {
+      const float2 pair = unpack2(acc[r / 2]);
+      out[r * kXN + threadIdx.x] = (r & 1) ? pair.y : pair.x;
     }
-    if (ok) {
-      const float* b = p.B + static_cast<size_t>(min(n0 + n, p.N - 1)) * p.ldb;
-#pragma unroll
-      for (int w = 0; w < (kT + 31) / 32; ++w)
-        for (uint32_t left = again[w]; left != 0u; left &= left - 1) {
-          const int t = w * 32 + __ffs(left) - 1;
-          const float* a = p.A + static_cast<size_t>(min(m0 + t, p.M - 1)) * p.lda;
-          float sum = 0.f;
-          for (int k = k_begin; k < k_end; ++k) sum = fmaf(a[k], b[k], sum);
-          out[t * kXN + n] = sum;
-        }
-    }
-    tc_fence_before_sync();
+    f32_finish<kT>(p, tmem_base, out, warp, 0, m0, n0, k_begin, k_end, steps, abort_flag, tiny);
   } else if (warp < 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp == 4 && elect_one()) {
@@ -385,6 +396,8 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
         mbar_arrive(full_bar + st);
       }
     }
+    if (steps > 0 && ok) mbar_wait(done_bar, 0, abort_flag, kTimeout);
+    f32_finish<kT>(p, tmem_base, reinterpret_cast<float*>(smem), warp, (warp >> 2) - 1, m0, n0, k_begin, k_end, steps, abort_flag, tiny);
   }
   __syncwarp();
   tc_fence_before_sync();
@@ -399,12 +412,17 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
       const int r = i / (kXN / 4), n = i % (kXN / 4) * 4;
       if (m0 + r >= p.M || n0 + n >= p.N) continue;
       float v[4] = {};
-      for (int q = 0; q < p.parts; ++q) {
-        float4 x;
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
-                     : "r"(mapa_u32(out + r * kXN + n, q)));
-        v[0] += x.x, v[1] += x.y, v[2] += x.z, v[3] += x.w;
+      for (int q0 = 0; q0 < p.parts; q0 += 4) {   // four reads on their way at a time
+        float4 x[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q0 + q < p.parts)
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(x[q].x), "=f"(x[q].y), "=f"(x[q].z), "=f"(x[q].w)
+                         : "r"(mapa_u32(out + r * kXN + n, q0 + q)));
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q0 + q < p.parts) v[0] += x[q].x, v[1] += x[q].y, v[2] += x[q].z, v[3] += x[q].w;
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e)
