@@ -115,8 +115,9 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(const uint4* __restrict__ 
 //   k heads  -> norm(gamma_k), rope -> k_cache[slot[t], h, :]
 //   v heads  -> v_cache[slot[t], h, :]
 // cos_sin is [max_pos, 128] = cos(64) | sin(64) in fp32. gamma pointers may be null (no head norm).
-// What bounds it: instructions. One warp per head re-read 512 bytes of cos and sin for 256 of the head and spent its instructions on
-// indices and on shuffles between partners. Here a group of heads shares indices, position, cos and sin, and no partner leaves its lane.
+// What bounds it: instructions (issue slots 62 %, 4.3 TB/s). One warp per head re-read 512 bytes of cos and sin for 256 of the head and spent
+// its instructions on indices and on shuffles between partners. Here a group of heads shares indices, position, cos and sin, and no
+// partner leaves its lane. 32 + 8 + 8 heads: 16384 tokens 244 us -> 94, 1167 tokens 19.4 -> 9.8, 8 tokens 1.5 either way.
 template <bool BF16, int kPairs>
 __global__ void __launch_bounds__(256) qk_norm_rope_kernel(const uint2* __restrict__ qkv, const int* __restrict__ positions,
                                                            const int64_t* __restrict__ slots, const uint2* q_gamma,
