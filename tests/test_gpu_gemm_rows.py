@@ -52,28 +52,6 @@ def test_gemm_rows_norm(M, N, K, swiglu):
     torch.testing.assert_close(y.double(), ref, rtol=2 ** -7, atol=2e-5)
 
 
-@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("M", [17, 32, 33, 250, 256])
-@pytest.mark.parametrize("N,K", [(1, 64), (8, 2048), (100, 192), (128, 4096), (592, 4096), (338, 7168)])
-def test_gemm_rows_groups(M, N, K, dtype):
-    """Groups of 16 tokens, the last one ragged, into a wider output; a row's result is that of 16 tokens alone."""
-    from triton_distributed_b200 import _lib, ops
-    torch.manual_seed(8)
-    x = torch.randn(M, K + 8, device="cuda").to(dtype)[:, :K]
-    w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(dtype)
-    wide = torch.full((M + 3, N + 5), 7.0, device="cuda", dtype=dtype)
-    seen, call = [], _lib.call
-    with pytest.MonkeyPatch.context() as m:
-        m.setattr(_lib, "call", lambda name, *args: (seen.append(name), call(name, *args)))
-        y = ops.gemm_skinny(x, w, wide[:M, :N])
-    assert seen == ["b200_gemm_rows_groups"]
-    # sums of K products of values around one in fp32, one rounding of the result
-    torch.testing.assert_close(y.double(), x.double() @ w.double().T, rtol=torch.finfo(dtype).eps, atol=2e-5)
-    assert torch.all(wide[M:] == 7.0) and torch.all(wide[:, N:] == 7.0)
-    for at in range(0, M - 15, 16):
-        assert torch.equal(ops.gemm_rows(x[at:at + 16], w), y[at:at + 16])
-
-
 def test_gemm_rows_refuses():
     from triton_distributed_b200 import _lib, ops
     x = torch.zeros(4, 128, device="cuda", dtype=torch.float16)

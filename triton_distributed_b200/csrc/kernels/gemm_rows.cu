@@ -21,9 +21,6 @@
 // result is), sums the squares of what it holds, and the row's factor is applied to the complete sums in fp32. The product with the gain must
 // stay finite in the storage type, so this is for bf16.
 //
-// For W of few rows (a router) the grid's second axis takes more tokens, 16 per CTA: the stream-K kernel shares a tile's sums of up to 256
-// tokens among its CTAs in global memory, which took 33 us at 256 tokens of 128 x 2048 (3.6 here, 7.4 -> 2.8 at 24).
-//
 // Role in the reference: F.linear, RMSNorm and the residual add of a decode step (python/triton_dist/layers/nvidia/tp_mlp.py:177-191,
 // tp_attn.py:240-271, models/qwen.py:92-120).
 #include "b200/elem.cuh"
@@ -89,7 +86,6 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   if (threadIdx.x == 0) abort_word = 0;
   // The first lane of a warp requests what the warp reads, into places that are the warp's own: at the start all of them (the
   // weights before the wait for the kernels in front), then each one again as soon as the warp has read it.
-  const int m0 = blockIdx.y * MB, tokens = min(MB, p.M - m0);   // this CTA's tokens
   int ask_tile = blockIdx.x, ask_span = warp, asked = warp;
   auto ask_next = [&]() {
     asked += kRowsWarps;
@@ -102,7 +98,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     tma_load_3d(s, &tmW, full + slot, 0, tile * R, span * p.kbs);
     if (kDual) tma_load_3d(s + p.w_bytes / 2, &tmW, full + slot, 0, p.N + tile * R, span * p.kbs);
   };
-  auto ask_x = [&](int slot, int span) { tma_load_3d(ring + slot * p.stage_bytes + p.w_bytes, &tmX, full + slot, 0, m0, span * p.kbs); };
+  auto ask_x = [&](int slot, int span) { tma_load_3d(ring + slot * p.stage_bytes + p.w_bytes, &tmX, full + slot, 0, 0, span * p.kbs); };
   while (ask_span >= p.spans) { ask_span -= p.spans; ask_tile += gridDim.x; }
   const int span0 = ask_span;
   if (lane == 0) {
@@ -232,13 +228,13 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll
     for (int j = 0; j < kOut; ++j) {
       const int i = threadIdx.x + j * 256, m = i / R, n = tile * R + i % R;
-      res[j] = p.residual != nullptr && m < tokens && n < p.N ? to_float(static_cast<const T*>(p.residual)[static_cast<size_t>(m0 + m) * p.ldc + n]) : 0.f;
+      res[j] = p.residual != nullptr && m < p.M && n < p.N ? to_float(static_cast<const T*>(p.residual)[static_cast<size_t>(m) * p.ldc + n]) : 0.f;
     }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < kOut; ++j) {
       const int i = threadIdx.x + j * 256, m = i / R, n = tile * R + i % R;
-      if (m >= tokens || n >= p.N || !ok) continue;
+      if (m >= p.M || n >= p.N || !ok) continue;
       float v = 0.f, u = 0.f;
 #pragma unroll
       for (int w = 0; w < kRowsWarps; ++w) {
@@ -256,7 +252,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
       if (kDual) v = v / (1.f + __expf(-v)) * u;
       const T y = from_float<T>(v + res[j]);
-      const size_t to = static_cast<size_t>(m0 + m) * p.ldc + n;
+      const size_t to = static_cast<size_t>(m) * p.ldc + n;
       if (p.out_f32) static_cast<float*>(p.C)[to] = to_float(y);
       else static_cast<T*>(p.C)[to] = y;
     }
@@ -282,10 +278,13 @@ constexpr int kRowsMaxGranules = 6;
 
 using namespace b200;
 
-static int gemm_rows_impl(const void* X, const void* W, void* C, int M, int N, int K, int ldx, int ldw, int ldc, int dual,
-                          const void* gamma, float eps, const void* residual, int out_f32, int dtype, uint32_t* status, void* stream) {
+// X [M <= 16, K] (pitch ldx), W [N, K] or [2 N, K] (dual; pitch ldw), C [M, N] (pitch ldc) of the same type (fp32 with out_f32).
+// gamma [K] (bf16 only) and residual [M, N] (pitch ldc) may be null. K must be a multiple of 64. dtype + kSettled: see host.h.
+B200_API int b200_gemm_rows(const void* X, const void* W, void* C, int M, int N, int K, int ldx, int ldw, int ldc, int dual,
+                            const void* gamma, float eps, const void* residual, int out_f32, int dtype, uint32_t* status, void* stream) {
   const bool settled = take_settled(dtype);
   B200_REQUIRE(dtype == kBF16 || dtype == kF16, "gemm_rows supports bf16/f16");
+  B200_REQUIRE(M >= 1 && M <= 16 && N >= 1, "gemm_rows handles 1..16 tokens, got %d", M);
   B200_REQUIRE(K >= 64 && K % 64 == 0, "gemm_rows: K (%d) must be a multiple of 64", K);
   B200_REQUIRE(gamma == nullptr || (dtype == kBF16 && K <= 16384 && reinterpret_cast<uintptr_t>(gamma) % 16 == 0),
                "gemm_rows: the norm is for bf16, K <= 16384 and a gain on a 16-byte boundary");
@@ -339,20 +338,6 @@ static int gemm_rows_impl(const void* X, const void* W, void* C, int M, int N, i
                   : (mb == 8 ? rows_kernel<false, 8, false>(granules) : rows_kernel<false, 16, false>(granules));
   // (one value for all calls: another thread's launch of the same kernel may need more than this one)
   B200_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem));
-  B200_CHECK_CUDA(launch_pdl(kernel, dim3(grid, (M + mb - 1) / mb), dim3(kRowsThreads), static_cast<size_t>(smem), static_cast<cudaStream_t>(stream), tw, tx, p));
+  B200_CHECK_CUDA(launch_pdl(kernel, dim3(grid), dim3(kRowsThreads), static_cast<size_t>(smem), static_cast<cudaStream_t>(stream), tw, tx, p));
   return kOk;
-}
-
-// X [M <= 16, K] (pitch ldx), W [N, K] or [2 N, K] (dual; pitch ldw), C [M, N] (pitch ldc) of the same type (fp32 with out_f32).
-// gamma [K] (bf16 only) and residual [M, N] (pitch ldc) may be null. K must be a multiple of 64. dtype + kSettled: see host.h.
-B200_API int b200_gemm_rows(const void* X, const void* W, void* C, int M, int N, int K, int ldx, int ldw, int ldc, int dual,
-                            const void* gamma, float eps, const void* residual, int out_f32, int dtype, uint32_t* status, void* stream) {
-  B200_REQUIRE(M >= 1 && M <= 16 && N >= 1, "gemm_rows handles 1..16 tokens, got %d", M);
-  return gemm_rows_impl(X, W, C, M, N, K, ldx, ldw, ldc, dual, gamma, eps, residual, out_f32, dtype, status, stream);
-}
-// The plain product for up to 256 tokens, 16 of them per CTA: for W of so few rows that the groups of tokens find SMs of their own.
-B200_API int b200_gemm_rows_groups(const void* X, const void* W, void* C, int M, int N, int K, int ldx, int ldw, int ldc, int dtype,
-                                   uint32_t* status, void* stream) {
-  B200_REQUIRE(M >= 1 && M <= 256 && N >= 1, "gemm_rows_groups handles 1..256 tokens, got %d", M);
-  return gemm_rows_impl(X, W, C, M, N, K, ldx, ldw, ldc, 0, nullptr, 0.f, nullptr, 0, dtype, status, stream);
 }

@@ -178,15 +178,6 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = Non
             and n_rows % (2 if swiglu else 1) == 0
             and (out is None or (out.shape == (M, N) and out.stride(1) == 1 and out.dtype == x.dtype))):
         return gemm_rows(x, w, out, swiglu, settled=settled)
-    # Few rows of w, a router's for one: groups of 16 tokens on SMs of their own, which read w once each. us, this and before: 128 x 2048
-    # at 24 tokens 2.8 and 7.4, at 128 3.2 and 18.9, at 256 3.6 and 33; 592 x 4096 at 24 tokens 4.1 and 9.7, at 256 30 and 50.
-    if (16 < M <= 256 and not swiglu and splits == 0 and epilogue is None and K % 64 == 0 and 64 <= K <= 7168 and 1 <= N <= 592 and N * K <= 592 * 4096
-            and w.shape[1] == K and w.dtype == x.dtype and (out is None or (out.shape == (M, N) and out.stride(1) == 1 and out.dtype == x.dtype))):
-        out = torch.empty((M, N), dtype=x.dtype, device=x.device) if out is None else out
-        _lib.call("b200_gemm_rows_groups", ptr(x), ptr(w), ptr(out), M, N, K, x.stride(0), w.stride(0), out.stride(0), dtype_code(x.dtype, settled),
-                  ptr(_pipeline_status(x.device)), stream_ptr())
-        _count()
-        return out
     own_output = epilogue is not None and epilogue.kind in (1, 2)
     if out is None and not own_output:
         out = torch.empty((M, N), dtype=x.dtype, device=x.device)
