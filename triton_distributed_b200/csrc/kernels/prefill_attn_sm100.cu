@@ -32,10 +32,11 @@
 // exponentials 370, without the rescaling 390), and in long calls the power cap. The special-function unit and the tensor core are busy 42 % of
 // the time each. Rescaling and storing by the softmax warps themselves took 450 us where it is 424 now; stored row by row from the registers
 // it was 525, since a warp that stores 32 rows at a time keeps the next item's rescaling waiting. Two threads per row (16 softmax warps)
-// took 470, steps of 64 keys with the next step's scores in front of this step's product 524: products of 64 columns are slow.
+// took 524 us for 508 over changing inputs, steps of 64 keys with the next step's scores in front of this step's product 565 for 500: products of
+// 64 columns are slow.
 // One query tile per CTA, P through shared memory, O in registers and a launch that transposed V
 // before it took 769 us for five causal sequences of 1 K to 3 K tokens (64 / 8 heads, bf16) and 851 for one of 16384 (8 / 1 heads);
-// this form 424 and 516 or less.
+// the softmax warps rescaling 450 and 516.
 //
 // Role in the reference: flash_attn_with_kvcache in layers/nvidia/tp_attn.py:194-195 (prefill) and the Triton
 // flash-attention consumer of the sequence-parallel all-gather path, kernels/nvidia/sp_ag_attention_intra_node.py:255-425.
