@@ -8,8 +8,9 @@ producer and consumer threads under thousands of random interleavings. The same 
 fail, which shows that the checker can see the hazard it is guarding against.
 
 What is modelled: the push gather of AG-GEMM (`csrc/kernels/gemm_sm100.cu`, communication warps and TMA producer), the
-slot / counter scheme of GEMM-RS (epilogue stores, signalling warp, reduce phase), and the barrier-free packet
-all-reduce (`csrc/kernels/allreduce_ll.cu`).
+slot / counter scheme of GEMM-RS (epilogue stores, signalling warp, reduce phase), the barrier-free packet
+all-reduce (`csrc/kernels/allreduce_ll.cu`), and the stage rings of the decode GEMMs (`csrc/kernels/gemm_skinny_sm100.cu`,
+`gemm_rows.cu`), the latter with waits that run out.
 """
 from __future__ import annotations
 
@@ -368,6 +369,86 @@ def test_decode_gemm_ring_publishing_before_arming_is_caught():
     with pytest.raises(Violation):
         for seed in range(300):
             _two_producer_ring_model(2, 12, random.Random(seed), publish_after_arming=False)
+
+
+# ---------------------------------------------------------------------------------------------- ring of the decode GEMM of few tokens
+def _rows_ring_model(warps, places, tiles, spans, late, rng, drain=True, by_cta=True):
+    """A CTA of `csrc/kernels/gemm_rows.cu` some of whose boxes (`late`, numbers of stages) land only after a wait for them has run
+    out. Stage i is warp i % warps', which has `places` places. Checked: no box is still on its way when the CTA gives its shared
+    memory back, every stored tile is complete or marked, and a mark comes with a raised status. `drain` / `by_cta` off: warps end
+    without waiting for what they requested / a thread looks at its own warp's waits alone."""
+    total = tiles * spans
+    flying, landed = set(), set()
+    sums = [[set() for _ in range(tiles)] for _ in range(warps)]   # stages that a warp has multiplied
+    arrived = [0] * (2 * tiles)                                    # of the CTA's barriers, two per tile
+    state = {"abort": False, "status": False, "out": 0}
+    stored = {}
+
+    def engine():
+        while state["out"] < warps:
+            ready = [i for i in flying if i not in late or state["abort"]]
+            if ready and rng.random() < 0.5:
+                i = rng.choice(sorted(ready))
+                flying.discard(i)
+                landed.add(i)
+            yield True
+
+    def warp(w):
+        asked, ok, at = w, True, w
+        while asked < total and asked < w + warps * places:
+            flying.add(asked)
+            asked += warps
+            yield True
+        for tile in range(tiles):
+            while at < (tile + 1) * spans:
+                while ok and at not in landed:
+                    if state["abort"] or (at in late and rng.random() < 0.2):   # somebody gave up, or this wait's budget is over
+                        state["abort"], ok = True, False
+                        for i in range(at, asked if drain else 0, warps):
+                            while i not in landed:
+                                yield True
+                    yield True
+                if ok:
+                    sums[w][tile].add(at)
+                    if asked < total:
+                        flying.add(asked)
+                        asked += warps
+                at += warps
+            for step in range(2):   # sums are in shared memory; they have been read
+                arrived[2 * tile + step] += 1
+                while arrived[2 * tile + step] < warps:
+                    yield False
+                if step == 0:
+                    whole = not state["abort"] if by_cta else ok
+                    stored[tile, w] = set().union(*(sums[v][tile] for v in range(warps))) if whole else None
+                yield True
+        if state["abort"]:
+            state["status"] = True
+        state["out"] += 1
+        if state["out"] == warps and flying:
+            raise Violation(f"boxes {sorted(flying)} land in shared memory that was given back")
+
+    _run([warp(w) for w in range(warps)] + [engine()], rng)
+    for (tile, w), got in stored.items():
+        if got is not None and got != set(range(tile * spans, (tile + 1) * spans)):
+            raise Violation(f"tile {tile} is stored without stages {set(range(tile * spans, (tile + 1) * spans)) - got}")
+    if any(got is None for got in stored.values()) != state["status"]:
+        raise Violation("incomplete results without a status, or a status without any")
+
+
+@pytest.mark.parametrize("warps,places,tiles,spans", [(2, 1, 1, 1), (4, 2, 3, 5), (8, 4, 2, 16), (8, 2, 3, 3)])
+def test_rows_gemm_expired_waits_leave_nothing_behind(warps, places, tiles, spans):
+    for seed in range(150):
+        rng = random.Random(seed)
+        late = set(rng.sample(range(tiles * spans), rng.randrange(0, min(4, tiles * spans) + 1)))
+        _rows_ring_model(warps, places, tiles, spans, late, rng)
+
+
+@pytest.mark.parametrize("fault", ["drain", "by_cta"])
+def test_rows_gemm_expired_waits_of_one_warp_alone_are_caught(fault):
+    with pytest.raises(Violation):
+        for seed in range(300):
+            _rows_ring_model(4, 2, 2, 8, {5, 11}, random.Random(seed), **{fault: False})
 
 
 # ---------------------------------------------------------------------------------------------- per-CTA call counters

@@ -51,7 +51,7 @@ struct RowsParams {
   const void* gamma;         // [K] or null
   const void* residual;      // [M, N], pitch ldc, or null
   void* C;
-  uint32_t* status;          // raised when a wait expires
+  uint32_t* status;          // raised when a wait expires; the tile's results are NaN then
 };
 
 __device__ __forceinline__ void ldmatrix_x2(uint32_t addr, uint32_t& r0, uint32_t& r1) {
@@ -149,8 +149,22 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       for (int e = 0; e < 4; ++e) acc[g][e] = 0.f;
     float sq[2] = {0.f, 0.f};   // squares of tokens lane / 4 and eight further, this lane's channels
     for (; at < first + p.spans; at += kRowsWarps) {
-      // after an expired wait the remaining rounds go by without work: all warps meet at the barriers below
-      ok = ok && mbar_wait(full + slot, phase, abort_flag, timeout_ns);
+      // after an expired wait the remaining rounds go by without work: all warps meet at the barriers below (one verdict per warp: the
+      // fragment loads and products are instructions of all its lanes)
+      if (ok) {
+        ok = __all_sync(0xffffffffu, mbar_wait(full + slot, phase, abort_flag, timeout_ns));
+        if (!ok && lane == 0) {   // boxes that are on their way have to land before shared memory is given back
+          volatile uint32_t never = 0;
+          int s = slot;
+          uint32_t ph = phase;
+          for (int i = at; i < asked; i += kRowsWarps) {
+            mbar_wait(full + s, ph, &never, timeout_ns);
+            s += kRowsWarps;
+            if (s >= p.stages) { s = warp; ph ^= 1; }
+          }
+        }
+        __syncwarp();
+      }
       if (ok) {
         uint32_t ws = smem_u32(ring + slot * p.stage_bytes), xs = ws + p.w_bytes;
         const uint32_t up = p.w_bytes / 2;
@@ -201,12 +215,11 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           ask_w(slot, ask_tile, ask_span);
           ask_x(slot, ask_span);
           ask_next();
-              }
+        }
       }
       slot += kRowsWarps;
       if (slot >= p.stages) { slot = warp; phase ^= 1; }
     }
-    if (!ok && lane == 0 && p.status != nullptr) *p.status = 1u;
     // ---- sums of the eight warps
     const int row = lane >> 2, col = (lane & 3) * 2;
 #pragma unroll
@@ -231,10 +244,11 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       res[j] = p.residual != nullptr && m < p.M && n < p.N ? to_float(static_cast<const T*>(p.residual)[static_cast<size_t>(m) * p.ldc + n]) : 0.f;
     }
     __syncthreads();
+    const bool whole = *abort_flag == 0u;   // no warp gave up: one that did left sums without its share
 #pragma unroll
     for (int j = 0; j < kOut; ++j) {
       const int i = threadIdx.x + j * 256, m = i / R, n = tile * R + i % R;
-      if (m >= p.M || n >= p.N || !ok) continue;
+      if (m >= p.M || n >= p.N) continue;
       float v = 0.f, u = 0.f;
 #pragma unroll
       for (int w = 0; w < kRowsWarps; ++w) {
@@ -251,13 +265,14 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         u *= s;
       }
       if (kDual) v = v / (1.f + __expf(-v)) * u;
-      const T y = from_float<T>(v + res[j]);
+      const T y = from_float<T>(whole ? v + res[j] : NAN);
       const size_t to = static_cast<size_t>(m) * p.ldc + n;
       if (p.out_f32) static_cast<float*>(p.C)[to] = to_float(y);
       else static_cast<T*>(p.C)[to] = y;
     }
     __syncthreads();   // the next tile's sums take the same place
   }
+  if (threadIdx.x == 0 && *abort_flag != 0u && p.status != nullptr) atomicMax(p.status, static_cast<uint32_t>(kStatusPipeTimeout));
 }
 
 using RowsKernel = void (*)(const CUtensorMap, const CUtensorMap, const RowsParams);
