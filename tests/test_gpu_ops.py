@@ -35,9 +35,11 @@ def test_gemm_skinny(M, N, K):
         y = ops.gemm_skinny(x, w, splits=splits)
         torch.cuda.synchronize()
         torch.testing.assert_close(y.float(), _ref_mm(x, w), rtol=2e-2, atol=2e-2)
-    # the scratch must be left clean: a second call gives the same answer
-    y2 = ops.gemm_skinny(x, w)
-    torch.testing.assert_close(y2.float(), _ref_mm(x, w), rtol=2e-2, atol=2e-2)
+    # the scratch must be left clean: another call (of at most 16 tokens without `splits` often runs on a kernel that has none) gives
+    # the same answer
+    for splits in (0, 3):
+        y2 = ops.gemm_skinny(x, w, splits=splits)
+        torch.testing.assert_close(y2.float(), _ref_mm(x, w), rtol=2e-2, atol=2e-2)
 
 
 @pytest.mark.parametrize("M,I,K", [(8, 3200, 5120), (4, 256, 128), (40, 1000, 520)])
@@ -109,10 +111,10 @@ def test_qk_norm_rope_and_cache_write():
     torch.testing.assert_close(vc[slots], qkv.view(T, -1, D)[:, Hq + Hkv:])
 
 
-@pytest.mark.parametrize("T,Hq,Hkv", [(1, 1, 1), (3, 8, 1), (2367, 4, 2), (2368, 4, 2), (1200, 8, 1), (800, 16, 8)])
+@pytest.mark.parametrize("T,Hq,Hkv", [(1, 1, 1), (3, 8, 1), (1184, 4, 2), (1185, 4, 2), (2367, 4, 2), (2368, 4, 2), (1200, 8, 1), (800, 16, 8)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_qk_norm_rope_groups_of_heads(T, Hq, Hkv, dtype):
-    """Two and eight heads a warp (eight from 16 warps an SM on), with groups that q, k and v share and that no head fills."""
+    """One and eight heads a warp (eight above 64 heads an SM), with groups that q, k and v share and that no head fills."""
     from triton_distributed_b200 import ops
     torch.manual_seed(14)
     D, n = 128, Hq + 2 * Hkv

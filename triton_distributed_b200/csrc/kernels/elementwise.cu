@@ -109,21 +109,89 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(const uint4* __restrict__ 
   }
 }
 
-// The fused projection qkv[T, (Hq + 2 Hkv) * 128], 2 * kPairs heads of a token per warp and half a warp per head: lane l of a half owns
-// elements 4l..4l+3 and their rotary partners, 64 further.
-//   q heads  -> norm(gamma_q), rope -> q_out[T, Hq, 128]
-//   k heads  -> norm(gamma_k), rope -> k_cache[slot[t], h, :]
+// One warp per (token, head) of the fused projection qkv[T, (Hq + 2 Hkv) * 128]. Lane l owns elements
+// 4l..4l+3 of the head; the rotary partner (i +- 64) sits in lane l ^ 16.
+//   q heads  -> RMSNorm(q_gamma) -> RoPE -> q_out[T, Hq, 128]
+//   k heads  -> RMSNorm(k_gamma) -> RoPE -> k_cache[slot[t], h, :]
 //   v heads  -> v_cache[slot[t], h, :]
 // cos_sin is [max_pos, 128] = cos(64) | sin(64) in fp32. gamma pointers may be null (no head norm).
-// What bounds it: instructions (issue slots 62 %, 4.3 TB/s). One warp per head re-read 512 bytes of cos and sin for 256 of the head and spent
-// its instructions on indices and on shuffles between partners. Here a group of heads shares indices, position, cos and sin, and no
-// partner leaves its lane. 32 + 8 + 8 heads: 16384 tokens 244 us -> 94, 1167 tokens 19.4 -> 9.8, 8 tokens 1.5 either way.
-template <bool BF16, int kPairs>
+template <bool BF16>
 __global__ void __launch_bounds__(256) qk_norm_rope_kernel(const uint2* __restrict__ qkv, const int* __restrict__ positions,
                                                            const int64_t* __restrict__ slots, const uint2* q_gamma,
                                                            const uint2* k_gamma, const float* __restrict__ cos_sin,
                                                            uint2* __restrict__ q_out, uint2* k_cache, uint2* v_cache,
                                                            int T, int Hq, int Hkv, float eps, bool settled) {
+  const int heads = Hq + 2 * Hkv;
+  griddep_launch_dependents();
+  const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  const int t = warp_global / heads;
+  const int h = warp_global - t * heads;
+  const uint2* gamma = h < Hq ? q_gamma : k_gamma;
+  // settled gains are fetched before the wait; past L1
+  if (!settled) griddep_wait();
+  const uint2 g = (gamma != nullptr && warp_global < T * heads && h < Hq + Hkv) ? __ldcg(gamma + lane) : make_uint2(0, 0);
+  griddep_wait();
+  if (warp_global >= T * heads) return;
+  const uint2 raw = qkv[(static_cast<size_t>(t) * heads + h) * 32 + lane];
+  const int64_t slot = slots ? slots[t] : t;
+  const int pos = positions[t];
+  if (h >= Hq + Hkv) {  // v: straight copy into the cache
+    if (slot >= 0) v_cache[(static_cast<size_t>(slot) * Hkv + (h - Hq - Hkv)) * 32 + lane] = raw;
+    return;
+  }
+  float x[4];
+  {
+    const float2 a = BF16 ? unpack_bf16x2(raw.x) : unpack_f16x2(raw.x);
+    const float2 b = BF16 ? unpack_bf16x2(raw.y) : unpack_f16x2(raw.y);
+    x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+  }
+  if (gamma) {
+    float ss = x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
+    ss = warp_sum(ss);
+    const float inv = rsqrtf(ss / 128.f + eps);
+    const float2 ga = BF16 ? unpack_bf16x2(g.x) : unpack_f16x2(g.x);
+    const float2 gb = BF16 ? unpack_bf16x2(g.y) : unpack_f16x2(g.y);
+    // round to the storage dtype after the norm, as a separate norm kernel would
+    float n0 = x[0] * inv * ga.x, n1 = x[1] * inv * ga.y, n2 = x[2] * inv * gb.x, n3 = x[3] * inv * gb.y;
+    const float2 r0 = BF16 ? unpack_bf16x2(pack_bf16x2(n0, n1)) : unpack_f16x2(pack_f16x2(n0, n1));
+    const float2 r1 = BF16 ? unpack_bf16x2(pack_bf16x2(n2, n3)) : unpack_f16x2(pack_f16x2(n2, n3));
+    x[0] = r0.x; x[1] = r0.y; x[2] = r1.x; x[3] = r1.y;
+  }
+  // neox rotation: out[i] = x[i] cos[i] - x[i+64] sin[i] (i < 64); out[i+64] = x[i+64] cos[i] + x[i] sin[i]
+  const int fi = (lane & 15) * 4;  // frequency index of this lane's first element
+  const float4 c = *reinterpret_cast<const float4*>(cos_sin + static_cast<size_t>(pos) * 128 + fi);
+  const float4 s = *reinterpret_cast<const float4*>(cos_sin + static_cast<size_t>(pos) * 128 + 64 + fi);
+  const float cs[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
+  float o[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float partner = __shfl_xor_sync(0xffffffffu, x[e], 16);
+    o[e] = lane < 16 ? x[e] * cs[e] - partner * sn[e] : x[e] * cs[e] + partner * sn[e];
+  }
+  uint2 outv;
+  outv.x = BF16 ? pack_bf16x2(o[0], o[1]) : pack_f16x2(o[0], o[1]);
+  outv.y = BF16 ? pack_bf16x2(o[2], o[3]) : pack_f16x2(o[2], o[3]);
+  if (h < Hq) {
+    q_out[(static_cast<size_t>(t) * Hq + h) * 32 + lane] = outv;
+  } else if (slot >= 0) {
+    k_cache[(static_cast<size_t>(slot) * Hkv + (h - Hq)) * 32 + lane] = outv;
+  }
+}
+
+// The same for many tokens: eight heads of a token per warp and half a warp per head, lane l of a half owns elements 4l..4l+3 and their rotary
+// partners, 64 further.
+// What bounds it: instructions (issue slots 62 %, 4.3 TB/s). One warp per head re-reads 512 bytes of cos and sin for 256 of the head and spends
+// its instructions on indices and on shuffles between partners. Here a group of heads shares indices, position, cos and sin, and no
+// partner leaves its lane. 32 + 8 + 8 heads: 16384 tokens 244 us -> 94, 1167 tokens 19.4 -> 9.8.
+constexpr int kRopePairs = 4;   // of heads per warp
+template <bool BF16>
+__global__ void __launch_bounds__(256) qk_norm_rope_groups_kernel(const uint2* __restrict__ qkv, const int* __restrict__ positions,
+                                                           const int64_t* __restrict__ slots, const uint2* q_gamma,
+                                                           const uint2* k_gamma, const float* __restrict__ cos_sin,
+                                                           uint2* __restrict__ q_out, uint2* k_cache, uint2* v_cache,
+                                                           int T, int Hq, int Hkv, float eps, bool settled) {
+  constexpr int kPairs = kRopePairs;
   const int heads = Hq + 2 * Hkv, groups = (heads + 2 * kPairs - 1) / (2 * kPairs);
   griddep_launch_dependents();
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -496,15 +564,16 @@ B200_API int b200_qk_norm_rope(const void* qkv, const int* positions, const int6
   B200_REQUIRE(dtype == kBF16 || dtype == kF16, "qk_norm_rope supports bf16/f16");
   B200_REQUIRE(head_dim == 128, "qk_norm_rope is specialised for head_dim 128, got %d", head_dim);
   if (T == 0) return kOk;
-  // Eight heads a warp where that leaves every SM 16 warps or more, two where the step is small and every warp's chain counts.
-  const int heads = Hq + 2 * Hkv;
-  const bool many = static_cast<long long>(T) * ((heads + 7) / 8) >= 16ll * sm_count();
-  const int per = many ? 8 : 2;
-  const long long warps = static_cast<long long>(T) * ((heads + per - 1) / per);
+  // Eight heads a warp where one warp per head would need a second wave (64 warps run on an SM). us with one and with eight, by heads per SM:
+  // 35 (16 + 4 heads, 256 tokens) 2.7, 2.9; 41 (32 + 16, 128) 2.9, 2.8; 55 (4 + 4, 1024) 3.1, 3.2; 54 (8 + 2, 800) 3.8, 3.9; 69 (8 + 2, 1024) 5.2,
+  // 4.2; 83 (32 + 16, 256) 5.6, 3.7. Two heads a warp were 3 to 24 % slower than one below that.
+  const int heads = Hq + 2 * Hkv, groups = (heads + 2 * kRopePairs - 1) / (2 * kRopePairs);
+  const bool many = static_cast<long long>(T) * heads > 64ll * sm_count();
+  const long long warps = static_cast<long long>(T) * (many ? groups : heads);
   const int grid = static_cast<int>((warps + 7) / 8);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  auto* kernel = dtype == kBF16 ? (many ? qk_norm_rope_kernel<true, 4> : qk_norm_rope_kernel<true, 1>)
-                                : (many ? qk_norm_rope_kernel<false, 4> : qk_norm_rope_kernel<false, 1>);
+  auto* kernel = dtype == kBF16 ? (many ? qk_norm_rope_groups_kernel<true> : qk_norm_rope_kernel<true>)
+                                : (many ? qk_norm_rope_groups_kernel<false> : qk_norm_rope_kernel<false>);
   B200_CHECK_CUDA(launch_pdl(kernel, grid, 256, 0, s, static_cast<const uint2*>(qkv), positions, slots, static_cast<const uint2*>(q_gamma),
                              static_cast<const uint2*>(k_gamma), cos_sin, static_cast<uint2*>(q_out), static_cast<uint2*>(k_cache),
                              static_cast<uint2*>(v_cache), T, Hq, Hkv, eps, settled));
