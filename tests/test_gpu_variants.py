@@ -90,6 +90,33 @@ def test_prefill_attention_matches_reference(lens_q, lens_k, Hq, Hkv, causal):
         torch.testing.assert_close(out[qs:qs + lq].float(), want, rtol=3e-2, atol=3e-2)
 
 
+@pytest.mark.parametrize("lens_q,lens_k,Hq,Hkv,dk,dv", [
+    ([1, 16, 128], [1, 16, 128], 8, 2, 128, 128),              # one step
+    ([129, 389, 40], [129, 389, 40], 8, 2, 128, 128), ([300, 5], [300, 700], 8, 8, 128, 136),   # two row blocks of a head; a cached prefix
+    ([100, 1, 500], [100, 300, 500], 4, 4, 72, 72), ([700, 260], [1200, 260], 8, 1, 64, 64), ([40], [1000], 6, 2, 40, 200)])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_prefill_attention_forms_agree(lens_q, lens_k, Hq, Hkv, dk, dv, causal, dtype):
+    """Small calls have the softmax warps rescale and store, larger ones warps of their own: the same bits, and those of the formula."""
+    from itertools import accumulate
+    from triton_distributed_b200 import ops
+    torch.manual_seed(31)
+    cu_q, cu_k = (torch.tensor([0, *accumulate(n)], dtype=torch.int32, device="cuda") for n in (lens_q, lens_k))
+    q, k, v = (torch.randn(sum(n), h, d, device="cuda").to(dtype) for n, h, d in ((lens_q, Hq, dk), (lens_k, Hkv, dk), (lens_k, Hkv, dv)))
+    gate = torch.randn(sum(lens_q), Hq, device="cuda").to(dtype)
+    small = ops.prefill_attention(q, k, v, cu_q, cu_k, max(lens_q), max(lens_k), dk ** -0.5, causal, gate=gate)
+    assert torch.equal(small, ops.prefill_attention(q, k, v, cu_q, cu_k, max(lens_q), 1 << 20, dk ** -0.5, causal, gate=gate))
+    ops.check_pipeline_status()
+    for b, (n, m) in enumerate(zip(lens_q, lens_k)):
+        qs, ks, vs = q[cu_q[b]:cu_q[b] + n].double(), k[cu_k[b]:cu_k[b] + m].double(), v[cu_k[b]:cu_k[b] + m].double()
+        s = torch.einsum("qhd,khd->hqk", qs, ks.repeat_interleave(Hq // Hkv, 1)) * dk ** -0.5
+        if causal:
+            s.masked_fill_(torch.ones(n, m, dtype=torch.bool, device="cuda").triu(m - n + 1), -torch.inf)
+        want = torch.einsum("hqk,khd->qhd", s.softmax(-1), vs.repeat_interleave(Hq // Hkv, 1)) * torch.sigmoid(gate[cu_q[b]:cu_q[b] + n].double())[..., None]
+        # probabilities and result are rounded once each: half a unit in the last place of both
+        assert (small[cu_q[b]:cu_q[b] + n].double() - want).norm() <= torch.finfo(dtype).eps * want.norm()
+
+
 def test_prefill_attention_reads_keys_in_place():
     """Keys of every sequence start at a fixed stride in a larger slot array (a cache whose sequences own contiguous
     runs of slots); rows beyond a sequence's length hold garbage that must not be read into the result."""

@@ -9,7 +9,8 @@
 // turn: published as ping-pong scheduling, FlashAttention-3, Shah et al. 2024):
 //   warps 0-3   softmax of tile 0, one thread per query row
 //   warps 4-7   softmax of tile 1
-//   warps 8-11  rescale O of either tile while the softmax warps compute the exponentials, and store the finished rows
+//   warps 8-11  rescale O of either tile while the softmax warps compute the exponentials, and store the finished rows (not in small
+//               calls, where the softmax warps do both: prefill_helped; the warps below are 8 to 10 then)
 //   warp 12     TMA producer: both Q tiles of an item, then K and V tiles through their rings (128-byte swizzle)
 //   warp 13     one elected thread issues tcgen05.mma, for each step and tile O += P V of this step, then S = Q K^T of the next
 //   warp 14     asks the hardware for the next item (cluster launch control) while the current one is worked on
@@ -57,13 +58,14 @@ constexpr int prefill_k_stages(int dk_atoms) { return dk_atoms <= 3 ? 2 : 1; }
 constexpr int prefill_v_stages(int dk_atoms) { return dk_atoms <= 2 ? 2 : 1; }
 // Output rows go to memory through shared memory, a warp's 32 rows at once, where rows of Q and K leave 32 KB for it.
 constexpr bool prefill_staged(int dk_atoms) { return dk_atoms <= 2; }
-constexpr int prefill_smem(int dk_atoms) {
+constexpr int prefill_smem(int dk_atoms, bool helped) {
   return 2 * dk_atoms * kPAtom /*Q*/ + prefill_k_stages(dk_atoms) * dk_atoms * kPAtom /*K*/ + prefill_v_stages(dk_atoms) * kPTile /*V*/ +
-         1024 + 256 + 2 * kPM * 4 /*factors*/ + (prefill_staged(dk_atoms) ? kPM * kPD * 2 : 0);
+         1024 + 256 + (helped ? 2 * kPM * 4 /*factors*/ + (prefill_staged(dk_atoms) ? kPM * kPD * 2 : 0) : 0);
 }
-constexpr int kPThreads = 512;
 // 512 threads start with 128 registers each; 2 x 128 x softmax + 128 x rescaling + 128 x others is the same total. Who stores needs more.
-constexpr int prefill_softmax_regs(int dk_atoms) { return prefill_staged(dk_atoms) ? 176 : 184; }
+// 384 threads (without the rescaling warps) start with 168: 2 x 128 x 216 + 128 x 72.
+constexpr int prefill_threads(bool helped) { return helped ? 512 : 384; }
+constexpr int prefill_softmax_regs(int dk_atoms, bool helped) { return !helped ? 216 : prefill_staged(dk_atoms) ? 176 : 184; }
 constexpr int prefill_scale_regs(int dk_atoms) { return prefill_staged(dk_atoms) ? 88 : 72; }
 constexpr int kPOtherRegs = 72;
 
@@ -183,12 +185,15 @@ __device__ __forceinline__ void prefill_store(const PrefillParams& p, const Pref
   }
 }
 
-template <int kDkAtoms, bool BF16>
-__global__ void __launch_bounds__(kPThreads, 1)
+// kHelped: four more warps rescale and, where shared memory allows, store
+template <int kDkAtoms, bool BF16, bool kHelped>
+__global__ void __launch_bounds__(prefill_threads(kHelped), 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const PrefillParams p) {
   constexpr int kKSt = prefill_k_stages(kDkAtoms), kVSt = prefill_v_stages(kDkAtoms);
   constexpr int kQkTile = kDkAtoms * kPAtom;
+  constexpr bool kStaged = kHelped && prefill_staged(kDkAtoms);
+  constexpr int kProducer = kHelped ? 12 : 8;   // the first warp behind those of the rows
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;                   // [2 tiles][atoms]
@@ -227,21 +232,21 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(v_full + i, 1);
       mbar_init(v_empty + i, 1);
       mbar_init(s_full + i, 1);
-      mbar_init(p_full + i, 8);
+      mbar_init(p_full + i, kHelped ? 8 : 4);
       mbar_init(o_full + i, 1);
       mbar_init(o_empty + i, 4);
       mbar_init(c_full + i, 4);
       mbar_init(f_full + i, 4);
     }
     mbar_init(next_full, 1);
-    mbar_init(next_empty, 14);  // producer, MMA issuer, eight softmax warps, four that rescale
+    mbar_init(next_empty, kProducer + 2);  // producer, MMA issuer and all warps in front of them
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
   }
-  if (warp == 15) tmem_alloc(tmem_slot, 512);
+  if (warp == kProducer + 3) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -260,9 +265,9 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     return more;
   };
 
-  if (warp >= 12) {
+  if (warp >= kProducer) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPOtherRegs));
-    if (warp == 12) {
+    if (warp == kProducer) {
       // ---------------------------------------------------------------- TMA producer
       if (elect_one()) {
         int kc = 0, vc = 0, qc = 0;
@@ -310,7 +315,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       }
       __syncwarp();
-    } else if (warp == 13) {
+    } else if (warp == kProducer + 1) {
       // ---------------------------------------------------------------- MMA issuer
       if (elect_one()) {
         const uint32_t idesc_s = umma_idesc_f16(kPM, kPN, BF16);
@@ -388,7 +393,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       }
       __syncwarp();
-    } else if (warp == 14) {
+    } else if (warp == kProducer + 2) {
       // ---------------------------------------------------------------- next items
       if (elect_one()) {
         bool more = true;
@@ -407,7 +412,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       __syncwarp();
     }
-  } else if (warp >= 8) {
+  } else if (kHelped && warp >= 8) {
     // ------------------------------------------------------------------ rescaling and output, one thread per query row of either tile
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(prefill_scale_regs(kDkAtoms)));
     const int row = (warp & 3) * 32 + lane;
@@ -446,7 +451,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       }
       // ---- the rows' output
-      for (int t = 0; t < 2 && ok && prefill_staged(kDkAtoms); ++t) {
+      for (int t = 0; t < 2 && ok && kStaged; ++t) {
         const int steps = w.steps_of(t);
         float inv = 0.f;
         if (steps > 0) {
@@ -457,17 +462,17 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           tc_fence_after_sync();
           inv = s_factor[t * kPM + row];
         }
-        prefill_store<prefill_staged(kDkAtoms), BF16>(p, w, t, steps, o_lanes + t * kPD, inv, s_out + (warp & 3) * 32 * 256, o_empty + t);
+        prefill_store<kStaged, BF16>(p, w, t, steps, o_lanes + t * kPD, inv, s_out + (warp & 3) * 32 * 256, o_empty + t);
       }
       if (!ok || !advance(i, true)) break;
     }
   } else {
     // ------------------------------------------------------------------ softmax, one thread per query row
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(prefill_softmax_regs(kDkAtoms)));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(prefill_softmax_regs(kDkAtoms, kHelped)));
     const int t = warp >> 2;  // tile
     const int row = (warp & 3) * 32 + lane;
     const uint32_t lanes = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-    const uint32_t s_addr = lanes + t * kPN;
+    const uint32_t s_addr = lanes + t * kPN, o_addr = lanes + 2 * kPN + t * kPD;
     int sc = 0, oc = 0, vc = 0;
     bool ok = true;
     for (int i = 0; ok; ++i) {
@@ -502,7 +507,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2e;
         if (j == 0) {
           ref = top;
-        } else {
+        } else if (kHelped) {
           // (the factors of the step before have been used: this step's scores were issued behind that step's product)
           float corr = 1.f;
           if (top > ref) {
@@ -513,6 +518,24 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           s_factor[t * kPM + row] = corr;
           __syncwarp();
           if (lane == 0) mbar_arrive(c_full + t);
+        } else if (__any_sync(0xffffffffu, top > ref)) {
+          // the scores of this step were issued after the tile's last product, so O is complete and nothing writes it now
+          float corr = 1.f;
+          if (top > ref) {
+            corr = fast_exp2(ref - top);
+            ref = top;
+          }
+          sum *= corr;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32(o_addr + c * 32, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
+            tmem_st_32x32(o_addr + c * 32, o);
+          }
+          tmem_st_wait();
         }
         const float base = ref == -INFINITY ? 0.f : ref;
         const f32x2 scale2 = pack2(p.scale_log2e, p.scale_log2e), base2 = pack2(-base, -base);
@@ -546,7 +569,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(p_full + t);
-          if (j == 0) mbar_arrive(p_full + t);   // for the warp that rescales: nothing to do yet
+          if (kHelped && j == 0) mbar_arrive(p_full + t);   // for the warp that rescales: nothing to do yet
         }
       }
       vc += w.n;
@@ -563,15 +586,15 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // The last step's factor may still be needed: it has been used once the item's last product is done.
         ok = __all_sync(0xffffffffu, mbar_wait(o_full + t, oc++ & 1, abort_flag, timeout_ns));
         if (!ok) break;
-        if (prefill_staged(kDkAtoms)) {
+        if (kStaged) {
           s_factor[t * kPM + row] = inv;
           __syncwarp();
           if (lane == 0) mbar_arrive(f_full + t);
         }
       }
-      if (!prefill_staged(kDkAtoms)) {   // eight warps store faster than four
+      if (!kStaged) {   // eight warps store faster than four
         tc_fence_after_sync();
-        prefill_store<false, BF16>(p, w, t, steps, tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 2 * kPN + t * kPD, steps > 0 ? inv : 0.f, nullptr, o_empty + t);
+        prefill_store<false, BF16>(p, w, t, steps, o_addr, inv, nullptr, o_empty + t);
       }
       if (!advance(i, true)) break;
     }
@@ -580,29 +603,42 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // ---------------------------------------------------------------------- teardown
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 15) tmem_dealloc(tmem_base, 512);
+  if (warp == kProducer + 3) tmem_dealloc(tmem_base, 512);
   if (threadIdx.x == 0 && *abort_flag != 0u && p.status != nullptr) atomicMax(p.status, static_cast<uint32_t>(kStatusPipeTimeout));
 }
 
-template <int kDkAtoms>
-static int launch_prefill_atoms(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p, dim3 grid,
-                                cudaStream_t s) {
+// Whether the rescaling warps pay: their hand-overs and the rows' way through shared memory add to the time of an item, which is all there is
+// when the items run at once over few keys. us without them and with them (8 / 2 heads, causal, 128 columns): 16 tokens 7.8, 9.2; 300 tokens
+// 12.3, 13.5; 3 x 389 14.7, 15.7; 2 x 700 19.3, 20.0; 1000 24.4, 24.2; 2000 41.6, 41.1; 8 x 16 tokens of 64 / 8 heads (256 items) 13.2, 14.5; 3 x 389
+// tokens of 32 / 8 heads (192 items) 25.3, 23.8. Not causal: 100 tokens 8.8, 9.5; 300 tokens 13.6, 13.6. Rows of 64 columns, causal: 1000 tokens
+// 22.4, 23.1; 1400 29.1, 29.1; 1400 of 32 / 8 heads (176 items, of which those of the first rows are short) 32.6, 33.8; not causal: 1000 tokens
+// 22.6, 23.0; 1400 29.5, 29.3. Wider rows are no slower with them at any size (192 x 192, 3 x 389 tokens: 30.0, 27.6).
+static bool prefill_helped(int dk_atoms, long long items, bool causal, int max_k) {
+  if (!prefill_staged(dk_atoms)) return true;
+  if (max_k <= kPN) return false;
+  const int few = dk_atoms == 1 ? (causal ? 1536 : 1280) : (causal ? 768 : 0);
+  return max_k > few || items > (dk_atoms == 1 && causal ? 3 * sm_count() / 2 : sm_count());
+}
+
+template <int kDkAtoms, bool kHelped>
+static int launch_prefill_form(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p, dim3 grid, cudaStream_t s) {
+  constexpr int kSmem = prefill_smem(kDkAtoms, kHelped), kThreads = prefill_threads(kHelped);
   static bool configured[64] = {false};
   int dev = 0;
   B200_CHECK_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    B200_CHECK_CUDA(cudaFuncSetAttribute(prefill_attn_kernel<kDkAtoms, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, prefill_smem(kDkAtoms)));
-    B200_CHECK_CUDA(cudaFuncSetAttribute(prefill_attn_kernel<kDkAtoms, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, prefill_smem(kDkAtoms)));
+    B200_CHECK_CUDA(cudaFuncSetAttribute(prefill_attn_kernel<kDkAtoms, true, kHelped>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    B200_CHECK_CUDA(cudaFuncSetAttribute(prefill_attn_kernel<kDkAtoms, false, kHelped>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     configured[dev & 63] = true;
   }
-  if (p.bf16) prefill_attn_kernel<kDkAtoms, true><<<grid, kPThreads, prefill_smem(kDkAtoms), s>>>(tq, tk, tv, p);
-  else prefill_attn_kernel<kDkAtoms, false><<<grid, kPThreads, prefill_smem(kDkAtoms), s>>>(tq, tk, tv, p);
+  if (p.bf16) prefill_attn_kernel<kDkAtoms, true, kHelped><<<grid, kThreads, kSmem, s>>>(tq, tk, tv, p);
+  else prefill_attn_kernel<kDkAtoms, false, kHelped><<<grid, kThreads, kSmem, s>>>(tq, tk, tv, p);
   B200_CHECK_CUDA(cudaGetLastError());
   return kOk;
 }
 
 static int prefill_launch(const void* q, int64_t ldq, const void* k, const void* v, int v_packed, const int* cu_q,
-                          const int* cu_k, const int* k_lens, int B, int total_q, int total_k, int max_q, int Hq, int Hkv, int dk, int dv, float scale,
+                          const int* cu_k, const int* k_lens, int B, int total_q, int total_k, int max_q, int max_k, int Hq, int Hkv, int dk, int dv, float scale,
                           int causal, const float* sink, const void* gate, int ldg, void* out, int dtype, uint32_t* status, cudaStream_t s) {
   CUtensorMap tq, tk, tv;
   int rc = make_tma_3d(&tq, q, dtype, dk, Hq, total_q, dk, static_cast<uint64_t>(ldq), 64, 1, kPM, true);
@@ -623,11 +659,13 @@ static int prefill_launch(const void* q, int64_t ldq, const void* k, const void*
   const int rows = p.pair_heads ? kPM : 2 * kPM;
   const dim3 grid((p.pair_heads ? Hq / 2 : Hq) * p.v_chunks, (max_q + rows - 1) / rows, B);
   B200_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "prefill attention grid is too large");
-  switch ((dk + 63) / 64) {
-    case 1: return launch_prefill_atoms<1>(tq, tk, tv, p, grid, s);
-    case 2: return launch_prefill_atoms<2>(tq, tk, tv, p, grid, s);
-    case 3: return launch_prefill_atoms<3>(tq, tk, tv, p, grid, s);
-    default: return launch_prefill_atoms<4>(tq, tk, tv, p, grid, s);
+  const int atoms = (dk + 63) / 64;
+  const bool helped = prefill_helped(atoms, static_cast<long long>(grid.x) * grid.y * grid.z, causal != 0, max_k);
+  switch (atoms) {
+    case 1: return helped ? launch_prefill_form<1, true>(tq, tk, tv, p, grid, s) : launch_prefill_form<1, false>(tq, tk, tv, p, grid, s);
+    case 2: return helped ? launch_prefill_form<2, true>(tq, tk, tv, p, grid, s) : launch_prefill_form<2, false>(tq, tk, tv, p, grid, s);
+    case 3: return launch_prefill_form<3, true>(tq, tk, tv, p, grid, s);
+    default: return launch_prefill_form<4, true>(tq, tk, tv, p, grid, s);
   }
 }
 
@@ -652,7 +690,7 @@ B200_API int b200_prefill_attention_direct(const void* q, const void* k, const v
   B200_REQUIRE(Hkv > 0 && Hq % Hkv == 0, "Hq (%d) must be a multiple of Hkv (%d)", Hq, Hkv);
   B200_REQUIRE(B >= 1 && max_q >= 1 && max_k >= 1 && total_q >= 1 && total_k >= 1, "empty problem");
   B200_REQUIRE(scale > 0.f, "the score scale must be positive");
-  return prefill_launch(q, static_cast<int64_t>(Hq) * dk, k, v, 0, cu_q, cu_k, k_lens, B, total_q, total_k, max_q, Hq, Hkv, dk, dv, scale,
+  return prefill_launch(q, static_cast<int64_t>(Hq) * dk, k, v, 0, cu_q, cu_k, k_lens, B, total_q, total_k, max_q, max_k, Hq, Hkv, dk, dv, scale,
                         causal, nullptr, gate, ldg, out, dtype, status, static_cast<cudaStream_t>(stream));
 }
 
@@ -698,6 +736,6 @@ B200_API int b200_prefill_attention_vt(const void* q, long long ldq, const void*
   B200_REQUIRE(dk >= 8 && dk % 8 == 0 && dk <= 256 && dv >= 8 && dv % 8 == 0 && ldq % 8 == 0 && total_k % 8 == 0,
                "prefill attention needs dk (%d) <= 256, and dk, dv (%d), ldq, total_k (%d) in multiples of 8", dk, dv, total_k);
   B200_REQUIRE(scale > 0.f, "the score scale must be positive");
-  return prefill_launch(q, ldq, k, vt, 1, cu_q, cu_k, k_lens, B, total_q, total_k, max_q, Hq, Hkv, dk, dv, scale, causal, sink,
+  return prefill_launch(q, ldq, k, vt, 1, cu_q, cu_k, k_lens, B, total_q, total_k, max_q, total_k, Hq, Hkv, dk, dv, scale, causal, sink,
                         nullptr, 0, out, dtype, status, static_cast<cudaStream_t>(stream));
 }
