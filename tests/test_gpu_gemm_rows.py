@@ -52,6 +52,24 @@ def test_gemm_rows_norm(M, N, K, swiglu):
     torch.testing.assert_close(y.double(), ref, rtol=2 ** -7, atol=2e-5)
 
 
+def test_status_word_is_made_in_front_of_a_capture(monkeypatch):
+    """A word that a capture made would be cleared by every replay, and read before the first."""
+    from triton_distributed_b200 import ops
+    x, w = torch.randn(8, 256, device="cuda").bfloat16(), torch.randn(512, 256, device="cuda").bfloat16()
+    monkeypatch.setattr(ops, "_pipe_status", {})
+    ops.reserve_skinny_scratch(x.device, 1, 1)
+    words = dict(ops._pipe_status)
+    assert len(words) == 1
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.gemm_skinny(x, w)
+    assert ops._pipe_status == words
+    words[x.device.index].fill_(3)
+    graph.replay()
+    with pytest.raises(RuntimeError):
+        ops.check_pipeline_status()
+
+
 def test_gemm_rows_refuses():
     from triton_distributed_b200 import _lib, ops
     x = torch.zeros(4, 128, device="cuda", dtype=torch.float16)

@@ -89,8 +89,10 @@ _skinny_scratch = _SkinnyScratch()
 
 
 def reserve_skinny_scratch(device, floats: int, tiles: int) -> None:
-    """Pre-size the split-K scratch (call before CUDA-graph capture so no allocation happens inside)."""
+    """Pre-size the split-K scratch and make the status word of the decode GEMM that needs no scratch (call before CUDA-graph capture
+    so no allocation happens inside)."""
     _skinny_scratch.get(torch.device(device), floats, tiles)
+    _pipeline_status(torch.device(device))
 
 
 class SkinnyEpilogue(ctypes.Structure):
