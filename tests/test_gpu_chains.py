@@ -13,16 +13,26 @@ def _rnd(*shape, dtype=BF):
     return torch.randn(shape, device="cuda").to(dtype)
 
 
-def _linear(p):
-    from triton_distributed_b200 import ops
-    x = _rnd(5, 256)
-    return lambda: ops.linear(x, p)
+def _linear(rows):   # at most 16 rows and more run on kernels of their own
+    def make(p):
+        from triton_distributed_b200 import ops
+        x = _rnd(rows, 256)
+        return lambda: ops.linear(x, p)
+    return make
 
 
-def _swiglu(p):
+def _swiglu(rows):
+    def make(p):
+        from triton_distributed_b200 import ops
+        x = _rnd(rows, 256)
+        return lambda: ops.gemm_skinny(x, p, swiglu=True)
+    return make
+
+
+def _normed(p):
     from triton_distributed_b200 import ops
-    x = _rnd(5, 256)
-    return lambda: ops.gemm_skinny(x, p, swiglu=True)
+    x, w = _rnd(5, 2048), _rnd(512, 2048)
+    return lambda: ops.gemm_rows(x, w, gamma=p.view(-1), eps=1e-6)
 
 
 def _groups(p):
@@ -107,7 +117,8 @@ def _sink(p):
     return lambda: ops.latent_attention(q, cache, lens, table, 1, 0.05, p.view(-1), 3, 16)
 
 
-CONSUMERS = {"linear": (_linear, (512, 256), BF), "swiglu": (_swiglu, (512, 256), BF), "groups": (_groups, (512, 256), BF),
+CONSUMERS = {"linear": (_linear(5), (512, 256), BF), "swiglu": (_swiglu(5), (512, 256), BF), "linear, 24 rows": (_linear(24), (512, 256), BF),
+             "swiglu, 24 rows": (_swiglu(24), (512, 256), BF), "normed": (_normed, (1, 2048), BF), "groups": (_groups, (512, 256), BF),
              "head_linear": (_heads, (512, 256), BF), "tanh_linear": (_tanh, (512, 256), BF), "rmsnorm": (_rmsnorm, (1, 2048), BF),
              "qk_norm_rope": (_rope, (1, 256), BF), "embed_norm": (_embed, (1, 2048), BF), "residual_norm": (_residual, (1, 2048), BF),
              "residual_post": (_post, (1, 2048), BF), "token_mix": (_mix, (3, 512), BF), "short_conv": (_conv, (4, 512), F32),

@@ -7,10 +7,12 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,N,K,swiglu", [
-    (1, 8, 64, False),          # one granule, one k-block (a stage has two)
-    (8, 1280, 5120, False),     # a tile per SM or less
-    (9, 1001, 192, False),      # the second half of the tokens, a ragged last tile, a ragged last stage
+    (1, 8, 64, False),          # one granule, one k-block
+    (8, 1280, 5120, False),     # a tile per SM or less, two stages of five k-blocks a warp
+    (9, 1001, 192, False),      # the second half of the tokens, a ragged last tile, warps without a stage
     (16, 6144, 1088, False),
+    (8, 1280, 4160, False),     # 65 k-blocks in stages of four: a ragged last stage
+    (16, 3000, 4160, False), (5, 700, 704, True),
     (3, 60000, 128, False),     # several tiles per CTA
     (1, 3200, 5120, True), (8, 12288, 256, True), (16, 100, 320, True),
 ])
@@ -50,6 +52,36 @@ def test_gemm_rows_norm(M, N, K, swiglu):
     if swiglu:
         ref = torch.nn.functional.silu(ref[:, :N]) * ref[:, N:]
     torch.testing.assert_close(y.double(), ref, rtol=2 ** -7, atol=2e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,swiglu", [(1, 130, 64, False), (8, 999, 4160, False), (13, 1280, 704, False), (16, 333, 1024, True)])
+def test_gemm_rows_pitches(M, N, K, swiglu, dtype):
+    """Rows of x, w, the result and the residual inside wider ones, through the entry that chooses the kernel; nothing beside them is
+    written, and a token's result does not depend on the tokens beside it."""
+    from triton_distributed_b200 import _lib, ops
+    torch.manual_seed(8)
+    rows = N * (2 if swiglu else 1)
+    x = torch.randn(M + 1, K + 16, device="cuda").to(dtype)[1:, 8:K + 8]
+    w = (torch.randn(rows, K + 24, device="cuda") * K ** -0.5).to(dtype)[:, 16:K + 16]
+    wide = torch.full((M + 3, N + 5), 7.0, device="cuda", dtype=dtype)
+    seen, call = [], _lib.call
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(_lib, "call", lambda name, *args: (seen.append(name), call(name, *args)))
+        y = ops.gemm_skinny(x, w, wide[:M, 3:N + 3], swiglu=swiglu)
+    assert seen == ["b200_gemm_rows"] and y.data_ptr() == wide[:M, 3:].data_ptr()
+    ref = x.double() @ w.double().T
+    if swiglu:
+        ref = torch.nn.functional.silu(ref[:, :N]) * ref[:, N:]
+    eps = torch.finfo(dtype).eps
+    torch.testing.assert_close(y.double(), ref, rtol=eps, atol=2e-5)   # as in test_gemm_rows
+    assert torch.equal(ops.gemm_rows(x[M // 2:M // 2 + 1], w, swiglu=swiglu)[0], y[M // 2])
+    if not swiglu:
+        h = torch.randn(M, N, device="cuda").to(dtype)
+        wide[:M, 3:N + 3] = h
+        ops.gemm_rows(x, w, out=wide[:M, 3:N + 3], residual=wide[:M, 3:N + 3])
+        torch.testing.assert_close(wide[:M, 3:N + 3].double(), ref + h.double(), rtol=eps, atol=2e-5)
+    assert torch.all(wide[M:] == 7.0) and torch.all(wide[:, :3] == 7.0) and torch.all(wide[:, N + 3:] == 7.0)
 
 
 def test_status_word_is_made_in_front_of_a_capture(monkeypatch):

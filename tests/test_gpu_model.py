@@ -40,6 +40,44 @@ def test_native_forward_matches_torch_mode(dist1):
     model.finalize()
 
 
+@pytest.mark.parametrize("bsz,seqlen", [(9, 1), (16, 1), (1, 5), (2, 8), (1, 16)])
+def test_steps_of_few_tokens_match_separate_norms(dist1, bsz, seqlen):
+    """Up to 16 tokens of a bf16 model on one GPU have norms and residual adds inside the projections; the path with separate
+    kernels is the other side, behind a cached prompt."""
+    cfg, model = _mk(dist1)
+    model.set_fwd("triton_dist_AR")
+    model.init_triton_dist_AR_ctx(64)
+    torch.manual_seed(12)
+    ids = torch.randint(0, model.arch.vocab_size, (bsz, 20 + seqlen), device="cuda")
+    pos = torch.arange(20 + seqlen, device="cuda")[None].repeat(bsz, 1)
+    outs, paths = {}, []
+    rows = model._step_rows
+    for few in (True, False):
+        model._step_rows = lambda *a: (paths.append(few), rows(*a))[1]
+        if not few:
+            model._few_tokens = lambda tokens: False
+        for only_hidden in (False, True):
+            kv = model.make_cache(bsz)
+            model.inference(ids[:, :20], pos[:, :20], kv)
+            outs[few, only_hidden] = model.inference(ids[:, 20:].contiguous(), pos[:, 20:].contiguous(), kv, wo_lm_head=only_hidden).double()
+    assert paths == [True, True]
+    for only_hidden in (False, True):
+        got, want = outs[True, only_hidden], outs[False, only_hidden]
+        assert got.shape == want.shape
+        # three layers of four bf16 roundings each in other places: a few times 2^-9 of the norm
+        assert (got - want).norm() <= 0.02 * want.norm()
+    model.finalize()
+
+
+def test_which_steps_have_norms_inside_the_projections(dist1):
+    _, model = _mk(dist1)
+    assert model._few_tokens(1) and model._few_tokens(16) and not model._few_tokens(17)
+    model.dtype = torch.float16     # may not hold the product of the residual stream and a gain
+    assert not model._few_tokens(1)
+    _, moe = _mk(dist1, "tiny-qwen3-moe")
+    assert not moe._few_tokens(1)
+
+
 def test_engine_graph_equals_eager_and_torch(dist1):
     from triton_distributed_b200.models import Engine
     cfg, model = _mk(dist1)

@@ -24,8 +24,8 @@ def test_gemm_matches_fp32_reference(M, N, K, dtype):
     torch.testing.assert_close(c.float(), ref, rtol=2e-2, atol=2e-2)
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (8, 1280, 5120), (8, 5120, 1024), (16, 384, 4096), (33, 1000, 520),
-                                   (128, 512, 1024), (256, 256, 512)])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (8, 1280, 5120), (8, 5120, 1024), (16, 384, 4096), (5, 700, 1032), (33, 1000, 520),
+                                   (24, 1280, 5120), (128, 512, 1024), (256, 256, 512)])
 def test_gemm_skinny(M, N, K):
     from triton_distributed_b200 import ops
     torch.manual_seed(1)
