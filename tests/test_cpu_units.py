@@ -156,6 +156,19 @@ def test_trace_merge_and_helpers(capsys):
     assert "hello" in capsys.readouterr().out
 
 
+def test_gemm_f32_cuts_in_front_where_a_call_has_many_steps():
+    import ctypes
+    from triton_distributed_b200 import _lib
+    lib = _lib.load()
+    need, size = lib.b200_gemm_f32_planes_bytes, lib.b200_gemm_f32_workspace_bytes
+    need.restype = size.restype = ctypes.c_longlong
+    for M, N, K in [(1, 22016, 4096), (16, 4096, 11008), (17, 64, 64), (32, 1024, 4096), (48, 512, 2048), (100, 512, 1024), (256, 4096, 256),
+                    (0, 5, 5), (40, 0, 5), (40, 5, 0)]:
+        assert need(M, N, K) == 0
+    for M, N, K in [(17, 4096, 4096), (48, 512, 4096), (64, 2048, 2048), (100, 512, 2048), (100, 2048, 5632), (1024, 4096, 1024), (1 << 20, 1 << 20, 64)]:
+        assert need(M, N, K) == size(M, K) > 0
+
+
 def test_native_library_builds_and_reports_errors():
     """The shared object loads without a driver; entry points that need one fail with a message, not a crash."""
     import ctypes

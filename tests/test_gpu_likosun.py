@@ -527,8 +527,8 @@ def test_gemm_f32_range_of_values(M, N, K):
     assert torch.equal(got[odd].double().nan_to_num(7.0), want[odd].nan_to_num(7.0))
 
 
-@pytest.mark.parametrize("M", [1, 16, 17, 112, 113, 128, 129, 300])
-@pytest.mark.parametrize("N,K,pad", [(130, 1, 0), (70, 63, 1), (300, 64, 0), (2048, 257, 3), (129, 1030, 2)])
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 112, 113, 128, 129, 300])
+@pytest.mark.parametrize("N,K,pad", [(130, 1, 0), (70, 63, 1), (300, 64, 0), (2048, 257, 3), (129, 1030, 2), (2048, 4100, 1)])
 def test_gemm_f32_planes(M, N, K, pad):
     """A cut beforehand gives the bits of a cut inside, with infinities, NaNs and the smallest numbers in it, from a workspace that held
     something else."""

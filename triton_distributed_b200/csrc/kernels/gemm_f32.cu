@@ -24,16 +24,18 @@
 //   warps 0-3   promotion: x1 y1 from tensor memory into registers, then the partial tile     warp 4  MMA issuer
 //   warp 5      A's planes into shared memory by bulk copies, where A was cut beforehand
 //   warps 8-15  operands: global memory -> registers, one or two steps of 64 k ahead -> three planes in 128-byte-swizzled shared memory
-// More than 16 rows of A are cut once, by a kernel in front, when the caller brings room for the planes: every column tile would cut them again,
-// and without them the registers hold two steps of B's loads instead of one. The planes and their sums are the same either way.
+// In calls of many steps A is cut once, by a kernel in front, when the caller brings room for the planes (b200_gemm_f32_planes_bytes): every
+// column tile would cut it again, and without it the registers hold two steps of B's loads instead of one. The planes and their sums are the
+// same either way.
 // What bounds it: the products, 1830 of 2330 clocks a step at 100 rows (the planes' copies are asked for when their place is free and take
 // about as long as a step), and the start and end of a CTA. The rare cases are left to a
 // second look per step: a branch for every four values kept the loads, the arithmetic and the stores of neighbouring values apart.
-// us, back to back over several B, with A cut by every CTA and one step of loads -> now (planes from 17 rows on; parts by clusters that fit):
+// us, back to back over several B, with A cut by every CTA, one step of loads and parts for 148 CTAs at once -> now (parts by clusters that fit):
 //   11264 x 2048   1 row 40 -> 38    100 rows 61 -> 54    1024 rows 516 -> 411
 //   2048 x 5632    1 row 39 -> 24    100 rows 60 -> 34    1024 rows 297 -> 195
 //   22016 x 4096   1 row 154 -> 123  100 rows 223 -> 159  1024 rows 1954 -> 1347
-//   4096 x 11008   1 row 68 -> 62..68  100 rows 90 -> 82  1024 rows 925 -> 636
+//   4096 x 11008   1 row 62 -> 56    100 rows 90 -> 82    1024 rows 925 -> 636
+//   512 x 1024     1 row 6.2 -> 6.3  32 rows 7.6 -> 7.6   100 rows 14.2 -> 12.2
 // fp32 products on the CUDA cores with 4 x 4 outputs per thread took 227 us for 1 x 11264 x 2048 and 336 for 100 x 2048 x 5632.
 #include "b200/host.h"
 #include "b200/packed_f32.cuh"
@@ -152,8 +154,44 @@ __global__ void __launch_bounds__(256) f32_planes_kernel(const F32Params p) {
   if (threadIdx.x == 0) p.planes_tiny[at] = tiny;
 }
 
-// The partial tile from its sums of x1 y1 and the scaled groups in tensor memory: three warpgroups, every third 16 rows each, a thread
-// a column of C. (One warpgroup took 8800 of a CTA's 45000 clocks for it at 112 rows, with the other warps idle.)
+// 16 rows of a column of the partial tile from their sums of x1 y1 (`sum`, by row) and the scaled groups in tensor memory (`from`). Returns the
+// rows whose sum is finite in x1 y1 but not in the scaled groups, or is no number where an infinity may have met such a value (`small`).
+template <typename Sum>
+__device__ __forceinline__ uint32_t f32_join(uint32_t from, bool read, bool ok, bool small, float* at, const Sum& sum) {
+  uint32_t c1[16] = {}, c2[16] = {}, c3[16] = {}, again = 0;
+  if (read) {
+    tmem_ld_32x16(from, c1);
+    tmem_ld_32x16(from + 128, c2);
+    tmem_ld_32x16(from + 256, c3);
+    tmem_ld_wait();
+  }
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const float main = sum(q);
+    const float rest = fmaf(fmaf(__uint_as_float(c3[q]), 0x1p-8f, __uint_as_float(c2[q])), 0x1p-8f, __uint_as_float(c1[q]));
+    const bool finite = fabsf(main) <= FLT_MAX;
+    const float v = finite ? fmaf(rest, 0x1p-8f, main) : main;
+    if (finite ? !(fabsf(rest) <= FLT_MAX) : small && main != main) again |= 1u << q;
+    at[q * kXN] = ok ? v : NAN;
+  }
+  return ok ? again : 0u;
+}
+// takes the marked rows of column n once more, one product after the other
+__device__ __forceinline__ void f32_again(const F32Params& p, uint32_t left, float* at, int m0, int n0, int n, int k_begin, int k_end) {
+  const float* b = p.B + static_cast<size_t>(min(n0 + n, p.N - 1)) * p.ldb;
+  for (; left != 0u; left &= left - 1) {
+    const int q = __ffs(left) - 1;
+    const float* a = p.A + static_cast<size_t>(min(m0 + q, p.M - 1)) * p.lda;
+    float sum = 0.f;
+    for (int k = k_begin; k < k_end; ++k) sum = fmaf(a[k], b[k], sum);
+    at[q * kXN] = sum;
+  }
+}
+
+// The partial tile is finished by three warpgroups, every third 16 rows each, a thread a column of C. (One warpgroup took 8800 of a CTA's
+// 45000 clocks for it at 112 rows, with the other warps idle.) 16 rows are finished by the warps that hold x1 y1, straight from their
+// registers.
+constexpr bool f32_alone(int rows) { return rows <= 16; }
 template <int kT>
 __device__ __forceinline__ void f32_finish(const F32Params& p, uint32_t tmem_base, float* out, int warp, int group, int m0, int n0, int k_begin,
                                            int k_end, int steps, volatile uint32_t* abort_flag, volatile uint32_t* tiny) {
@@ -165,34 +203,9 @@ __device__ __forceinline__ void f32_finish(const F32Params& p, uint32_t tmem_bas
 #pragma unroll 1
   for (int h = group; h < kT / 16; h += 3) {
     float* at = out + h * 16 * kXN + n;
-    uint32_t c1[16] = {}, c2[16] = {}, c3[16] = {};
     __syncwarp();
-    if (steps > 0 && ok) {
-      tmem_ld_32x16(lanes + 128 + h * 16, c1);
-      tmem_ld_32x16(lanes + 256 + h * 16, c2);
-      tmem_ld_32x16(lanes + 384 + h * 16, c3);
-      tmem_ld_wait();
-    }
-    // rows whose sum is finite in x1 y1 but not in the scaled groups, or is no number where an infinity may have met such a value
-    uint32_t again = 0;
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const float main = at[q * kXN];
-      const float rest = fmaf(fmaf(__uint_as_float(c3[q]), 0x1p-8f, __uint_as_float(c2[q])), 0x1p-8f, __uint_as_float(c1[q]));
-      const bool finite = fabsf(main) <= FLT_MAX;
-      const float v = finite ? fmaf(rest, 0x1p-8f, main) : main;
-      if (finite ? !(fabsf(rest) <= FLT_MAX) : small && main != main) again |= 1u << q;
-      at[q * kXN] = ok ? v : NAN;
-    }
-    if (!ok) again = 0u;
-    const float* b = p.B + static_cast<size_t>(min(n0 + n, p.N - 1)) * p.ldb;
-    for (uint32_t left = again; left != 0u; left &= left - 1) {
-      const int q = __ffs(left) - 1;
-      const float* a = p.A + static_cast<size_t>(min(m0 + h * 16 + q, p.M - 1)) * p.lda;
-      float sum = 0.f;
-      for (int k = k_begin; k < k_end; ++k) sum = fmaf(a[k], b[k], sum);
-      at[q * kXN] = sum;
-    }
+    const uint32_t again = f32_join(lanes + 128 + h * 16, steps > 0 && ok, ok, small, at, [&](int q) { return at[q * kXN]; });
+    f32_again(p, again, at, m0 + h * 16, n0, n, k_begin, k_end);
   }
   tc_fence_before_sync();
 }
@@ -202,8 +215,8 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes,
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
-// kPlanes: A has been cut by f32_planes_kernel and arrives by bulk copies
-template <int kT, bool kPlanes>
+// kPlanes: A has been cut by f32_planes_kernel and arrives by bulk copies. kDepth: steps of loads in flight
+template <int kT, bool kPlanes, int kDepth>
 __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params p) {
   using T = F32Tile<kT>;
   extern __shared__ uint8_t smem_raw[];
@@ -272,15 +285,25 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
       __syncwarp();
       if (lane == 0) mbar_arrive(dempty_bar + at);
     }
-    if (steps > 0 && ok) mbar_wait(done_bar, 0, abort_flag, kTimeout);
-    // all products are done: the stages give way to the partial tile [kT][128], first of x1 y1
+    if (steps > 0 && ok) ok = mbar_wait(done_bar, 0, abort_flag, kTimeout);
+    // all products are done: the stages give way to the partial tile [kT][128]
     float* out = reinterpret_cast<float*>(smem);
-#pragma unroll
-    for (int r = 0; r < kT; ++r) {
+    auto sum = [&](int r) {   // of x1 y1
       const float2 pair = unpack2(acc[r / 2]);
-      out[r * kXN + threadIdx.x] = (r & 1) ? pair.y : pair.x;
+      return (r & 1) ? pair.y : pair.x;
+    };
+    if (f32_alone(kT)) {
+      ok = __all_sync(0xffffffffu, ok);
+      tc_fence_after_sync();
+      const bool small = *tiny != 0u;
+      const uint32_t again = f32_join(lanes + 128, steps > 0 && ok, ok, small, out + threadIdx.x, sum);
+      f32_again(p, again, out + threadIdx.x, m0, n0, threadIdx.x, k_begin, k_end);
+      tc_fence_before_sync();
+    } else {
+#pragma unroll
+      for (int r = 0; r < kT; ++r) out[r * kXN + threadIdx.x] = sum(r);
+      f32_finish<kT>(p, tmem_base, out, warp, 0, m0, n0, k_begin, k_end, steps, abort_flag, tiny);
     }
-    f32_finish<kT>(p, tmem_base, out, warp, 0, m0, n0, k_begin, k_end, steps, abort_flag, tiny);
   } else if (warp < 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp == 4 && elect_one()) {
@@ -345,7 +368,6 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
     // eight rows down the swizzle repeats: the offset inside a row is the same for all rows of this thread
     const uint32_t off = static_cast<uint32_t>(r0 * 128 + (((c >> 1) ^ (r0 & 7)) * 16) + (c & 1) * 8);
     constexpr int kRowsB = kXN / 16, kRowsA = kPlanes ? 0 : kT / 16;
-    constexpr int kDepth = kRowsA <= 2 ? 2 : 1;   // steps of loads in flight, as many as the registers hold
     const float *rb[kRowsB], *ra[kRowsA + 1];
     float4 vb[kDepth][kRowsB], va[kDepth][kRowsA + 1];
 #pragma unroll
@@ -360,12 +382,10 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
       for (int i = 0; i < kRowsA; ++i) va[d][i] = f32_load4(ra[i], k0 + d * kXK, k_end, p.vec_a);
     }
     bool ok = true;
-    for (int s0 = 0; s0 < steps && ok; s0 += 2) {
+    for (int s0 = 0; s0 < steps && ok; s0 += kDepth) {
 #pragma unroll
-      for (int st = 0; st < 2; ++st) {
-        const int s = s0 + st, next = k0 + (s + kDepth) * kXK;
-        constexpr int kSets = kDepth - 1;
-        const int d = st & kSets;
+      for (int d = 0; d < kDepth; ++d) {
+        const int s = s0 + d, st = s & 1, next = k0 + (s + kDepth) * kXK;
         if (s >= steps) break;
         ok = mbar_wait(empty_bar + st, ((s >> 1) & 1) ^ 1, abort_flag, kTimeout);
         if (!ok) break;
@@ -396,8 +416,10 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
         mbar_arrive(full_bar + st);
       }
     }
-    if (steps > 0 && ok) mbar_wait(done_bar, 0, abort_flag, kTimeout);
-    f32_finish<kT>(p, tmem_base, reinterpret_cast<float*>(smem), warp, (warp >> 2) - 1, m0, n0, k_begin, k_end, steps, abort_flag, tiny);
+    if (!f32_alone(kT)) {
+      if (steps > 0 && ok) mbar_wait(done_bar, 0, abort_flag, kTimeout);
+      f32_finish<kT>(p, tmem_base, reinterpret_cast<float*>(smem), warp, (warp >> 2) - 1, m0, n0, k_begin, k_end, steps, abort_flag, tiny);
+    }
   }
   __syncwarp();
   tc_fence_before_sync();
@@ -412,16 +434,17 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
       const int r = i / (kXN / 4), n = i % (kXN / 4) * 4;
       if (m0 + r >= p.M || n0 + n >= p.N) continue;
       float v[4] = {};
-      for (int q0 = 0; q0 < p.parts; q0 += 4) {   // four reads on their way at a time
-        float4 x[4];
+      constexpr int kReads = kT <= 16 && kDepth == 1 ? 1 : 4;   // on their way at a time; a short sum of few rows gains nothing by more
+      for (int q0 = 0; q0 < p.parts; q0 += kReads) {
+        float4 x[kReads];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < kReads; ++q)
           if (q0 + q < p.parts)
             asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
                          : "=f"(x[q].x), "=f"(x[q].y), "=f"(x[q].z), "=f"(x[q].w)
                          : "r"(mapa_u32(out + r * kXN + n, q0 + q)));
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < kReads; ++q)
           if (q0 + q < p.parts) v[0] += x[q].x, v[1] += x[q].y, v[2] += x[q].z, v[3] += x[q].w;
       }
 #pragma unroll
@@ -437,27 +460,40 @@ __global__ void __launch_bounds__(kXThreads, 1) gemm_f32_kernel(const F32Params 
 // as much as four steps. A cluster's CTAs, one per SM, lie in one part of the chip, so clusters leave SMs over: 15 of eight run at a time
 // and not 18 (2048 x 5632, 100 rows: 16 clusters of eight, two waves, 53 us; of six, one wave, 35). The counts are a B200's, whatever the
 // device has: the parts are part of the result's rounding.
+constexpr int kF32Clusters[kXMaxParts] = {148, 74, 45, 33, 26, 22, 15, 15};
 static int f32_parts(int N, int K) {
-  constexpr int kClusters[kXMaxParts] = {148, 74, 45, 33, 26, 22, 15, 15};
   const int tiles = (N + kXN - 1) / kXN, steps = (K + kXK - 1) / kXK;
   int best = 1;
   long long least = 1ll << 62;
   for (int parts = 1; parts <= kXMaxParts && parts <= steps; ++parts) {
-    const long long waves = (tiles + kClusters[parts - 1] - 1) / kClusters[parts - 1];
+    const long long waves = (tiles + kF32Clusters[parts - 1] - 1) / kF32Clusters[parts - 1];
     const long long cost = waves * ((steps + parts - 1) / parts + 4);
     if (cost < least) least = cost, best = parts;
   }
   return best;
 }
 
-template <int kT, bool kPlanes>
+// row tiles of even height: 100 rows are one of 112, 150 two of 80
+static int f32_rows(int M) {
+  const int tiles = (M + 127) / 128;
+  return ((M + tiles - 1) / tiles + 15) / 16 * 16;
+}
+// steps of 64 k that the busiest SM takes in all its waves
+static int f32_steps(int M, int N, int K) {
+  const int parts = f32_parts(N, K), at_once = kF32Clusters[parts - 1];
+  const long long tiles = static_cast<long long>((N + kXN - 1) / kXN) * ((M + f32_rows(M) - 1) / f32_rows(M));
+  const long long steps = (tiles + at_once - 1) / at_once * (((K + kXK - 1) / kXK + parts - 1) / parts);
+  return steps > 1 << 20 ? 1 << 20 : static_cast<int>(steps);
+}
+
+template <int kT, bool kPlanes, int kDepth>
 static int launch_gemm_f32_form(const F32Params& p, cudaStream_t stream) {
   using T = F32Tile<kT>;
   static bool configured[64] = {false};
   int dev = 0;
   B200_CHECK_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    B200_CHECK_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<kT, kPlanes>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem));
+    B200_CHECK_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<kT, kPlanes, kDepth>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem));
     configured[dev & 63] = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -476,33 +512,42 @@ static int launch_gemm_f32_form(const F32Params& p, cudaStream_t stream) {
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   if (kPlanes)
     B200_CHECK_CUDA(launch_pdl(f32_planes_kernel<kT>, dim3((p.K + kXK - 1) / kXK, cfg.gridDim.y), dim3(256), 0, stream, p));
-  B200_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<kT, kPlanes>, p));
+  B200_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<kT, kPlanes, kDepth>, p));
   return kOk;
 }
 template <int kT>
 static int launch_gemm_f32(F32Params& p, void* workspace, cudaStream_t stream) {
-  if (workspace == nullptr) return launch_gemm_f32_form<kT, false>(p, stream);
+  if (workspace == nullptr) {
+    // Two steps of B in flight beside 16 rows of A, where a CTA has steps enough to need them. us with one and with two, one row: 64 x 256
+    // 5.0, 5.3; 256 x 4096 (8 steps) 12.8, 13.2; 2048 x 4096 (11) 20.0, 19.2; 4096 x 4096 (16) 26.7, 25.4. More rows leave no registers for it.
+    if (kT == 16 && f32_steps(p.M, p.N, p.K) > 8) return launch_gemm_f32_form<kT, false, kT == 16 ? 2 : 1>(p, stream);
+    return launch_gemm_f32_form<kT, false, 1>(p, stream);
+  }
   const size_t stages = static_cast<size_t>((p.M + kT - 1) / kT) * ((p.K + kXK - 1) / kXK);
   p.planes = static_cast<uint8_t*>(workspace);
   p.planes_tiny = reinterpret_cast<uint32_t*>(p.planes + stages * (3 * F32Tile<kT>::kPlaneA));
-  return launch_gemm_f32_form<kT, true>(p, stream);
+  return launch_gemm_f32_form<kT, true, 2>(p, stream);
 }
 
 }  // namespace b200
 
 using namespace b200;
 
-// row tiles of even height: 100 rows are one of 112, 150 two of 80
-static int f32_rows(int M) {
-  const int tiles = (M + 127) / 128;
-  return ((M + tiles - 1) / tiles + 15) / 16 * 16;
-}
-
 // Bytes of b200_gemm_f32_planes' workspace.
 B200_API long long b200_gemm_f32_workspace_bytes(int M, int K) {
   if (M <= 0 || K <= 0) return 0;
   const int rows = f32_rows(M);
   return static_cast<long long>((M + rows - 1) / rows) * ((K + kXK - 1) / kXK) * (3ll * rows * kXK * 2 + 4);
+}
+
+// Bytes of a workspace that makes the call faster, or none: the launch in front costs about 1.2 us, and a step of few rows is no shorter with A's
+// planes at hand. us with A cut inside and in front, by rows x N x K (steps of the busiest SM): 32 x 256 x 1024 (2) 7.8, 8.7; 32 x 1024 x 4096
+// (8) 16.5, 17.0; 32 x 4096 x 4096 (16) 28.3, 27.7; 48 x 512 x 2048 (4) 11.3, 11.7; 48 x 512 x 4096 (8) 17.8, 17.3; 64 x 2048 x 1024 (3) 12.6, 13.3; 64 x
+// 2048 x 2048 (6) 16.8, 17.1; 64 x 512 x 4096 (8) 19.4, 18.3; 100 x 512 x 1024 (2) 12.5, 13.2; 100 x 512 x 2048 (4) 16.1, 16.0; 100 x 2048 x 2048 (6) 21.0,
+// 20.2; 256 x 1024 x 1024 (4) 27.1, 27.1; 256 x 4096 x 4096 (32) 83, 70.
+B200_API long long b200_gemm_f32_planes_bytes(int M, int N, int K) {
+  if (M <= 16 || N <= 0 || K <= 0 || f32_steps(M, N, K) * f32_rows(M) < 384) return 0;
+  return b200_gemm_f32_workspace_bytes(M, K);
 }
 
 // workspace (nullable, on a 16-byte boundary): A is cut into its planes there, once for all column tiles; results are the same. status

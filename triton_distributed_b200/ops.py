@@ -271,9 +271,8 @@ def linear_groups(x: torch.Tensor, w: torch.Tensor, rows: list[int], settled: bo
     return out
 
 
-# A row tile of 16 is cut beside the 128 rows of B at no cost (1 x 22016 x 4096: 140 us either way); more rows are cut once in front of the
-# product (100 x 11264 x 2048: 57 us for 61, 1024 x 4096 x 11008: 673 for 925), as long as their planes, six bytes a value, stay small.
-_F32_ROWS_CUT_INSIDE = 16
+# A is cut once in front of the product where that is faster (b200_gemm_f32_planes_bytes: from 17 rows on in calls of many steps) and as long as
+# its planes, six bytes a value, stay small.
 _F32_WORKSPACE = 256 << 20
 
 
@@ -288,11 +287,11 @@ def gemm_f32(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None) 
     if out is None:
         out = torch.empty((M, N), dtype=a.dtype, device=a.device)
     ws = None
-    if M > _F32_ROWS_CUT_INSIDE and K > 0 and N > 0:
-        fn = _lib.load().b200_gemm_f32_workspace_bytes
+    if M > 16:
+        fn = _lib.load().b200_gemm_f32_planes_bytes
         fn.restype = ctypes.c_longlong
-        need = fn(M, K)
-        ws = torch.empty(need, dtype=torch.uint8, device=a.device) if need <= _F32_WORKSPACE else None
+        need = fn(M, N, K)
+        ws = torch.empty(need, dtype=torch.uint8, device=a.device) if 0 < need <= _F32_WORKSPACE else None
     if ws is None:
         _lib.call("b200_gemm_f32_checked", ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
                   ptr(_pipeline_status(a.device)), stream_ptr())
