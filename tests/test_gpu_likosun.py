@@ -550,6 +550,23 @@ def test_gemm_f32_planes(M, N, K, pad):
     ops.check_pipeline_status()
 
 
+def test_gemm_f32_without_room_for_the_planes(monkeypatch):
+    """Calls whose workspace finds no memory run without it, to the same bits."""
+    from triton_distributed_b200 import _lib, ops
+    a, b = torch.randn(200, 4096, device="cuda"), torch.randn(2048, 4096, device="cuda")
+    seen, call, empty = [], _lib.call, torch.empty
+    monkeypatch.setattr(_lib, "call", lambda name, *args: (seen.append(name), call(name, *args)))
+    want = ops.gemm_f32(a, b)
+
+    def full(*args, **kw):
+        if kw.get("dtype") == torch.uint8:
+            raise torch.OutOfMemoryError("none left")
+        return empty(*args, **kw)
+    monkeypatch.setattr(torch, "empty", full)
+    assert torch.equal(ops.gemm_f32(a, b), want)
+    assert seen == ["b200_gemm_f32_planes", "b200_gemm_f32_checked"]
+
+
 @pytest.mark.parametrize("K", [1, 2, 3, 5, 8, 40])
 @pytest.mark.parametrize("kind", ["full mantissas", "any", "one sign"])
 def test_gemm_f32_short_sums(K, kind):

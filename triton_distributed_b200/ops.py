@@ -291,7 +291,11 @@ def gemm_f32(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None) 
         fn = _lib.load().b200_gemm_f32_planes_bytes
         fn.restype = ctypes.c_longlong
         need = fn(M, N, K)
-        ws = torch.empty(need, dtype=torch.uint8, device=a.device) if 0 < need <= _F32_WORKSPACE else None
+        if 0 < need <= _F32_WORKSPACE:
+            try:
+                ws = torch.empty(need, dtype=torch.uint8, device=a.device)
+            except torch.OutOfMemoryError:   # nothing but time depends on it
+                pass
     if ws is None:
         _lib.call("b200_gemm_f32_checked", ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
                   ptr(_pipeline_status(a.device)), stream_ptr())
