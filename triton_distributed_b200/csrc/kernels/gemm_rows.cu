@@ -351,8 +351,15 @@ B200_API int b200_gemm_rows(const void* X, const void* W, void* C, int M, int N,
   else
     kernel = dual ? (mb == 8 ? rows_kernel<false, 8, true>(granules) : rows_kernel<false, 16, true>(granules))
                   : (mb == 8 ? rows_kernel<false, 8, false>(granules) : rows_kernel<false, 16, false>(granules));
-  // (one value for all calls: another thread's launch of the same kernel may need more than this one)
-  B200_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem));
+  // once per device and kernel, with what the largest launch needs (about 1 us of host time)
+  static bool configured[64][2][2][2][kRowsMaxGranules] = {};
+  int dev = 0;
+  B200_CHECK_CUDA(cudaGetDevice(&dev));
+  bool& done = configured[dev & 63][dtype == kBF16][dual != 0][mb == 16][granules - 1];
+  if (!done) {
+    B200_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem));
+    done = true;
+  }
   B200_CHECK_CUDA(launch_pdl(kernel, dim3(grid), dim3(kRowsThreads), static_cast<size_t>(smem), static_cast<cudaStream_t>(stream), tw, tx, p));
   return kOk;
 }

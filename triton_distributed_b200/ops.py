@@ -174,12 +174,15 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = Non
     M, K = x.shape
     n_rows = w.shape[0]
     N = n_rows // 2 if swiglu else n_rows
-    # Few tokens and all of K on one SM: 1.1 to 2.3 times as fast at the projections of 1280 x 5120 to 151936 x 4096. A long K with
-    # few rows to it stays with the kernel that spreads K over the SMs.
+    # Few tokens and all of K on one SM: no slower at any of 1, 8, 9, 16 tokens x 8 ... 12288 rows x 256 ... 12288 of K that the rule takes. us in
+    # a chain of such calls, stream-K and this, 1 / 8 / 9 / 16 tokens: 8 x 1024 4.7 / 5.2 / 5.5 / 5.7, 1.7 / 1.7 / 1.8 / 1.8; 128 x 2048 (on the edge)
+    # 4.7 / 5.1 / 5.4 / 5.6, 2.2 / 2.2 / 2.4 / 2.4; 512 x 4096 5.4 / 6.0 / 6.2 / 6.8, 3.6 / 3.6 / 3.8 / 3.7; 1024 x 8192 8.4 / 9.2 / 9.5 / 10.0, 6.6 / 6.3 /
+    # 6.4 / 6.4; 5120 x 12288 23.0 / 23.6 / 24.1 / 24.6, 20.8 / 21.1 / 21.1 / 21.4; 12288 x 8192 gated (1, 8, 9) 62.4 / 64.7 / 66.2, 62.1 / 62.6 / 61.9.
+    # A longer K with few rows to it stays with the kernel that spreads K over the SMs.
     if (1 <= M <= 16 and K % 64 == 0 and 64 <= K <= 1024 + 8 * N and splits == 0 and epilogue is None and w.shape[1] == K and w.dtype == x.dtype
             and n_rows % (2 if swiglu else 1) == 0
             and (out is None or (out.shape == (M, N) and out.stride(1) == 1 and out.dtype == x.dtype))):
-        return gemm_rows(x, w, out, swiglu, settled=settled)
+        return _gemm_rows(x, w, out, M, N, K, swiglu, None, 0.0, None, False, settled)
     own_output = epilogue is not None and epilogue.kind in (1, 2)
     if out is None and not own_output:
         out = torch.empty((M, N), dtype=x.dtype, device=x.device)
@@ -213,14 +216,19 @@ def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None,
     N = w.shape[0] // 2 if swiglu else w.shape[0]
     if w.shape[1] != K or w.dtype != x.dtype or (swiglu and w.shape[0] % 2):
         raise ValueError("gemm_rows: shape/dtype mismatch")
-    if out is None:
-        out = torch.empty((M, N), dtype=torch.float32 if out_f32 else x.dtype, device=x.device)
-    if out.shape != (M, N) or out.stride(1) != 1 or out.dtype != (torch.float32 if out_f32 else x.dtype):
+    if out is not None and (out.shape != (M, N) or out.stride(1) != 1 or out.dtype != (torch.float32 if out_f32 else x.dtype)):
         raise ValueError("gemm_rows: the output is [M, N] with unit inner stride")
     if gamma is not None and (gamma.shape != (K,) or gamma.dtype != x.dtype or not gamma.is_contiguous()):
         raise ValueError("gemm_rows: gamma is [K] in the type of x")
-    if residual is not None and (residual.shape != (M, N) or residual.dtype != x.dtype or residual.stride() != out.stride()):
+    if residual is not None and (residual.shape != (M, N) or residual.dtype != x.dtype or residual.stride() != ((N, 1) if out is None else out.stride())):
         raise ValueError("gemm_rows: the residual is laid out like the output")
+    return _gemm_rows(x, w, out, M, N, K, swiglu, gamma, eps, residual, out_f32, settled)
+
+
+def _gemm_rows(x, w, out, M, N, K, swiglu, gamma, eps, residual, out_f32, settled):
+    """``gemm_rows`` of arguments that have been looked at."""
+    if out is None:
+        out = torch.empty((M, N), dtype=torch.float32 if out_f32 else x.dtype, device=x.device)
     _lib.call("b200_gemm_rows", ptr(x), ptr(w), ptr(out), M, N, K, x.stride(0), w.stride(0), out.stride(0), 1 if swiglu else 0, ptr(gamma),
               c_float(eps), ptr(residual), 1 if out_f32 else 0, dtype_code(x.dtype, settled), ptr(_pipeline_status(x.device)), stream_ptr())
     _count()
