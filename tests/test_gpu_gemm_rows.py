@@ -84,6 +84,44 @@ def test_gemm_rows_pitches(M, N, K, swiglu, dtype):
     assert torch.all(wide[M:] == 7.0) and torch.all(wide[:, :3] == 7.0) and torch.all(wide[:, N + 3:] == 7.0)
 
 
+@pytest.mark.parametrize("settled", [False, True])
+def test_gemm_rows_repeats_itself_in_chains(settled):
+    """Launches of several sizes that start under one another, with another stream's work on the SMs: every result has the bits of the
+    call alone, which is right against 64 bits."""
+    from triton_distributed_b200 import ops
+    torch.manual_seed(9)
+    cases = []
+    for M, N, K, gated, normed in [(1, 1280, 5120, False, True), (8, 592, 4096, False, False), (16, 128, 2048, False, False), (5, 3200, 1024, True, True),
+                                   (16, 3000, 4160, False, False), (9, 8, 64, False, False)]:
+        x, w = torch.randn(M, K).bfloat16(), (torch.randn(N * (2 if gated else 1), K) * K ** -0.5).bfloat16()
+        gamma = (1 + torch.randn(K)).bfloat16() if normed else None
+        ref = (x.double() * gamma.double()).bfloat16().double() @ w.double().T if normed else x.double() @ w.double().T   # on the host
+        if normed:
+            ref *= torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6)
+        if gated:
+            ref = torch.nn.functional.silu(ref[:, :N]) * ref[:, N:]
+        args = [t.cuda() if t is not None else None for t in (x, w, gamma)]
+        cases.append((args, gated, ref))
+    torch.cuda.synchronize()   # the operands are settled
+    call = lambda a, gated: ops.gemm_rows(a[0], a[1], swiglu=gated, gamma=a[2], eps=1e-6, settled=settled)
+    alone = [call(a, gated) for a, gated, _ in cases]
+    for got, (_, _, ref) in zip(alone, cases):   # (as in test_gemm_rows_norm)
+        torch.testing.assert_close(got.cpu().double(), ref, rtol=2 ** -7, atol=2e-5)
+    side, busy = torch.cuda.Stream(), torch.randn(2048, 2048, device="cuda").bfloat16()
+    torch.cuda.synchronize()
+    wrong = torch.zeros(len(cases), dtype=torch.int32, device="cuda")
+    for _ in range(20):
+        with torch.cuda.stream(side):
+            for _ in range(4):
+                busy @ busy
+        got = [[call(a, gated) for a, gated, _ in cases] for _ in range(10)]
+        for ys in got:
+            for i, y in enumerate(ys):
+                wrong[i] += (y.view(torch.int16) != alone[i].view(torch.int16)).any()
+    assert wrong.tolist() == [0] * len(cases)
+    ops.check_pipeline_status()
+
+
 def test_status_word_is_made_in_front_of_a_capture(monkeypatch):
     """A word that a capture made would be cleared by every replay, and read before the first."""
     from triton_distributed_b200 import ops
