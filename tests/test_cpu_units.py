@@ -169,6 +169,20 @@ def test_gemm_f32_cuts_in_front_where_a_call_has_many_steps():
         assert need(M, N, K) == size(M, K) > 0
 
 
+def test_seeding_leaves_the_library_workspace_of_a_running_process_alone(monkeypatch):
+    import os
+    import torch
+    from triton_distributed_b200 import utils
+    for running in (True, False):
+        monkeypatch.delenv("CUBLAS_WORKSPACE_CONFIG", raising=False)
+        monkeypatch.setattr(torch.cuda, "is_initialized", lambda: running)
+        utils.init_seed(3)
+        assert ("CUBLAS_WORKSPACE_CONFIG" in os.environ) == (not running)
+    monkeypatch.setenv("CUBLAS_WORKSPACE_CONFIG", ":16:8")   # the user's own choice stays
+    utils.init_seed(3)
+    assert os.environ["CUBLAS_WORKSPACE_CONFIG"] == ":16:8"
+
+
 def test_native_library_builds_and_reports_errors():
     """The shared object loads without a driver; entry points that need one fail with a message, not a crash."""
     import ctypes

@@ -34,6 +34,18 @@ def test_heap_alloc_free_and_views(dist1):
     heap.check_status()
 
 
+def test_library_products_stay_in_their_workspace(dist1):
+    """A split product in double (13 MB of partial sums) leaves live tensors alone, also in a process that used cuBLAS before the
+    bring-up."""
+    torch.manual_seed(8)
+    for _ in range(60):
+        x, w = torch.randn(250, 4104, device="cuda").bfloat16()[:, :4096], (torch.randn(592, 4096, device="cuda") / 64).bfloat16()
+        held = torch.randn(250, 592, device="cuda").double()
+        kept = held.float()
+        x.double() @ w.double().T
+        assert torch.equal(held, kept.double())
+
+
 def test_bounded_wait_reports_timeout_instead_of_hanging(dist1):
     """A wait on a flag that nobody sets must come back with an error status."""
     from triton_distributed_b200 import _lib
