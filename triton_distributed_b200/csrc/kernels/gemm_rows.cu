@@ -76,6 +76,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   uint32_t* s_gamma = reinterpret_cast<uint32_t*>(red + kRowsWarps * MB * kPitch);      // [K / 2] pairs
   __shared__ uint64_t full[kRowsMaxStages];
   __shared__ float s_sq[kRowsWarps][16];
+  __shared__ int s_lost[kRowsWarps];   // stage whose wait a warp gave up
   __shared__ uint32_t abort_word;
   volatile uint32_t* abort_flag = &abort_word;
   const uint64_t timeout_ns = 4000000000ull;
@@ -149,21 +150,12 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       for (int e = 0; e < 4; ++e) acc[g][e] = 0.f;
     float sq[2] = {0.f, 0.f};   // squares of tokens lane / 4 and eight further, this lane's channels
     for (; at < first + p.spans; at += kRowsWarps) {
-      // after an expired wait the remaining rounds go by without work: all warps meet at the barriers below (one verdict per warp: the
-      // fragment loads and products are instructions of all its lanes)
+      // After an expired wait the remaining rounds go by without work: all warps meet at the barriers below. One verdict per warp: the
+      // fragment loads and products are instructions of all its lanes.
       if (ok) {
-        ok = __all_sync(0xffffffffu, mbar_wait(full + slot, phase, abort_flag, timeout_ns));
-        if (!ok && lane == 0) {   // boxes that are on their way have to land before shared memory is given back
-          volatile uint32_t never = 0;
-          int s = slot;
-          uint32_t ph = phase;
-          for (int i = at; i < asked; i += kRowsWarps) {
-            mbar_wait(full + s, ph, &never, timeout_ns);
-            s += kRowsWarps;
-            if (s >= p.stages) { s = warp; ph ^= 1; }
-          }
-        }
-        __syncwarp();
+        const bool got = mbar_wait(full + slot, phase, abort_flag, timeout_ns);
+        ok = __all_sync(0xffffffffu, got);
+        if (!ok) s_lost[warp] = at;
       }
       if (ok) {
         uint32_t ws = smem_u32(ring + slot * p.stage_bytes), xs = ws + p.w_bytes;
@@ -243,8 +235,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       const int i = threadIdx.x + j * 256, m = i / R, n = tile * R + i % R;
       res[j] = p.residual != nullptr && m < p.M && n < p.N ? to_float(static_cast<const T*>(p.residual)[static_cast<size_t>(m) * p.ldc + n]) : 0.f;
     }
-    __syncthreads();
-    const bool whole = *abort_flag == 0u;   // no warp gave up: one that did left sums without its share
+    const bool whole = __syncthreads_and(ok);   // no warp gave up, or the sums lack its share
 #pragma unroll
     for (int j = 0; j < kOut; ++j) {
       const int i = threadIdx.x + j * 256, m = i / R, n = tile * R + i % R;
@@ -272,7 +263,14 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     }
     __syncthreads();   // the next tile's sums take the same place
   }
-  if (threadIdx.x == 0 && *abort_flag != 0u && p.status != nullptr) atomicMax(p.status, static_cast<uint32_t>(kStatusPipeTimeout));
+  if (!ok && lane == 0) {   // boxes that are on their way have to land before shared memory is given back
+    volatile uint32_t never = 0;
+    for (int i = s_lost[warp]; i < asked; i += kRowsWarps) {
+      const int round = i / kRowsWarps, places = p.stages / kRowsWarps;   // of this warp
+      mbar_wait(full + warp + round % places * kRowsWarps, round / places & 1, &never, timeout_ns);
+    }
+  }
+  if (threadIdx.x == 0 && abort_word != 0u && p.status != nullptr) atomicMax(p.status, static_cast<uint32_t>(kStatusPipeTimeout));
 }
 
 using RowsKernel = void (*)(const CUtensorMap, const CUtensorMap, const RowsParams);
